@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
 #include <vector>
 
 #include "../../include/xfold_b200.h"
@@ -63,9 +64,25 @@ struct ProfScope {
 int fail(Ctx* c, int code, const char* fmt, ...);
 int check_launch(Ctx* c, const char* what);
 
+// Launch that may start while the previous kernel of the stream still runs (see pdl_wait in umma.cuh).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 // ---- tensor maps --------------------------------------------------------------------------
 // bf16 tensor of rank 3, innermost stride 1; s1/s2 are strides of dims 1/2 in ELEMENTS.
-// 128-byte swizzle (or 64-byte, for boxes whose rows are 64 bytes), zero fill outside the extents.
+// 128-byte swizzle (64-byte for boxes whose rows are 64 bytes, 0 for none), zero fill outside the extents.
 bool make_tmap_bf16_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
                        uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, int swizzle_bytes = 128);
 

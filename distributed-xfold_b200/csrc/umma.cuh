@@ -263,6 +263,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel launched with the attribute (launch_pdl in internal.h) may start while its
+// predecessor in the stream still runs; everything up to pdl_wait() -- barriers, tensor memory, weights that no kernel of
+// the call writes -- overlaps the predecessor's tail.  Rules that keep it safe: EVERY thread of such a kernel calls
+// pdl_wait() before it touches anything a predecessor wrote or still reads (so that the completion of a kernel implies
+// the completion of all before it), and pdl_launch() comes after the tensor memory allocation (a successor that got the
+// tensor memory first would wait for this kernel, and this kernel for the tensor memory).
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ------------------------------------------------------------------------------------
 // misc math
 // ------------------------------------------------------------------------------------
 // sigmoid(x) = 0.5 * tanh(0.5 x) + 0.5: one MUFU op (tanh.approx, rel. error ~2^-11) instead of ex2 + rcp
@@ -274,6 +285,15 @@ __device__ __forceinline__ float sigmoidf_fast(float x) {
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
+}
+// two float32 FMAs in one instruction: d = a * b + c, element by element
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
 }
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }

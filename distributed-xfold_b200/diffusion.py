@@ -76,8 +76,8 @@ class PackedDiffusionTransformer:
         self.num_head, self.num_blocks, self.sb = num_head, num_blocks, super_block_size
         self.pair_ln_g = ops._f32(state.get(prefix + "pair_input_layer_norm.weight"), device)
         self.pair_ln_b = ops._f32(state.get(prefix + "pair_input_layer_norm.bias"), device)
-        self.pl_w = [ops._f32(state[prefix + f"pair_logits_projection.{i}.weight"], device)
-                     for i in range(num_blocks // super_block_size)]
+        self.pl_w = ops._f32(torch.cat([state[prefix + f"pair_logits_projection.{i}.weight"]
+                                        for i in range(num_blocks // super_block_size)], 0), device)
         self.blocks = [PackedDiffusionBlock(state, prefix + f"self_attention.{i}.", prefix + f"transition_block.{i}.",
                                             device, num_head) for i in range(num_blocks)]
 
@@ -85,14 +85,8 @@ class PackedDiffusionTransformer:
         """[N, N, 128] bf16 -> per super-block float16 [super_block_size, heads, N, pad8(N)], the prepared operand of the
         attention kernel (values times log2(e)): half the resident bytes of the float32 logits, and no conversion inside
         the 200 denoising steps.  ('n s (b h) -> b h n s', nn/d_diffusion_transformer.py:301-305.)"""
-        n = pair_cond.shape[0]
-        out = []
-        for w in self.pl_w:
-            _, proj = ops.layernorm(pair_cond, self.pair_ln_g, self.pair_ln_b, proj_w=w, want_y=False)
-            prepared = ops.prepare_pair_bias(proj.reshape(self.sb * self.num_head, n, n))
-            del proj
-            out.append(prepared.reshape(self.sb, self.num_head, n, prepared.shape[-1]))
-        return out
+        prepared = ops.pair_logits_prepared(pair_cond, self.pair_ln_g, self.pair_ln_b, self.pl_w)
+        return list(prepared.reshape(-1, self.sb, self.num_head, *prepared.shape[1:]))
 
     def forward(self, act: torch.Tensor, mask: Optional[torch.Tensor], single_cond: torch.Tensor,
                 pair_logits: List[torch.Tensor]) -> torch.Tensor:

@@ -333,6 +333,19 @@ def prepare_pair_bias(pair_bias: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def pair_logits_prepared(pair: torch.Tensor, gamma, beta, w: torch.Tensor) -> torch.Tensor:
+    """pair bf16 [N, N, 128], w float32 [H, 128] -> float16 [H, N, pad8(N)]: the projection of LayerNorm(pair) to H heads in
+    the form of ``prepare_pair_bias``."""
+    _need_cuda(pair, gamma, beta, w)
+    assert pair.dtype == BF16 and pair.is_contiguous() and pair.shape[0] == pair.shape[1] and pair.shape[2] == 128
+    dev = _dev(pair)
+    n, h = pair.shape[0], w.shape[0]
+    out = torch.empty(h, n, (n + 7) // 8 * 8, dtype=torch.float16, device=pair.device)
+    check(load().xfold_pair_logits_prepared_fwd(ctx(dev), _ptr(pair), n, _ptr(gamma), _ptr(beta), _ptr(w), h, _ptr(out),
+                                                _stream(dev)), dev, "xfold_pair_logits_prepared_fwd")
+    return out
+
+
 def attention_pair_bias_core(xn: torch.Tensor, w: PackedSelfAttention, pair_bias: torch.Tensor,
                              mask: Optional[torch.Tensor]) -> torch.Tensor:
     """xn bf16 [B, S, C] (normalised input), pair_bias float32 [H, S, S] or the float16 [H, S, pad8(S)] tensor of

@@ -175,6 +175,11 @@ int xfold_attention_pair_bias_core_fwd(xfold_ctx* ctx, const void* xn, int B, in
  * all 200 denoising steps (nn/d_diffusion_transformer.py:296-305 recomputes them per call) -- converts it once with
  * xfold_pair_bias_prepare_fwd (prepared: H * S * pad8(S) * 2 bytes) and passes it to the _prepared_ form of the core. */
 int xfold_pair_bias_prepare_fwd(xfold_ctx* ctx, const float* pair_bias, int H, int S, void* prepared, void* stream);
+/* LayerNorm (eps 1e-5) of a whole pair representation [N][N][128] and its projection to H heads (w float32 [H][128], H a
+ * multiple of 16), written as prepared pair bias [H][N][pad8(N)]: every block's logits of the diffusion transformer in one
+ * launch ('n s (b h) -> b h n s', nn/d_diffusion_transformer.py:299-305). */
+int xfold_pair_logits_prepared_fwd(xfold_ctx* ctx, const void* pair, int N, const float* ln_gamma, const float* ln_beta,
+                                   const float* w, int H, void* prepared, void* stream);
 int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* ctx, const void* xn, int B, int S, int C, int H, int Dp,
                                                 const void* w_qkvg, const float* qkvg_bias, const float* qkvg_scale,
                                                 const void* prepared_bias, const float* mask, void* out, void* ws,

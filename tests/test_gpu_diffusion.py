@@ -107,3 +107,20 @@ def test_sampler_loop_around_the_gpu_transformer(ops, oracle):
     ref = dh.sample_diffusion(denoiser(cpu_transformer), sched, atom_mask, samples, generator=torch.Generator().manual_seed(5))
     assert got.shape == (samples, n, atoms, 3) and torch.isfinite(got).all()
     assert relf(got, ref) < 2e-2
+
+
+@pytest.mark.parametrize("n,h", [(1, 16), (77, 64), (128, 144), (130, 128), (257, 384)])
+def test_pair_logits_prepared(ops, n, h):
+    """LayerNorm + projection to the prepared pair bias at tile edges, ragged rows and head counts that fill the last
+    group of heads only in part; rows with a mean well away from zero; zero in the padding columns."""
+    g = torch.Generator().manual_seed(n + h)
+    pair = (2.0 * torch.randn(n, n, 128, generator=g) + 0.7).to(BF)
+    gamma, beta = torch.rand(128, generator=g) + 0.5, 0.3 * torch.randn(128, generator=g)
+    w = torch.randn(h, 128, generator=g) / 11
+    out = ops.pair_logits_prepared(pair.cuda(), gamma.cuda(), beta.cuda(), w.cuda())
+    ops.synchronize_and_check()
+    assert tuple(out.shape) == (h, n, (n + 7) // 8 * 8)
+    ref = torch.nn.functional.layer_norm(pair.double(), (128,), gamma.double(), beta.double(), 1e-5) @ w.double().T
+    ref = ref.permute(2, 0, 1) * 1.4426950408889634
+    assert relf(out[..., :n].cpu(), ref) < 4e-4  # float16 output rounding only
+    assert float(out[..., n:].float().abs().sum()) == 0.0
