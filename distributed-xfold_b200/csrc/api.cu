@@ -66,11 +66,12 @@ bool make_tmap_bf16_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d
 static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M, int K, const bf16* w, int wrows, int ldw,
                      GemmArgs a, int bn, cudaStream_t st) {
   if (M <= 0) return XFOLD_OK;
+  if (M >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "linear: too many rows");
   if ((K & 7) || (ldx & 7) || (ldw & 7)) return fail(c, XFOLD_ERR_ARG, "linear: K and leading dimensions must be multiples of 8");
   CUtensorMap tA, tB;
   if (!make_tmap_bf16_3d(&tA, x, K, M, 1, ldx, (uint64_t)ldx * M, 64, 128, 1))
     return fail(c, XFOLD_ERR_ARG, "linear: cannot encode the activation tensor map (base 16 B aligned?)");
-  if (!make_tmap_bf16_3d(&tB, w, K, wrows, 1, ldw, (uint64_t)ldw * wrows, 64, bn, 1))
+  if (!make_tmap_bf16_3d(&tB, w, K, wrows, 1, ldw, (uint64_t)ldw * wrows, 64, epi == EPI_SWIGLU && bn < 256 ? bn / 2 : bn, 1))
     return fail(c, XFOLD_ERR_ARG, "linear: cannot encode the weight tensor map");
   a.M = (int)M;
   a.K = K;
@@ -82,9 +83,9 @@ static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M,
 
 static int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
                         const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0) {
-  if (M >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "linear: too many rows");
   GemmArgs a;
-  const int bn = (N > 128) ? 256 : 128;
+  const int bn = gemm_tile_n(c, M, N, K, 1, 256, 64);
+  a.static_b = c->static_weights;
   a.N = N;
   a.tiles_n = (N + bn - 1) / bn;
   a.out = out;
@@ -105,14 +106,14 @@ int linear_plain_fwd(Ctx* c, const bf16* x, long long ldx, long long M, int K, c
 static int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N,
                              const bf16* gate, long long ldg, int row_gate_mod, const bf16* resid, long long ldr,
                              bf16* out, long long ldo, cudaStream_t st) {
-  if (M >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "linear: too many rows");
   GemmArgs a;
-  const int bn = 128;
+  const int bn = gemm_tile_n(c, M, N, K, 1, 128, 64);
+  a.static_b = c->static_weights;
   a.N = N;
   a.tiles_n = (N + bn - 1) / bn;
   a.out = out;
   a.ldo = ldo;
-  if (row_gate_mod > 0) { a.row_gate = gate; a.row_gate_mod = row_gate_mod; }
+  if (row_gate_mod > 0 && row_gate_mod < M) { a.row_gate = gate; a.row_gate_mod = row_gate_mod; }
   else a.gate = gate;
   a.ldg = ldg;
   a.resid = resid;
@@ -153,13 +154,14 @@ static int linear_gate_resid_chunked(Ctx* c, const bf16* x, long long ldx, long 
 static int linear_swiglu(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* wp, int F, bf16* out,
                          long long ldo, cudaStream_t st) {
   if (F % 128) return fail(c, XFOLD_ERR_ARG, "linear_swiglu: F must be a multiple of 128");
-  if (M >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "linear: too many rows");
   GemmArgs a;
+  const int bn = gemm_tile_n(c, M, 2 * F, K, 1, 256, 128);
+  a.static_b = c->static_weights;
   a.N = 2 * F;
-  a.tiles_n = F / 128;
+  a.tiles_n = 2 * F / bn;
   a.out = out;
   a.ldo = ldo;
-  return gemm_rows(c, EPI_SWIGLU, x, ldx, M, K, wp, 2 * F, K, a, 256, st);
+  return gemm_rows(c, EPI_SWIGLU, x, ldx, M, K, wp, 2 * F, K, a, bn, st);
 }
 
 static int batched_contract(Ctx* c, const bf16* a_, const bf16* b_, bf16* out, int channels, int Mi, int Nj, int Kk,
@@ -313,6 +315,7 @@ static TriMulWs carve_trimul(void* ws, size_t cap, int N) {
 
 static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, const xfold_trimul_weights* w, void* ws,
                       size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr) {
+  StaticWeights sw(c);
   if (!z || !w || !w->w_in || !w->w_out) return fail(c, XFOLD_ERR_ARG, "trimul: null argument");
   if (N <= 0) return XFOLD_OK;
   TriMulWs W = carve_trimul(ws, ws_bytes, N);
@@ -378,6 +381,7 @@ int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask,
 
 static int triattn_fwd(Ctx* c, bf16* z, const float* mask, int N, int transpose, const xfold_triattn_weights* w, void* ws,
                        size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr) {
+  StaticWeights sw(c);
   if (!z || !w || !w->w_qkvg || !w->w_out || !w->w_bias) return fail(c, XFOLD_ERR_ARG, "triattn: null argument");
   if (N <= 0) return XFOLD_OK;
   TriAttnWs W = carve_triattn(ws, ws_bytes, N, N);
@@ -390,6 +394,7 @@ static int triattn_fwd(Ctx* c, bf16* z, const float* mask, int N, int transpose,
 
 int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_transition_weights* w, void* ws,
                           size_t ws_bytes, cudaStream_t st, bf16* upd, const ChunkHook* hook) {
+  StaticWeights sw(c);
   if (!x || !w || !w->w1_packed || !w->w2) return fail(c, XFOLD_ERR_ARG, "transition: null argument");
   if (rows <= 0) return XFOLD_OK;
   // before any size arithmetic or launch: row counts the kernels cannot index, or whose byte sizes would wrap
@@ -469,6 +474,7 @@ size_t single_ws_bytes(int N) {
 // plT: bf16 [16][N][ldq] pair logits, [h][query][key].
 int single_update(Ctx* c, bf16* s, const bf16* plT, int ldq, const float* seq_mask, int N,
                          const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, cudaStream_t st) {
+  StaticWeights sw(c);
   Carver cv(ws, ws_bytes);
   bf16* xn = (bf16*)cv.take((size_t)N * 384 * 2);
   bf16* o = (bf16*)cv.take((size_t)N * 512 * 2);
@@ -498,6 +504,7 @@ static size_t pairformer_ws_bytes(int N) {
 
 static int pairformer_fwd(Ctx* c, bf16* z, bf16* s, const float* pair_mask, const float* seq_mask, int N,
                           const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, cudaStream_t st) {
+  StaticWeights sw(c);
   if (!z || !w) return fail(c, XFOLD_ERR_ARG, "pairformer: null argument");
   if (ws_bytes < pairformer_ws_bytes(N)) return fail(c, XFOLD_ERR_ARG, "pairformer: workspace too small (%zu < %zu)", ws_bytes, pairformer_ws_bytes(N));
   int rc;

@@ -202,6 +202,8 @@ attn3_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  pdl_wait();
+  pdl_launch();
 
   // Register re-balancing (whole warpgroups): the control warps run single threads with a handful of values, the
   // softmax threads hold a block's 64 logits and 16 packed probabilities.
@@ -591,8 +593,10 @@ attn3_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CU
 // Mask-bias tiles: out[b][kb] is an un-swizzled K-major [128 keys][16] bf16 tile (core matrices of
 // 8 keys x 8 columns, 128 B each; the two column halves 128 B apart, 8-key groups 256 B apart) whose
 // column 0 holds 1e9 * (mask[b][k] - 1) for k < S and -1e30 for the padding of the last tile.
-__global__ void mext_kernel(const float* __restrict__ mask, long long mask_ld, bf16* __restrict__ out, int B, int S,
+__global__ void mext_kernel(const float* mask, long long mask_ld, bf16* __restrict__ out, int B, int S,
                             int KB) {
+  pdl_wait();
+  pdl_launch();
   const long long n = (long long)B * KB * 128;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -620,13 +624,15 @@ int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, 
   long long blocks = (n + 255) / 256;
   if (blocks > 8192) blocks = 8192;
   ProfScope ps(c, XFOLD_K_MASK_BIAS, st);
-  mext_kernel<<<(int)blocks, 256, 0, st>>>(mask, mask_ld, out, B, S, KB);
+  launch_pdl(mext_kernel, (int)blocks, 256, 0, st, mask, mask_ld, out, B, S, KB);
   return check_launch(c, "mext_kernel");
 }
 
 // fp32 [H][S][S] -> 16-bit [H][S][ldq] (same query-major order, padded row pitch): FP16 values times log2(e), the operand
 // the kernel's pair-bias tensor map expects (the kernel works in base 2 and adds the tile as it is).
-__global__ void bias_convert_kernel(const float* __restrict__ in, __half* __restrict__ out, long long rows, int S, int ldq) {
+__global__ void bias_convert_kernel(const float* in, __half* __restrict__ out, long long rows, int S, int ldq) {
+  pdl_wait();
+  pdl_launch();
   const long long n = rows * ldq;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -642,7 +648,7 @@ int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int 
   long long blocks = (rows * ldq + 255) / 256;
   if (blocks > 16384) blocks = 16384;
   ProfScope ps(c, XFOLD_K_MASK_BIAS, st);
-  bias_convert_kernel<<<(int)blocks, 256, 0, st>>>(in, reinterpret_cast<__half*>(out), rows, S, ldq);
+  launch_pdl(bias_convert_kernel, (int)blocks, 256, 0, st, in, reinterpret_cast<__half*>(out), rows, S, ldq);
   return check_launch(c, "bias_convert_kernel");
 }
 
@@ -658,7 +664,7 @@ static int launch_attn3(Ctx* c, int grid, const CUtensorMap& tmq, const CUtensor
     attr_done[c->device & 7] = true;
   }
   ProfScope ps(c, c->attn_tag, st);
-  attn3_kernel<D><<<grid, (A3_CTRL + 4 * (128 / D)) * 32, A3_SMEM, st>>>(tmq, tmkv, tmb, a);
+  launch_pdl(attn3_kernel<D>, grid, (A3_CTRL + 4 * (128 / D)) * 32, A3_SMEM, st, tmq, tmkv, tmb, a);
   return check_launch(c, "attn3_kernel");
 }
 

@@ -30,15 +30,15 @@ constexpr uint32_t EPI_TILE = 128 * 64 * 2;  // one staged [128 rows][64 columns
 
 template <int BN>
 struct GemmCfg {
-  static constexpr int STAGES = 4;
+  static constexpr int STAGES = BN == 64 ? 5 : 4;
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  // after the operand ring: 2 output chunks; with 128-wide tiles also 2 residual and 2 gate chunks
+  // after the operand ring: 2 output chunks; with 128- and 64-wide tiles also 2 residual and 2 gate chunks
   static constexpr uint32_t OFF_OUT = STAGES * STAGE_BYTES;
   static constexpr uint32_t OFF_RES = OFF_OUT + 2 * EPI_TILE;
   static constexpr uint32_t OFF_GATE = OFF_RES + 2 * EPI_TILE;
-  static constexpr uint32_t OFF_BAR = (BN == 128) ? OFF_GATE + 2 * EPI_TILE : OFF_RES;
+  static constexpr uint32_t OFF_BAR = (BN <= 128) ? OFF_GATE + 2 * EPI_TILE : OFF_RES;
   static constexpr uint32_t SMEM_BYTES = OFF_BAR + 256 /*barriers*/ + 1024 /*align slack*/;
 };
 
@@ -72,8 +72,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmG, const GemmArgs p) {
   using Cfg = GemmCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
-  // residual / gate chunks are prefetched by TMA only in the 128-wide gate/residual configuration
-  constexpr bool EPI_LOADS = (EPI == EPI_GATE_RESID) && (BN == 128);
+  // residual / gate chunks are prefetched by TMA
+  constexpr bool EPI_LOADS = EPI == EPI_GATE_RESID;
+  static_assert(!EPI_LOADS || BN <= 128, "no room for the residual / gate chunks beside 256-wide operand tiles");
+  // SWIGLU weights come in groups of [128 SiLU rows | 128 linear rows]: a tile takes BN / 2 rows of either half
+  constexpr bool B_SPLIT = EPI == EPI_SWIGLU && BN < 256;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -123,6 +126,25 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t stage = 0, phase = 0, echunk = 0;
       bool okay = true;
       (void)echunk;
+      auto load_b = [&](uint8_t* sB, uint64_t* bar, int kb, int tn, int bb) {
+        if constexpr (B_SPLIT) {
+          const int r0 = tn * (BN / 2) / 128 * 256 + tn * (BN / 2) % 128;
+          tma_load_3d(sB, &tmB, bar, kb * BK, r0, bb);
+          tma_load_3d(sB + Cfg::B_BYTES / 2, &tmB, bar, kb * BK, r0 + 128, bb);
+        } else {
+          tma_load_3d(sB, &tmB, bar, kb * BK, tn * BN, bb);
+        }
+      };
+      // Weights that no kernel of this call writes are fetched before the wait for the previous kernel: with a few rows
+      // of activations the launch is a latency chain and the weights' trip from HBM is the longest link of it.
+      int pre = 0;
+      if (p.static_b && (long long)blockIdx.x < total)
+        for (; pre < STAGES && pre < KB; ++pre) {
+          mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
+          load_b(smem + pre * Cfg::STAGE_BYTES + Cfg::A_BYTES, &full[pre], pre, int(blockIdx.x % p.tiles_n), 0);
+        }
+      pdl_wait();
+      pdl_launch();
       for (long long t = blockIdx.x; t < total && okay; t += gridDim.x) {
         const int tn = int(t % p.tiles_n);
         const int tm = int((t / p.tiles_n) % p.tiles_m);
@@ -134,7 +156,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if constexpr (EPI_LOADS) {
           const uint32_t nload = (p.resid ? 1u : 0u) + (p.gate ? 1u : 0u);
           if (nload) {
-            for (int c = 0; c < BN / 64 && okay; ++c, ++echunk) {
+            for (int c = 0; c < BN / 64 && tn * BN + c * 64 < p.N && okay; ++c, ++echunk) {
               const uint32_t eb = echunk & 1u;
               if (!mbar_wait(&eempty[eb], ((echunk >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
               mbar_arrive_expect_tx(&efull[eb], nload * EPI_TILE);
@@ -145,12 +167,18 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         for (int kb = 0; kb < KB; ++kb) {
+          uint8_t* sA = smem + stage * Cfg::STAGE_BYTES;
+          if (pre > 0) {  // the first tile's first stages: announced, and B on its way
+            --pre;
+            tma_load_3d(sA, &tmA, &full[stage], kb * BK, a1, a2);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            continue;
+          }
           if (!mbar_wait(&empty[stage], phase ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
           mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          uint8_t* sA = smem + stage * Cfg::STAGE_BYTES;
           if (!p.mn_major) {
             tma_load_3d(sA, &tmA, &full[stage], kb * BK, a1, a2);
-            tma_load_3d(sA + Cfg::A_BYTES, &tmB, &full[stage], kb * BK, tn * BN, bb);
+            load_b(sA + Cfg::A_BYTES, &full[stage], kb, tn, bb);
           } else {
             // operands stored [k][m] / [k][n]: one [64 k][64 m] box (8 KB, 128-byte rows) per 64 rows of the tile
 #pragma unroll
@@ -163,7 +191,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
     }
+    pdl_wait();
+    pdl_launch();
   } else if (warp == 1) {
+    pdl_wait();
+    pdl_launch();
     if (lane == 0) {
       // MN-major operands (rows of the smem tile are K indices): 64-element chunks along M / N are 8 KB apart, a step of
       // 16 along K is 16 rows of 128 B
@@ -192,6 +224,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     }
   } else {
+    pdl_wait();
+    pdl_launch();
     const int q = warp & 3;          // TMEM lane quarter this warp may read
     const int ch = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
     const int row = q * 32 + lane;
@@ -222,6 +256,20 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         if (tn < 2 && rvalid && p.mask) mk = p.mask[tok];
       }
+      // GATE_RESID with a gate row per (row % mod): the first chunk's gate values, fetched before the wait as well
+      const bool row_gate_vec = EPI == EPI_GATE_RESID && p.row_gate && (p.ldg & 7) == 0 && (p.N & 31) == 0;
+      uint4 rg[4];
+      auto fetch_row_gate = [&](int c) {
+        const long long m = (long long)tm * BM + row;
+        const int col = tn * BN + c * 64 + ch * 32;
+        if (m < p.M && col < p.N) {
+          const uint4* src = reinterpret_cast<const uint4*>(p.row_gate + (m % p.row_gate_mod) * p.ldg + col);
+#pragma unroll
+          for (int g = 0; g < 4; ++g) rg[g] = src[g];
+        }
+      };
+      if constexpr (EPI == EPI_GATE_RESID)
+        if (row_gate_vec) fetch_row_gate(0);
       if (!mbar_wait(&tfull[buf], aphase, ab, XF_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(q * 32) << 16);
@@ -236,8 +284,12 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const long long m = (long long)tm * BM + row;
         const uint32_t rsw = uint32_t(row & 7);
         const bool elected = (warp == 2 && lane == 0);
+        // Chunks beyond the output's last column are left out.  (They must not pass through the staging buffers without a
+        // store of their own either: the wait below counts committed stores, and a chunk that commits none would let the
+        // one after it overwrite a tile that is still being read.)
+        const int nch = min(NCH, (n_out - tn * WOUT + 63) / 64);
 #pragma unroll 1
-        for (int c = 0; c < NCH; ++c, ++ochunk) {
+        for (int c = 0; c < nch; ++c, ++ochunk) {
           const int col0 = tn * WOUT + c * 64;          // first output column of the chunk
           const int colw = col0 + ch * 32;              // first output column of this warp
           uint8_t* so = smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE + row * 128;
@@ -307,7 +359,18 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
               }
             }
-            if (p.row_gate) {  // gate shared by rows with equal (row % mod): AdaLN-Zero conditioning of several samples
+            if (row_gate_vec) {
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const uint32_t w4[4] = {rg[g].x, rg[g].y, rg[g].z, rg[g].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
+                  v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
+                }
+              }
+              if (c + 1 < nch) fetch_row_gate(c + 1);
+            } else if (p.row_gate) {  // gate shared by rows with equal (row % mod): AdaLN-Zero conditioning of several samples
 #pragma unroll
               for (int g = 0; g < 4; ++g) {
                 const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
@@ -371,7 +434,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           fence_proxy_async_smem();
           named_bar_sync(2, 256);
-          if (elected && col0 < n_out) {
+          if (elected) {
             tma_store_3d(&tmO, smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE, col0, tm * BM, b);
             tma_store_commit();
           }
@@ -417,7 +480,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
     }
-    if (warp == 2 && lane == 0) tma_store_wait_read<0>();  // staged tiles must be read out before the CTA exits
+    if (warp == 2 && lane == 0) tma_store_wait_all();  // written, not only read out: the next kernel may be waiting already
   }
 
   tc_fence_before();
@@ -452,7 +515,7 @@ static int launch_one(Ctx* c, const CUtensorMap& tmA, const CUtensorMap& tmB, co
     const uint64_t bstride = a.batches > 1 ? (uint64_t)a.out_batch_stride : (uint64_t)a.ldo * (uint64_t)a.M;
     if (!make_tmap_bf16_3d(&tmO, a.out, n_out, a.M, a.batches, a.ldo, bstride, 64, 128, 1))
       return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the output tensor map (16-byte aligned base, ld multiple of 8?)");
-    if (EPI == EPI_GATE_RESID && BN == 128) {
+    if (EPI == EPI_GATE_RESID) {
       if (a.resid && !make_tmap_bf16_3d(&tmR, a.resid, a.N, a.M, 1, a.ldr, (uint64_t)a.ldr * a.M, 64, 128, 1))
         return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the residual tensor map");
       if (a.gate && !make_tmap_bf16_3d(&tmG, a.gate, a.N, a.M, 1, a.ldg, (uint64_t)a.ldg * a.M, 64, 128, 1))
@@ -466,26 +529,45 @@ static int launch_one(Ctx* c, const CUtensorMap& tmA, const CUtensorMap& tmB, co
                   : EPI == EPI_GATE_RESID ? XFOLD_K_LINEAR_GATE_RESID
                   : (a.batches > 1 ? XFOLD_K_TRIMUL_CONTRACT : XFOLD_K_LINEAR);
   ProfScope ps(c, tag, st);
-  kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(tmA, tmB, tmO, tmR, tmG, a);
+  launch_pdl(kern, grid, GEMM_THREADS, Cfg::SMEM_BYTES, st, tmA, tmB, tmO, tmR, tmG, a);
   return check_launch(c, "gemm_tn_kernel");
 }
 
 int launch_gemm(Ctx* c, int epi, int bn, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a,
                 cudaStream_t st) {
-  if (bn == 256) {
-    switch (epi) {
-      case EPI_PLAIN: return launch_one<256, EPI_PLAIN>(c, tmA, tmB, a, st);
-      case EPI_GATE_RESID: return launch_one<256, EPI_GATE_RESID>(c, tmA, tmB, a, st);
-      case EPI_SWIGLU: return launch_one<256, EPI_SWIGLU>(c, tmA, tmB, a, st);
-      case EPI_TRIMUL_AB: return launch_one<256, EPI_TRIMUL_AB>(c, tmA, tmB, a, st);
-    }
-  } else if (bn == 128) {
-    switch (epi) {
-      case EPI_PLAIN: return launch_one<128, EPI_PLAIN>(c, tmA, tmB, a, st);
-      case EPI_GATE_RESID: return launch_one<128, EPI_GATE_RESID>(c, tmA, tmB, a, st);
-    }
+  switch (epi * 1000 + bn) {
+    case EPI_PLAIN * 1000 + 256: return launch_one<256, EPI_PLAIN>(c, tmA, tmB, a, st);
+    case EPI_PLAIN * 1000 + 128: return launch_one<128, EPI_PLAIN>(c, tmA, tmB, a, st);
+    case EPI_PLAIN * 1000 + 64: return launch_one<64, EPI_PLAIN>(c, tmA, tmB, a, st);
+    case EPI_GATE_RESID * 1000 + 128: return launch_one<128, EPI_GATE_RESID>(c, tmA, tmB, a, st);
+    case EPI_GATE_RESID * 1000 + 64: return launch_one<64, EPI_GATE_RESID>(c, tmA, tmB, a, st);
+    case EPI_SWIGLU * 1000 + 256: return launch_one<256, EPI_SWIGLU>(c, tmA, tmB, a, st);
+    case EPI_SWIGLU * 1000 + 128: return launch_one<128, EPI_SWIGLU>(c, tmA, tmB, a, st);
+    case EPI_TRIMUL_AB * 1000 + 256: return launch_one<256, EPI_TRIMUL_AB>(c, tmA, tmB, a, st);
   }
   return fail(c, XFOLD_ERR_ARG, "gemm: unsupported tile %d / epilogue %d", bn, epi);
+}
+
+// Width of the output tiles.  A CTA's time is its number of tiles times what a tile costs, in clocks: the shared-memory
+// reads of the products' operands (128 bytes per clock: 128 + BN of them per 64-wide step of K; they, not the tensor pipe,
+// bound one CTA's products) or the epilogue (about 10 per column, it runs beside the next tile's products), and once the
+// first tile's latency.  Wide tiles win when there are many (fewer operand reads), narrow ones when a wide tile would
+// leave most SMs without work.
+int gemm_tile_n(const Ctx* c, long long M, int N, int K, int batches, int widest, int narrowest) {
+  const long long tm = (M + BM - 1) / BM * batches;
+  const int kb = (K + BK - 1) / BK;
+  int best = widest;
+  double best_cost = 1e30;
+  for (int bn = widest; bn >= narrowest; bn /= 2) {
+    const long long tiles = tm * ((N + bn - 1) / bn), waves = (tiles + c->sm_count - 1) / c->sm_count;
+    const double main_loop = double(kb) * (128 + bn), epi = 10.0 * bn;
+    const double cost = waves * (main_loop > epi ? main_loop : epi) + (main_loop > epi ? epi : main_loop);
+    if (cost < best_cost * 0.98) {
+      best_cost = cost;
+      best = bn;
+    }
+  }
+  return best;
 }
 
 }  // namespace xf

@@ -27,6 +27,9 @@ struct Ctx {
   long long launch_count = 0;  // kernels launched through this context
   int prof_on = 0;             // when set, every launch is bracketed by a pair of CUDA events
   int attn_tag = XFOLD_K_ATTENTION;  // kernel class the attention launchers account their launch to
+  // Set while an operator made of several kernels runs: its weights are older than its first kernel, so that the later
+  // ones may fetch them before their predecessor has finished.
+  int static_weights = 0;
   // While a stage's exchange kernels are meant to run beside its GEMMs (second stream), the persistent GEMMs leave some
   // SMs free and the exchange kernels are sized for them: a GEMM CTA fills its SM, so without free SMs the two serialise.
   int gemm_sms = 0;      // SMs a GEMM launch may take (0: all)
@@ -58,6 +61,13 @@ struct ProfScope {
     cudaEventRecord(r.b, st);
     c->prof_recs.push_back(r);
   }
+};
+
+struct StaticWeights {
+  Ctx* c;
+  int before;
+  explicit StaticWeights(Ctx* c_) : c(c_), before(c_->static_weights) { c->static_weights = 1; }
+  ~StaticWeights() { c->static_weights = before; }
 };
 
 // returns XFOLD_OK or sets ctx->last_error and returns a status code
@@ -95,6 +105,7 @@ struct GemmArgs {
   int a_row_mode = 0;  // 0: tile rows are consecutive rows of A; 1: tile rows step along dim 2, dim 1 fixed
   int a_dim1 = 1;      // row mode 1: extent of dim 1
   int b_batched = 0;
+  int static_b = 0;    // B is written by no kernel that may still run: its first tiles may be fetched before pdl_wait
   int mn_major = 0;    // operands are stored [k][m] and [k][n] (tensor maps: inner dim = m / n, boxes of 64 x 64)
   // PLAIN / SWIGLU / GATE_RESID output
   bf16* out = nullptr;
@@ -119,8 +130,11 @@ struct GemmArgs {
   int* status = nullptr;
 };
 
-// A is described by tmA (box 64 x 128 rows), B by tmB (box 64 x BN rows); BN is 128 or 256.
+// A is described by tmA (box 64 x 128 rows), B by tmB (box 64 x BN rows; SWIGLU below 256: 64 x BN / 2); BN is 64, 128 or
+// 256 (GATE_RESID up to 128, SWIGLU from 128).
 int launch_gemm(Ctx* c, int epi, int bn, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a,
                 cudaStream_t st);
+// the tile width BN to use for an [M x N x K] product (see gemm.cu)
+int gemm_tile_n(const Ctx* c, long long M, int N, int K, int batches, int widest, int narrowest);
 
 }  // namespace xf

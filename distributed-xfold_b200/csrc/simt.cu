@@ -32,10 +32,10 @@ __device__ __forceinline__ bf16 bias16(float v) {
 
 template <int C, int H>
 __global__ void __launch_bounds__(256)
-ln_rows_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
+ln_rows_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
                const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                const float* __restrict__ pw, float* __restrict__ proj, long long proj_plane,
-               const bf16* __restrict__ mod_scale, const bf16* __restrict__ mod_shift, int mod_rows,
+               const bf16* mod_scale, const bf16* mod_shift, int mod_rows,
                bf16* __restrict__ proj_bf16, int trav_inner, int trav_outer, int proj_pitch) {
   constexpr int V = C / 128;  // uint2 (4 x bf16) vectors per lane
   // rows a warp keeps in flight at once: the loads of all of them are issued before any is reduced
@@ -43,6 +43,8 @@ ln_rows_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y, 
   const int lane = threadIdx.x & 31;
   const long long warp_global = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  pdl_wait();
+  pdl_launch();
   for (long long base = warp_global; base < rows; base += nwarps * RPW) {
     uint2 raw[RPW][V];
     long long srow[RPW], pidx[RPW];
@@ -173,15 +175,17 @@ ln_rows_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y, 
 // ---------------------------------------------------------------------------------------------
 template <int H>
 __global__ void __launch_bounds__(256, 3)
-ln128_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
+ln128_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
              const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
              const float* __restrict__ pw, float* __restrict__ proj, long long proj_plane,
-             const bf16* __restrict__ mod_scale, const bf16* __restrict__ mod_shift, int mod_rows,
+             const bf16* mod_scale, const bf16* mod_shift, int mod_rows,
              bf16* __restrict__ proj_bf16, int trav_inner, int trav_outer, int proj_pitch) {
   // dynamic shared memory: H x 128 projection weights, then two tiles of 128 rows x 256 B.  The tile of the next
   // iteration is fetched with cp.async while the current one is processed, so loads stay in flight all the time.
   extern __shared__ __align__(16) float s_pw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>(s_pw + H * 128);
+  pdl_wait();
+  pdl_launch();
   if constexpr (H > 0) {
     // stored as [head][half][lane16][4] so that the 16 lanes of a row read consecutive 16-byte words
     for (int i = threadIdx.x; i < H * 128; i += blockDim.x) {
@@ -335,7 +339,7 @@ constexpr uint32_t LNTC_SMEM = LNTC_OFF_MISC + 2048 + 1024;
 
 template <int H>
 __global__ void __launch_bounds__(256, 3)
-ln128_tc_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
+ln128_tc_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ldy, long long rows,
                 const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                 const float* __restrict__ pw, long long proj_plane, bf16* __restrict__ proj_bf16, int trav_inner,
                 int trav_outer, int proj_pitch, int* status) {
@@ -351,6 +355,11 @@ ln128_tc_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y,
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int lane = threadIdx.x & 31, half = lane >> 4, l16 = lane & 15, warp = threadIdx.x >> 5;
   const AbortCtx ab{cta_abort, status};
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, 32);
+    tmem_relinquish();
+  }
+  pdl_wait();
 
   // folded weights: one head per half-warp pass
   for (int h = warp * 2 + half; h < 16; h += 16) {
@@ -389,13 +398,10 @@ ln128_tc_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ y,
     fence_barrier_init();
   }
   fence_proxy_async_smem();
-  if (warp == 0) {
-    tmem_alloc(tmem_slot, 32);
-    tmem_relinquish();
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch();
   const uint32_t tmem_base = *tmem_slot;
 
   const int c0 = l16 * 8;
@@ -541,7 +547,7 @@ static int launch_ln128_tc(Ctx* c, const bf16* x, long long ldx, bf16* y, long l
     attr_done[c->device & 7] = true;
   }
   ProfScope ps(c, XFOLD_K_LAYERNORM, st);
-  ln128_tc_kernel<H><<<(int)blocks, 256, LNTC_SMEM, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, plane, pbf, tin, tout, tpitch,
+  launch_pdl(ln128_tc_kernel<H>, (int)blocks, 256, LNTC_SMEM, st, x, ldx, y, ldy, rows, g, b, eps, pw, plane, pbf, tin, tout, tpitch,
                                                           c->d_status);
   return check_launch(c, "ln128_tc_kernel");
 }
@@ -578,10 +584,10 @@ static int launch_ln128(Ctx* c, const bf16* x, long long ldx, bf16* y, long long
   }
   ProfScope ps(c, XFOLD_K_LAYERNORM, st);
   switch (H) {
-    case 0: ln128_kernel<0><<<(int)blocks, 256, sm, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 4: ln128_kernel<4><<<(int)blocks, 256, sm, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 16: ln128_kernel<16><<<(int)blocks, 256, sm, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 64: ln128_kernel<64><<<(int)blocks, 256, sm, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 0: launch_pdl(ln128_kernel<0>, (int)blocks, 256, sm, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 4: launch_pdl(ln128_kernel<4>, (int)blocks, 256, sm, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 16: launch_pdl(ln128_kernel<16>, (int)blocks, 256, sm, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 64: launch_pdl(ln128_kernel<64>, (int)blocks, 256, sm, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
     default: return fail(c, XFOLD_ERR_ARG, "layernorm: fused projection supports 0, 4, 16 or 64 outputs, got %d", H);
   }
   return check_launch(c, "ln128_kernel");
@@ -598,10 +604,10 @@ static int launch_ln_c(Ctx* c, const bf16* x, long long ldx, bf16* y, long long 
   if (blocks <= 0) return XFOLD_OK;
   ProfScope ps(c, XFOLD_K_LAYERNORM, st);
   switch (H) {
-    case 0: ln_rows_kernel<C, 0><<<(int)blocks, 256, 0, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 4: ln_rows_kernel<C, 4><<<(int)blocks, 256, 0, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 16: ln_rows_kernel<C, 16><<<(int)blocks, 256, 0, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
-    case 64: ln_rows_kernel<C, 64><<<(int)blocks, 256, 0, st>>>(x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 0: launch_pdl(ln_rows_kernel<C, 0>, (int)blocks, 256, 0, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 4: launch_pdl(ln_rows_kernel<C, 4>, (int)blocks, 256, 0, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 16: launch_pdl(ln_rows_kernel<C, 16>, (int)blocks, 256, 0, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
+    case 64: launch_pdl(ln_rows_kernel<C, 64>, (int)blocks, 256, 0, st, x, ldx, y, ldy, rows, g, b, eps, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch); break;
     default: return fail(c, XFOLD_ERR_ARG, "layernorm: fused projection supports 0, 4, 16 or 64 outputs, got %d", H);
   }
   return check_launch(c, "ln_rows_kernel");
@@ -635,12 +641,14 @@ constexpr size_t CMLN_SMEM = 2 * CMLN_TILE_BYTES + 2 * 4 * CMLN_TOK * sizeof(flo
 // The tile of the NEXT iteration is fetched with cp.async (global -> shared without passing through registers) while
 // the current one is normalised and stored, so loads stay in flight through the compute and store phases.
 __global__ void __launch_bounds__(256, 3)
-cm_ln_kernel(const bf16* __restrict__ in, long long chan_stride, long long row_stride, int R, int N,
+cm_ln_kernel(const bf16* in, long long chan_stride, long long row_stride, int R, int N,
              bf16* __restrict__ out, const float* __restrict__ gamma, const float* __restrict__ beta, float eps) {
   extern __shared__ __align__(16) uint8_t cmln_smem[];
   bf16 (*tiles)[128][CMLN_PITCH] = reinterpret_cast<bf16 (*)[128][CMLN_PITCH]>(cmln_smem);
   float (*psum)[CMLN_TOK] = reinterpret_cast<float (*)[CMLN_TOK]>(cmln_smem + 2 * CMLN_TILE_BYTES);
   float (*psq)[CMLN_TOK] = psum + 4;
+  pdl_wait();
+  pdl_launch();
   const int tiles_j = (N + CMLN_TOK - 1) / CMLN_TOK;
   const long long ntiles = (long long)R * tiles_j;
   const bool vec_ok = ((chan_stride | row_stride) & 7) == 0;
@@ -748,7 +756,7 @@ int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_st
     if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "channel LayerNorm smem attribute: %s", cudaGetErrorString(e));
     attr_done[c->device & 7] = true;
   }
-  cm_ln_kernel<<<(int)blocks, 256, CMLN_SMEM, st>>>(in, chan_stride, row_stride, R, N, out, gamma, beta, eps);
+  launch_pdl(cm_ln_kernel, (int)blocks, 256, CMLN_SMEM, st, in, chan_stride, row_stride, R, N, out, gamma, beta, eps);
   return check_launch(c, "cm_ln_kernel");
 }
 
@@ -756,7 +764,9 @@ int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_st
 // SwiGLU over rows: in [rows][2F] -> out [rows][F] = silu(in[:, :F]) * in[:, F:]
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-swiglu_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, long long rows, int F) {
+swiglu_kernel(const bf16* in, bf16* __restrict__ out, long long rows, int F) {
+  pdl_wait();
+  pdl_launch();
   const long long n8 = rows * (F / 8);
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n8;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -783,7 +793,7 @@ int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cuda
   const long long cap = (long long)c->sm_count * 16;
   if (blocks > cap) blocks = cap;
   ProfScope ps(c, XFOLD_K_SWIGLU, st);
-  swiglu_kernel<<<(int)blocks, 256, 0, st>>>(in, out, rows, F);
+  launch_pdl(swiglu_kernel, (int)blocks, 256, 0, st, in, out, rows, F);
   return check_launch(c, "swiglu_kernel");
 }
 

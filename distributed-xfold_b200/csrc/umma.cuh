@@ -157,6 +157,8 @@ template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
+// waits until this thread's bulk stores have been written (the .read form: only read out of shared memory)
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -265,10 +267,14 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // ------------------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with the attribute (launch_pdl in internal.h) may start while its
 // predecessor in the stream still runs; everything up to pdl_wait() -- barriers, tensor memory, weights that no kernel of
-// the call writes -- overlaps the predecessor's tail.  Rules that keep it safe: EVERY thread of such a kernel calls
-// pdl_wait() before it touches anything a predecessor wrote or still reads (so that the completion of a kernel implies
-// the completion of all before it), and pdl_launch() comes after the tensor memory allocation (a successor that got the
-// tensor memory first would wait for this kernel, and this kernel for the tensor memory).
+// the call writes -- overlaps the predecessor's tail.  Rules that keep it safe:
+//   * every thread calls pdl_wait() before it touches anything a predecessor wrote or still reads, so that the completion
+//     of a kernel implies the completion of all before it;
+//   * pdl_launch() comes after the tensor memory allocation (a successor that got the tensor memory first would wait for
+//     this kernel, and this kernel for the tensor memory) and after pdl_wait(): L1 is invalidated when a kernel starts, and
+//     a kernel two places ahead must not start while this kernel's predecessor still reads what this kernel overwrites;
+//   * no kernel reads through L1 a buffer that it also writes, and no pointer to activations is const __restrict__: the
+//     compiler treats such loads as invariant and may move them above pdl_wait().
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
