@@ -60,6 +60,15 @@ class PairformerWeightsF32(C.Structure):
                 ("sa_qkvg", vp), ("sa_qkvg_bias", vp), ("sa_out", vp), ("single_transition", TransitionWeightsF32)]
 
 
+class DiffusionBlockWeights(C.Structure):
+    _fields_ = [(n, vp) for n in ("w_qkvg", "qkvg_bias", "qkvg_scale", "w_out", "w1_packed", "w2")]
+
+
+class DiffusionWeights(C.Structure):
+    _fields_ = [(n, ci) for n in ("C", "C_cond", "H", "Dp", "F", "num_blocks")] + \
+               [(n, vp) for n in ("w_mod", "b_mod", "w_gate", "b_gate")] + [("blocks", C.POINTER(DiffusionBlockWeights))]
+
+
 class ShardDesc(C.Structure):
     _fields_ = [("world", ci), ("rank", ci), ("n_tokens", ci), ("row_starts", C.POINTER(ci)),
                 ("zbuf0", C.POINTER(vp)), ("zbuf1", C.POINTER(vp)), ("plane_a", C.POINTER(vp)), ("plane_b", C.POINTER(vp)),
@@ -119,6 +128,8 @@ SIGNATURES = {
     "xfold_pair_bias_prepare_fwd": (ci, [vp, vp, ci, ci, vp, vp]),
     "xfold_pair_logits_prepared_fwd": (ci, [vp, vp, ci, vp, vp, vp, ci, vp, vp]),
     "xfold_attention_pair_bias_core_prepared_fwd": (ci, [vp, vp, ci, ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
+    "xfold_diffusion_workspace_bytes": (sz, [ci, ci, C.POINTER(DiffusionWeights)]),
+    "xfold_diffusion_transformer_fwd": (ci, [vp, vp, ci, ci, vp, vp, C.POINTER(DiffusionWeights), C.POINTER(vp), vp, sz, vp]),
     "xfold_cross_attention_workspace_bytes": (sz, [ci, ci, ci, ci, ci]),
     "xfold_cross_attention_fwd": (ci, [vp, vp, vp, ci, ci, ci, ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "xfold_pairformer_f32_workspace_bytes": (sz, [ci]),

@@ -81,8 +81,8 @@ static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M,
   return launch_gemm(c, epi, bn, tA, tB, a, st);
 }
 
-static int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
-                        const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0) {
+int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
+                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0, int f16_col1) {
   GemmArgs a;
   const int bn = gemm_tile_n(c, M, N, K, 1, 256, 64);
   a.static_b = c->static_weights;
@@ -97,13 +97,7 @@ static int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K
   return gemm_rows(c, EPI_PLAIN, x, ldx, M, K, w, N, K, a, bn, st);
 }
 
-// for the translation units that compose operators out of plain projections
-int linear_plain_fwd(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
-                     const float* scale, bf16* out, long long ldo, cudaStream_t st) {
-  return linear_plain(c, x, ldx, M, K, w, N, bias, scale, out, ldo, st);
-}
-
-static int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N,
+int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N,
                              const bf16* gate, long long ldg, int row_gate_mod, const bf16* resid, long long ldr,
                              bf16* out, long long ldo, cudaStream_t st) {
   GemmArgs a;
@@ -151,7 +145,7 @@ static int linear_gate_resid_chunked(Ctx* c, const bf16* x, long long ldx, long 
   return rc;
 }
 
-static int linear_swiglu(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* wp, int F, bf16* out,
+int linear_swiglu(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* wp, int F, bf16* out,
                          long long ldo, cudaStream_t st) {
   if (F % 128) return fail(c, XFOLD_ERR_ARG, "linear_swiglu: F must be a multiple of 128");
   GemmArgs a;

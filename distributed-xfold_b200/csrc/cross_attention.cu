@@ -109,9 +109,6 @@ __global__ void __launch_bounds__(256) xattn_kernel(XAttnArgs p) {
   }
 }
 
-int linear_plain_fwd(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
-                     const float* scale, bf16* out, long long ldo, cudaStream_t st);
-
 }  // namespace xf
 
 using namespace xf;
@@ -136,9 +133,9 @@ int xfold_cross_attention_fwd(xfold_ctx* cx, const void* q_data, const void* m_d
   if (!ws || !cv.ok()) return fail(c, XFOLD_ERR_ARG, "cross attention: workspace too small (%zu < %zu)", ws_bytes, cv.off);
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
-  if ((rc = linear_plain_fwd(c, (const bf16*)q_data, Ca, (long long)B * S, Ca, (const bf16*)w_qg, 2 * W, qg_bias, qg_scale, qg,
+  if ((rc = linear_plain(c, (const bf16*)q_data, Ca, (long long)B * S, Ca, (const bf16*)w_qg, 2 * W, qg_bias, qg_scale, qg,
                              2 * W, st))) return rc;
-  if ((rc = linear_plain_fwd(c, (const bf16*)m_data, Cm, (long long)B * K, Cm, (const bf16*)w_kv, 2 * W, nullptr, nullptr, kv,
+  if ((rc = linear_plain(c, (const bf16*)m_data, Cm, (long long)B * K, Cm, (const bf16*)w_kv, 2 * W, nullptr, nullptr, kv,
                              2 * W, st))) return rc;
   XAttnArgs a{qg, kv, bias, (bf16*)out, B, S, K, H};
   const long long total = (long long)B * H * S;

@@ -48,6 +48,14 @@ int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int tra
 int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_stride, int R, int N, bf16* out,
                  const float* gamma, const float* beta, float eps, cudaStream_t st);
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
+// ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
+int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
+                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0);
+int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const bf16* gate,
+                      long long ldg, int row_gate_mod, const bf16* resid, long long ldr, bf16* out, long long ldo,
+                      cudaStream_t st);
+int linear_swiglu(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* wp, int F, bf16* out, long long ldo,
+                  cudaStream_t st);
 // ---- stages of the operators (api.cu); (chan, row) strides are in elements -------------------------------
 int trimul_project(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed_store,
                    const xfold_trimul_weights* w, bf16* x, bf16* a_out, bf16* b_out, bf16* g, long long chan_stride,

@@ -1,11 +1,12 @@
 """DiffusionTransformer on the sm_100a kernels (reference: nn/d_diffusion_transformer.py:37-310).
 
 24 blocks in 6 super-blocks; per block  act += AttentionPairBias(act, mask, pair_logits, single_cond)
-and  act += DiffusionTransition(act, single_cond).  Everything below is a composition of C-ABI calls:
+and  act += DiffusionTransition(act, single_cond).  A step is one C-ABI call (``xfold_diffusion_transformer_fwd``):
 
-    AdaptiveLayerNorm        -> conditioning GEMM on LN(single_cond), then LayerNorm with fused modulation
+    conditioning             -> one LayerNorm of single_cond and two GEMMs for the modulations and gates of many blocks
+    AdaptiveLayerNorm        -> LayerNorm with fused modulation
     q/k/v/gate projections   -> one GEMM with query bias and D^-0.5 folded into the epilogue
-    attention (16 x 48 -> 64)-> flash kernel with the fp32 pair bias
+    attention (16 x 48 -> 64)-> flash kernel with the prepared pair logits
     AdaLNZero                -> output GEMM whose epilogue multiplies by sigmoid(cond) per token row and adds the residual
     DiffusionTransition      -> GEMM with SwiGLU epilogue, then the AdaLNZero GEMM
 
@@ -16,11 +17,12 @@ reference's ShardInfo rule (d_alphafold3.py:381-385); no collective is needed in
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Dict, List, Optional
 
 import torch
 
-from . import ops
+from . import _cabi, ops
 from .distribute_utils import ShardInfo
 
 State = Dict[str, torch.Tensor]
@@ -47,27 +49,30 @@ class _PackedAdaLN:
         return ops.layernorm(x, mod_scale=sc, mod_shift=sh)       # sigmoid(scale) * LN(x) + shift
 
 
-class _PackedAdaLNZero:
-    def __init__(self, state: State, prefix: str, device, w_out: torch.Tensor):
-        self.w_out = w_out
-        self.wc = ops._b16(state[prefix + "adaptive_zero_cond.weight"], device)
-        bc = state.get(prefix + "adaptive_zero_cond.bias")
-        self.bc = None if bc is None else ops._f32(bc, device)
-
-    def __call__(self, x: torch.Tensor, cond: torch.Tensor, resid: torch.Tensor, n_tokens: int) -> torch.Tensor:
-        gate = ops.linear(cond, self.wc, self.bc)                 # [N, c]; the kernel applies the sigmoid
-        return ops.linear_gate_residual(x, self.w_out, gate, resid, row_gate_mod=n_tokens, out=resid)
+def _conditioning(state: State, p_att: str, p_tr: str):
+    """The conditioning projections of one block: (mod [4c, c_cond], its bias [4c], gate [2c, c_cond], its bias [2c]).  The
+    scale of the conditioning's LayerNorm goes into the columns of the first, so that all blocks share one LayerNorm."""
+    mod, mod_b, gate, gate_b = [], [], [], []
+    for p in (p_att, p_tr):
+        ln = p + "adaptive_layernorm."
+        g = state[ln + "single_cond_layer_norm.weight"].detach().float()
+        scale_b = state[ln + "single_cond_scale.bias"].detach().float()
+        mod += [state[ln + n + ".weight"].detach().float() * g for n in ("single_cond_scale", "single_cond_bias")]
+        mod_b += [scale_b, torch.zeros_like(scale_b)]
+        w = state[p + "adaptive_zero_init.adaptive_zero_cond.weight"].detach().float()
+        b = state.get(p + "adaptive_zero_init.adaptive_zero_cond.bias")
+        gate.append(w)
+        gate_b.append(w.new_zeros(w.shape[0]) if b is None else b.detach().float())
+    return mod, mod_b, gate, gate_b
 
 
 class PackedDiffusionBlock:
     def __init__(self, state: State, p_att: str, p_tr: str, device, num_head: int = 16):
         self.att = ops.PackedSelfAttention(state, p_att, device, num_head)
-        self.att_ln = _PackedAdaLN(state, p_att + "adaptive_layernorm.", device)
-        self.att_zero = _PackedAdaLNZero(state, p_att + "adaptive_zero_init.", device, self.att.w_out)
-        self.tr_ln = _PackedAdaLN(state, p_tr + "adaptive_layernorm.", device)
         self.tr_w1 = ops._b16(ops.pack_swiglu_weight(state[p_tr + "transition1.weight"]), device)
-        self.tr_zero = _PackedAdaLNZero(state, p_tr + "adaptive_zero_init.", device,
-                                        ops._b16(state[p_tr + "adaptive_zero_init.transition2.weight"], device))
+        self.tr_w2 = ops._b16(state[p_tr + "adaptive_zero_init.transition2.weight"], device)
+        self.c = _cabi.DiffusionBlockWeights(ops._ptr(self.att.w_qkvg), ops._ptr(self.att.bias), ops._ptr(self.att.scale),
+                                             ops._ptr(self.att.w_out), ops._ptr(self.tr_w1), ops._ptr(self.tr_w2))
 
 
 class PackedDiffusionTransformer:
@@ -78,8 +83,17 @@ class PackedDiffusionTransformer:
         self.pair_ln_b = ops._f32(state.get(prefix + "pair_input_layer_norm.bias"), device)
         self.pl_w = ops._f32(torch.cat([state[prefix + f"pair_logits_projection.{i}.weight"]
                                         for i in range(num_blocks // super_block_size)], 0), device)
-        self.blocks = [PackedDiffusionBlock(state, prefix + f"self_attention.{i}.", prefix + f"transition_block.{i}.",
-                                            device, num_head) for i in range(num_blocks)]
+        names = [(prefix + f"self_attention.{i}.", prefix + f"transition_block.{i}.") for i in range(num_blocks)]
+        self.blocks = [PackedDiffusionBlock(state, p_att, p_tr, device, num_head) for p_att, p_tr in names]
+        parts = [_conditioning(state, p_att, p_tr) for p_att, p_tr in names]
+        stack = [torch.cat([t for p in parts for t in p[k]], 0) for k in range(4)]
+        self.w_mod, self.w_gate = ops._b16(stack[0], device), ops._b16(stack[2], device)
+        self.b_mod, self.b_gate = ops._f32(stack[1], device), ops._f32(stack[3], device)
+        a = self.blocks[0].att
+        self._arr = (_cabi.DiffusionBlockWeights * num_blocks)(*[b.c for b in self.blocks])
+        self.c = _cabi.DiffusionWeights(a.C, self.w_mod.shape[1], a.H, a.Dp, self.blocks[0].tr_w2.shape[1], num_blocks,
+                                        ops._ptr(self.w_mod), ops._ptr(self.b_mod), ops._ptr(self.w_gate),
+                                        ops._ptr(self.b_gate), self._arr)
 
     def pair_logits(self, pair_cond: torch.Tensor) -> List[torch.Tensor]:
         """[N, N, 128] bf16 -> per super-block float16 [super_block_size, heads, N, pad8(N)], the prepared operand of the
@@ -91,17 +105,30 @@ class PackedDiffusionTransformer:
     def forward(self, act: torch.Tensor, mask: Optional[torch.Tensor], single_cond: torch.Tensor,
                 pair_logits: List[torch.Tensor]) -> torch.Tensor:
         """act bf16 [S, N, 768] or [N, 768] (updated in place and returned); single_cond bf16 [N, 384]."""
-        squeeze = act.dim() == 2
-        a = act[None] if squeeze else act
-        n = a.shape[1]
-        for i, blk in enumerate(self.blocks):
-            pl = pair_logits[i // self.sb][i % self.sb]
-            xn = blk.att_ln(a, single_cond)
-            o = ops.attention_pair_bias_core(xn, blk.att, pl, mask)
-            blk.att_zero(o, single_cond, a, n)
-            xn = blk.tr_ln(a, single_cond)
-            h = ops.linear_swiglu(xn, blk.tr_w1)
-            blk.tr_zero(h, single_cond, a, n)
+        ops._need_cuda(act, mask, single_cond, *pair_logits)
+        assert act.dtype == BF16 and act.is_contiguous() and act.shape[-1] == self.c.C
+        assert single_cond.dtype == BF16 and single_cond.is_contiguous()
+        s = 1 if act.dim() == 2 else act.shape[0]
+        n = act.shape[-2]
+        assert tuple(single_cond.shape) == (n, self.c.C_cond)
+        shape = (self.sb, self.num_head, n, (n + 7) // 8 * 8)
+        if any(t.dtype == torch.float32 for t in pair_logits):   # plain logits [super_block_size, heads, N, N]
+            pair_logits = [ops.prepare_pair_bias(t.reshape(-1, n, n).contiguous()).reshape(shape)
+                           if t.dtype == torch.float32 else t for t in pair_logits]
+        ptrs = (C.c_void_p * self.num_blocks)()
+        for i, t in enumerate(pair_logits):
+            assert t.dtype == torch.float16 and tuple(t.shape) == shape and t.is_contiguous()
+            base, step = t.data_ptr(), t.stride(0) * 2
+            for j in range(self.sb):
+                ptrs[i * self.sb + j] = base + j * step
+        if mask is not None:
+            mask = mask.to(torch.float32).contiguous()
+        dev = ops._dev(act)
+        lib = _cabi.load()
+        ws = ops._Workspace.get(dev, lib.xfold_diffusion_workspace_bytes(s, n, C.byref(self.c)))
+        rc = lib.xfold_diffusion_transformer_fwd(_cabi.ctx(dev), ops._ptr(act), s, n, ops._ptr(mask), ops._ptr(single_cond),
+                                                 C.byref(self.c), ptrs, ops._ptr(ws), ws.numel(), ops._stream(dev))
+        _cabi.check(rc, dev, "xfold_diffusion_transformer_fwd")
         return act
 
 

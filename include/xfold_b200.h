@@ -185,6 +185,34 @@ int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* ctx, const void* xn, 
                                                 const void* prepared_bias, const float* mask, void* out, void* ws,
                                                 size_t ws_bytes, void* stream);
 
+/* All blocks of the DiffusionTransformer (nn/d_diffusion_transformer.py:267-310) for one denoising step of S samples, in
+ * place on act bf16 [S][N][C].  The conditioning projections of all blocks are stacked:
+ *   w_mod  bf16 [num_blocks * 4C][C_cond]: per block scale, shift (attention), scale, shift (transition), every column
+ *          multiplied by the block's single_cond_layer_norm scale; b_mod float32 [num_blocks * 4C] (zero for the shifts)
+ *   w_gate bf16 [num_blocks * 2C][C_cond]: per block the AdaLN-Zero gates of attention and transition; b_gate or null
+ * w_qkvg / w_out as for xfold_attention_pair_bias_core_fwd (heads padded to Dp), w1_packed [2F][C], w2 [C][F] as for
+ * xfold_linear_swiglu_fwd; pair_logits: per block the prepared bias [H][N][pad8(N)]; mask float32 [N] or null. */
+typedef struct {
+  const void* w_qkvg;
+  const float* qkvg_bias;
+  const float* qkvg_scale;
+  const void* w_out;
+  const void* w1_packed;
+  const void* w2;
+} xfold_diffusion_block_weights;
+typedef struct {
+  int C, C_cond, H, Dp, F, num_blocks;
+  const void* w_mod;
+  const float* b_mod;
+  const void* w_gate;
+  const float* b_gate;
+  const xfold_diffusion_block_weights* blocks;
+} xfold_diffusion_weights;
+size_t xfold_diffusion_workspace_bytes(int S, int N, const xfold_diffusion_weights* w);
+int xfold_diffusion_transformer_fwd(xfold_ctx* ctx, void* act, int S, int N, const float* mask, const void* single_cond,
+                                    const xfold_diffusion_weights* w, const void* const* pair_logits, void* ws,
+                                    size_t ws_bytes, void* stream);
+
 /* The same core with one mask row per batch entry (mask float32, row b at mask + b * mask_ld; mask_ld = 0: one row for
  * all), which is what `_alpha_attention::grid_self_attn_forward` takes as its `bias` [B, 1, 1, S]
  * (csrc/Alpha_Attention.cpp:50-70). */
