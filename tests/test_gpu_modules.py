@@ -242,3 +242,23 @@ def test_cross_attention(ops, oracle, golden, case):
     out = ops.cross_attention(qd.to(BF).cuda(), md.to(BF).cuda(), bb.cuda(), w)
     ops.synchronize_and_check()
     assert relf(out.float().cpu(), ref) < 2e-2
+
+
+@pytest.mark.parametrize("B,S,K,H,D", [(2, 1, 1, 1, 16), (1, 16, 128, 4, 64), (3, 33, 129, 5, 16), (2, 47, 260, 3, 32)])
+def test_cross_attention_tile_edges(ops, oracle, B, S, K, H, D):
+    """Sizes around the 16-query, 32-query, 4-head and 128-key steps of the kernel, with keys masked through the bias."""
+    c = H * D if (H * D) % 8 == 0 else 128
+    g = torch.Generator().manual_seed(B + S + K)
+    ws = {n: torch.randn(shape, generator=g) / c ** 0.5 for n, shape in (("query_w", (c, H, D)), ("query_b", (1, H, D)),
+          ("key_w", (c, H, D)), ("value_w", (c, H, D)), ("gating_w", (c, H, D)))}
+    qd, md = torch.randn(B, S, c, generator=g), torch.randn(B, K, c, generator=g)
+    keep = torch.rand(B, 1, 1, K, generator=g) > 0.2
+    keep[..., 0] = True
+    bb = torch.randn(B, H, S, K, generator=g) + 1e9 * (keep.float() - 1)
+    rb = lambda t: t.to(BF).float()
+    ref = oracle.cross_attention(rb(qd), rb(md), bb, rb(ws["query_w"]), ws["query_b"], rb(ws["key_w"]), rb(ws["value_w"]),
+                                 rb(ws["gating_w"]))
+    w = ops.PackedCrossAttention(ws["query_w"], ws["query_b"], ws["key_w"], ws["value_w"], ws["gating_w"], "cuda")
+    out = ops.cross_attention(qd.to(BF).cuda(), md.to(BF).cuda(), bb.cuda(), w)
+    ops.synchronize_and_check()
+    assert relf(out.float().cpu(), ref) < 2e-2
