@@ -82,7 +82,8 @@ static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M,
 }
 
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
-                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0, int f16_col1) {
+                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0, int f16_col1,
+                 int log2e_cols) {
   GemmArgs a;
   const int bn = gemm_tile_n(c, M, N, K, 1, 256, 64);
   a.static_b = c->static_weights;
@@ -94,6 +95,7 @@ int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const
   a.col_scale = scale;
   a.f16_col0 = f16_col0;
   a.f16_col1 = f16_col1;
+  a.log2e_cols = log2e_cols;
   return gemm_rows(c, EPI_PLAIN, x, ldx, M, K, w, N, K, a, bn, st);
 }
 
@@ -361,7 +363,7 @@ int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask,
                         bf16* upd, const ChunkHook* hook) {
   const long long M = (long long)R * N;
   // the v columns are stored as fp16: the attention kernel's P V product runs with fp16 operands
-  int rc = linear_plain(c, x, 128, M, 128, (const bf16*)w->w_qkvg, 512, nullptr, w->qkvg_scale, qkvg, 512, st, 256, 384);
+  int rc = linear_plain(c, x, 128, M, 128, (const bf16*)w->w_qkvg, 512, nullptr, w->qkvg_scale, qkvg, 512, st, 256, 384, 128);
   if (rc) return rc;
   if ((rc = launch_mext(c, mask, mask_ld, mext, R, N, st))) return rc;
   const long long seq_stride = transposed ? (long long)R * 128 : 128;
@@ -446,7 +448,7 @@ static int apb_core_fwd_(Ctx* c, const bf16* xn, int B, int S, int C, int H, int
   if (!ws || !cv.ok()) return fail(c, XFOLD_ERR_ARG, "apb: workspace too small (%zu < %zu)", ws_bytes, cv.off);
   const int Wd = H * Dp;
   // the v columns leave the projection as fp16: P and V are the fp16 operands of the P V product
-  int rc = linear_plain(c, xn, C, (long long)B * S, C, w_qkvg, 4 * Wd, qkvg_bias, qkvg_scale, W.qkvg, 4 * Wd, st, 2 * Wd, 3 * Wd);
+  int rc = linear_plain(c, xn, C, (long long)B * S, C, w_qkvg, 4 * Wd, qkvg_bias, qkvg_scale, W.qkvg, 4 * Wd, st, 2 * Wd, 3 * Wd, Wd);
   if (rc) return rc;
   if (!pair_biasT) {
     if ((rc = launch_bias_transpose(c, pair_bias, W.biasT, H, S, W.ldq, st))) return rc;

@@ -130,7 +130,7 @@ static int diffusion_fwd(Ctx* c, bf16* act, int S, int N, const float* mask, con
     if ((rc = launch_adaln(c, act, D.xn, M, C, mod, mod + C, ldm, N, st))) return rc;
     // the v columns leave the projection as fp16: P and V are the fp16 operands of the P V product
     if ((rc = linear_plain(c, D.xn, C, M, C, (const bf16*)k.w_qkvg, 4 * Wd, k.qkvg_bias, k.qkvg_scale, D.qkvg, 4 * Wd, st,
-                           2 * Wd, 3 * Wd))) return rc;
+                           2 * Wd, 3 * Wd, Wd))) return rc;
     c->attn_tag = XFOLD_K_APB_ATTENTION;
     rc = launch_attention2(c, D.qkvg, 4 * Wd, N, S, 0, 0, Wd, 2 * Wd, 3 * Wd, w->H, (const bf16*)logits[b], ldq, D.mext, 1, D.o,
                            Wd, (long long)N * Wd, st, w->Dp);

@@ -321,6 +321,12 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               for (int e = 0; e < 32; ++e) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
             }
           }
+          if constexpr (EPI == EPI_PLAIN) {
+            if (colw < p.log2e_cols) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e) v[e] *= 1.4426950408889634f;
+            }
+          }
           if constexpr (EPI == EPI_GATE_RESID) {
             // order: v * sigmoid(gate) first, residual added last
             const bool rvalid = m < p.M;

@@ -113,6 +113,7 @@ struct GemmArgs {
   const float* col_bias = nullptr;
   const float* col_scale = nullptr;
   int f16_col0 = 0, f16_col1 = 0;  // PLAIN: output columns [f16_col0, f16_col1) are stored as fp16 (multiples of 32)
+  int log2e_cols = 0;  // PLAIN: output columns [0, log2e_cols) times log2(e) (a multiple of 32): the attention works in base 2
   const bf16* resid = nullptr;
   long long ldr = 0;
   const bf16* gate = nullptr;

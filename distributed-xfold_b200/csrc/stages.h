@@ -50,7 +50,8 @@ int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_st
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
 // ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
-                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0);
+                 const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0,
+                 int log2e_cols = 0);
 int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const bf16* gate,
                       long long ldg, int row_gate_mod, const bf16* resid, long long ldr, bf16* out, long long ldo,
                       cudaStream_t st);

@@ -120,6 +120,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// The same for a converged warp that stays converged: every branch depends on a vote.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const AbortCtx& ab, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (uint32_t spin = 1;; ++spin) {
+    if (__all_sync(0xffffffffu, mbar_try_wait_parked(bar, parity, XF_PARK_NS))) return true;
+    if ((spin & 15u) == 0) {
+      if (__any_sync(0xffffffffu, *ab.cta_abort != 0)) return false;
+      if (__any_sync(0xffffffffu, clock64() - t0 > XF_WAIT_CYCLES)) {
+        *ab.cta_abort = 1;
+        atomicCAS(ab.status, 0, code);
+        return false;
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------
 // TMA (tensor maps are passed as __grid_constant__ kernel parameters)
 // ------------------------------------------------------------------------------------
@@ -205,6 +222,33 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same, issued by the lanes with go != 0 (one, elected by the caller) of a converged warp: no branch, so that operands
+// can stay in uniform registers.
+__device__ __forceinline__ void umma_ss_if(uint32_t go, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(go)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_if(uint32_t go, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(go)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t go, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(smem_u32(bar)), "r"(go)
       : "memory");
 }
 // Arrives (count 1) on the mbarrier once every MMA issued so far by this thread is done.
