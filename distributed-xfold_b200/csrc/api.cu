@@ -395,6 +395,13 @@ int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_tr
   if (rows <= 0) return XFOLD_OK;
   // before any size arithmetic or launch: row counts the kernels cannot index, or whose byte sizes would wrap
   if (C <= 0 || F <= 0 || rows >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "transition: bad shape (%lld rows, C=%d, F=%d)", rows, C, F);
+  // 128-wide rows (the pair representation): one kernel, no scratch.  With a hook (the caller's work after each chunk of
+  // rows) only for a single chunk.
+  if (C == 128 && F % 128 == 0 && (!hook || !hook->after || hook->parts <= 1)) {
+    const int rc = launch_transition128(c, x, upd ? upd : x, rows, F, w->ln_gamma, w->ln_beta, (const bf16*)w->w1_packed,
+                                        (const bf16*)w->w2, upd != nullptr, st);
+    return rc || !hook || !hook->after ? rc : hook->after(0, rows);
+  }
   Carver cv(ws, ws_bytes);
   bf16* xn = (bf16*)cv.take((size_t)rows * C * 2);
   bf16* h = (bf16*)cv.take((size_t)rows * F * 2);

@@ -118,12 +118,6 @@ __device__ __forceinline__ void tmem_st16_(uint32_t taddr, const uint32_t (&r)[1
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait_() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// true in exactly one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
-}
 // Which of a sweep's 16 pairs take the polynomial: two.  (TriangleAttention, 1024 tokens: none 1.33 ms, two or three 1.27,
 // four or five 1.32, six 1.44 -- the FMA pipe and the issue slots are then the longer queue.)
 __host__ __device__ constexpr bool poly_pair(int e) { return (e & 7) == 7; }

@@ -47,6 +47,8 @@ int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int tra
                       bf16* out, long long out_seq_stride, long long out_batch_stride, cudaStream_t st, int head_dim = 32);
 int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_stride, int R, int N, bf16* out,
                  const float* gamma, const float* beta, float eps, cudaStream_t st);
+int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F, const float* gamma, const float* beta,
+                         const bf16* w1, const bf16* w2, int update_only, cudaStream_t st);
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
 // ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,

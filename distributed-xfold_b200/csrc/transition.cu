@@ -1,0 +1,342 @@
+// Transition of the pair representation in one kernel:  x += W2 swiglu(W1 LN(x))  for rows of 128, F hidden units
+// (csrc/Alpha_Attention.cpp:72-92, kernel_test/transition.py:22-48 state the operator).
+//
+// Bound: the tensor core.  Per tile of 128 rows 25 M multiply-adds (6100 clocks) and 65536 sigmoids (4096 clocks of the
+// special-function unit); the weights are 384 KB at F = 512, so two tiles share each block of them.  The only HBM traffic is
+// x itself.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) the normalised rows and the hidden activations made six
+// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows; this kernel 0.47 ms (one tile at a time: 0.49 ms).
+//
+// Persistent CTAs, a pair of tiles (A, B) of 128 rows at a time, hidden units in blocks of 64; per tile
+//     D1 = LN(x) W1(block)^T   [128 x (64 SiLU | 64 linear)]      tensor memory
+//     h  = silu(D1a) * D1b     bf16, shared memory (K-major, 128-byte swizzle)
+//     D2 += h W2(block)^T      [128 x 128]                        tensor memory
+//   warp 0         : TMA -- x tiles, weight blocks of 32 KB (W1, free after D1) and 16 KB (W2), two of each
+//   warp 1         : tcgen05.mma issuer; D1 of a block is issued ahead of D2 of the block before it
+//   warps 2 - 9    : LayerNorm in place, one thread per row
+//   warps 10 - 17  : one set of four per tile: D1 -> h; finally D2 + x -> the h buffer in two halves, which leave by TMA
+// With no more tiles than SMs a CTA takes one tile (B is left out).
+#include "internal.h"
+#include "stages.h"
+#include "umma.cuh"
+
+namespace xf {
+
+constexpr uint32_t TR_TILE = 32768;                       // [2 halves][128 rows][64 columns], swizzled
+constexpr uint32_t TR_W1 = 32768, TR_W2 = 16384;          // a block's weights: [2 K halves][128 rows][64], [128 rows][64]
+constexpr uint32_t TR_H = 16384;
+constexpr uint32_t TR_OFF_N = 0, TR_OFF_W1 = 2 * TR_TILE, TR_OFF_W2 = TR_OFF_W1 + 2 * TR_W1, TR_OFF_H = TR_OFF_W2 + 2 * TR_W2,
+                   TR_OFF_GB = TR_OFF_H + 2 * TR_H, TR_OFF_BAR = TR_OFF_GB + 1024, TR_SMEM = TR_OFF_BAR + 256 + 1024;
+constexpr int TR_THREADS = 18 * 32;
+static_assert(TR_SMEM <= 232448, "shared memory");
+
+struct TransitionArgs {
+  const float *gamma, *beta;
+  const bf16* x;
+  long long rows;
+  int items, pair, blocks;  // items of one tile (pair = 0) or two; hidden blocks of 64
+  int update_only;          // out = the update alone (x is not added)
+  int* status;
+};
+
+__global__ void __launch_bounds__(TR_THREADS, 1)
+transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmo,
+                  const __grid_constant__ CUtensorMap tmw1, const __grid_constant__ CUtensorMap tmw2, const TransitionArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  float* gb = reinterpret_cast<float*>(smem + TR_OFF_GB);  // gamma[128], beta[128]
+  uint64_t* x_full = reinterpret_cast<uint64_t*>(smem + TR_OFF_BAR);  // [tile] x has landed
+  uint64_t* n_full = x_full + 2;     // [tile] normalised in place
+  uint64_t* n_empty = n_full + 2;    // [tile] the item's last D1 product is complete
+  uint64_t* w1_full = n_empty + 2;   // [2]
+  uint64_t* w1_empty = w1_full + 2;  // [2] the block's D1 products are complete
+  uint64_t* w2_full = w1_empty + 2;  // [2]
+  uint64_t* w2_empty = w2_full + 2;  // [2] the block's D2 products are complete
+  uint64_t* d1_full = w2_empty + 2;  // [tile]
+  uint64_t* d1_empty = d1_full + 2;  // [tile] in registers
+  uint64_t* h_full = d1_empty + 2;   // [tile]
+  uint64_t* h_empty = h_full + 2;    // [tile] D2 has read h
+  uint64_t* d2_full = h_empty + 2;   // [tile]
+  uint64_t* d2_empty = d2_full + 2;  // [tile]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d2_empty + 2);
+  volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = int(__reduce_max_sync(0xffffffffu, threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const AbortCtx ab{cta_abort, p.status};
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&x_full[s], 1);
+      mbar_init(&n_full[s], 4);
+      mbar_init(&n_empty[s], 1);
+      mbar_init(&w1_full[s], 1);
+      mbar_init(&w1_empty[s], 1);
+      mbar_init(&w2_full[s], 1);
+      mbar_init(&w2_empty[s], 1);
+      mbar_init(&d1_full[s], 1);
+      mbar_init(&d1_empty[s], 4);
+      mbar_init(&h_full[s], 4);
+      mbar_init(&h_empty[s], 1);
+      mbar_init(&d2_full[s], 1);
+      mbar_init(&d2_empty[s], 4);
+    }
+    *cta_abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmx);
+    tma_prefetch_desc(&tmo);
+    tma_prefetch_desc(&tmw1);
+    tma_prefetch_desc(&tmw2);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (threadIdx.x >= 64 && threadIdx.x < 192) {
+    gb[threadIdx.x - 64] = p.gamma ? p.gamma[threadIdx.x - 64] : 1.f;
+    gb[threadIdx.x + 64] = p.beta ? p.beta[threadIdx.x - 64] : 0.f;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __reduce_max_sync(0xffffffffu, *tmem_slot);  // D1 of A, B; D2 of A, B: 128 columns each
+  const uint32_t base = smem_u32(smem);
+  const int NBK = p.blocks, NT = p.pair ? 2 : 1;
+  const int mine = (p.items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
+
+  if (warp == 0) {
+    pdl_wait();
+    pdl_launch();
+    if (lane == 0) {
+      const long long nblk = (long long)mine * NBK;
+      int hb1 = 0, hb2 = 0, t = blockIdx.x, xt = 0;
+      bool okay = true;
+      auto load_w1 = [&](long long i) {
+        const uint32_t st = uint32_t(i) & 1u;
+        if (!mbar_wait(&w1_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
+        mbar_arrive_expect_tx(&w1_full[st], TR_W1);
+        uint8_t* sw = smem + TR_OFF_W1 + st * TR_W1;
+        const int r0 = (hb1 >> 1) * 256 + (hb1 & 1) * 64;  // 64 SiLU units and their 64 linear partners
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh) {
+          tma_load_3d(sw + kh * 16384, &tmw1, &w1_full[st], kh * 64, r0, 0);
+          tma_load_3d(sw + kh * 16384 + 8192, &tmw1, &w1_full[st], kh * 64, r0 + 128, 0);
+        }
+        if (++hb1 == NBK) hb1 = 0;
+      };
+      auto load_w2 = [&](long long i) {
+        const uint32_t st = uint32_t(i) & 1u;
+        if (!mbar_wait(&w2_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
+        mbar_arrive_expect_tx(&w2_full[st], TR_W2);
+        tma_load_3d(smem + TR_OFF_W2 + st * TR_W2, &tmw2, &w2_full[st], hb2 * 64, 0, 0);
+        if (++hb2 == NBK) hb2 = 0;
+      };
+      load_w1(0);
+      // W2 runs one block behind W1, and the next item's x goes out with the item's last blocks: no load waits for a
+      // buffer that is freed later than the one after it needs
+      for (long long i = 0; i <= nblk && okay; ++i) {
+        if (xt < mine && (long long)xt * NBK <= i) {  // i == first block of item xt: its W1 is on its way
+          for (int s = 0; s < NT && okay; ++s) {
+            if (!mbar_wait(&n_empty[s], (uint32_t(xt) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
+            mbar_arrive_expect_tx(&x_full[s], TR_TILE);
+            uint8_t* sx = smem + TR_OFF_N + s * TR_TILE;
+            const int r = (t * NT + s) * 128;
+            tma_load_3d(sx, &tmx, &x_full[s], 0, r, 0);
+            tma_load_3d(sx + 16384, &tmx, &x_full[s], 64, r, 0);
+          }
+          t += gridDim.x;
+          ++xt;
+        }
+        if (okay && i > 0) load_w2(i - 1);
+        if (okay && i + 1 < nblk) load_w1(i + 1);
+      }
+    }
+  } else if (warp == 1) {
+    pdl_wait();
+    pdl_launch();
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc = make_idesc(128, 128);
+    uint32_t g1 = 0, g2 = 0;  // blocks whose D1 / D2 have been issued
+    auto d1 = [&](int hb, uint32_t item) -> bool {
+      const uint32_t b = g1 & 1u;
+      if (!mbar_wait_warp(&w1_full[b], (g1 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) return false;
+      const uint64_t wd = make_sdesc(base + TR_OFF_W1 + b * TR_W1, 16, 1024);
+      for (int s = 0; s < NT; ++s) {
+        if (hb == 0 && !mbar_wait_warp(&n_full[s], item & 1u, ab, XF_ERR_WAIT_FULL)) return false;
+        if (!mbar_wait_warp(&d1_empty[s], (g1 & 1u) ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) return false;
+        tc_fence_after();
+        const uint64_t nd = make_sdesc(base + TR_OFF_N + s * TR_TILE, 16, 1024);
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_ss_if(leader, tmem_base + s * 128, nd + uint64_t(kh * 1024 + 2 * j), wd + uint64_t(kh * 1024 + 2 * j), idesc,
+                       (kh | j) ? 1u : 0u);
+        umma_commit_if(leader, &d1_full[s]);
+        if (hb == NBK - 1) umma_commit_if(leader, &n_empty[s]);
+      }
+      umma_commit_if(leader, &w1_empty[b]);
+      ++g1;
+      return true;
+    };
+    bool okay = mine > 0 ? d1(0, 0) : true;
+    for (int it = 0; it < mine && okay; ++it) {
+      for (int hb = 0; hb < NBK && okay; ++hb) {
+        // the next block's D1 first; at the item's end D2 (the next item's rows are still on their way)
+        if (hb + 1 < NBK && !d1(hb + 1, it)) { okay = false; break; }
+        const uint32_t b = g2 & 1u;
+        if (!mbar_wait_warp(&w2_full[b], (g2 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
+        const uint64_t wd = make_sdesc(base + TR_OFF_W2 + b * TR_W2, 16, 1024);
+        for (int s = 0; s < NT && okay; ++s) {
+          if (hb == 0 && !mbar_wait_warp(&d2_empty[s], (uint32_t(it) & 1u) ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) { okay = false; break; }
+          if (!mbar_wait_warp(&h_full[s], g2 & 1u, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
+          tc_fence_after();
+          const uint64_t hd = make_sdesc(base + TR_OFF_H + s * TR_H, 16, 1024);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_ss_if(leader, tmem_base + 256 + s * 128, hd + uint64_t(2 * j), wd + uint64_t(2 * j), idesc, (hb | j) ? 1u : 0u);
+          umma_commit_if(leader, hb == NBK - 1 ? &d2_full[s] : &h_empty[s]);  // after the last block D2's reader reuses h
+        }
+        umma_commit_if(leader, &w2_empty[b]);
+        ++g2;
+      }
+      if (okay && it + 1 < mine) okay = d1(0, it + 1);
+    }
+  } else if (warp < 10) {
+    pdl_wait();
+    pdl_launch();
+    const int s = (warp - 2) >> 2, row = ((warp - 2) & 3) * 32 + lane;
+    for (int it = 0; it < mine && s < NT; ++it) {
+      if (!mbar_wait(&x_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL)) break;
+      ln_row_in_place(smem + TR_OFF_N + s * TR_TILE, row, gb);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&n_full[s]);
+    }
+  } else {
+    pdl_wait();
+    pdl_launch();
+    const int s = (warp - 10) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t rsw = uint32_t(row & 7), laddr = tmem_base + s * 128 + (uint32_t(quarter * 32) << 16);
+    uint8_t* sh = smem + TR_OFF_H + s * TR_H + row * 128;
+    uint32_t g = 0, gh = 0;  // blocks; h buffers handed to D2 with a notice (all but an item's last)
+    int t = blockIdx.x;
+    for (int it = 0; it < mine && s < NT; ++it, t += gridDim.x) {
+      for (int hb = 0; hb < NBK; ++hb, ++g) {
+        mbar_wait(&d1_full[s], g & 1u, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through: these warps meet at a barrier)
+        tc_fence_after();
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
+          uint32_t ra[32], rb[32];
+          tmem_ld32(laddr + c2 * 32, ra);
+          tmem_ld32(laddr + 64 + c2 * 32, rb);
+          tmem_ld_wait();
+          if (c2 == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&d1_empty[s]);
+          }
+          uint32_t o[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float a0 = __uint_as_float(ra[2 * e]), a1 = __uint_as_float(ra[2 * e + 1]);
+            o[e] = pack_bf16x2(a0 * sigmoidf_fast(a0) * __uint_as_float(rb[2 * e]), a1 * sigmoidf_fast(a1) * __uint_as_float(rb[2 * e + 1]));
+          }
+          if (c2 == 0 && hb > 0) {
+            mbar_wait(&h_empty[s], gh & 1u, ab, XF_ERR_WAIT_EMPTY);
+            ++gh;
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<uint4*>(sh + ((uint32_t(c2 * 4 + c) ^ rsw) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&h_full[s]);
+      }
+      // the tile's result: D2 + x, through the h buffer, 64 columns at a time
+      const long long tile_row = (long long)(t * NT + s) * 128;
+      const bool valid = tile_row + row < p.rows && !p.update_only;
+      const uint4* xg = reinterpret_cast<const uint4*>(p.x + (tile_row + row) * 128);
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+        uint4 xv[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) xv[q] = valid ? __ldcg(xg + hf * 8 + q) : make_uint4(0, 0, 0, 0);
+        if (hf == 0) {
+          mbar_wait(&d2_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
+          tc_fence_after();
+        } else {
+          if (quarter == 0 && lane == 0) tma_store_wait_read<0>();
+          named_bar_sync(1 + s, 128);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t r[32];
+          tmem_ld32(laddr + 256 + hf * 64 + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint4 u = xv[q];
+            const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              o[e] = pack_bf16x2(__uint_as_float(r[q * 8 + 2 * e]) + bf16_lo(w4[e]), __uint_as_float(r[q * 8 + 2 * e + 1]) + bf16_hi(w4[e]));
+            *reinterpret_cast<uint4*>(sh + ((uint32_t(c * 4 + q) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+            if (c == 0) xv[q] = valid ? __ldcg(xg + hf * 8 + 4 + q) : make_uint4(0, 0, 0, 0);
+          }
+        }
+        if (hf == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&d2_empty[s]);
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(1 + s, 128);
+        if (quarter == 0 && lane == 0 && tile_row < p.rows) {
+          tma_store_3d(&tmo, smem + TR_OFF_H + s * TR_H, hf * 64, (int)tile_row, 0);
+          tma_store_commit();
+        }
+      }
+      if (quarter == 0 && lane == 0) tma_store_wait_read<0>();
+      named_bar_sync(1 + s, 128);  // h is free for the next item
+    }
+    if (quarter == 0 && lane == 0) tma_store_wait_all();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*cta_abort && threadIdx.x == 0) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {}
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// x, out: [rows][128]; w1: [2F][128] in groups of [128 SiLU | 128 linear] rows, w2: [128][F]
+int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F, const float* gamma, const float* beta,
+                         const bf16* w1, const bf16* w2, int update_only, cudaStream_t st) {
+  CUtensorMap tmx, tmo, tmw1, tmw2;
+  if (!make_tmap_bf16_3d(&tmx, x, 128, rows, 1, 128, (uint64_t)128 * rows, 64, 128, 1) ||
+      !make_tmap_bf16_3d(&tmo, out, 128, rows, 1, 128, (uint64_t)128 * rows, 64, 128, 1) ||
+      !make_tmap_bf16_3d(&tmw1, w1, 128, 2 * F, 1, 128, (uint64_t)256 * F, 64, 64, 1) ||
+      !make_tmap_bf16_3d(&tmw2, w2, F, 128, 1, F, (uint64_t)128 * F, 64, 128, 1))
+    return fail(c, XFOLD_ERR_ARG, "transition: cannot encode tensor maps (16-byte aligned bases?)");
+  static bool attr_done[8] = {false};
+  if (!attr_done[c->device & 7]) {
+    cudaError_t e = cudaFuncSetAttribute(transition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM);
+    if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "transition smem attribute: %s", cudaGetErrorString(e));
+    attr_done[c->device & 7] = true;
+  }
+  const int sms = c->gemm_sms > 0 && c->gemm_sms < c->sm_count ? c->gemm_sms : c->sm_count;
+  const int tiles = (int)((rows + 127) / 128), pair = tiles > sms ? 1 : 0, items = pair ? (tiles + 1) / 2 : tiles;
+  TransitionArgs a{gamma, beta, x, rows, items, pair, F / 64, update_only, c->d_status};
+  ProfScope ps(c, XFOLD_K_LINEAR_SWIGLU, st);
+  launch_pdl(transition_kernel, items < sms ? items : sms, TR_THREADS, TR_SMEM, st, tmx, tmo, tmw1, tmw2, a);
+  return check_launch(c, "transition_kernel");
+}
+
+}  // namespace xf

@@ -348,6 +348,64 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 
+// true in exactly one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+// Pieces of a LayerNorm over rows of bf16.  Mixed-precision adds take the packed halves as they are: once for the sum, once
+// to centre.
+__device__ __forceinline__ void sum2(uint32_t x, float2& s) {
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;\n\t}"
+      : "+f"(s.x), "+f"(s.y) : "r"(x));
+}
+__device__ __forceinline__ float2 centre2(uint32_t x, float nmean) {
+  float2 v;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %3;\n\tadd.rn.f32.bf16 %1, h, %3;\n\t}"
+      : "=f"(v.x), "=f"(v.y) : "r"(x), "f"(nmean));
+  return v;
+}
+// Row `row` of a [2 halves][128 rows][64 columns] 128-byte-swizzled tile of 128 bf16 columns, by one thread: statistics, then
+// (x - mean) * rstd * gamma + beta in place; gb = gamma[128], beta[128].  Three passes over shared memory: holding the row
+// would take 64 registers.
+__device__ __forceinline__ void ln_row_in_place(uint8_t* tile, int row, const float* gb) {
+  const uint32_t rsw = uint32_t(row & 7);
+  auto piece = [&](int g) { return reinterpret_cast<uint4*>(tile + (g >> 3) * 16384 + row * 128 + ((uint32_t(g & 7) ^ rsw) << 4)); };
+  float2 sm = make_float2(0.f, 0.f), sq = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int g = 0; g < 16; ++g) {
+    const uint4 u = *piece(g);
+    sum2(u.x, sm); sum2(u.y, sm); sum2(u.z, sm); sum2(u.w, sm);
+  }
+  const float nmean = -(sm.x + sm.y) * (1.f / 128);
+#pragma unroll
+  for (int g = 0; g < 16; ++g) {
+    const uint4 u = *piece(g);
+    const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = centre2(w4[e], nmean);
+      sq = ffma2(v, v, sq);
+    }
+  }
+  const float rstd = rsqrtf((sq.x + sq.y) * (1.f / 128) + 1e-5f);
+  const float2 r2 = make_float2(rstd, rstd);
+#pragma unroll 4
+  for (int g = 0; g < 16; ++g) {
+    const uint4 u = *piece(g);
+    const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 ga = *reinterpret_cast<const float2*>(gb + g * 8 + 2 * e), be = *reinterpret_cast<const float2*>(gb + 128 + g * 8 + 2 * e);
+      const float2 v = ffma2(ffma2(centre2(w4[e], nmean), r2, make_float2(0.f, 0.f)), ga, be);
+      o[e] = pack_bf16x2(v.x, v.y);
+    }
+    *piece(g) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // Byte offset of element (row, col) inside a K-major / MN-major 128B-swizzled tile whose rows are
 // 64 bf16 wide: 16-byte chunk index is XORed with (row & 7).  The tile base must be 1024 B aligned.
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t col_elem) {

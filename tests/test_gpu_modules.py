@@ -288,3 +288,43 @@ def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
     out = out.float().cpu().reshape(B, S, H, w.Dp)[..., :d]
     # the prepared bias is fp16 times log2(e): an absolute error of up to 0.18 in a logit near 300 * log2(e)
     assert torch.isfinite(out).all() and relf(out, ref) < 0.15
+
+
+@pytest.mark.parametrize("B,S,C,H", [(4, 65, 384, 16), (3, 33, 384, 16), (1, 129, 384, 16), (2, 1100, 384, 16), (1, 64, 768, 16),
+                                     (3, 400, 768, 16)])
+def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
+    """Logits of several dozen that grow along the keys: the running reference exponent has to move (output and stored
+    probabilities rescaled) in every row, for slots over batch rows and over query tiles, at block edges and remainders."""
+    g = torch.Generator().manual_seed(900 + S)
+    st = oracle.make_self_attention_state(g, "", C, 0, False)
+    xn = torch.randn(B, S, C, generator=g).to(BF)
+    pb = torch.randn(H, S, S, generator=g) + 60.0 * (torch.arange(S) // 24)[None, None, :] / max(S // 24, 1)
+    pb[:, ::3] = pb[:, ::3].flip(-1)   # a third of the rows with the maximum first
+    mask = (torch.rand(S, generator=g) > 0.1).float()
+    r = rounded(st)
+    d = C // H
+    shp = (C, H, d)
+    ref = oracle.gated_attention(xn.float(), 1e9 * (mask[None, None, None, :] - 1), pb.half().float(),
+                                 r["q_projection.weight"].T.reshape(shp), r["k_projection.weight"].T.reshape(shp),
+                                 r["v_projection.weight"].T.reshape(shp), r["gating_query.weight"].T.reshape(shp), None,
+                                 query_b=st["q_projection.bias"].reshape(H, d))
+    w = ops.PackedSelfAttention(st, "", "cuda", H)
+    out = ops.attention_pair_bias_core(xn.cuda().contiguous(), w, pb.cuda().contiguous(), mask.cuda())
+    ops.synchronize_and_check()
+    out = out.float().cpu().reshape(B, S, H, w.Dp)[..., :d]
+    # the prepared bias is fp16 times log2(e): an absolute error of up to 0.03 in a logit near 60 * log2(e)
+    assert torch.isfinite(out).all() and relf(out, ref) < 4e-2
+
+
+@pytest.mark.parametrize("rows", [1, 127, 129, 148 * 128, 148 * 128 + 1, 297 * 128 + 5])
+def test_transition_tile_pairs(ops, oracle, rows):
+    """Around the tile, the switch from one to two tiles per CTA, and an odd number of tiles."""
+    g = torch.Generator().manual_seed(rows)
+    st = with_affine_norms(oracle.make_transition_state(g, "", 128), rows + 1)
+    x = (1.5 * torch.randn(rows, 128, generator=g) - 0.5).to(BF)
+    ref = x.float() + oracle.transition(rounded(st), "", x.float())
+    w = ops.PackedTransition(st, "", "cuda")
+    xd = x.cuda().contiguous()
+    ops.transition_(xd, w)
+    ops.synchronize_and_check()
+    check_update(x, xd, ref)
