@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -35,6 +36,11 @@ struct Ctx {
   int gemm_sms = 0;      // SMs a GEMM launch may take (0: all)
   int peer_cta_cap = 0;  // CTAs of a peer exchange kernel (0: its own default)
   std::vector<ProfRec> prof_recs, prof_pool;
+  // Second stream of the one-GPU trunk: the single representation's kernels of a block run beside the next block's.  One
+  // call at a time uses it (side_mu is held while the call issues its work; events are captured by the waits as they are issued).
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  std::mutex side_mu;
 };
 
 // Brackets one kernel launch with events on its stream while profiling is enabled, and counts it.

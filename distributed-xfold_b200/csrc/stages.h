@@ -75,12 +75,12 @@ int triattn_bias(Ctx* c, const bf16* z, int R, int N, const xfold_triattn_weight
                  long long plane, int rows_are_keys, cudaStream_t st);
 int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask, long long mask_ld, int R, int N,
                  int transposed, const xfold_triattn_weights* w, bf16* qkvg, bf16* mext, bf16* z, cudaStream_t st,
-                 bf16* upd = nullptr, const ChunkHook* hook = nullptr);
+                 bf16* upd = nullptr, const ChunkHook* hook = nullptr, bool mext_ready = false);
 int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_transition_weights* w, void* ws,
                    size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr, const ChunkHook* hook = nullptr);
 size_t single_ws_bytes(int N);
 int single_update(Ctx* c, bf16* s, const bf16* plT, int ldq, const float* seq_mask, int N,
-                  const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, cudaStream_t st);
+                  const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, cudaStream_t st, const bf16* mext = nullptr);
 
 // ---- peer-memory exchange launchers (peer.cu); pointer arrays are host arrays of `world` peer-mapped addresses ----
 int launch_transpose_scatter(Ctx* c, const bf16* z, int R, int N, int row0, void* const* dst, const int* col_starts,
