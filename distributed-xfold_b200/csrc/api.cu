@@ -190,41 +190,11 @@ static int batched_contract(Ctx* c, const bf16* a_, const bf16* b_, bf16* out, i
 // a / b are stored "row-interleaved channel-major": element (row i, channel c, k) at (i * 128 + c) * ld + k.
 // A rank's rows are one contiguous block, so the all-gather of b over the row-shard group is a plain
 // concatenation, and the per-channel operand of the contraction is a strided 2-D slice for TMA.
-int trimul_project(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed_store,
-                          const xfold_trimul_weights* w, bf16* x, bf16* a_out, bf16* b_out, bf16* g, long long chan_stride,
-                          long long row_stride, cudaStream_t st) {
-  const long long M = (long long)R * N;
-  int rc = launch_ln_rows(c, z, 128, x, 128, M, 128, w->ln_in_gamma, w->ln_in_beta, 1e-5f, 0, nullptr, nullptr, 0,
-                          nullptr, nullptr, 0, st);
-  if (rc) return rc;
-  CUtensorMap tA, tB;
-  bool ok;
-  GemmArgs a;
-  if (!transposed_store) {
-    ok = make_tmap_bf16_3d(&tA, x, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1);
-    a.a_row_mode = 0;
-    a.tiles_m = (int)((M + 127) / 128);
-  } else {  // tile rows step along the first token axis, second axis fixed: a[j][c][i] (needs R == N)
-    ok = make_tmap_bf16_3d(&tA, x, 128, N, R, 128, (uint64_t)128 * N, 64, 1, 128);
-    a.a_row_mode = 1;
-    a.a_dim1 = N;
-    a.tiles_m = N * ((R + 127) / 128);
-  }
-  ok = ok && make_tmap_bf16_3d(&tB, w->w_in, 128, 640, 1, 128, 128 * 640, 64, 256, 1);
-  if (!ok) return fail(c, XFOLD_ERR_ARG, "trimul: cannot encode projection tensor maps");
-  a.M = (int)M;
-  a.N = 640;
-  a.K = 128;
-  a.tiles_n = 3;
-  a.out_a = a_out;
-  a.out_b = b_out;
-  a.out_g = g;
-  a.cm_chan_stride = chan_stride;
-  a.cm_ld = row_stride;
-  a.ntok = N;
-  a.mask = mask;
-  a.status = c->d_status;
-  return launch_gemm(c, EPI_TRIMUL_AB, 256, tA, tB, a, st);
+int trimul_project(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed_store, const xfold_trimul_weights* w,
+                   bf16* a_out, bf16* b_out, bf16* g, long long chan_stride, long long row_stride, cudaStream_t st) {
+  if (R <= 0 || N <= 0) return XFOLD_OK;
+  return launch_row_project_trimul(c, z, mask, R, N, transposed_store, w->ln_in_gamma, w->ln_in_beta, (const bf16*)w->w_in, a_out,
+                                   b_out, g, chan_stride, row_stride, st);
 }
 
 // o[i][c][j] = sum_k a[i][c][k] * b[j][c][k]   (a: Ri rows, b: Nj rows, both [.][128][ld]; o: [Ri][128][ldo])
@@ -311,7 +281,6 @@ static TriMulWs carve_trimul(void* ws, size_t cap, int N) {
 
 static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, const xfold_trimul_weights* w, void* ws,
                       size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr) {
-  StaticWeights sw(c);
   if (!z || !w || !w->w_in || !w->w_out) return fail(c, XFOLD_ERR_ARG, "trimul: null argument");
   if (N <= 0) return XFOLD_OK;
   TriMulWs W = carve_trimul(ws, ws_bytes, N);
@@ -319,8 +288,9 @@ static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, c
   // incoming: a and b are stored transposed, so that o[i][c][j] = sum_k bT[i][c][k] aT[j][c][k] is the same product
   // one GPU: plain channel-major planes [128][N][ld] (rows of a tile are 2 KB apart, best DRAM locality)
   const long long cs = (long long)N * W.ld, rs = W.ld;
-  int rc = trimul_project(c, z, mask, N, N, outgoing ? 0 : 1, w, W.x, W.a, W.b, W.g, cs, rs, st);
+  int rc = trimul_project(c, z, mask, N, N, outgoing ? 0 : 1, w, W.a, W.b, W.g, cs, rs, st);
   if (rc) return rc;
+  StaticWeights sw(c);
   rc = trimul_contract(c, outgoing ? W.a : W.b, cs, rs, outgoing ? W.b : W.a, cs, rs, N, N, N, W.o, cs, rs, st);
   if (rc) return rc;
   return trimul_output(c, W.o, cs, rs, W.g, N, N, w, W.x, z, st, upd);
@@ -358,35 +328,42 @@ int triattn_bias(Ctx* c, const bf16* z, int R, int N, const xfold_triattn_weight
 
 // z (+)= out_proj(gated attention(x)) for R batch rows (sequence length N); biasT: bf16 [4][N][ldq], [h][query][key].
 // transposed: the R x N token grid is stored [N][R] (sequence index outermost), used by the single-GPU ending node.
+// mext: mask-bias tiles of the R rows; x receives the attention's output.
+static int triattn_attend(Ctx* c, bf16* x, const bf16* biasT, int ldq, int R, int N, int transposed, const xfold_triattn_weights* w,
+                          const bf16* qkvg, const bf16* mext, bf16* z, cudaStream_t st, bf16* upd, const ChunkHook* hook) {
+  const long long seq_stride = transposed ? (long long)R * 128 : 128;
+  const long long batch_stride = transposed ? 128 : (long long)N * 128;
+  const int rc = launch_attention2(c, qkvg, 512, N, R, transposed, 0, 128, 256, 384, 4, biasT, ldq, mext, R, x, seq_stride,
+                                   batch_stride, st);
+  if (rc) return rc;
+  return linear_gate_resid_chunked(c, x, 128, (long long)R * N, 128, (const bf16*)w->w_out, 128, upd ? nullptr : z, 128,
+                                   upd ? upd : z, 128, st, hook);
+}
 int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask, long long mask_ld, int R, int N,
                         int transposed, const xfold_triattn_weights* w, bf16* qkvg, bf16* mext, bf16* z, cudaStream_t st,
-                        bf16* upd, const ChunkHook* hook, bool mext_ready) {
+                        bf16* upd, const ChunkHook* hook) {
   const long long M = (long long)R * N;
   // the v columns are stored as fp16: the attention kernel's P V product runs with fp16 operands
   int rc = linear_plain(c, x, 128, M, 128, (const bf16*)w->w_qkvg, 512, nullptr, w->qkvg_scale, qkvg, 512, st, 256, 384, 128);
   if (rc) return rc;
-  if (!mext_ready && (rc = launch_mext(c, mask, mask_ld, mext, R, N, st))) return rc;
-  const long long seq_stride = transposed ? (long long)R * 128 : 128;
-  const long long batch_stride = transposed ? 128 : (long long)N * 128;
-  rc = launch_attention2(c, qkvg, 512, N, R, transposed, 0, 128, 256, 384, 4, biasT, ldq, mext, R, x, seq_stride,
-                         batch_stride, st);
-  if (rc) return rc;
-  return linear_gate_resid_chunked(c, x, 128, M, 128, (const bf16*)w->w_out, 128, upd ? nullptr : z, 128, upd ? upd : z, 128,
-                                   st, hook);
+  if ((rc = launch_mext(c, mask, mask_ld, mext, R, N, st))) return rc;
+  return triattn_attend(c, x, biasT, ldq, R, N, transposed, w, qkvg, mext, z, st, upd, hook);
 }
 
 // mext: mask-bias tiles made beforehand (launch_mext over the N mask rows), or null
 static int triattn_fwd(Ctx* c, bf16* z, const float* mask, int N, int transpose, const xfold_triattn_weights* w, void* ws,
                        size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr, bf16* mext = nullptr) {
-  StaticWeights sw(c);
   if (!z || !w || !w->w_qkvg || !w->w_out || !w->w_bias) return fail(c, XFOLD_ERR_ARG, "triattn: null argument");
   if (N <= 0) return XFOLD_OK;
   TriAttnWs W = carve_triattn(ws, ws_bytes, N, N);
   if (!ws || W.bytes > ws_bytes) return fail(c, XFOLD_ERR_ARG, "triattn: workspace too small (%zu < %zu)", ws_bytes, W.bytes);
   // both nodes use bias(q, k) = projection of token (q, k), not transposed for the ending node
-  int rc = triattn_bias(c, z, N, N, w, W.x, W.nbT, W.ldq, (long long)N * W.ldq, 0, st);
+  int rc = launch_row_project_attn(c, z, N, N, w->ln_gamma, w->ln_beta, (const bf16*)w->w_qkvg, w->qkvg_scale, w->w_bias, W.qkvg,
+                                   W.nbT, W.ldq, (long long)N * W.ldq, st);
   if (rc) return rc;
-  return triattn_core(c, W.x, W.nbT, W.ldq, mask, N, N, N, transpose, w, W.qkvg, mext ? mext : W.mext, z, st, upd, nullptr, mext != nullptr);
+  StaticWeights sw(c);
+  if (!mext && (rc = launch_mext(c, mask, N, mext = W.mext, N, N, st))) return rc;
+  return triattn_attend(c, W.x, W.nbT, W.ldq, N, N, transpose, w, W.qkvg, mext, z, st, upd, nullptr);
 }
 
 int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_transition_weights* w, void* ws,
@@ -400,7 +377,7 @@ int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_tr
   // rows) only for a single chunk.
   if (C == 128 && F % 128 == 0 && (!hook || !hook->after || hook->parts <= 1)) {
     const int rc = launch_transition128(c, x, upd ? upd : x, rows, F, w->ln_gamma, w->ln_beta, (const bf16*)w->w1_packed,
-                                        (const bf16*)w->w2, upd != nullptr, st);
+                                        (const bf16*)w->w2, sw.before, upd != nullptr, st);
     return rc || !hook || !hook->after ? rc : hook->after(0, rows);
   }
   Carver cv(ws, ws_bytes);
@@ -788,7 +765,7 @@ int xfold_trimul_project_fwd(xfold_ctx* c, const void* z, const float* mask, int
                              void* x_scratch, void* a, void* b, void* g, int ld, void* stream) {
   if (!c || !z || !w || !x_scratch || !a || !b || !g) return XFOLD_ERR_ARG;
   if (ld < N || (ld & 7)) return fail(c, XFOLD_ERR_ARG, "trimul project: ld must be >= N and a multiple of 8");
-  return trimul_project(c, (const bf16*)z, mask, R, N, 0, w, (bf16*)x_scratch, (bf16*)a, (bf16*)b, (bf16*)g, ld,
+  return trimul_project(c, (const bf16*)z, mask, R, N, 0, w, (bf16*)a, (bf16*)b, (bf16*)g, ld,
                         (long long)128 * ld, (cudaStream_t)stream);
 }
 int xfold_trimul_contract_fwd(xfold_ctx* c, const void* a, const void* b_full, int R, int Nj, int K, int ld, void* o, int ldo,

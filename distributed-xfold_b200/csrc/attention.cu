@@ -102,14 +102,6 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   return make_float2(__uint_as_float(__float_as_uint(q.x) + (__float_as_uint(t.x) << 23)),
                      __uint_as_float(__float_as_uint(q.y) + (__float_as_uint(t.y) << 23)));
 }
-__device__ __forceinline__ void tmem_ld16_(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st16_(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -393,7 +385,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
                     uint32_t o[16];
 #pragma unroll 1
                     for (int oc = 0; oc < D; oc += 16) {
-                      tmem_ld16_(o_addr + oc, o);
+                      tmem_ld16(o_addr + oc, o);
                       tmem_ld_wait();
 #pragma unroll
                       for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
@@ -404,7 +396,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
                     const __half2 a2 = __float2half2_rn(alpha);
                     uint32_t q[16];
                     tmem_st_wait_();
-                    tmem_ld16_(buf, q);
+                    tmem_ld16(buf, q);
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {

@@ -7,9 +7,9 @@
 //                 the other buffer.  Row-major outputs leave through 128-byte-swizzled staging tiles
 //                 and TMA stores; residual and gate tiles of the 128-wide configuration come in by TMA.
 //
-// Every projection of the Pairformer block, the SwiGLU transition and the per-channel N x N x N
-// TriangleMultiplication contraction (batched over the 128 channels) run through this kernel; they
-// differ only in the tensor maps and in the epilogue that is fused behind the accumulator.
+// The output projections, the single representation's and the diffusion transformer's projections and the per-channel
+// N x N x N TriangleMultiplication contraction (batched over the 128 channels) run through this kernel; they differ only in
+// the tensor maps and in the epilogue that is fused behind the accumulator.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -42,19 +42,6 @@ struct GemmCfg {
   static constexpr uint32_t SMEM_BYTES = OFF_BAR + 256 /*barriers*/ + 1024 /*align slack*/;
 };
 
-__device__ __forceinline__ void store8_bf16(bf16* dst, const float* v, int nvalid, bool vec_ok) {
-  if (nvalid >= 8 && vec_ok) {
-    uint4 u;
-    u.x = pack_bf16x2(v[0], v[1]);
-    u.y = pack_bf16x2(v[2], v[3]);
-    u.z = pack_bf16x2(v[4], v[5]);
-    u.w = pack_bf16x2(v[6], v[7]);
-    *reinterpret_cast<uint4*>(dst) = u;
-  } else {
-    for (int e = 0; e < 8; ++e)
-      if (e < nvalid) dst[e] = __float2bfloat16(v[e]);
-  }
-}
 __device__ __forceinline__ void load8_bf16(const bf16* src, float* v, int nvalid, bool vec_ok) {
   if (nvalid >= 8 && vec_ok) {
     const uint4 u = *reinterpret_cast<const uint4*>(src);
@@ -149,9 +136,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int tn = int(t % p.tiles_n);
         const int tm = int((t / p.tiles_n) % p.tiles_m);
         const int b = int(t / ((long long)p.tiles_n * p.tiles_m));
-        int a1, a2;
-        if (p.a_row_mode == 0) { a1 = tm * BM; a2 = b; }
-        else { a1 = tm % p.a_dim1; a2 = (tm / p.a_dim1) * BM; }
+        const int a1 = tm * BM, a2 = b;
         const int bb = p.b_batched ? b : 0;
         if constexpr (EPI_LOADS) {
           const uint32_t nload = (p.resid ? 1u : 0u) + (p.gate ? 1u : 0u);
@@ -237,25 +222,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int tm = int((t / p.tiles_n) % p.tiles_m);
       const int b = int(t / ((long long)p.tiles_n * p.tiles_m));
       const uint32_t buf = it & 1u, aphase = (it >> 1) & 1u;
-      // TRIMUL_AB: where this thread's token goes, and its mask value, fetched BEFORE the wait for the accumulator so
-      // that the load's latency hides behind the product instead of heading every tile's epilogue
-      long long tok = 0, cm_off = 0;
-      bool rvalid = false;
-      float mk = 1.f;
-      if constexpr (EPI == EPI_TRIMUL_AB) {
-        if (p.a_row_mode == 0) {
-          tok = (long long)tm * BM + row;
-          rvalid = tok < p.M;
-          const long long i = tok / p.ntok, j = tok - i * p.ntok;
-          cm_off = i * p.cm_ld + j;
-        } else {
-          const long long jf = tm % p.a_dim1, i = (long long)(tm / p.a_dim1) * BM + row;
-          rvalid = i * p.ntok < p.M;  // M = rows * ntok
-          tok = i * p.ntok + jf;
-          cm_off = jf * p.cm_ld + i;
-        }
-        if (tn < 2 && rvalid && p.mask) mk = p.mask[tok];
-      }
       // GATE_RESID with a gate row per (row % mod): the first chunk's gate values, fetched before the wait as well
       const bool row_gate_vec = EPI == EPI_GATE_RESID && p.row_gate && (p.ldg & 7) == 0 && (p.N & 31) == 0;
       uint4 rg[4];
@@ -274,212 +240,174 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(q * 32) << 16);
 
-      if constexpr (EPI != EPI_TRIMUL_AB) {
-        // Staged epilogue: the tile leaves in 64-column chunks.  Each of the 8 warps converts its 32 rows x 32
-        // columns of the chunk into a 128-byte-swizzled shared-memory tile (conflict-free 16-byte stores), then
-        // one thread hands the tile to TMA.  Residual / gate chunks arrive the same way in the other direction.
-        constexpr int NCH = (EPI == EPI_SWIGLU) ? BN / 128 : BN / 64;  // output chunks per tile
-        constexpr int WOUT = (EPI == EPI_SWIGLU) ? BN / 2 : BN;        // output columns per tile
-        const int n_out = (EPI == EPI_SWIGLU) ? p.N / 2 : p.N;
-        const long long m = (long long)tm * BM + row;
-        const uint32_t rsw = uint32_t(row & 7);
-        const bool elected = (warp == 2 && lane == 0);
-        // Chunks beyond the output's last column are left out.  (They must not pass through the staging buffers without a
-        // store of their own either: the wait below counts committed stores, and a chunk that commits none would let the
-        // one after it overwrite a tile that is still being read.)
-        const int nch = min(NCH, (n_out - tn * WOUT + 63) / 64);
+      // Staged epilogue: the tile leaves in 64-column chunks.  Each of the 8 warps converts its 32 rows x 32
+      // columns of the chunk into a 128-byte-swizzled shared-memory tile (conflict-free 16-byte stores), then
+      // one thread hands the tile to TMA.  Residual / gate chunks arrive the same way in the other direction.
+      constexpr int NCH = (EPI == EPI_SWIGLU) ? BN / 128 : BN / 64;  // output chunks per tile
+      constexpr int WOUT = (EPI == EPI_SWIGLU) ? BN / 2 : BN;        // output columns per tile
+      const int n_out = (EPI == EPI_SWIGLU) ? p.N / 2 : p.N;
+      const long long m = (long long)tm * BM + row;
+      const uint32_t rsw = uint32_t(row & 7);
+      const bool elected = (warp == 2 && lane == 0);
+      // Chunks beyond the output's last column are left out.  (They must not pass through the staging buffers without a
+      // store of their own either: the wait below counts committed stores, and a chunk that commits none would let the
+      // one after it overwrite a tile that is still being read.)
+      const int nch = min(NCH, (n_out - tn * WOUT + 63) / 64);
 #pragma unroll 1
-        for (int c = 0; c < nch; ++c, ++ochunk) {
-          const int col0 = tn * WOUT + c * 64;          // first output column of the chunk
-          const int colw = col0 + ch * 32;              // first output column of this warp
-          uint8_t* so = smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE + row * 128;
-          float v[32];
-          if constexpr (EPI == EPI_SWIGLU) {
-            uint32_t ra[32], rb[32];
-            tmem_ld32(taddr + c * 64 + ch * 32, ra);
-            tmem_ld32(taddr + BN / 2 + c * 64 + ch * 32, rb);
-            tmem_ld_wait();
+      for (int c = 0; c < nch; ++c, ++ochunk) {
+        const int col0 = tn * WOUT + c * 64;          // first output column of the chunk
+        const int colw = col0 + ch * 32;              // first output column of this warp
+        uint8_t* so = smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE + row * 128;
+        float v[32];
+        if constexpr (EPI == EPI_SWIGLU) {
+          uint32_t ra[32], rb[32];
+          tmem_ld32(taddr + c * 64 + ch * 32, ra);
+          tmem_ld32(taddr + BN / 2 + c * 64 + ch * 32, rb);
+          tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              const float x = __uint_as_float(ra[e]);
-              v[e] = x * sigmoidf_fast(x) * __uint_as_float(rb[e]);
-            }
-          } else {
-            uint32_t r[32];
-            tmem_ld32(taddr + c * 64 + ch * 32, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+          for (int e = 0; e < 32; ++e) {
+            const float x = __uint_as_float(ra[e]);
+            v[e] = x * sigmoidf_fast(x) * __uint_as_float(rb[e]);
           }
-          if constexpr (EPI == EPI_PLAIN) {
-            if (p.col_bias) {
+        } else {
+          uint32_t r[32];
+          tmem_ld32(taddr + c * 64 + ch * 32, r);
+          tmem_ld_wait();
 #pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] += (colw + e < n_out) ? p.col_bias[colw + e] : 0.f;
-            }
-            if (p.col_scale) {
+          for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+        }
+        if constexpr (EPI == EPI_PLAIN) {
+          if (p.col_bias) {
 #pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
+            for (int e = 0; e < 32; ++e) v[e] += (colw + e < n_out) ? p.col_bias[colw + e] : 0.f;
+          }
+          if (p.col_scale) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
+          }
+        }
+        if constexpr (EPI == EPI_PLAIN) {
+          if (colw < p.log2e_cols) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] *= 1.4426950408889634f;
+          }
+        }
+        if constexpr (EPI == EPI_GATE_RESID) {
+          // order: v * sigmoid(gate) first, residual added last
+          const bool rvalid = m < p.M;
+          bool staged = false;
+          uint32_t eb = 0;
+          if constexpr (EPI_LOADS) {
+            if (p.resid || p.gate) {
+              staged = true;
+              eb = echunk & 1u;
+              if (!mbar_wait(&efull[eb], (echunk >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) dead = true;
+              ++echunk;
             }
           }
-          if constexpr (EPI == EPI_PLAIN) {
-            if (colw < p.log2e_cols) {
-#pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] *= 1.4426950408889634f;
-            }
-          }
-          if constexpr (EPI == EPI_GATE_RESID) {
-            // order: v * sigmoid(gate) first, residual added last
-            const bool rvalid = m < p.M;
-            bool staged = false;
-            uint32_t eb = 0;
-            if constexpr (EPI_LOADS) {
-              if (p.resid || p.gate) {
-                staged = true;
-                eb = echunk & 1u;
-                if (!mbar_wait(&efull[eb], (echunk >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) dead = true;
-                ++echunk;
-              }
-            }
-            if (p.gate) {
-              if (staged) {
-                const uint8_t* sg = smem + Cfg::OFF_GATE + eb * EPI_TILE + row * 128;
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const uint4 u = *reinterpret_cast<const uint4*>(sg + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
-                  const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
-                    v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
-                  }
-                }
-              } else {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
-                  if (nvalid <= 0) continue;
-                  float t8[8];
-                  load8_bf16(p.gate + m * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) v[g * 8 + e] *= sigmoidf_fast(t8[e]);
-                }
-              }
-            }
-            if (row_gate_vec) {
+          if (p.gate) {
+            if (staged) {
+              const uint8_t* sg = smem + Cfg::OFF_GATE + eb * EPI_TILE + row * 128;
 #pragma unroll
               for (int g = 0; g < 4; ++g) {
-                const uint32_t w4[4] = {rg[g].x, rg[g].y, rg[g].z, rg[g].w};
+                const uint4 u = *reinterpret_cast<const uint4*>(sg + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
+                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
                   v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
                 }
               }
-              if (c + 1 < nch) fetch_row_gate(c + 1);
-            } else if (p.row_gate) {  // gate shared by rows with equal (row % mod): AdaLN-Zero conditioning of several samples
+            } else {
 #pragma unroll
               for (int g = 0; g < 4; ++g) {
                 const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
                 if (nvalid <= 0) continue;
                 float t8[8];
-                load8_bf16(p.row_gate + (m % p.row_gate_mod) * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
+                load8_bf16(p.gate + m * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[g * 8 + e] *= sigmoidf_fast(t8[e]);
               }
             }
-            if (p.resid) {
-              if (staged) {
-                const uint8_t* sr = smem + Cfg::OFF_RES + eb * EPI_TILE + row * 128;
+          }
+          if (row_gate_vec) {
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const uint4 u = *reinterpret_cast<const uint4*>(sr + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
-                  const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+            for (int g = 0; g < 4; ++g) {
+              const uint32_t w4[4] = {rg[g].x, rg[g].y, rg[g].z, rg[g].w};
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    v[g * 8 + 2 * e] += bf16_lo(w4[e]);
-                    v[g * 8 + 2 * e + 1] += bf16_hi(w4[e]);
-                  }
-                }
-              } else {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                  const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
-                  if (nvalid <= 0) continue;
-                  float t8[8];
-                  load8_bf16(p.resid + m * p.ldr + col, t8, nvalid, (p.ldr & 7) == 0);
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) v[g * 8 + e] += t8[e];
-                }
+              for (int e = 0; e < 4; ++e) {
+                v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
+                v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
               }
             }
-            if (staged) {
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&eempty[eb]);
-            }
-          }
-          // the TMA store that last used this staging buffer (two chunks ago) must have read it out
-          if (elected) tma_store_wait_read<1>();
-          named_bar_sync(1, 256);
-          bool as_f16 = false;
-          if constexpr (EPI == EPI_PLAIN) as_f16 = colw >= p.f16_col0 && colw < p.f16_col1;
+            if (c + 1 < nch) fetch_row_gate(c + 1);
+          } else if (p.row_gate) {  // gate shared by rows with equal (row % mod): AdaLN-Zero conditioning of several samples
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 u;
-            if (as_f16) {
-              u.x = pack_f16x2(v[g * 8 + 0], v[g * 8 + 1]);
-              u.y = pack_f16x2(v[g * 8 + 2], v[g * 8 + 3]);
-              u.z = pack_f16x2(v[g * 8 + 4], v[g * 8 + 5]);
-              u.w = pack_f16x2(v[g * 8 + 6], v[g * 8 + 7]);
-            } else {
-              u.x = pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]);
-              u.y = pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]);
-              u.z = pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]);
-              u.w = pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]);
+            for (int g = 0; g < 4; ++g) {
+              const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
+              if (nvalid <= 0) continue;
+              float t8[8];
+              load8_bf16(p.row_gate + (m % p.row_gate_mod) * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[g * 8 + e] *= sigmoidf_fast(t8[e]);
             }
-            *reinterpret_cast<uint4*>(so + ((uint32_t(ch * 4 + g) ^ rsw) << 4)) = u;
           }
-          fence_proxy_async_smem();
-          named_bar_sync(2, 256);
-          if (elected) {
-            tma_store_3d(&tmO, smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE, col0, tm * BM, b);
-            tma_store_commit();
+          if (p.resid) {
+            if (staged) {
+              const uint8_t* sr = smem + Cfg::OFF_RES + eb * EPI_TILE + row * 128;
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const uint4 u = *reinterpret_cast<const uint4*>(sr + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
+                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  v[g * 8 + 2 * e] += bf16_lo(w4[e]);
+                  v[g * 8 + 2 * e + 1] += bf16_hi(w4[e]);
+                }
+              }
+            } else {
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
+                if (nvalid <= 0) continue;
+                float t8[8];
+                load8_bf16(p.resid + m * p.ldr + col, t8, nvalid, (p.ldr & 7) == 0);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[g * 8 + e] += t8[e];
+              }
+            }
+          }
+          if (staged) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&eempty[eb]);
           }
         }
-      } else {  // EPI_TRIMUL_AB
-        // tile_n 0: [projection | gate] rows of a; 1: the same for b; 2: gating_linear (first 128 columns)
-        if (tn < 2) {
-          bf16* dst = (tn == 0 ? p.out_a : p.out_b) + cm_off;
-#pragma unroll 1
-          for (int cc = ch * 2; cc < ch * 2 + 2; ++cc) {
-            uint32_t rp[32], rg[32];
-            tmem_ld32(taddr + cc * 32, rp);
-            tmem_ld32(taddr + 128 + cc * 32, rg);
-            tmem_ld_wait();
-            if (rvalid) {
+        // the TMA store that last used this staging buffer (two chunks ago) must have read it out
+        if (elected) tma_store_wait_read<1>();
+        named_bar_sync(1, 256);
+        bool as_f16 = false;
+        if constexpr (EPI == EPI_PLAIN) as_f16 = colw >= p.f16_col0 && colw < p.f16_col1;
 #pragma unroll
-              for (int e = 0; e < 32; ++e) {
-                const float v = __uint_as_float(rp[e]) * mk * sigmoidf_fast(__uint_as_float(rg[e]));
-                dst[(long long)(cc * 32 + e) * p.cm_chan_stride] = __float2bfloat16(v);
-              }
-            }
+        for (int g = 0; g < 4; ++g) {
+          uint4 u;
+          if (as_f16) {
+            u.x = pack_f16x2(v[g * 8 + 0], v[g * 8 + 1]);
+            u.y = pack_f16x2(v[g * 8 + 2], v[g * 8 + 3]);
+            u.z = pack_f16x2(v[g * 8 + 4], v[g * 8 + 5]);
+            u.w = pack_f16x2(v[g * 8 + 6], v[g * 8 + 7]);
+          } else {
+            u.x = pack_bf16x2(v[g * 8 + 0], v[g * 8 + 1]);
+            u.y = pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]);
+            u.z = pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]);
+            u.w = pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]);
           }
-        } else {
-          bf16* orow = p.out_g + tok * 128;
-#pragma unroll 1
-          for (int cc = ch * 2; cc < ch * 2 + 2; ++cc) {
-            uint32_t r[32];
-            tmem_ld32(taddr + cc * 32, r);
-            tmem_ld_wait();
-            if (rvalid) {
-#pragma unroll
-              for (int g8 = 0; g8 < 4; ++g8) {
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[g8 * 8 + e]);
-                store8_bf16(orow + cc * 32 + g8 * 8, v, 8, true);
-              }
-            }
-          }
+          *reinterpret_cast<uint4*>(so + ((uint32_t(ch * 4 + g) ^ rsw) << 4)) = u;
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(2, 256);
+        if (elected) {
+          tma_store_3d(&tmO, smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE, col0, tm * BM, b);
+          tma_store_commit();
         }
       }
       tc_fence_before();
@@ -516,22 +444,19 @@ static int launch_one(Ctx* c, const CUtensorMap& tmA, const CUtensorMap& tmB, co
   const long long total = (long long)a.batches * a.tiles_m * a.tiles_n;
   if (total <= 0) return XFOLD_OK;
   CUtensorMap tmO = tmA, tmR = tmA, tmG = tmA;  // placeholders when unused
-  if (EPI != EPI_TRIMUL_AB) {
-    const int n_out = (EPI == EPI_SWIGLU) ? a.N / 2 : a.N;
-    const uint64_t bstride = a.batches > 1 ? (uint64_t)a.out_batch_stride : (uint64_t)a.ldo * (uint64_t)a.M;
-    if (!make_tmap_bf16_3d(&tmO, a.out, n_out, a.M, a.batches, a.ldo, bstride, 64, 128, 1))
-      return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the output tensor map (16-byte aligned base, ld multiple of 8?)");
-    if (EPI == EPI_GATE_RESID) {
-      if (a.resid && !make_tmap_bf16_3d(&tmR, a.resid, a.N, a.M, 1, a.ldr, (uint64_t)a.ldr * a.M, 64, 128, 1))
-        return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the residual tensor map");
-      if (a.gate && !make_tmap_bf16_3d(&tmG, a.gate, a.N, a.M, 1, a.ldg, (uint64_t)a.ldg * a.M, 64, 128, 1))
-        return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the gate tensor map");
-    }
+  const int n_out = (EPI == EPI_SWIGLU) ? a.N / 2 : a.N;
+  const uint64_t bstride = a.batches > 1 ? (uint64_t)a.out_batch_stride : (uint64_t)a.ldo * (uint64_t)a.M;
+  if (!make_tmap_bf16_3d(&tmO, a.out, n_out, a.M, a.batches, a.ldo, bstride, 64, 128, 1))
+    return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the output tensor map (16-byte aligned base, ld multiple of 8?)");
+  if (EPI == EPI_GATE_RESID) {
+    if (a.resid && !make_tmap_bf16_3d(&tmR, a.resid, a.N, a.M, 1, a.ldr, (uint64_t)a.ldr * a.M, 64, 128, 1))
+      return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the residual tensor map");
+    if (a.gate && !make_tmap_bf16_3d(&tmG, a.gate, a.N, a.M, 1, a.ldg, (uint64_t)a.ldg * a.M, 64, 128, 1))
+      return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the gate tensor map");
   }
   const int sms = c->gemm_sms > 0 && c->gemm_sms < c->sm_count ? c->gemm_sms : c->sm_count;
   const int grid = (int)(total < sms ? total : sms);
-  const int tag = EPI == EPI_TRIMUL_AB ? XFOLD_K_TRIMUL_PROJ
-                  : EPI == EPI_SWIGLU  ? XFOLD_K_LINEAR_SWIGLU
+  const int tag = EPI == EPI_SWIGLU ? XFOLD_K_LINEAR_SWIGLU
                   : EPI == EPI_GATE_RESID ? XFOLD_K_LINEAR_GATE_RESID
                   : (a.batches > 1 ? XFOLD_K_TRIMUL_CONTRACT : XFOLD_K_LINEAR);
   ProfScope ps(c, tag, st);
@@ -549,7 +474,6 @@ int launch_gemm(Ctx* c, int epi, int bn, const CUtensorMap& tmA, const CUtensorM
     case EPI_GATE_RESID * 1000 + 64: return launch_one<64, EPI_GATE_RESID>(c, tmA, tmB, a, st);
     case EPI_SWIGLU * 1000 + 256: return launch_one<256, EPI_SWIGLU>(c, tmA, tmB, a, st);
     case EPI_SWIGLU * 1000 + 128: return launch_one<128, EPI_SWIGLU>(c, tmA, tmB, a, st);
-    case EPI_TRIMUL_AB * 1000 + 256: return launch_one<256, EPI_TRIMUL_AB>(c, tmA, tmB, a, st);
   }
   return fail(c, XFOLD_ERR_ARG, "gemm: unsupported tile %d / epilogue %d", bn, epi);
 }

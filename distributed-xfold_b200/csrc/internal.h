@@ -103,13 +103,11 @@ bool make_tmap_bf16_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d
                        uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, int swizzle_bytes = 128);
 
 // ---- GEMM ---------------------------------------------------------------------------------
-enum GemmEpi : int { EPI_PLAIN = 0, EPI_GATE_RESID = 1, EPI_SWIGLU = 2, EPI_TRIMUL_AB = 3 };
+enum GemmEpi : int { EPI_PLAIN = 0, EPI_GATE_RESID = 1, EPI_SWIGLU = 2 };
 
 struct GemmArgs {
   int M = 0, N = 0, K = 0, batches = 1;
   int tiles_m = 0, tiles_n = 0;
-  int a_row_mode = 0;  // 0: tile rows are consecutive rows of A; 1: tile rows step along dim 2, dim 1 fixed
-  int a_dim1 = 1;      // row mode 1: extent of dim 1
   int b_batched = 0;
   int static_b = 0;    // B is written by no kernel that may still run: its first tiles may be fetched before pdl_wait
   int mn_major = 0;    // operands are stored [k][m] and [k][n] (tensor maps: inner dim = m / n, boxes of 64 x 64)
@@ -126,14 +124,6 @@ struct GemmArgs {
   long long ldg = 0;
   const bf16* row_gate = nullptr;  // GATE_RESID: gate indexed by (m % row_gate_mod), for conditioning shared by samples
   int row_gate_mod = 0;
-  // TRIMUL_AB
-  bf16* out_a = nullptr;
-  bf16* out_b = nullptr;
-  bf16* out_g = nullptr;
-  long long cm_chan_stride = 0;
-  int cm_ld = 0;
-  int ntok = 0;
-  const float* mask = nullptr;
   int* status = nullptr;
 };
 

@@ -135,7 +135,7 @@ static int trimul_sharded(Ctx* c, ShardCtx* sc, bf16* z, const float* mask_rows,
   for (int r0 = 0; r0 < R; r0 += rper) {
     const int rr = R - r0 < rper ? R - r0 : rper;
     const long long t0 = (long long)r0 * N;
-    if ((rc = trimul_project(c, z + t0 * 128, mask_rows ? mask_rows + t0 : nullptr, rr, N, 0, w, W.x + t0 * 128,
+    if ((rc = trimul_project(c, z + t0 * 128, mask_rows ? mask_rows + t0 : nullptr, rr, N, 0, w,
                              W.a + (long long)r0 * 128 * ld, W.b + (long long)r0 * 128 * ld, W.g + t0 * 128, ld,
                              (long long)128 * ld, st))) return rc;
     if ((rc = fork_to_side(c, sc, st))) return rc;

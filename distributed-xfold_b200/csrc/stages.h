@@ -48,7 +48,14 @@ int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int tra
 int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_stride, int R, int N, bf16* out,
                  const float* gamma, const float* beta, float eps, cudaStream_t st);
 int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F, const float* gamma, const float* beta,
-                         const bf16* w1, const bf16* w2, int update_only, cudaStream_t st);
+                         const bf16* w1, const bf16* w2, int static_w, int update_only, cudaStream_t st);
+// LayerNorm of the pair representation and its projections (row_project.cu)
+int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed, const float* gamma,
+                              const float* beta, const bf16* w_in, bf16* out_a, bf16* out_b, bf16* out_g, long long chan_stride,
+                              long long row_stride, cudaStream_t st);
+int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* gamma, const float* beta, const bf16* w_qkvg,
+                            const float* scale, const float* w_bias, bf16* qkvg, bf16* bias, int pitch, long long plane,
+                            cudaStream_t st);
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
 // ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
@@ -61,7 +68,7 @@ int linear_swiglu(Ctx* c, const bf16* x, long long ldx, long long M, int K, cons
                   cudaStream_t st);
 // ---- stages of the operators (api.cu); (chan, row) strides are in elements -------------------------------
 int trimul_project(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed_store,
-                   const xfold_trimul_weights* w, bf16* x, bf16* a_out, bf16* b_out, bf16* g, long long chan_stride,
+                   const xfold_trimul_weights* w, bf16* a_out, bf16* b_out, bf16* g, long long chan_stride,
                    long long row_stride, cudaStream_t st);
 int trimul_contract(Ctx* c, const bf16* a_, long long a_cs, long long a_rs, const bf16* b_, long long b_cs,
                     long long b_rs, int Ri, int Nj, int K, bf16* o, long long o_cs, long long o_rs, cudaStream_t st,
@@ -75,7 +82,7 @@ int triattn_bias(Ctx* c, const bf16* z, int R, int N, const xfold_triattn_weight
                  long long plane, int rows_are_keys, cudaStream_t st);
 int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask, long long mask_ld, int R, int N,
                  int transposed, const xfold_triattn_weights* w, bf16* qkvg, bf16* mext, bf16* z, cudaStream_t st,
-                 bf16* upd = nullptr, const ChunkHook* hook = nullptr, bool mext_ready = false);
+                 bf16* upd = nullptr, const ChunkHook* hook = nullptr);
 int transition_fwd(Ctx* c, bf16* x, long long rows, int C, int F, const xfold_transition_weights* w, void* ws,
                    size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr, const ChunkHook* hook = nullptr);
 size_t single_ws_bytes(int N);

@@ -34,6 +34,7 @@ struct TransitionArgs {
   const bf16* x;
   long long rows;
   int items, pair, blocks;  // items of one tile (pair = 0) or two; hidden blocks of 64
+  int static_w;             // see GemmArgs::static_b
   int update_only;          // out = the update alone (x is not added)
   int* status;
 };
@@ -103,8 +104,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   const int mine = (p.items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
 
   if (warp == 0) {
-    pdl_wait();
-    pdl_launch();
+    if (!p.static_w) pdl_wait();
     if (lane == 0) {
       const long long nblk = (long long)mine * NBK;
       int hb1 = 0, hb2 = 0, t = blockIdx.x, xt = 0;
@@ -129,7 +129,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
         tma_load_3d(smem + TR_OFF_W2 + st * TR_W2, &tmw2, &w2_full[st], hb2 * 64, 0, 0);
         if (++hb2 == NBK) hb2 = 0;
       };
-      load_w1(0);
+      load_w1(0);  // (weights that no kernel of the call writes: on their way before the wait for the previous kernel)
+      pdl_wait();
+      pdl_launch();
       // W2 runs one block behind W1, and the next item's x goes out with the item's last blocks: no load waits for a
       // buffer that is freed later than the one after it needs
       for (long long i = 0; i <= nblk && okay; ++i) {
@@ -149,6 +151,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
         if (okay && i + 1 < nblk) load_w1(i + 1);
       }
     }
+    pdl_wait();
+    pdl_launch();
   } else if (warp == 1) {
     pdl_wait();
     pdl_launch();
@@ -206,7 +210,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const int s = (warp - 2) >> 2, row = ((warp - 2) & 3) * 32 + lane;
     for (int it = 0; it < mine && s < NT; ++it) {
       if (!mbar_wait(&x_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL)) break;
-      ln_row_in_place(smem + TR_OFF_N + s * TR_TILE, row, gb);
+      float nmean, rstd;
+      row_stats(smem + TR_OFF_N + s * TR_TILE, row, nmean, rstd);
+      row_normalise(smem + TR_OFF_N + s * TR_TILE, row, nmean, rstd, gb);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&n_full[s]);
@@ -318,7 +324,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
 
 // x, out: [rows][128]; w1: [2F][128] in groups of [128 SiLU | 128 linear] rows, w2: [128][F]
 int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F, const float* gamma, const float* beta,
-                         const bf16* w1, const bf16* w2, int update_only, cudaStream_t st) {
+                         const bf16* w1, const bf16* w2, int static_w, int update_only, cudaStream_t st) {
   CUtensorMap tmx, tmo, tmw1, tmw2;
   if (!make_tmap_bf16_3d(&tmx, x, 128, rows, 1, 128, (uint64_t)128 * rows, 64, 128, 1) ||
       !make_tmap_bf16_3d(&tmo, out, 128, rows, 1, 128, (uint64_t)128 * rows, 64, 128, 1) ||
@@ -333,7 +339,7 @@ int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F
   }
   const int sms = c->gemm_sms > 0 && c->gemm_sms < c->sm_count ? c->gemm_sms : c->sm_count;
   const int tiles = (int)((rows + 127) / 128), pair = tiles > sms ? 1 : 0, items = pair ? (tiles + 1) / 2 : tiles;
-  TransitionArgs a{gamma, beta, x, rows, items, pair, F / 64, update_only, c->d_status};
+  TransitionArgs a{gamma, beta, x, rows, items, pair, F / 64, static_w, update_only, c->d_status};
   ProfScope ps(c, XFOLD_K_LINEAR_SWIGLU, st);
   launch_pdl(transition_kernel, items < sms ? items : sms, TR_THREADS, TR_SMEM, st, tmx, tmo, tmw1, tmw2, a);
   return check_launch(c, "transition_kernel");

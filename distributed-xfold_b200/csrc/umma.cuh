@@ -306,6 +306,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------
@@ -369,19 +377,20 @@ __device__ __forceinline__ float2 centre2(uint32_t x, float nmean) {
 // Row `row` of a [2 halves][128 rows][64 columns] 128-byte-swizzled tile of 128 bf16 columns, by one thread: statistics, then
 // (x - mean) * rstd * gamma + beta in place; gb = gamma[128], beta[128].  Three passes over shared memory: holding the row
 // would take 64 registers.
-__device__ __forceinline__ void ln_row_in_place(uint8_t* tile, int row, const float* gb) {
-  const uint32_t rsw = uint32_t(row & 7);
-  auto piece = [&](int g) { return reinterpret_cast<uint4*>(tile + (g >> 3) * 16384 + row * 128 + ((uint32_t(g & 7) ^ rsw) << 4)); };
+__device__ __forceinline__ uint4* row_piece(uint8_t* tile, int row, int g) {
+  return reinterpret_cast<uint4*>(tile + (g >> 3) * 16384 + row * 128 + ((uint32_t(g & 7) ^ uint32_t(row & 7)) << 4));
+}
+__device__ __forceinline__ void row_stats(uint8_t* tile, int row, float& nmean, float& rstd) {
   float2 sm = make_float2(0.f, 0.f), sq = make_float2(0.f, 0.f);
 #pragma unroll
   for (int g = 0; g < 16; ++g) {
-    const uint4 u = *piece(g);
+    const uint4 u = *row_piece(tile, row, g);
     sum2(u.x, sm); sum2(u.y, sm); sum2(u.z, sm); sum2(u.w, sm);
   }
-  const float nmean = -(sm.x + sm.y) * (1.f / 128);
+  nmean = -(sm.x + sm.y) * (1.f / 128);
 #pragma unroll
   for (int g = 0; g < 16; ++g) {
-    const uint4 u = *piece(g);
+    const uint4 u = *row_piece(tile, row, g);
     const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -389,11 +398,13 @@ __device__ __forceinline__ void ln_row_in_place(uint8_t* tile, int row, const fl
       sq = ffma2(v, v, sq);
     }
   }
-  const float rstd = rsqrtf((sq.x + sq.y) * (1.f / 128) + 1e-5f);
+  rstd = rsqrtf((sq.x + sq.y) * (1.f / 128) + 1e-5f);
+}
+__device__ __forceinline__ void row_normalise(uint8_t* tile, int row, float nmean, float rstd, const float* gb) {
   const float2 r2 = make_float2(rstd, rstd);
 #pragma unroll 4
   for (int g = 0; g < 16; ++g) {
-    const uint4 u = *piece(g);
+    const uint4 u = *row_piece(tile, row, g);
     const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
     uint32_t o[4];
 #pragma unroll
@@ -402,7 +413,7 @@ __device__ __forceinline__ void ln_row_in_place(uint8_t* tile, int row, const fl
       const float2 v = ffma2(ffma2(centre2(w4[e], nmean), r2, make_float2(0.f, 0.f)), ga, be);
       o[e] = pack_bf16x2(v.x, v.y);
     }
-    *piece(g) = make_uint4(o[0], o[1], o[2], o[3]);
+    *row_piece(tile, row, g) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
