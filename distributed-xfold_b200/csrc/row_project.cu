@@ -6,14 +6,17 @@
 // extra round trip, and the projections' epilogues -- eight warps in lock-step over two staging buffers -- left HBM half idle.
 //
 // Persistent CTAs keep the weights in shared memory and walk over tiles of 128 rows:
-//   warp 0              : TMA (weights once, then x tiles)
+//   warp 0              : TMA (weights once, then x tiles, two in flight)
 //   warp 1              : tcgen05.mma issuer; a tile's columns in units of 128 accumulator columns, a ring of NSET units
-//   warps 2 - 5         : LayerNorm in place, one thread per row.  For the pair bias the tensor core first multiplies the RAW
-//                         tile (exact bf16) by w * gamma; the normalisation enters through the row's statistics.
+//   warps 2 - 9         : LayerNorm in place, two threads per row.  For the pair bias the tensor core first multiplies the
+//                         RAW tile (exact bf16) by w * gamma; the normalisation enters through the row's statistics.
 //   then NSET x 4 warps : epilogue, one set of four per unit of the ring, each set on its own: no set waits for another
 // A unit is 128 weight rows; for the gated projections [64 projection rows | 64 gate rows], so that both halves of 64 outputs
-// meet in one accumulator.  With few tiles the units are divided over several CTAs per tile (`parts`; each normalises the
-// tile for itself), so that a short sequence still uses the whole chip.
+// meet in one accumulator; g is two units of 64.  With few tiles the units are divided over several CTAs per tile (`parts`;
+// each normalises the tile for itself), so that a short sequence still uses the whole chip.  trimul has at least two parts
+// (a with half of g, b with the other half): 160 KB of weights would leave no room for a second x tile, and with one, its
+// load and normalisation stood between a tile's last product and the next tile's first (11 700 clocks per tile instead of
+// the 7200 that HBM needs in the attn form).
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -42,14 +45,15 @@ struct RowProjectArgs {
 
 template <bool ATTN>
 struct RpCfg {
-  static constexpr int UNITS = ATTN ? 4 : 5, NSET = ATTN ? 3 : 4;
-  static constexpr int THREADS = (6 + 4 * NSET) * 32;
+  // units: attn q, k, v, gate; trimul a0, a1, g0, b0, b1, g1 (g: 64 columns)
+  static constexpr int UNITS = ATTN ? 4 : 6, NSET = ATTN ? 3 : 4, MIN_PARTS = ATTN ? 1 : 2;
+  static constexpr int THREADS = (10 + 4 * NSET) * 32;
   static constexpr uint32_t W_UNIT = 32768, X_TILE = 32768;      // [2 K halves][128 rows][64], swizzled
-  static constexpr int STG_COLS = ATTN ? 64 : 32;
-  static constexpr uint32_t STG = 128 * STG_COLS * 2;            // a set's staging tile [128 rows][STG_COLS]
-  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + UNITS * W_UNIT, OFF_STG = OFF_X + X_TILE, OFF_WB = OFF_STG + NSET * STG,
-                            OFF_GB = OFF_WB + (ATTN ? 4096 : 0), OFF_SC = OFF_GB + 1024, OFF_CB = OFF_SC + (ATTN ? 2048 : 0),
-                            OFF_BAR = OFF_CB + (ATTN ? 128 : 0), SMEM = OFF_BAR + 256 + 1024;
+  static constexpr uint32_t STG = 128 * 32 * 2;                  // a set's staging tile [128 rows][32 columns]
+  static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + UNITS / MIN_PARTS * W_UNIT, OFF_STG = OFF_X + 2 * X_TILE,
+                            OFF_WB = OFF_STG + NSET * STG, OFF_GB = OFF_WB + (ATTN ? 4096 : 0), OFF_SC = OFF_GB + 1024,
+                            OFF_CB = OFF_SC + (ATTN ? 2048 : 0), OFF_ST = OFF_CB + (ATTN ? 128 : 0),
+                            OFF_BAR = OFF_ST + (ATTN ? 1024 : 0), SMEM = OFF_BAR + 256 + 1024;
   static_assert(SMEM <= 232448, "shared memory");
 };
 
@@ -67,11 +71,11 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   float* colsum = reinterpret_cast<float*>(smem + Cfg::OFF_CB);  // [16], colbias[16]
   float* colbias = colsum + 16;
   uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* x_full = w_full + 1;
-  uint64_t* x_free = x_full + 1;   // the tile's last product is complete
-  uint64_t* n_full = x_free + 1;   // normalised in place
-  uint64_t* b_full = n_full + 1;   // bias product complete
-  uint64_t* t_full = b_full + 1;   // [NSET] a unit's accumulator is complete
+  uint64_t* x_full = w_full + 1;   // [2]
+  uint64_t* x_free = x_full + 2;   // [2] the tile's last product is complete
+  uint64_t* n_full = x_free + 2;   // [2] normalised in place
+  uint64_t* b_full = n_full + 2;   // [2] bias product complete
+  uint64_t* t_full = b_full + 2;   // [NSET] a unit's accumulator is complete
   uint64_t* t_empty = t_full + NSET;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + NSET);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -80,10 +84,12 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(w_full, 1);
-    mbar_init(x_full, 1);
-    mbar_init(x_free, 1);
-    mbar_init(n_full, 4);
-    mbar_init(b_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&x_full[s], 1);
+      mbar_init(&x_free[s], 1);
+      mbar_init(&n_full[s], 8);
+      mbar_init(&b_full[s], 1);
+    }
     for (int s = 0; s < NSET; ++s) {
       mbar_init(&t_full[s], 1);
       mbar_init(&t_empty[s], 4);
@@ -146,31 +152,35 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   const int t0 = int(blockIdx.x) / p.parts, step = int(gridDim.x) / p.parts;
   const int mine = t0 < p.tiles ? (p.tiles - t0 + step - 1) / step : 0;
   const bool with_bias = ATTN && part == 0;
+  auto unit_g = [](int g) { return !ATTN && g % 3 == 2; };
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_arrive_expect_tx(w_full, U * Cfg::W_UNIT);
+      uint32_t bytes = 0;
+      for (int u = 0; u < U; ++u) bytes += unit_g(u0 + u) ? Cfg::W_UNIT / 2 : Cfg::W_UNIT;
+      mbar_arrive_expect_tx(w_full, bytes);
       for (int u = 0; u < U; ++u) {
         uint8_t* sw = smem + Cfg::OFF_W + u * Cfg::W_UNIT;
         const int g = u0 + u;
-        // first 64 and last 64 weight rows of the unit
-        const int r0 = ATTN || g == 4 ? g * 128 : (g >> 1) * 256 + (g & 1) * 64, r1 = ATTN || g == 4 ? r0 + 64 : r0 + 128;
+        // first 64 and last 64 weight rows of the unit (g: 64 in all)
+        const int r0 = ATTN ? g * 128 : unit_g(g) ? 512 + (g / 3) * 64 : (g / 3) * 256 + (g % 3) * 64, r1 = ATTN ? r0 + 64 : r0 + 128;
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) {
           tma_load_3d(sw + kh * 16384, &tmw, w_full, kh * 64, r0, 0);
-          tma_load_3d(sw + kh * 16384 + 8192, &tmw, w_full, kh * 64, r1, 0);
+          if (!unit_g(g)) tma_load_3d(sw + kh * 16384 + 8192, &tmw, w_full, kh * 64, r1, 0);
         }
       }
       pdl_wait();
       pdl_launch();
       for (int it = 0; it < mine; ++it) {
         const int t = t0 + it * step;
-        if (!mbar_wait(x_free, (uint32_t(it) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-        mbar_arrive_expect_tx(x_full, Cfg::X_TILE);
-        uint8_t* sx = smem + Cfg::OFF_X;
+        const uint32_t xb = it & 1;
+        if (!mbar_wait(&x_free[xb], ((uint32_t(it) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+        mbar_arrive_expect_tx(&x_full[xb], Cfg::X_TILE);
+        uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
         const int c1 = p.mode1 ? t % p.dim1 : t * 128, c2 = p.mode1 ? t / p.dim1 * 128 : 0;
-        tma_load_3d(sx, &tmx, x_full, 0, c1, c2);
-        tma_load_3d(sx + 16384, &tmx, x_full, 64, c1, c2);
+        tma_load_3d(sx, &tmx, &x_full[xb], 0, c1, c2);
+        tma_load_3d(sx + 16384, &tmx, &x_full[xb], 64, c1, c2);
       }
     }
     pdl_wait();
@@ -180,127 +190,176 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     pdl_launch();
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc = make_idesc(128, 128), idesc_b = make_idesc(128, 16);
-    const uint64_t xd = make_sdesc(base + Cfg::OFF_X, 16, 1024), wbd = make_sdesc(base + Cfg::OFF_WB, 16, 1024);
+    const uint64_t wbd = make_sdesc(base + Cfg::OFF_WB, 16, 1024);
     uint32_t set = 0, ph = 0;
     bool okay = mbar_wait_warp(w_full, 0, ab, XF_ERR_WAIT_FULL);
+    int nb = 0;  // tiles whose bias product has been issued; it runs ahead of the tile's other products
+    auto bias_product = [&]() {
+      tc_fence_after();
+      const uint32_t xb = nb & 1;
+      const uint64_t xd = make_sdesc(base + Cfg::OFF_X + xb * Cfg::X_TILE, 16, 1024);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          umma_ss_if(leader, tmem_base + 384 + xb * 16, xd + uint64_t(kh * 1024 + 2 * j), wbd + uint64_t(kh * 128 + 2 * j), idesc_b,
+                     (kh | j) ? 1u : 0u);
+      umma_commit_if(leader, &b_full[xb]);
+      ++nb;
+    };
     for (int it = 0; it < mine && okay; ++it) {
-      if (with_bias) {
-        if (!mbar_wait_warp(x_full, uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_ss_if(leader, tmem_base + 384, xd + uint64_t(kh * 1024 + 2 * j), wbd + uint64_t(kh * 128 + 2 * j), idesc_b,
-                       (kh | j) ? 1u : 0u);
-        umma_commit_if(leader, b_full);
+      const uint32_t xb = it & 1, xph = (uint32_t(it) >> 1) & 1u;
+      if (with_bias && nb == it) {
+        if (!mbar_wait_warp(&x_full[xb], xph, ab, XF_ERR_WAIT_FULL)) break;
+        bias_product();
       }
-      if (!mbar_wait_warp(n_full, uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL)) break;
+      if (!mbar_wait_warp(&n_full[xb], xph, ab, XF_ERR_WAIT_FULL)) break;
+      const uint64_t xd = make_sdesc(base + Cfg::OFF_X + xb * Cfg::X_TILE, 16, 1024);
       for (int u = 0; u < U; ++u) {
+        if (with_bias && nb == it + 1 && nb < mine &&
+            __all_sync(0xffffffffu, mbar_test_wait(&x_full[nb & 1], (uint32_t(nb) >> 1) & 1u)))
+          bias_product();
         if (!mbar_wait_warp(&t_empty[set], ph ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) { okay = false; break; }
         tc_fence_after();
         const uint64_t wd = make_sdesc(base + Cfg::OFF_W + u * Cfg::W_UNIT, 16, 1024);
+        const uint32_t id = unit_g(u0 + u) ? make_idesc(128, 64) : idesc;
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_ss_if(leader, tmem_base + set * 128, xd + uint64_t(kh * 1024 + 2 * j), wd + uint64_t(kh * 1024 + 2 * j), idesc,
+            umma_ss_if(leader, tmem_base + set * 128, xd + uint64_t(kh * 1024 + 2 * j), wd + uint64_t(kh * 1024 + 2 * j), id,
                        (kh | j) ? 1u : 0u);
         umma_commit_if(leader, &t_full[set]);
         if (++set == NSET) { set = 0; ph ^= 1u; }
       }
-      if (okay) umma_commit_if(leader, x_free);
+      if (okay) umma_commit_if(leader, &x_free[xb]);
     }
-  } else if (warp < 6) {
+  } else if (warp < 10) {
     pdl_wait();
     pdl_launch();
-    // (warp & 3) is the quarter of tensor memory's lanes this warp may read: row = lane there
-    const int row = (warp & 3) * 32 + lane;
-    uint8_t* sx = smem + Cfg::OFF_X;
+    // 16 rows per warp; the two halves of a row in lanes l and l + 16
+    const int row = (warp - 2) * 16 + (lane & 15), half = lane >> 4;
+    float2* rstat = reinterpret_cast<float2*>(smem + Cfg::OFF_ST);
     for (int it = 0; it < mine; ++it) {
-      if (!mbar_wait(x_full, uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL)) break;
-      float nmean, rstd;
-      row_stats(sx, row, nmean, rstd);
-      if (with_bias) {
-        if (!__all_sync(0xffffffffu, mbar_wait(b_full, uint32_t(it) & 1u, ab, XF_ERR_WAIT_TMEM_FULL))) break;
-        tc_fence_after();
-        uint32_t d[4];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                     : "r"(tmem_base + 384 + (uint32_t((warp & 3) * 32) << 16)) : "memory");
-        tmem_ld_wait();
-        tc_fence_before();
-        const long long r = (long long)(t0 + it * step) * 128 + row;
-        if (r < p.rows) {
-          const int q = int(r / p.inner), k = int(r - (long long)q * p.inner);
-          __half* dst = reinterpret_cast<__half*>(p.bias) + (long long)q * p.pitch + k;
+      const uint32_t xb = it & 1, xph = (uint32_t(it) >> 1) & 1u;
+      mbar_wait(&x_full[xb], xph, ab, XF_ERR_WAIT_FULL);  // (a failed wait runs through: these warps may meet at a barrier)
+      uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
+      uint32_t xr[32];
+      float2 sm[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const float v = fmaf(rstd, fmaf(nmean, colsum[h], __uint_as_float(d[h])), colbias[h]) * 1.4426950408889634f;
-            dst[h * p.plane] = __float2half_rn(fminf(fmaxf(v, -60000.f), 60000.f));
+      for (int q = 0; q < 8; ++q) {
+        const uint4 u = *row_piece(sx, row, half * 8 + q);
+        xr[q * 4] = u.x; xr[q * 4 + 1] = u.y; xr[q * 4 + 2] = u.z; xr[q * 4 + 3] = u.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 32; ++e) sum2(xr[e], sm[e & 1]);
+      float s = (sm[0].x + sm[0].y) + (sm[1].x + sm[1].y);
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      const float nmean = -s * (1.f / 128);
+      float2 sq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        const float2 v = centre2(xr[e], nmean);
+        sq[e & 1] = ffma2(v, v, sq[e & 1]);
+      }
+      s = (sq[0].x + sq[0].y) + (sq[1].x + sq[1].y);
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      const float rstd = rsqrtf(s * (1.f / 128) + 1e-5f);
+      if (with_bias) {
+        if (half == 0) rstat[row] = make_float2(nmean, rstd);
+        named_bar_sync(NSET + 1, 256);
+        mbar_wait(&b_full[xb], xph, ab, XF_ERR_WAIT_TMEM_FULL);
+        if (warp < 6) {  // (warp & 3) is the quarter of tensor memory's lanes this warp may read: row = lane there
+          tc_fence_after();
+          uint32_t d[4];
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                       : "r"(tmem_base + 384 + xb * 16 + (uint32_t((warp & 3) * 32) << 16)) : "memory");
+          tmem_ld_wait();
+          tc_fence_before();
+          const int rr = (warp & 3) * 32 + lane;
+          const long long r = (long long)(t0 + it * step) * 128 + rr;
+          if (r < p.rows) {
+            const float2 st = rstat[rr];
+            const int q = int(r / p.inner), k = int(r - (long long)q * p.inner);
+            __half* dst = reinterpret_cast<__half*>(p.bias) + (long long)q * p.pitch + k;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+              const float v = fmaf(st.y, fmaf(st.x, colsum[h], __uint_as_float(d[h])), colbias[h]) * 1.4426950408889634f;
+              dst[h * p.plane] = __float2half_rn(fminf(fmaxf(v, -60000.f), 60000.f));
+            }
           }
         }
       }
-      row_normalise(sx, row, nmean, rstd, gb);
+      const float2 r2 = make_float2(rstd, rstd);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = half * 64 + q * 8 + 2 * e;
+          const float2 ga = *reinterpret_cast<const float2*>(gb + c), be = *reinterpret_cast<const float2*>(gb + 128 + c);
+          const float2 v = ffma2(ffma2(centre2(xr[q * 4 + e], nmean), r2, make_float2(0.f, 0.f)), ga, be);
+          o[e] = pack_bf16x2(v.x, v.y);
+        }
+        *row_piece(sx, row, half * 8 + q) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(n_full);
+      if (lane == 0) mbar_arrive(&n_full[xb]);
     }
   } else {
     pdl_wait();
     pdl_launch();
-    const int set = (warp - 6) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+    const int set = (warp - 10) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t laddr = tmem_base + set * 128 + (uint32_t(quarter * 32) << 16);
     uint8_t* stg = smem + Cfg::OFF_STG + set * Cfg::STG;
-    const bool elected = ((warp - 6) & 3) == 0 && lane == 0;
+    const bool elected = ((warp - 10) & 3) == 0 && lane == 0;
     uint32_t k = 0;  // units this set has taken
     for (int n = set; n < mine * U; n += NSET, ++k) {
       const int it = n / U, g = u0 + n % U, t = t0 + it * step;
       const int c1 = p.mode1 ? t % p.dim1 : t * 128, c2 = p.mode1 ? t / p.dim1 * 128 : 0;
-      if constexpr (ATTN) {
+      const uint32_t rsw = uint32_t(row >> 1) & 3u;  // 64-byte swizzle of the staging tile
+      if (ATTN || unit_g(g)) {
+        const int chunks = ATTN ? 4 : 2, col0 = ATTN ? g * 128 : (g / 3) * 64;
         mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through: the set meets at barriers)
         tc_fence_after();
-        const uint32_t rsw = uint32_t(row & 7);
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < chunks; ++c) {
+          uint32_t r[32];
+          tmem_ld32(laddr + c * 32, r);
           if (elected) tma_store_wait_read<0>();
           named_bar_sync(1 + set, 128);
+          tmem_ld_wait();
+          if (c == chunks - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&t_empty[set]);
+          }
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t r[32];
-            tmem_ld32(laddr + c * 64 + hf * 32, r);
-            tmem_ld_wait();
-            if (c == 1 && hf == 1) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&t_empty[set]);
-            }
-            const float* s0 = sc + g * 128 + c * 64 + hf * 32;
+          for (int q = 0; q < 4; ++q) {
+            uint32_t o[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint32_t o[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 s2 = *reinterpret_cast<const float2*>(s0 + q * 8 + 2 * e);
-                const float v0 = __uint_as_float(r[q * 8 + 2 * e]) * s2.x, v1 = __uint_as_float(r[q * 8 + 2 * e + 1]) * s2.y;
-                if (g == 2) {  // the v columns leave as fp16
-                  const __half2 h2 = __floats2half2_rn(v0, v1);
-                  o[e] = *reinterpret_cast<const uint32_t*>(&h2);
-                } else {
-                  o[e] = pack_bf16x2(v0, v1);
-                }
+            for (int e = 0; e < 4; ++e) {
+              float v0 = __uint_as_float(r[q * 8 + 2 * e]), v1 = __uint_as_float(r[q * 8 + 2 * e + 1]);
+              if constexpr (ATTN) {
+                const float2 s2 = *reinterpret_cast<const float2*>(sc + col0 + c * 32 + q * 8 + 2 * e);
+                v0 *= s2.x;
+                v1 *= s2.y;
               }
-              *reinterpret_cast<uint4*>(stg + row * 128 + ((uint32_t(hf * 4 + q) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+              const __half2 h2 = __floats2half2_rn(v0, v1);  // the v columns leave as fp16
+              o[e] = ATTN && g == 2 ? *reinterpret_cast<const uint32_t*>(&h2) : pack_bf16x2(v0, v1);
             }
+            *reinterpret_cast<uint4*>(stg + row * 64 + ((uint32_t(q) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
           }
           fence_proxy_async_smem();
           named_bar_sync(1 + set, 128);
           if (elected) {
-            tma_store_3d(&tmo, stg, g * 128 + c * 64, c1, c2);
+            tma_store_3d(&tmo, stg, col0 + c * 32, c1, c2);
             tma_store_commit();
           }
         }
-      } else if (g < 4) {
+      } else {
         // where this thread's token goes, and its mask value, before the wait
         long long off = 0;
         bool valid;
@@ -316,7 +375,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
           off = (long long)c1 * p.row_stride + i;
           if (valid && p.mask) mk = p.mask[i * p.ntok + c1];
         }
-        bf16* dst = (g < 2 ? p.out_a : p.out_b) + off + (long long)((g & 1) * 64) * p.chan_stride;
+        bf16* dst = (g < 3 ? p.out_a : p.out_b) + off + (long long)(g % 3 * 64) * p.chan_stride;
         mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
         tc_fence_after();
 #pragma unroll 1
@@ -336,36 +395,6 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
               *dst = __float2bfloat16(__uint_as_float(rp[e]) * mk * sigmoidf_fast(__uint_as_float(rg[e])));
               dst += p.chan_stride;
             }
-          }
-        }
-      } else {
-        mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
-        tc_fence_after();
-        const uint32_t rsw = uint32_t(row >> 1) & 3u;  // 64-byte swizzle
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(laddr + c * 32, r);
-          if (elected) tma_store_wait_read<0>();
-          named_bar_sync(1 + set, 128);
-          tmem_ld_wait();
-          if (c == 3) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&t_empty[set]);
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t o[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(__uint_as_float(r[q * 8 + 2 * e]), __uint_as_float(r[q * 8 + 2 * e + 1]));
-            *reinterpret_cast<uint4*>(stg + row * 64 + ((uint32_t(q) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-          fence_proxy_async_smem();
-          named_bar_sync(1 + set, 128);
-          if (elected) {
-            tma_store_3d(&tmo, stg, c * 32, c1, c2);
-            tma_store_commit();
           }
         }
       }
@@ -398,7 +427,8 @@ static int launch_row_project(Ctx* c, const CUtensorMap& tmx, const CUtensorMap&
   }
   const int sms = c->gemm_sms > 0 && c->gemm_sms < c->sm_count ? c->gemm_sms : c->sm_count;
   // units divided over CTAs as long as a tile per CTA group leaves SMs without work
-  a.parts = sms / a.tiles < 1 ? 1 : sms / a.tiles > Cfg::UNITS ? Cfg::UNITS : sms / a.tiles;
+  const int spread = sms / a.tiles;
+  a.parts = spread < Cfg::MIN_PARTS ? Cfg::MIN_PARTS : spread > Cfg::UNITS ? Cfg::UNITS : spread;
   const int groups = a.tiles < sms / a.parts ? a.tiles : sms / a.parts;
   a.static_w = c->static_weights;
   a.status = c->d_status;
@@ -446,7 +476,7 @@ int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* ga
   CUtensorMap tmx, tmw, tmo;
   RowProjectArgs a = {};
   if (!make_tmap_bf16_3d(&tmx, z, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) ||
-      !make_tmap_bf16_3d(&tmo, qkvg, 512, M, 1, 512, (uint64_t)512 * M, 64, 128, 1) ||
+      !make_tmap_bf16_3d(&tmo, qkvg, 512, M, 1, 512, (uint64_t)512 * M, 32, 128, 1, 64) ||
       !make_tmap_bf16_3d(&tmw, w_qkvg, 128, 512, 1, 128, 128 * 512, 64, 64, 1))
     return fail(c, XFOLD_ERR_ARG, "triattn: cannot encode projection tensor maps");
   a.tiles = (int)((M + 127) / 128);
