@@ -249,18 +249,15 @@ int trimul_contract_mn(Ctx* c, const bf16* at, long long at_cs, long long at_rs,
   return launch_gemm(c, EPI_PLAIN, 256, tA, tB, a, st);
 }
 
-// z (+)= Linear(LN_c(o)) * sigmoid(g); o: [R][128][ldo]; x: scratch [R*N][128]
-int trimul_output(Ctx* c, const bf16* o, long long o_cs, long long o_rs, const bf16* g, int R, int N,
-                         const xfold_trimul_weights* w, bf16* x, bf16* z, cudaStream_t st, bf16* upd) {
-  int rc = launch_cm_ln(c, o, o_cs, o_rs, R, N, x, w->ln_c_gamma, w->ln_c_beta, 1e-5f, st);
-  if (rc) return rc;
-  // upd given: write the update alone there and leave z untouched; else z += update
-  return linear_gate_resid(c, x, 128, (long long)R * N, 128, (const bf16*)w->w_out, 128, g, 128, 0, upd ? nullptr : z, 128,
-                           upd ? upd : z, 128, st);
+// z (+)= Linear(LN_c(o)) * sigmoid(g); o: channel-major.  upd given: write the update alone there and leave z untouched.
+int trimul_output(Ctx* c, const bf16* o, long long o_cs, long long o_rs, const bf16* g, int R, int N, const xfold_trimul_weights* w,
+                  bf16* z, cudaStream_t st, bf16* upd) {
+  return launch_row_output_cm(c, o, o_cs, o_rs, R, N, w->ln_c_gamma, w->ln_c_beta, (const bf16*)w->w_out, g, upd ? nullptr : z,
+                              upd ? upd : z, st);
 }
 
 struct TriMulWs {
-  bf16 *x, *a, *b, *g, *o;
+  bf16 *a, *b, *g, *o;
   int ld;
   size_t bytes;
 };
@@ -270,7 +267,6 @@ static TriMulWs carve_trimul(void* ws, size_t cap, int N) {
   w.ld = pad8(N);
   const size_t tok = (size_t)N * N * 128 * 2;
   const size_t cm = (size_t)128 * N * w.ld * 2;
-  w.x = (bf16*)cv.take(tok);
   w.g = (bf16*)cv.take(tok);
   w.a = (bf16*)cv.take(cm);
   w.b = (bf16*)cv.take(cm);
@@ -293,7 +289,7 @@ static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, c
   StaticWeights sw(c);
   rc = trimul_contract(c, outgoing ? W.a : W.b, cs, rs, outgoing ? W.b : W.a, cs, rs, N, N, N, W.o, cs, rs, st);
   if (rc) return rc;
-  return trimul_output(c, W.o, cs, rs, W.g, N, N, w, W.x, z, st, upd);
+  return trimul_output(c, W.o, cs, rs, W.g, N, N, w, z, st, upd);
 }
 
 struct TriAttnWs {
@@ -336,8 +332,11 @@ static int triattn_attend(Ctx* c, bf16* x, const bf16* biasT, int ldq, int R, in
   const int rc = launch_attention2(c, qkvg, 512, N, R, transposed, 0, 128, 256, 384, 4, biasT, ldq, mext, R, x, seq_stride,
                                    batch_stride, st);
   if (rc) return rc;
-  return linear_gate_resid_chunked(c, x, 128, (long long)R * N, 128, (const bf16*)w->w_out, 128, upd ? nullptr : z, 128,
-                                   upd ? upd : z, 128, st, hook);
+  const long long M = (long long)R * N;
+  if (hook && hook->after && hook->parts > 1)
+    return linear_gate_resid_chunked(c, x, 128, M, 128, (const bf16*)w->w_out, 128, z, 128, z, 128, st, hook);
+  const int rc2 = launch_row_output(c, x, M, (const bf16*)w->w_out, upd ? nullptr : z, upd ? upd : z, st);
+  return rc2 || !hook || !hook->after ? rc2 : hook->after(0, M);
 }
 int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask, long long mask_ld, int R, int N,
                         int transposed, const xfold_triattn_weights* w, bf16* qkvg, bf16* mext, bf16* z, cudaStream_t st,
@@ -785,8 +784,7 @@ int xfold_trimul_contract_planes_fwd(xfold_ctx* c, const void* a, const void* b,
 int xfold_trimul_output_fwd(xfold_ctx* c, const void* o, int ldo, const void* g, int R, int N, const xfold_trimul_weights* w,
                             void* x_scratch, void* z, void* stream) {
   if (!c || !o || !g || !w || !x_scratch || !z) return XFOLD_ERR_ARG;
-  return trimul_output(c, (const bf16*)o, ldo, (long long)128 * ldo, (const bf16*)g, R, N, w, (bf16*)x_scratch, (bf16*)z,
-                       (cudaStream_t)stream);
+  return trimul_output(c, (const bf16*)o, ldo, (long long)128 * ldo, (const bf16*)g, R, N, w, (bf16*)z, (cudaStream_t)stream);
 }
 int xfold_triattn_bias_fwd(xfold_ctx* c, const void* z, int R, int N, const xfold_triattn_weights* w, void* x, void* biasT,
                            int pitch, long long plane, int rows_are_keys, void* stream) {

@@ -79,12 +79,6 @@ __device__ __forceinline__ float ex2f_(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tadd.rn.f32x2 rd, ra, rb;\n\t"
-      "mov.b64 {%0, %1}, rd;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
 // 2^y for a pair of float32 on the FMA pipe: y = n + f with n the nearest integer, 2^f by a degree-5 polynomial on
 // [-1/2, 1/2] (minimax in relative error, 7.5e-8, fitted with the Remez exchange), n added to the exponent field.
 __device__ __forceinline__ float2 ex2_poly2(float2 y) {

@@ -165,7 +165,7 @@ static int trimul_sharded(Ctx* c, ShardCtx* sc, bf16* z, const float* mask_rows,
   }
   if ((rc = join_side(c, sc, st))) return rc;
   if ((rc = barrier(c, sc, st))) return rc;
-  return trimul_output(c, (const bf16*)sc->po[me], ld, (long long)128 * ld, W.g, R, N, w, W.x, z, st);
+  return trimul_output(c, (const bf16*)sc->po[me], ld, (long long)128 * ld, W.g, R, N, w, z, st);
 }
 
 static int block_sharded(Ctx* c, ShardCtx* sc, int* slot, bf16* s, const float* pair_mask, const float* seq_mask,

@@ -1,6 +1,5 @@
 // Bandwidth-bound kernels: LayerNorm over rows (optionally with a small fused projection that
-// produces the attention pair bias), LayerNorm of a channel-major tensor with a transposing
-// write-back, and the element-wise pieces of the diffusion transformer (AdaLN modulation, gates).
+// produces the attention pair bias) and the element-wise pieces of the diffusion transformer (AdaLN modulation, gates).
 // One warp per row, 8-byte vector accesses, fp32 statistics, warp-shuffle reductions.
 #include <cuda_fp16.h>
 
@@ -626,138 +625,6 @@ int launch_ln_rows(Ctx* c, const bf16* x, long long ldx, bf16* y, long long ldy,
     case 768: return launch_ln_c<768>(c, x, ldx, y, ldy, rows, g, b, eps, H, pw, proj, plane, msc, msh, mod_rows, pbf, tin, tout, tpitch, st);
   }
   return fail(c, XFOLD_ERR_ARG, "layernorm: unsupported width %d (128, 384, 768)", C);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Channel-major -> token-major LayerNorm: in [128][R][ld] bf16, out [R*N][128] bf16.
-// A block stages 128 channels x 64 tokens in shared memory (rows padded to 66 elements so that
-// the per-token reads below are bank-conflict free), 4 threads share a token.
-// ---------------------------------------------------------------------------------------------
-constexpr int CMLN_TOK = 128;
-constexpr int CMLN_PITCH = CMLN_TOK + 8;  // elements; keeps every row 16-byte aligned
-constexpr size_t CMLN_TILE_BYTES = (size_t)128 * CMLN_PITCH * sizeof(bf16);
-constexpr size_t CMLN_SMEM = 2 * CMLN_TILE_BYTES + 2 * 4 * CMLN_TOK * sizeof(float);
-
-// The tile of the NEXT iteration is fetched with cp.async (global -> shared without passing through registers) while
-// the current one is normalised and stored, so loads stay in flight through the compute and store phases.
-__global__ void __launch_bounds__(256, 3)
-cm_ln_kernel(const bf16* in, long long chan_stride, long long row_stride, int R, int N,
-             bf16* __restrict__ out, const float* __restrict__ gamma, const float* __restrict__ beta, float eps) {
-  extern __shared__ __align__(16) uint8_t cmln_smem[];
-  bf16 (*tiles)[128][CMLN_PITCH] = reinterpret_cast<bf16 (*)[128][CMLN_PITCH]>(cmln_smem);
-  float (*psum)[CMLN_TOK] = reinterpret_cast<float (*)[CMLN_TOK]>(cmln_smem + 2 * CMLN_TILE_BYTES);
-  float (*psq)[CMLN_TOK] = psum + 4;
-  pdl_wait();
-  pdl_launch();
-  const int tiles_j = (N + CMLN_TOK - 1) / CMLN_TOK;
-  const long long ntiles = (long long)R * tiles_j;
-  const bool vec_ok = ((chan_stride | row_stride) & 7) == 0;
-  // 128 channel rows x 128 tokens: 16 x 16-byte pieces per row
-  auto fetch = [&](long long t, int buf) {
-    const int i = int(t / tiles_j);
-    const int j0 = int(t % tiles_j) * CMLN_TOK;
-    for (int idx = threadIdx.x; idx < 128 * 16; idx += 256) {
-      const int ch = idx >> 4, w = idx & 15;
-      const int j = j0 + 8 * w;
-      const bf16* src = in + ch * chan_stride + (long long)i * row_stride + j;
-      bf16* dst = &tiles[buf][ch][8 * w];
-      if (vec_ok && j + 7 < N) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-      } else {
-        bf16 tmp[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) tmp[e] = (j + e < N) ? src[e] : __float2bfloat16(0.f);
-        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(tmp);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  int buf = 0;
-  if ((long long)blockIdx.x < ntiles) fetch(blockIdx.x, 0);
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, buf ^= 1) {
-    const int i = int(t / tiles_j);
-    const int j0 = int(t % tiles_j) * CMLN_TOK;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // tile t has landed for every thread; everybody is done with the other buffer and with psum
-    if (t + gridDim.x < ntiles) fetch(t + gridDim.x, buf ^ 1);
-    bf16 (*tile)[CMLN_PITCH] = tiles[buf];
-    // thread = (token pair tp, quarter of the channels): a warp reads 32 consecutive 4-byte words per channel row
-    const int tp = threadIdx.x & 63, part = threadIdx.x >> 6;
-    float v0[32], v1[32];
-    float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll
-    for (int e = 0; e < 32; ++e) {
-      const uint32_t u = *reinterpret_cast<const uint32_t*>(&tile[part * 32 + e][2 * tp]);
-      v0[e] = bf16_lo(u);
-      v1[e] = bf16_hi(u);
-      s0 += v0[e]; s1 += v1[e];
-      q0 += v0[e] * v0[e]; q1 += v1[e] * v1[e];
-    }
-    psum[part][2 * tp] = s0; psum[part][2 * tp + 1] = s1;
-    psq[part][2 * tp] = q0; psq[part][2 * tp + 1] = q1;
-    __syncthreads();
-    float mean[2], rstd[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int tk = 2 * tp + u;
-      const float sm = psum[0][tk] + psum[1][tk] + psum[2][tk] + psum[3][tk];
-      const float sq = psq[0][tk] + psq[1][tk] + psq[2][tk] + psq[3][tk];
-      mean[u] = sm * (1.f / 128);
-      rstd[u] = rsqrtf(fmaxf(sq * (1.f / 128) - mean[u] * mean[u], 0.f) + eps);
-    }
-    // Every thread holds its values in registers and the statistics are exchanged: the tile's buffer is free.  The
-    // normalised tokens are staged there token-major, so that they leave as whole 256-byte rows (a thread's own 2 x 64
-    // bytes written straight to global memory use half of every 128-byte line they touch).
-    bf16 (*stage)[CMLN_PITCH] = tile;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      bf16* srow = &stage[2 * tp + u][part * 32];
-#pragma unroll
-      for (int g8 = 0; g8 < 4; ++g8) {
-        float o[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int ch = part * 32 + g8 * 8 + e;
-          float tv = ((u ? v1[g8 * 8 + e] : v0[g8 * 8 + e]) - mean[u]) * rstd[u];
-          if (gamma) tv *= gamma[ch];
-          if (beta) tv += beta[ch];
-          o[e] = tv;
-        }
-        uint4 w4;
-        w4.x = pack_bf16x2(o[0], o[1]); w4.y = pack_bf16x2(o[2], o[3]);
-        w4.z = pack_bf16x2(o[4], o[5]); w4.w = pack_bf16x2(o[6], o[7]);
-        *reinterpret_cast<uint4*>(srow + g8 * 8) = w4;
-      }
-    }
-    __syncthreads();
-    // 128 tokens x 16 pieces of 16 bytes: a warp writes two whole token rows per instruction
-    for (int idx = threadIdx.x; idx < CMLN_TOK * 16; idx += 256) {
-      const int tk = idx >> 4, piece = idx & 15;
-      const int j = j0 + tk;
-      if (j < N)
-        *reinterpret_cast<uint4*>(out + ((long long)i * N + j) * 128 + piece * 8) =
-            *reinterpret_cast<const uint4*>(&stage[tk][piece * 8]);
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_stride, int R, int N, bf16* out,
-                 const float* gamma, const float* beta, float eps, cudaStream_t st) {
-  const long long ntiles = (long long)R * ((N + CMLN_TOK - 1) / CMLN_TOK);
-  if (ntiles <= 0) return XFOLD_OK;
-  long long blocks = ntiles;
-  const long long cap = (long long)c->sm_count * 3;  // one wave of resident CTAs (3 per SM): the loop is grid-strided
-  if (blocks > cap) blocks = cap;
-  ProfScope ps(c, XFOLD_K_CHANNEL_LN, st);
-  static bool attr_done[8] = {false};
-  if (!attr_done[c->device & 7]) {
-    cudaError_t e = cudaFuncSetAttribute(cm_ln_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CMLN_SMEM);
-    if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "channel LayerNorm smem attribute: %s", cudaGetErrorString(e));
-    attr_done[c->device & 7] = true;
-  }
-  launch_pdl(cm_ln_kernel, (int)blocks, 256, CMLN_SMEM, st, in, chan_stride, row_stride, R, N, out, gamma, beta, eps);
-  return check_launch(c, "cm_ln_kernel");
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -45,8 +45,6 @@ int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int 
 int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int transposed, int q_col0, int k_col0,
                       int v_col0, int g_col0, int heads, const bf16* biasT, int ldq, const bf16* mext, int mext_rows,
                       bf16* out, long long out_seq_stride, long long out_batch_stride, cudaStream_t st, int head_dim = 32);
-int launch_cm_ln(Ctx* c, const bf16* in, long long chan_stride, long long row_stride, int R, int N, bf16* out,
-                 const float* gamma, const float* beta, float eps, cudaStream_t st);
 int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F, const float* gamma, const float* beta,
                          const bf16* w1, const bf16* w2, int static_w, int update_only, cudaStream_t st);
 // LayerNorm of the pair representation and its projections (row_project.cu)
@@ -56,6 +54,10 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
 int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* gamma, const float* beta, const bf16* w_qkvg,
                             const float* scale, const float* w_bias, bf16* qkvg, bf16* bias, int pitch, long long plane,
                             cudaStream_t st);
+// output projections of the pair representation (row_output.cu)
+int launch_row_output(Ctx* c, const bf16* x, long long M, const bf16* w, const bf16* resid, bf16* out, cudaStream_t st);
+int launch_row_output_cm(Ctx* c, const bf16* o, long long o_cs, long long o_rs, int R, int N, const float* gamma, const float* beta,
+                         const bf16* w, const bf16* g, const bf16* resid, bf16* out, cudaStream_t st);
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
 // ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
@@ -77,7 +79,7 @@ int trimul_contract_mn(Ctx* c, const bf16* at, long long at_cs, long long at_rs,
                        long long bt_rs, int Mi, int Nj, int K, bf16* o, long long o_cs, long long o_rs, cudaStream_t st,
                        int channels = 128);
 int trimul_output(Ctx* c, const bf16* o, long long o_cs, long long o_rs, const bf16* g, int R, int N,
-                  const xfold_trimul_weights* w, bf16* x, bf16* z, cudaStream_t st, bf16* upd = nullptr);
+                  const xfold_trimul_weights* w, bf16* z, cudaStream_t st, bf16* upd = nullptr);
 int triattn_bias(Ctx* c, const bf16* z, int R, int N, const xfold_triattn_weights* w, bf16* x, bf16* bias, int pitch,
                  long long plane, int rows_are_keys, cudaStream_t st);
 int triattn_core(Ctx* c, bf16* x, const bf16* biasT, int ldq, const float* mask, long long mask_ld, int R, int N,
