@@ -53,7 +53,7 @@ struct RpCfg {
   static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + UNITS / MIN_PARTS * W_UNIT, OFF_STG = OFF_X + 2 * X_TILE,
                             OFF_WB = OFF_STG + NSET * STG, OFF_GB = OFF_WB + (ATTN ? 4096 : 0), OFF_SC = OFF_GB + 1024,
                             OFF_CB = OFF_SC + (ATTN ? 2048 : 0), OFF_ST = OFF_CB + (ATTN ? 128 : 0),
-                            OFF_BAR = OFF_ST + (ATTN ? 1024 : 0), SMEM = OFF_BAR + 256 + 1024;
+                            OFF_BAR = OFF_ST + (ATTN ? 2048 : 0), SMEM = OFF_BAR + 256 + 1024;
   static_assert(SMEM <= 232448, "shared memory");
 };
 
@@ -239,7 +239,6 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     pdl_launch();
     // 16 rows per warp; the two halves of a row in lanes l and l + 16
     const int row = (warp - 2) * 16 + (lane & 15), half = lane >> 4;
-    float2* rstat = reinterpret_cast<float2*>(smem + Cfg::OFF_ST);
     for (int it = 0; it < mine; ++it) {
       const uint32_t xb = it & 1, xph = (uint32_t(it) >> 1) & 1u;
       mbar_wait(&x_full[xb], xph, ab, XF_ERR_WAIT_FULL);  // (a failed wait runs through: these warps may meet at a barrier)
@@ -266,6 +265,8 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       s += __shfl_xor_sync(0xffffffffu, s, 16);
       const float rstd = rsqrtf(s * (1.f / 128) + 1e-5f);
       if (with_bias) {
+        // (by tile parity: a warp may be one tile ahead of the readers, not two -- the barrier is in between)
+        float2* rstat = reinterpret_cast<float2*>(smem + Cfg::OFF_ST) + xb * 128;
         if (half == 0) rstat[row] = make_float2(nmean, rstd);
         named_bar_sync(NSET + 1, 256);
         mbar_wait(&b_full[xb], xph, ab, XF_ERR_WAIT_TMEM_FULL);
