@@ -316,6 +316,23 @@ def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
     assert torch.isfinite(out).all() and relf(out, ref) < 4e-2
 
 
+@pytest.mark.parametrize("n", [129, 137, 310])
+def test_triangle_multiplication_ragged_contraction_tiles(ops, oracle, n):
+    """Token counts whose last 256-wide contraction tile is mostly empty, and row counts that are no multiple of a tile."""
+    g = torch.Generator().manual_seed(n)
+    st = with_affine_norms(oracle.make_trimul_state(g, ""), n)
+    z = torch.randn(n, n, 128, generator=g).to(BF)
+    mask = (torch.rand(n, n, generator=g) > 0.2).float()
+    w = ops.PackedTriMul(st, "", "cuda")
+    for outgoing in (True, False):
+        ref = z.float() + oracle.triangle_multiplication(rounded(st), "", z.float(), mask, outgoing)
+        for _ in range(3):
+            zd = z.cuda().contiguous()
+            ops.triangle_multiplication_(zd, mask.cuda(), w, outgoing)
+            ops.synchronize_and_check()
+            check_update(z, zd, ref)
+
+
 @pytest.mark.parametrize("rows", [1, 127, 129, 148 * 128, 148 * 128 + 1, 297 * 128 + 5])
 def test_transition_tile_pairs(ops, oracle, rows):
     """Around the tile, the switch from one to two tiles per CTA, and an odd number of tiles."""
