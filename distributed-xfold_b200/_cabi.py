@@ -128,6 +128,8 @@ SIGNATURES = {
     "xfold_pair_bias_prepare_fwd": (ci, [vp, vp, ci, ci, vp, vp]),
     "xfold_pair_logits_prepared_fwd": (ci, [vp, vp, ci, vp, vp, vp, ci, vp, vp]),
     "xfold_attention_pair_bias_core_prepared_fwd": (ci, [vp, vp, ci, ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
+    "xfold_grid_attention_workspace_bytes": (sz, [ci, ci, ci, ci]),
+    "xfold_grid_attention_fwd": (ci, [vp, vp, ci, ci, ci, ci, vp, vp, vp, vp, ll, vp, ci, vp, ci, vp, sz, vp]),
     "xfold_diffusion_workspace_bytes": (sz, [ci, ci, C.POINTER(DiffusionWeights)]),
     "xfold_diffusion_transformer_fwd": (ci, [vp, vp, ci, ci, vp, vp, C.POINTER(DiffusionWeights), C.POINTER(vp), vp, sz, vp]),
     "xfold_cross_attention_workspace_bytes": (sz, [ci, ci, ci, ci, ci]),

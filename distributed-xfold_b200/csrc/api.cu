@@ -357,7 +357,7 @@ static int triattn_fwd(Ctx* c, bf16* z, const float* mask, int N, int transpose,
   TriAttnWs W = carve_triattn(ws, ws_bytes, N, N);
   if (!ws || W.bytes > ws_bytes) return fail(c, XFOLD_ERR_ARG, "triattn: workspace too small (%zu < %zu)", ws_bytes, W.bytes);
   // both nodes use bias(q, k) = projection of token (q, k), not transposed for the ending node
-  int rc = launch_row_project_attn(c, z, N, N, w->ln_gamma, w->ln_beta, (const bf16*)w->w_qkvg, w->qkvg_scale, w->w_bias, W.qkvg,
+  int rc = launch_row_project_attn(c, z, N, N, 1, w->ln_gamma, w->ln_beta, (const bf16*)w->w_qkvg, w->qkvg_scale, w->w_bias, W.qkvg,
                                    W.nbT, W.ldq, (long long)N * W.ldq, st);
   if (rc) return rc;
   StaticWeights sw(c);
@@ -449,6 +449,48 @@ static int apb_core_fwd_(Ctx* c, const bf16* xn, int B, int S, int C, int H, int
   }
   return launch_attention2(c, W.qkvg, 4 * Wd, S, B, 0, 0, Wd, 2 * Wd, 3 * Wd, H, pair_biasT, W.ldq, mext, mrows, out, Wd,
                            (long long)S * Wd, st, Dp);
+}
+
+// The whole TriangleAttention operator on normalised rows: projections, gated attention, output projection, with the
+// sequence axis of the result padded to SP (zeros).  mask_bias: additive, one row per batch entry (ld > 0) or one for all.
+struct GridWs {
+  bf16 *qkvg, *biasT, *mext, *att;
+  size_t bytes;
+};
+static GridWs carve_grid(void* ws, size_t cap, int B, int S, int SP, int H) {
+  GridWs W;
+  Carver cv(ws, cap);
+  W.qkvg = (bf16*)cv.take((size_t)B * S * 4 * H * 32 * 2);
+  W.biasT = (bf16*)cv.take((size_t)H * S * pad8(S) * 2);
+  W.mext = (bf16*)cv.take((size_t)B * ((S + 127) / 128) * 4096);
+  W.att = (bf16*)cv.take((size_t)B * SP * H * 32 * 2);
+  W.bytes = cv.off;
+  return W;
+}
+static int grid_attention_fwd(Ctx* c, const bf16* x, int B, int S, int C, int H, const bf16* w_qkvg, const float* scale,
+                              const float* pair_bias, const float* mask_bias, long long mask_ld, const bf16* w_out, int C_out,
+                              bf16* out, int SP, void* ws, size_t ws_bytes, cudaStream_t st) {
+  if (B <= 0 || S <= 0) return XFOLD_OK;
+  if (SP < S || H % 4) return fail(c, XFOLD_ERR_ARG, "grid attention: SP >= S and a multiple of four heads");
+  const GridWs W = carve_grid(ws, ws_bytes, B, S, SP, H);
+  if (!ws || W.bytes > ws_bytes) return fail(c, XFOLD_ERR_ARG, "grid attention: workspace too small (%zu < %zu)", ws_bytes, W.bytes);
+  const int Wd = H * 32, ldq = pad8(S), mrows = mask_bias && mask_ld > 0 ? B : 1;
+  int rc;
+  // padded rows of the attention's output: zero rows project to zero rows
+  if (SP > S && cudaMemset2DAsync(W.att + (size_t)S * Wd, (size_t)SP * Wd * 2, 0, (size_t)(SP - S) * Wd * 2, B, st) != cudaSuccess)
+    return fail(c, XFOLD_ERR_LAUNCH, "grid attention: memset");
+  if (C == 128 && Wd == 128)
+    rc = launch_row_project_attn(c, x, B, S, 0, nullptr, nullptr, w_qkvg, scale, nullptr, W.qkvg, nullptr, 0, 0, st);
+  else
+    rc = linear_plain(c, x, C, (long long)B * S, C, w_qkvg, 4 * Wd, nullptr, scale, W.qkvg, 4 * Wd, st, 2 * Wd, 3 * Wd, Wd);
+  if (rc) return rc;
+  StaticWeights sw(c);
+  if ((rc = launch_bias_transpose(c, pair_bias, W.biasT, H, S, ldq, st))) return rc;
+  if ((rc = launch_mext(c, mask_bias, mask_ld, W.mext, mrows, S, st, 1))) return rc;
+  if ((rc = launch_attention2(c, W.qkvg, 4 * Wd, S, B, 0, 0, Wd, 2 * Wd, 3 * Wd, H, W.biasT, ldq, W.mext, mrows, W.att, Wd,
+                              (long long)SP * Wd, st, 32))) return rc;
+  if (Wd == 128 && C_out == 128) return launch_row_output(c, W.att, (long long)B * SP, w_out, nullptr, out, st);
+  return linear_plain(c, W.att, Wd, (long long)B * SP, Wd, w_out, C_out, nullptr, nullptr, out, C_out, st);
 }
 
 size_t single_ws_bytes(int N) {
@@ -749,6 +791,17 @@ int xfold_gated_attention_core_fwd(xfold_ctx* c, const void* xn, int B, int S, i
   if (!c) return XFOLD_ERR_ARG;
   return apb_core_fwd(c, (const bf16*)xn, B, S, C, H, Dp, (const bf16*)w_qkvg, qkvg_bias, qkvg_scale, pair_bias, nullptr,
                       mask, (bf16*)out, ws, ws_bytes, (cudaStream_t)stream, mask_ld);
+}
+
+size_t xfold_grid_attention_workspace_bytes(int B, int S, int SP, int H) {
+  return B > 0 && S > 0 ? carve_grid(nullptr, 0, B, S, SP, H).bytes + 1024 : 0;
+}
+int xfold_grid_attention_fwd(xfold_ctx* c, const void* x, int B, int S, int C, int H, const void* w_qkvg, const float* qkvg_scale,
+                             const float* pair_bias, const float* mask_bias, long long mask_ld, const void* w_out, int C_out,
+                             void* out, int SP, void* ws, size_t ws_bytes, void* stream) {
+  if (!c || !x || !w_qkvg || !pair_bias || !w_out || !out) return XFOLD_ERR_ARG;
+  return grid_attention_fwd(c, (const bf16*)x, B, S, C, H, (const bf16*)w_qkvg, qkvg_scale, pair_bias, mask_bias, mask_ld,
+                            (const bf16*)w_out, C_out, (bf16*)out, SP, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 int xfold_pairformer_stack_fwd(xfold_ctx* c, void* z, void* s, const float* pair_mask, const float* seq_mask, int N,

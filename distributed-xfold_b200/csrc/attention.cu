@@ -485,7 +485,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
 // holds 1e9 * (mask[b][k] - 1) for k < S and -1e30 for the padding of the last tile; its other columns are zero.
 // 1e9 * (mask - 1) as in the reference, floored at -60000: any such logit still exponentiates to exactly 0 next to an
 // unmasked one, while a row whose keys are ALL masked keeps fp32-resolvable logits (at 1e9 the fp32 spacing is 64).
-__global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restrict__ out, int B, int S, int KS) {
+// additive: the mask is given as that additive bias.
+__global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restrict__ out, int B, int S, int KS, int additive) {
   pdl_wait();
   pdl_launch();
   const long long n = (long long)B * KS * 64;
@@ -493,19 +494,22 @@ __global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restr
     const long long bb = idx / (KS * 64);
     const int k = int(idx - bb * (KS * 64));
     float v = -1.0e30f;
-    if (k < S) v = mask ? fmaxf(1.0e9f * (mask[bb * mask_ld + k] - 1.f), -60000.f) : 0.f;
+    if (k < S) {
+      v = mask ? mask[bb * mask_ld + k] : additive ? 0.f : 1.f;
+      v = fminf(fmaxf(additive ? v : 1.0e9f * (v - 1.f), -60000.f), additive ? 0.f : 3.0e38f);
+    }
     out[idx] = make_uint4(uint32_t(__bfloat16_as_ushort(__float2bfloat16(v))), 0, 0, 0);
   }
 }
 
-int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st) {
+int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st, int additive) {
   const int KS = (S + 63) / 64;
   const long long n = (long long)B * KS * 64;
   if (n <= 0) return XFOLD_OK;
   long long blocks = (n + 255) / 256;
   if (blocks > 8192) blocks = 8192;
   ProfScope ps(c, XFOLD_K_MASK_BIAS, st);
-  launch_pdl(mext_kernel, (int)blocks, 256, 0, st, mask, mask_ld, reinterpret_cast<uint4*>(out), B, S, KS);
+  launch_pdl(mext_kernel, (int)blocks, 256, 0, st, mask, mask_ld, reinterpret_cast<uint4*>(out), B, S, KS, additive);
   return check_launch(c, "mext_kernel");
 }
 

@@ -28,6 +28,7 @@ namespace xf {
 struct RowProjectArgs {
   const float *gamma, *beta;
   int tiles, parts, static_w;
+  int norm;         // 0: the rows come normalised, nothing is done to them
   long long rows;
   int mode1, dim1;  // mode1: tile rows step along the first token axis, second axis fixed (transposed planes)
   // trimul
@@ -122,7 +123,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int c = l16 * 8 + e * 2 + u;
-          const float w = h < 4 ? p.w_bias[h * 128 + c] : 0.f;
+          const float w = h < 4 && p.w_bias ? p.w_bias[h * 128 + c] : 0.f;
           w2[u] = __bfloat162float(__float2bfloat16(w * (p.gamma ? p.gamma[c] : 1.f)));
           s += w2[u];
           b += (p.beta ? p.beta[c] : 0.f) * w;
@@ -151,7 +152,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   const int part = int(blockIdx.x) % p.parts, u0 = part * UNITS / p.parts, U = (part + 1) * UNITS / p.parts - u0;
   const int t0 = int(blockIdx.x) / p.parts, step = int(gridDim.x) / p.parts;
   const int mine = t0 < p.tiles ? (p.tiles - t0 + step - 1) / step : 0;
-  const bool with_bias = ATTN && part == 0;
+  const bool with_bias = ATTN && part == 0 && p.w_bias;
   auto unit_g = [](int g) { return !ATTN && g % 3 == 2; };
 
   if (warp == 0) {
@@ -242,6 +243,11 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     for (int it = 0; it < mine; ++it) {
       const uint32_t xb = it & 1, xph = (uint32_t(it) >> 1) & 1u;
       mbar_wait(&x_full[xb], xph, ab, XF_ERR_WAIT_FULL);  // (a failed wait runs through: these warps may meet at a barrier)
+      if (!p.norm) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&n_full[xb]);
+        continue;
+      }
       uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
       uint32_t xr[32];
       float2 sm[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -458,6 +464,7 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   }
   ok = ok && make_tmap_bf16_3d(&tmw, w_in, 128, 640, 1, 128, 128 * 640, 64, 64, 1);
   if (!ok) return fail(c, XFOLD_ERR_ARG, "trimul: cannot encode projection tensor maps");
+  a.norm = 1;
   a.gamma = gamma;
   a.beta = beta;
   a.rows = M;
@@ -470,7 +477,8 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   return launch_row_project<false>(c, tmx, tmw, tmo, a, st);
 }
 
-int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* gamma, const float* beta, const bf16* w_qkvg,
+// norm = 0: z is normalised already, and w_bias (then null) has no output
+int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, int norm, const float* gamma, const float* beta, const bf16* w_qkvg,
                             const float* scale, const float* w_bias, bf16* qkvg, bf16* bias, int pitch, long long plane,
                             cudaStream_t st) {
   const long long M = (long long)R * N;
@@ -481,6 +489,7 @@ int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* ga
       !make_tmap_bf16_3d(&tmw, w_qkvg, 128, 512, 1, 128, 128 * 512, 64, 64, 1))
     return fail(c, XFOLD_ERR_ARG, "triattn: cannot encode projection tensor maps");
   a.tiles = (int)((M + 127) / 128);
+  a.norm = norm;
   a.gamma = gamma;
   a.beta = beta;
   a.rows = M;

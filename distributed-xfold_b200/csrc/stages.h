@@ -40,7 +40,7 @@ int launch_ln_rows(Ctx* c, const bf16* x, long long ldx, bf16* y, long long ldy,
                    const float* b, float eps, int H, const float* pw, float* proj, long long plane, const bf16* msc,
                    const bf16* msh, int mod_rows, cudaStream_t st, bf16* proj_bf16 = nullptr, int trav_inner = 0,
                    int trav_outer = 0, int proj_pitch = 0);
-int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st);
+int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st, int additive = 0);
 int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int ldq, cudaStream_t st);
 int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int transposed, int q_col0, int k_col0,
                       int v_col0, int g_col0, int heads, const bf16* biasT, int ldq, const bf16* mext, int mext_rows,
@@ -51,7 +51,7 @@ int launch_transition128(Ctx* c, const bf16* x, bf16* out, long long rows, int F
 int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed, const float* gamma,
                               const float* beta, const bf16* w_in, bf16* out_a, bf16* out_b, bf16* out_g, long long chan_stride,
                               long long row_stride, cudaStream_t st);
-int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, const float* gamma, const float* beta, const bf16* w_qkvg,
+int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, int norm, const float* gamma, const float* beta, const bf16* w_qkvg,
                             const float* scale, const float* w_bias, bf16* qkvg, bf16* bias, int pitch, long long plane,
                             cudaStream_t st);
 // output projections of the pair representation (row_output.cu)

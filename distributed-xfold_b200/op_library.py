@@ -78,7 +78,6 @@ def _mask_from_bias(bias: torch.Tensor, rows: int, s: int) -> torch.Tensor:
 # CUDA implementations
 # ---------------------------------------------------------------------------------------------------------------
 def _grid_self_attn(q_data, bias, nonbatched_bias, query_w, key_w, value_w, gating_w, output_w, key_dim, value_dim):
-    import ctypes as C
     from ._cabi import check, ctx, load
     b, s, c = q_data.shape
     _, h, d = query_w.shape
@@ -98,20 +97,17 @@ def _grid_self_attn(q_data, bias, nonbatched_bias, query_w, key_w, value_w, gati
 
     w_qkvg, scale, w_out = _cached("gsa", (query_w, key_w, value_w, gating_w, output_w), pack)
     x = q_data.to(BF16).contiguous()
-    mask = _mask_from_bias(bias, b, s)
+    bias = bias.float().reshape(-1, s).contiguous()      # additive: 1e9 * (mask - 1), per batch entry or shared
     nb = nonbatched_bias.float().contiguous() if nonbatched_bias.numel() else torch.zeros(h, s, s, device=dev)
     lib = load()
     di = dev.index if dev.index is not None else torch.cuda.current_device()
-    ws = ops._Workspace.get(di, lib.xfold_apb_workspace_bytes(b, s, h, 32))
-    att = torch.empty(b, s, h * 32, dtype=BF16, device=dev)
-    rc = lib.xfold_gated_attention_core_fwd(ctx(di), x.data_ptr(), b, s, c, h, 32, w_qkvg.data_ptr(), None, scale.data_ptr(),
-                                            nb.data_ptr(), mask.data_ptr(), s if mask.shape[0] == b else 0, att.data_ptr(),
-                                            ws.data_ptr(), ws.numel(), torch.cuda.current_stream(di).cuda_stream)
-    check(rc, di, "xfold_gated_attention_core_fwd")
-    out = ops.linear(att, w_out)                                                     # [B, S, c_out]
     sp = _pad_to(s, QKV_BLOCKSIZE)
-    if sp != s:
-        out = torch.nn.functional.pad(out, (0, 0, 0, sp - s))
+    ws = ops._Workspace.get(di, lib.xfold_grid_attention_workspace_bytes(b, s, sp, h))
+    out = torch.empty(b, sp, w_out.shape[0], dtype=BF16, device=dev)
+    rc = lib.xfold_grid_attention_fwd(ctx(di), x.data_ptr(), b, s, c, h, w_qkvg.data_ptr(), scale.data_ptr(), nb.data_ptr(),
+                                      bias.data_ptr(), s if bias.shape[0] >= b else 0, w_out.data_ptr(), w_out.shape[0],
+                                      out.data_ptr(), sp, ws.data_ptr(), ws.numel(), torch.cuda.current_stream(di).cuda_stream)
+    check(rc, di, "xfold_grid_attention_fwd")
     return out.to(q_data.dtype)
 
 

@@ -185,6 +185,14 @@ int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* ctx, const void* xn, 
                                                 const void* prepared_bias, const float* mask, void* out, void* ws,
                                                 size_t ws_bytes, void* stream);
 
+/* The TriangleAttention operator on already normalised rows (csrc/Alpha_Attention.cpp:50-70): x bf16 [B][S][C], w_qkvg bf16
+ * [4 * H * 32][C] (heads padded to 32), qkvg_scale float32 [4 * H * 32] or null, pair_bias float32 [H][S][S], mask_bias the
+ * ADDITIVE mask 1e9 * (mask - 1), float32, row b at mask_bias + b * mask_ld (0: one row for all; null: no mask), w_out bf16
+ * [C_out][H * 32] -> out bf16 [B][SP][C_out], rows S..SP-1 zero. */
+size_t xfold_grid_attention_workspace_bytes(int B, int S, int SP, int H);
+int xfold_grid_attention_fwd(xfold_ctx* ctx, const void* x, int B, int S, int C, int H, const void* w_qkvg,
+                             const float* qkvg_scale, const float* pair_bias, const float* mask_bias, long long mask_ld,
+                             const void* w_out, int C_out, void* out, int SP, void* ws, size_t ws_bytes, void* stream);
 /* All blocks of the DiffusionTransformer (nn/d_diffusion_transformer.py:267-310) for one denoising step of S samples, in
  * place on act bf16 [S][N][C].  The conditioning projections of all blocks are stacked:
  *   w_mod  bf16 [num_blocks * 4C][C_cond]: per block scale, shift (attention), scale, shift (transition), every column

@@ -116,3 +116,21 @@ def test_op_transition(lib, oracle):
     torch.cuda.synchronize()
     ref = oracle.transition({k: rb(v) for k, v in st.items()}, "", rb(x))
     assert tuple(out.shape) == tuple(x.shape) and relf(out.float().cpu(), ref) < 2e-2
+
+
+@pytest.mark.parametrize("b,s,c,h,d,shared", [(2, 64, 128, 4, 32, False), (5, 130, 128, 4, 24, True), (3, 33, 256, 8, 32, False)])
+def test_op_grid_self_attention_shapes(lib, oracle, b, s, c, h, d, shared):
+    """No padding, a mask row shared by the batch with padded heads, and widths beyond the pair representation's."""
+    g = torch.Generator().manual_seed(70 + s)
+    ws = _attn_weights(g, c, h, d, True)
+    x = torch.randn(b, s, c, generator=g)
+    bias = 1e9 * ((torch.rand(1 if shared else b, 1, 1, s, generator=g) > 0.2).float() - 1)
+    nb = torch.randn(h, s, s, generator=g)
+    out = lib.grid_self_attn_forward(x.to(BF).cuda(), bias.cuda(), nb.cuda(), *(ws[n].to(BF).cuda() for n in (
+        "query_w", "key_w", "value_w", "gating_w", "output_w")), d, d)
+    torch.cuda.synchronize()
+    sp = (s + 63) // 64 * 64
+    assert tuple(out.shape) == (b, sp, c) and float(out[:, s:].float().abs().sum()) == 0.0
+    ref = oracle.gated_attention(rb(x), bias, nb, rb(ws["query_w"]), rb(ws["key_w"]), rb(ws["value_w"]), rb(ws["gating_w"]),
+                                 rb(ws["output_w"]))
+    assert relf(out[:, :s].float().cpu(), ref) < 2e-2
