@@ -7,7 +7,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-SOURCES = ["api.cu", "gemm.cu", "simt.cu", "attention.cu", "peer.cu", "sharded.cu", "fp32_validation.cu", "cross_attention.cu", "pair_logits.cu",
+SOURCES = ["api.cu", "gemm.cu", "gemm_split.cu", "simt.cu", "attention.cu", "peer.cu", "sharded.cu", "fp32_validation.cu", "cross_attention.cu", "pair_logits.cu",
            "diffusion.cu", "transition.cu", "row_project.cu",
            "row_output.cu"]
 # the fp32 validation kernels want IEEE division, exact exponentials and denormals: no fast-math for that file

@@ -64,7 +64,7 @@ bool make_tmap_bf16_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d
 // generic linear layers on top of the GEMM kernel
 // ---------------------------------------------------------------------------------------------
 static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M, int K, const bf16* w, int wrows, int ldw,
-                     GemmArgs a, int bn, cudaStream_t st) {
+                     GemmArgs a, int bn, cudaStream_t st, int split = 1) {
   if (M <= 0) return XFOLD_OK;
   if (M >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "linear: too many rows");
   if ((K & 7) || (ldx & 7) || (ldw & 7)) return fail(c, XFOLD_ERR_ARG, "linear: K and leading dimensions must be multiples of 8");
@@ -78,7 +78,7 @@ static int gemm_rows(Ctx* c, int epi, const bf16* x, long long ldx, long long M,
   a.batches = 1;
   a.tiles_m = (int)((M + 127) / 128);
   a.status = c->d_status;
-  return launch_gemm(c, epi, bn, tA, tB, a, st);
+  return split > 1 ? launch_gemm_split(c, split, tA, tB, a, st) : launch_gemm(c, epi, bn, tA, tB, a, st);
 }
 
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
@@ -103,7 +103,11 @@ int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, 
                              const bf16* gate, long long ldg, int row_gate_mod, const bf16* resid, long long ldr,
                              bf16* out, long long ldo, cudaStream_t st) {
   GemmArgs a;
-  const int bn = gemm_tile_n(c, M, N, K, 1, 128, 64);
+  // the split kernel's epilogue reads and writes 16-byte pieces
+  const uintptr_t ptrs = (uintptr_t)out | (uintptr_t)resid | (uintptr_t)gate;
+  const long long lds = N | ldo | (resid ? ldr : 0) | (gate ? ldg : 0);
+  const int split = (ptrs & 15) || (lds & 7) ? 1 : gemm_split(c, M, N, K);
+  const int bn = split > 1 ? 64 : gemm_tile_n(c, M, N, K, 1, 128, 64);
   a.static_b = c->static_weights;
   a.N = N;
   a.tiles_n = (N + bn - 1) / bn;
@@ -114,7 +118,7 @@ int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, 
   a.ldg = ldg;
   a.resid = resid;
   a.ldr = ldr;
-  return gemm_rows(c, EPI_GATE_RESID, x, ldx, M, K, w, N, K, a, bn, st);
+  return gemm_rows(c, EPI_GATE_RESID, x, ldx, M, K, w, N, K, a, bn, st, split);
 }
 
 // The gated / residual projection in row chunks, with the caller's hook after each chunk's launch (see ChunkHook).

@@ -96,6 +96,26 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// The same with clusters of `cluster` CTAs.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), int grid, int cluster, int block, size_t smem, cudaStream_t st,
+                               Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 // ---- tensor maps --------------------------------------------------------------------------
 // bf16 tensor of rank 3, innermost stride 1; s1/s2 are strides of dims 1/2 in ELEMENTS.
 // 128-byte swizzle (64-byte for boxes whose rows are 64 bytes, 0 for none), zero fill outside the extents.
@@ -131,6 +151,10 @@ struct GemmArgs {
 // 256 (GATE_RESID up to 128, SWIGLU from 128).
 int launch_gemm(Ctx* c, int epi, int bn, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a,
                 cudaStream_t st);
+// GATE_RESID products of few tiles and a long K: `split` (2, 4, 8) CTAs share a tile 64 columns wide and add their parts of
+// K (gemm_split.cu).  N a multiple of 8, pointers of the epilogue 16-byte aligned, leading dimensions multiples of 8.
+int launch_gemm_split(Ctx* c, int split, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, cudaStream_t st);
+int gemm_split(const Ctx* c, long long M, int N, int K);
 // the tile width BN to use for an [M x N x K] product (see gemm.cu)
 int gemm_tile_n(const Ctx* c, long long M, int N, int K, int batches, int widest, int narrowest);
 
