@@ -96,6 +96,21 @@ def test_linear_gate_residual(ops, M, K, N):
     assert relf(y.float().cpu(), ref) < 4e-3
 
 
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 77, 128, 129, 300, 640])  # 8, 8, .. 8, 4, 2 and 1 CTAs to a tile
+@pytest.mark.parametrize("K,N", [(1024, 768), (1544, 392), (256, 72)])
+def test_linear_gate_residual_split_k(ops, M, K, N):
+    x, w, resid = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(M, N, seed=4)
+    mod = max(1, M // 3)
+    gate = rnd(mod, N, seed=8)
+    y = ops.linear_gate_residual(x.cuda(), w.cuda(), gate.cuda(), resid.cuda(), row_gate_mod=mod)
+    ops.synchronize_and_check()
+    ref = resid.float() + (x.float() @ w.float().T) * torch.sigmoid(gate.float()[torch.arange(M) % mod])
+    assert relf(y.float().cpu(), ref) < 4e-3
+    inplace = resid.cuda()
+    y = ops.linear_gate_residual(x.cuda(), w.cuda(), None, inplace, out=inplace)
+    assert relf(y.float().cpu(), resid.float() + x.float() @ w.float().T) < 4e-3
+
+
 @pytest.mark.parametrize("M,K,F", [(900, 128, 512), (260, 384, 1536), (100, 768, 1536)])
 def test_linear_swiglu(ops, M, K, F):
     x, w1 = rnd(M, K, seed=1), rnd(2 * F, K, seed=2, scale=K ** -0.5)
