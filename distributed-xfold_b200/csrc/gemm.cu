@@ -1,7 +1,7 @@
 // Persistent, warp-specialised bf16 GEMM  D[m][n] = sum_k A[m][k] * B[n][k]  for sm_100a.
 //
 //   warp 0      : TMA producer (one elected lane), 128-byte-swizzled K-major tiles, STAGES-deep ring
-//   warp 1      : tcgen05.mma issuer (one elected lane); owns the TMEM allocation (2 accumulators)
+//   warp 1      : tcgen05.mma issuer (one lane elected inside the instructions); owns the TMEM allocation (2 accumulators)
 //   warps 2..9  : epilogue; two warps share each 32-lane quarter of the 128-row accumulator (one per
 //                 half of the columns) and drain it with tcgen05.ld while the MMA warp already fills
 //                 the other buffer.  Row-major outputs leave through 128-byte-swizzled staging tiles
@@ -76,7 +76,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(eempty + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __reduce_max_sync(0xffffffffu, threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const AbortCtx ab{cta_abort, p.status};
 
@@ -103,7 +103,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __reduce_max_sync(0xffffffffu, *tmem_slot);
 
   const int KB = (p.K + BK - 1) / BK;
   const long long total = (long long)p.batches * p.tiles_m * p.tiles_n;
@@ -181,32 +181,33 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp == 1) {
     pdl_wait();
     pdl_launch();
-    if (lane == 0) {
-      // MN-major operands (rows of the smem tile are K indices): 64-element chunks along M / N are 8 KB apart, a step of
-      // 16 along K is 16 rows of 128 B
-      const uint32_t idesc = p.mn_major ? make_idesc(BM, BN, 1, 1) : make_idesc(BM, BN);
-      const uint32_t lbo = p.mn_major ? 8192u : 16u, kstep = p.mn_major ? 128u : 2u;
-      uint32_t stage = 0, phase = 0, it = 0;
-      bool okay = true;
-      for (long long t = blockIdx.x; t < total && okay; t += gridDim.x, ++it) {
-        const uint32_t buf = it & 1u, aphase = (it >> 1) & 1u;
-        if (!mbar_wait(&tempty[buf], aphase ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) break;
+    // Warp-uniform throughout: votes instead of per-lane branches, one elected lane predicated inside each instruction, so
+    // that descriptors and addresses stay in uniform registers.
+    // MN-major operands (rows of the smem tile are K indices): 64-element chunks along M / N are 8 KB apart, a step of
+    // 16 along K is 16 rows of 128 B
+    const uint32_t go = elect_one();
+    const uint32_t idesc = p.mn_major ? make_idesc(BM, BN, 1, 1) : make_idesc(BM, BN);
+    const uint32_t lbo = p.mn_major ? 8192u : 16u, kstep = p.mn_major ? 128u : 2u;
+    uint32_t stage = 0, phase = 0, it = 0;
+    bool okay = true;
+    for (long long t = blockIdx.x; t < total && okay; t += gridDim.x, ++it) {
+      const uint32_t buf = it & 1u, aphase = (it >> 1) & 1u;
+      if (!mbar_wait_warp(&tempty[buf], aphase ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + buf * BN;
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp(&full[stage], phase, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem_base + buf * BN;
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&full[stage], phase, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-          const uint64_t ad = make_sdesc(sA, lbo, 1024);
-          const uint64_t bd = make_sdesc(sA + Cfg::A_BYTES, lbo, 1024);
+        const uint32_t sA = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+        const uint64_t ad = make_sdesc(sA, lbo, 1024);
+        const uint64_t bd = make_sdesc(sA + Cfg::A_BYTES, lbo, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)  // K-major: 16 bf16 = 32 B along K inside the swizzled row
-            umma_ss(d, ad + kstep * k, bd + kstep * k, idesc, (kb | k) ? 1u : 0u);
-          umma_commit(&empty[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
-        if (okay) umma_commit(&tfull[buf]);
+        for (int k = 0; k < BK / 16; ++k)  // K-major: 16 bf16 = 32 B along K inside the swizzled row
+          umma_ss_if(go, d, ad + kstep * k, bd + kstep * k, idesc, (kb | k) ? 1u : 0u);
+        umma_commit_if(go, &empty[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (okay) umma_commit_if(go, &tfull[buf]);
     }
   } else {
     pdl_wait();
@@ -236,6 +237,12 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if constexpr (EPI == EPI_GATE_RESID)
         if (row_gate_vec) fetch_row_gate(0);
+      // column vectors: their lines, so that the epilogue does not begin with a trip to L2 or HBM
+      if constexpr (EPI == EPI_PLAIN)
+        if (lane < BN / 32 && tn * BN + lane * 32 < p.N) {
+          if (p.col_bias) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col_bias + tn * BN + lane * 32));
+          if (p.col_scale) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col_scale + tn * BN + lane * 32));
+        }
       if (!mbar_wait(&tfull[buf], aphase, ab, XF_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(q * 32) << 16);
@@ -277,13 +284,26 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
         }
         if constexpr (EPI == EPI_PLAIN) {
-          if (p.col_bias) {
+          // column vectors: one address for the whole warp, four columns per load where they are whole
+          const bool vec = colw + 32 <= n_out && !((reinterpret_cast<uintptr_t>(p.col_bias) | reinterpret_cast<uintptr_t>(p.col_scale)) & 15);
+          if (vec) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] += (colw + e < n_out) ? p.col_bias[colw + e] : 0.f;
-          }
-          if (p.col_scale) {
+            for (int e = 0; e < 8; ++e) {
+              if (p.col_bias) {
+                const float4 f = reinterpret_cast<const float4*>(p.col_bias + colw)[e];
+                v[4 * e] += f.x; v[4 * e + 1] += f.y; v[4 * e + 2] += f.z; v[4 * e + 3] += f.w;
+              }
+              if (p.col_scale) {
+                const float4 f = reinterpret_cast<const float4*>(p.col_scale + colw)[e];
+                v[4 * e] *= f.x; v[4 * e + 1] *= f.y; v[4 * e + 2] *= f.z; v[4 * e + 3] *= f.w;
+              }
+            }
+          } else {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
+            for (int e = 0; e < 32; ++e) {
+              if (p.col_bias) v[e] += (colw + e < n_out) ? p.col_bias[colw + e] : 0.f;
+              if (p.col_scale) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
+            }
           }
         }
         if constexpr (EPI == EPI_PLAIN) {
