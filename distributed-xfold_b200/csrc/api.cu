@@ -96,7 +96,8 @@ int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const
   a.f16_col0 = f16_col0;
   a.f16_col1 = f16_col1;
   a.log2e_cols = log2e_cols;
-  return gemm_rows(c, EPI_PLAIN, x, ldx, M, K, w, N, K, a, bn, st);
+  const bool cols = bias || scale || f16_col1 > f16_col0 || log2e_cols > 0;
+  return gemm_rows(c, cols ? EPI_COLS : EPI_PLAIN, x, ldx, M, K, w, N, K, a, bn, st);
 }
 
 int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N,

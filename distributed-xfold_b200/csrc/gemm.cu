@@ -4,7 +4,7 @@
 //   warp 1      : tcgen05.mma issuer (one lane elected inside the instructions); owns the TMEM allocation (2 accumulators)
 //   warps 2..9  : epilogue; two warps share each 32-lane quarter of the 128-row accumulator (one per
 //                 half of the columns) and drain it with tcgen05.ld while the MMA warp already fills
-//                 the other buffer.  Row-major outputs leave through 128-byte-swizzled staging tiles
+//                 the other buffer.  Row-major outputs leave through each warp's own staging tiles
 //                 and TMA stores; residual and gate tiles of the 128-wide configuration come in by TMA.
 //
 // The output projections, the single representation's and the diffusion transformer's projections and the per-channel
@@ -26,7 +26,8 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int GEMM_THREADS = 320;  // TMA warp, MMA warp, 8 epilogue warps
 
-constexpr uint32_t EPI_TILE = 128 * 64 * 2;  // one staged [128 rows][64 columns] bf16 chunk, 128-byte swizzled
+constexpr uint32_t EPI_TILE = 128 * 64 * 2;  // a residual / gate chunk: [128 rows][64 columns] bf16, 128-byte swizzled
+constexpr uint32_t OUT_TILE = 32 * 32 * 2;   // a warp's part of an output chunk: [32 rows][32 columns] bf16, 64-byte swizzled
 
 template <int BN>
 struct GemmCfg {
@@ -34,9 +35,9 @@ struct GemmCfg {
   static constexpr uint32_t A_BYTES = BM * BK * 2;
   static constexpr uint32_t B_BYTES = BN * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  // after the operand ring: 2 output chunks; with 128- and 64-wide tiles also 2 residual and 2 gate chunks
+  // after the operand ring: 2 output parts for each of 8 warps; with 128- and 64-wide tiles also 2 residual and 2 gate chunks
   static constexpr uint32_t OFF_OUT = STAGES * STAGE_BYTES;
-  static constexpr uint32_t OFF_RES = OFF_OUT + 2 * EPI_TILE;
+  static constexpr uint32_t OFF_RES = OFF_OUT + 8 * 2 * OUT_TILE;
   static constexpr uint32_t OFF_GATE = OFF_RES + 2 * EPI_TILE;
   static constexpr uint32_t OFF_BAR = (BN <= 128) ? OFF_GATE + 2 * EPI_TILE : OFF_RES;
   static constexpr uint32_t SMEM_BYTES = OFF_BAR + 256 /*barriers*/ + 1024 /*align slack*/;
@@ -237,35 +238,34 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if constexpr (EPI == EPI_GATE_RESID)
         if (row_gate_vec) fetch_row_gate(0);
-      // column vectors: their lines, so that the epilogue does not begin with a trip to L2 or HBM
-      if constexpr (EPI == EPI_PLAIN)
-        if (lane < BN / 32 && tn * BN + lane * 32 < p.N) {
-          if (p.col_bias) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col_bias + tn * BN + lane * 32));
-          if (p.col_scale) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col_scale + tn * BN + lane * 32));
-        }
       if (!mbar_wait(&tfull[buf], aphase, ab, XF_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(q * 32) << 16);
 
       // Staged epilogue: the tile leaves in 64-column chunks.  Each of the 8 warps converts its 32 rows x 32
-      // columns of the chunk into a 128-byte-swizzled shared-memory tile (conflict-free 16-byte stores), then
-      // one thread hands the tile to TMA.  Residual / gate chunks arrive the same way in the other direction.
+      // columns of the chunk into a 64-byte-swizzled shared-memory tile of its own (conflict-free 16-byte stores) and
+      // hands it to TMA, without waiting for the other warps.  Residual / gate chunks arrive by TMA as [128][64] tiles.
       constexpr int NCH = (EPI == EPI_SWIGLU) ? BN / 128 : BN / 64;  // output chunks per tile
       constexpr int WOUT = (EPI == EPI_SWIGLU) ? BN / 2 : BN;        // output columns per tile
       const int n_out = (EPI == EPI_SWIGLU) ? p.N / 2 : p.N;
       const long long m = (long long)tm * BM + row;
       const uint32_t rsw = uint32_t(row & 7);
-      const bool elected = (warp == 2 && lane == 0);
-      // Chunks beyond the output's last column are left out.  (They must not pass through the staging buffers without a
-      // store of their own either: the wait below counts committed stores, and a chunk that commits none would let the
-      // one after it overwrite a tile that is still being read.)
+      // Chunks beyond the output's last column are left out.  (A part that passes through the staging buffers commits a
+      // group even if it stores nothing: the wait below counts groups, and a part without one would let the next
+      // overwrite a tile that is still being read.)
       const int nch = min(NCH, (n_out - tn * WOUT + 63) / 64);
 #pragma unroll 1
       for (int c = 0; c < nch; ++c, ++ochunk) {
         const int col0 = tn * WOUT + c * 64;          // first output column of the chunk
         const int colw = col0 + ch * 32;              // first output column of this warp
-        uint8_t* so = smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE + row * 128;
+        uint8_t* so = smem + Cfg::OFF_OUT + ((warp - 2) * 2 + (ochunk & 1u)) * OUT_TILE;
         float v[32];
+        float cb = 0.f, cs = 1.f;  // this lane's element of the column vectors
+        if constexpr (EPI == EPI_COLS) {
+          if (p.col_bias && colw + lane < n_out) cb = p.col_bias[colw + lane];
+          if (p.col_scale && colw + lane < n_out) cs = p.col_scale[colw + lane];
+          if (colw < p.log2e_cols) cs *= 1.4426950408889634f;
+        }
         if constexpr (EPI == EPI_SWIGLU) {
           uint32_t ra[32], rb[32];
           tmem_ld32(taddr + c * 64 + ch * 32, ra);
@@ -282,35 +282,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tmem_ld_wait();
 #pragma unroll
           for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
-        }
-        if constexpr (EPI == EPI_PLAIN) {
-          // column vectors: one address for the whole warp, four columns per load where they are whole
-          const bool vec = colw + 32 <= n_out && !((reinterpret_cast<uintptr_t>(p.col_bias) | reinterpret_cast<uintptr_t>(p.col_scale)) & 15);
-          if (vec) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              if (p.col_bias) {
-                const float4 f = reinterpret_cast<const float4*>(p.col_bias + colw)[e];
-                v[4 * e] += f.x; v[4 * e + 1] += f.y; v[4 * e + 2] += f.z; v[4 * e + 3] += f.w;
-              }
-              if (p.col_scale) {
-                const float4 f = reinterpret_cast<const float4*>(p.col_scale + colw)[e];
-                v[4 * e] *= f.x; v[4 * e + 1] *= f.y; v[4 * e + 2] *= f.z; v[4 * e + 3] *= f.w;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              if (p.col_bias) v[e] += (colw + e < n_out) ? p.col_bias[colw + e] : 0.f;
-              if (p.col_scale) v[e] *= (colw + e < n_out) ? p.col_scale[colw + e] : 0.f;
-            }
-          }
-        }
-        if constexpr (EPI == EPI_PLAIN) {
-          if (colw < p.log2e_cols) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] *= 1.4426950408889634f;
-          }
         }
         if constexpr (EPI == EPI_GATE_RESID) {
           // order: v * sigmoid(gate) first, residual added last
@@ -403,10 +374,28 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         // the TMA store that last used this staging buffer (two chunks ago) must have read it out
-        if (elected) tma_store_wait_read<1>();
-        named_bar_sync(1, 256);
+        if (lane == 0) tma_store_wait_read<1>();
+        __syncwarp();
+        if constexpr (EPI == EPI_COLS) {
+          // Every row needs all 32 elements of the column vectors: they pass through the free staging buffer.  (Loaded by
+          // every thread from global memory they cost 1.3 us more in a launch of 128 tiles, and the code for columns that do
+          // not come in fours cost instruction fetches.)
+          float* sv = reinterpret_cast<float*>(so);
+          sv[lane] = cb;
+          sv[32 + lane] = cs;
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float4 fb = reinterpret_cast<const float4*>(sv)[e], fs = reinterpret_cast<const float4*>(sv)[8 + e];
+            v[4 * e] = (v[4 * e] + fb.x) * fs.x;
+            v[4 * e + 1] = (v[4 * e + 1] + fb.y) * fs.y;
+            v[4 * e + 2] = (v[4 * e + 2] + fb.z) * fs.z;
+            v[4 * e + 3] = (v[4 * e + 3] + fb.w) * fs.w;
+          }
+          __syncwarp();
+        }
         bool as_f16 = false;
-        if constexpr (EPI == EPI_PLAIN) as_f16 = colw >= p.f16_col0 && colw < p.f16_col1;
+        if constexpr (EPI == EPI_COLS) as_f16 = colw >= p.f16_col0 && colw < p.f16_col1;
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           uint4 u;
@@ -421,20 +410,20 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             u.z = pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]);
             u.w = pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]);
           }
-          *reinterpret_cast<uint4*>(so + ((uint32_t(ch * 4 + g) ^ rsw) << 4)) = u;
+          *reinterpret_cast<uint4*>(so + lane * 64 + ((uint32_t(g) ^ uint32_t((lane >> 1) & 3)) << 4)) = u;
         }
         fence_proxy_async_smem();
-        named_bar_sync(2, 256);
-        if (elected) {
-          tma_store_3d(&tmO, smem + Cfg::OFF_OUT + (ochunk & 1u) * EPI_TILE, col0, tm * BM, b);
-          tma_store_commit();
+        __syncwarp();
+        if (lane == 0) {
+          if (colw < n_out && tm * BM + q * 32 < p.M) tma_store_3d(&tmO, so, colw, tm * BM + q * 32, b);
+          tma_store_commit();  // an empty group counts too: the wait above is by number
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
     }
-    if (warp == 2 && lane == 0) tma_store_wait_all();  // written, not only read out: the next kernel may be waiting already
+    if (lane == 0) tma_store_wait_all();  // written, not only read out: the next kernel may be waiting already
   }
 
   tc_fence_before();
@@ -466,7 +455,7 @@ static int launch_one(Ctx* c, const CUtensorMap& tmA, const CUtensorMap& tmB, co
   CUtensorMap tmO = tmA, tmR = tmA, tmG = tmA;  // placeholders when unused
   const int n_out = (EPI == EPI_SWIGLU) ? a.N / 2 : a.N;
   const uint64_t bstride = a.batches > 1 ? (uint64_t)a.out_batch_stride : (uint64_t)a.ldo * (uint64_t)a.M;
-  if (!make_tmap_bf16_3d(&tmO, a.out, n_out, a.M, a.batches, a.ldo, bstride, 64, 128, 1))
+  if (!make_tmap_bf16_3d(&tmO, a.out, n_out, a.M, a.batches, a.ldo, bstride, 32, 32, 1, 64))
     return fail(c, XFOLD_ERR_ARG, "gemm: cannot encode the output tensor map (16-byte aligned base, ld multiple of 8?)");
   if (EPI == EPI_GATE_RESID) {
     if (a.resid && !make_tmap_bf16_3d(&tmR, a.resid, a.N, a.M, 1, a.ldr, (uint64_t)a.ldr * a.M, 64, 128, 1))
@@ -490,6 +479,9 @@ int launch_gemm(Ctx* c, int epi, int bn, const CUtensorMap& tmA, const CUtensorM
     case EPI_PLAIN * 1000 + 256: return launch_one<256, EPI_PLAIN>(c, tmA, tmB, a, st);
     case EPI_PLAIN * 1000 + 128: return launch_one<128, EPI_PLAIN>(c, tmA, tmB, a, st);
     case EPI_PLAIN * 1000 + 64: return launch_one<64, EPI_PLAIN>(c, tmA, tmB, a, st);
+    case EPI_COLS * 1000 + 256: return launch_one<256, EPI_COLS>(c, tmA, tmB, a, st);
+    case EPI_COLS * 1000 + 128: return launch_one<128, EPI_COLS>(c, tmA, tmB, a, st);
+    case EPI_COLS * 1000 + 64: return launch_one<64, EPI_COLS>(c, tmA, tmB, a, st);
     case EPI_GATE_RESID * 1000 + 128: return launch_one<128, EPI_GATE_RESID>(c, tmA, tmB, a, st);
     case EPI_GATE_RESID * 1000 + 64: return launch_one<64, EPI_GATE_RESID>(c, tmA, tmB, a, st);
     case EPI_SWIGLU * 1000 + 256: return launch_one<256, EPI_SWIGLU>(c, tmA, tmB, a, st);

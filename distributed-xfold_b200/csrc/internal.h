@@ -123,7 +123,9 @@ bool make_tmap_bf16_3d(CUtensorMap* m, const void* base, uint64_t d0, uint64_t d
                        uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, int swizzle_bytes = 128);
 
 // ---- GEMM ---------------------------------------------------------------------------------
-enum GemmEpi : int { EPI_PLAIN = 0, EPI_GATE_RESID = 1, EPI_SWIGLU = 2 };
+// COLS: PLAIN with column vectors or columns that leave in another form.  A kernel of its own: what PLAIN does not need would
+// cost it instruction fetches (contraction of 37 tokens 4.0 -> 3.5 us).
+enum GemmEpi : int { EPI_PLAIN = 0, EPI_GATE_RESID = 1, EPI_SWIGLU = 2, EPI_COLS = 3 };
 
 struct GemmArgs {
   int M = 0, N = 0, K = 0, batches = 1;
@@ -131,13 +133,13 @@ struct GemmArgs {
   int b_batched = 0;
   int static_b = 0;    // B is written by no kernel that may still run: its first tiles may be fetched before pdl_wait
   int mn_major = 0;    // operands are stored [k][m] and [k][n] (tensor maps: inner dim = m / n, boxes of 64 x 64)
-  // PLAIN / SWIGLU / GATE_RESID output
+  // output (row-major, all epilogues)
   bf16* out = nullptr;
   long long ldo = 0, out_batch_stride = 0;
-  const float* col_bias = nullptr;
+  const float* col_bias = nullptr;  // COLS: (product + col_bias) * col_scale
   const float* col_scale = nullptr;
-  int f16_col0 = 0, f16_col1 = 0;  // PLAIN: output columns [f16_col0, f16_col1) are stored as fp16 (multiples of 32)
-  int log2e_cols = 0;  // PLAIN: output columns [0, log2e_cols) times log2(e) (a multiple of 32): the attention works in base 2
+  int f16_col0 = 0, f16_col1 = 0;  // COLS: output columns [f16_col0, f16_col1) are stored as fp16 (multiples of 32)
+  int log2e_cols = 0;  // COLS: output columns [0, log2e_cols) times log2(e) (a multiple of 32): the attention works in base 2
   const bf16* resid = nullptr;
   long long ldr = 0;
   const bf16* gate = nullptr;
