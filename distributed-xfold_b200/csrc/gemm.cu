@@ -1,6 +1,6 @@
 // Persistent, warp-specialised bf16 GEMM  D[m][n] = sum_k A[m][k] * B[n][k]  for sm_100a.
 //
-//   warp 0      : TMA producer (one elected lane), 128-byte-swizzled K-major tiles, STAGES-deep ring
+//   warp 0      : TMA producer (one lane elected inside the instructions), 128-byte-swizzled K-major tiles, STAGES-deep ring
 //   warp 1      : tcgen05.mma issuer (one lane elected inside the instructions); owns the TMEM allocation (2 accumulators)
 //   warps 2..9  : epilogue; two warps share each 32-lane quarter of the 128-row accumulator (one per
 //                 half of the columns) and drain it with tcgen05.ld while the MMA warp already fills
@@ -42,16 +42,6 @@ struct GemmCfg {
   static constexpr uint32_t OFF_BAR = (BN <= 128) ? OFF_GATE + 2 * EPI_TILE : OFF_RES;
   static constexpr uint32_t SMEM_BYTES = OFF_BAR + 256 /*barriers*/ + 1024 /*align slack*/;
 };
-
-__device__ __forceinline__ void load8_bf16(const bf16* src, float* v, int nvalid, bool vec_ok) {
-  if (nvalid >= 8 && vec_ok) {
-    const uint4 u = *reinterpret_cast<const uint4*>(src);
-    v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
-    v[4] = bf16_lo(u.z); v[5] = bf16_hi(u.z); v[6] = bf16_lo(u.w); v[7] = bf16_hi(u.w);
-  } else {
-    for (int e = 0; e < 8; ++e) v[e] = (e < nvalid) ? __bfloat162float(src[e]) : 0.f;
-  }
-}
 
 template <int BN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -110,75 +100,73 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const long long total = (long long)p.batches * p.tiles_m * p.tiles_n;
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, echunk = 0;
-      bool okay = true;
-      (void)echunk;
-      auto load_b = [&](uint8_t* sB, uint64_t* bar, int kb, int tn, int bb) {
-        if constexpr (B_SPLIT) {
-          const int r0 = tn * (BN / 2) / 128 * 256 + tn * (BN / 2) % 128;
-          tma_load_3d(sB, &tmB, bar, kb * BK, r0, bb);
-          tma_load_3d(sB + Cfg::B_BYTES / 2, &tmB, bar, kb * BK, r0 + 128, bb);
-        } else {
-          tma_load_3d(sB, &tmB, bar, kb * BK, tn * BN, bb);
-        }
-      };
-      // Weights that no kernel of this call writes are fetched before the wait for the previous kernel: with a few rows
-      // of activations the launch is a latency chain and the weights' trip from HBM is the longest link of it.
-      int pre = 0;
-      if (p.static_b && (long long)blockIdx.x < total)
-        for (; pre < STAGES && pre < KB; ++pre) {
-          mbar_arrive_expect_tx(&full[pre], Cfg::STAGE_BYTES);
-          load_b(smem + pre * Cfg::STAGE_BYTES + Cfg::A_BYTES, &full[pre], pre, int(blockIdx.x % p.tiles_n), 0);
-        }
-      pdl_wait();
-      pdl_launch();
-      for (long long t = blockIdx.x; t < total && okay; t += gridDim.x) {
-        const int tn = int(t % p.tiles_n);
-        const int tm = int((t / p.tiles_n) % p.tiles_m);
-        const int b = int(t / ((long long)p.tiles_n * p.tiles_m));
-        const int a1 = tm * BM, a2 = b;
-        const int bb = p.b_batched ? b : 0;
-        if constexpr (EPI_LOADS) {
-          const uint32_t nload = (p.resid ? 1u : 0u) + (p.gate ? 1u : 0u);
-          if (nload) {
-            for (int c = 0; c < BN / 64 && tn * BN + c * 64 < p.N && okay; ++c, ++echunk) {
-              const uint32_t eb = echunk & 1u;
-              if (!mbar_wait(&eempty[eb], ((echunk >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
-              mbar_arrive_expect_tx(&efull[eb], nload * EPI_TILE);
-              if (p.resid) tma_load_3d(smem + Cfg::OFF_RES + eb * EPI_TILE, &tmR, &efull[eb], tn * BN + c * 64, tm * BM, 0);
-              if (p.gate) tma_load_3d(smem + Cfg::OFF_GATE + eb * EPI_TILE, &tmG, &efull[eb], tn * BN + c * 64, tm * BM, 0);
-            }
-            if (!okay) break;
-          }
-        }
-        for (int kb = 0; kb < KB; ++kb) {
-          uint8_t* sA = smem + stage * Cfg::STAGE_BYTES;
-          if (pre > 0) {  // the first tile's first stages: announced, and B on its way
-            --pre;
-            tma_load_3d(sA, &tmA, &full[stage], kb * BK, a1, a2);
-            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-            continue;
-          }
-          if (!mbar_wait(&empty[stage], phase ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
-          mbar_arrive_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          if (!p.mn_major) {
-            tma_load_3d(sA, &tmA, &full[stage], kb * BK, a1, a2);
-            load_b(sA + Cfg::A_BYTES, &full[stage], kb, tn, bb);
-          } else {
-            // operands stored [k][m] / [k][n]: one [64 k][64 m] box (8 KB, 128-byte rows) per 64 rows of the tile
-#pragma unroll
-            for (int x = 0; x < BM / 64; ++x) tma_load_3d(sA + x * 8192, &tmA, &full[stage], a1 + x * 64, kb * BK, a2);
-#pragma unroll
-            for (int x = 0; x < BN / 64; ++x)
-              tma_load_3d(sA + Cfg::A_BYTES + x * 8192, &tmB, &full[stage], tn * BN + x * 64, kb * BK, bb);
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
+    // warp-uniform, like the issuer below
+    const uint32_t go = elect_one();
+    uint32_t stage = 0, phase = 0, echunk = 0;
+    bool okay = true;
+    (void)echunk;
+    auto load_b = [&](uint8_t* sB, uint64_t* bar, int kb, int tn, int bb) {
+      if constexpr (B_SPLIT) {
+        const int r0 = tn * (BN / 2) / 128 * 256 + tn * (BN / 2) % 128;
+        tma_load_3d_if(go, sB, &tmB, bar, kb * BK, r0, bb);
+        tma_load_3d_if(go, sB + Cfg::B_BYTES / 2, &tmB, bar, kb * BK, r0 + 128, bb);
+      } else {
+        tma_load_3d_if(go, sB, &tmB, bar, kb * BK, tn * BN, bb);
       }
-    }
+    };
+    // Weights that no kernel of this call writes are fetched before the wait for the previous kernel: with a few rows
+    // of activations the launch is a latency chain and the weights' trip from HBM is the longest link of it.
+    int pre = 0;
+    if (p.static_b && (long long)blockIdx.x < total)
+      for (; pre < STAGES && pre < KB; ++pre) {
+        mbar_arrive_expect_tx_if(go, &full[pre], Cfg::STAGE_BYTES);
+        load_b(smem + pre * Cfg::STAGE_BYTES + Cfg::A_BYTES, &full[pre], pre, int(blockIdx.x % p.tiles_n), 0);
+      }
     pdl_wait();
     pdl_launch();
+    for (long long t = blockIdx.x; t < total && okay; t += gridDim.x) {
+      const int tn = int(t % p.tiles_n);
+      const int tm = int((t / p.tiles_n) % p.tiles_m);
+      const int b = int(t / ((long long)p.tiles_n * p.tiles_m));
+      const int a1 = tm * BM, a2 = b;
+      const int bb = p.b_batched ? b : 0;
+      if constexpr (EPI_LOADS) {
+        const uint32_t nload = (p.resid ? 1u : 0u) + (p.gate ? 1u : 0u);
+        if (nload) {
+          for (int c = 0; c < BN / 64 && tn * BN + c * 64 < p.N && okay; ++c, ++echunk) {
+            const uint32_t eb = echunk & 1u;
+            if (!mbar_wait_warp(&eempty[eb], ((echunk >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
+            mbar_arrive_expect_tx_if(go, &efull[eb], nload * EPI_TILE);
+            if (p.resid) tma_load_3d_if(go, smem + Cfg::OFF_RES + eb * EPI_TILE, &tmR, &efull[eb], tn * BN + c * 64, tm * BM, 0);
+            if (p.gate) tma_load_3d_if(go, smem + Cfg::OFF_GATE + eb * EPI_TILE, &tmG, &efull[eb], tn * BN + c * 64, tm * BM, 0);
+          }
+          if (!okay) break;
+        }
+      }
+      for (int kb = 0; kb < KB; ++kb) {
+        uint8_t* sA = smem + stage * Cfg::STAGE_BYTES;
+        if (pre > 0) {  // the first tile's first stages: announced, and B on its way
+          --pre;
+          tma_load_3d_if(go, sA, &tmA, &full[stage], kb * BK, a1, a2);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          continue;
+        }
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
+        mbar_arrive_expect_tx_if(go, &full[stage], Cfg::STAGE_BYTES);
+        if (!p.mn_major) {
+          tma_load_3d_if(go, sA, &tmA, &full[stage], kb * BK, a1, a2);
+          load_b(sA + Cfg::A_BYTES, &full[stage], kb, tn, bb);
+        } else {
+          // operands stored [k][m] / [k][n]: one [64 k][64 m] box (8 KB, 128-byte rows) per 64 rows of the tile
+#pragma unroll
+          for (int x = 0; x < BM / 64; ++x) tma_load_3d_if(go, sA + x * 8192, &tmA, &full[stage], a1 + x * 64, kb * BK, a2);
+#pragma unroll
+          for (int x = 0; x < BN / 64; ++x)
+            tma_load_3d_if(go, sA + Cfg::A_BYTES + x * 8192, &tmB, &full[stage], tn * BN + x * 64, kb * BK, bb);
+        }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
   } else if (warp == 1) {
     pdl_wait();
     pdl_launch();
@@ -285,86 +273,44 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         if constexpr (EPI == EPI_GATE_RESID) {
           // order: v * sigmoid(gate) first, residual added last
-          const bool rvalid = m < p.M;
-          bool staged = false;
-          uint32_t eb = 0;
-          if constexpr (EPI_LOADS) {
-            if (p.resid || p.gate) {
-              staged = true;
-              eb = echunk & 1u;
-              if (!mbar_wait(&efull[eb], (echunk >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) dead = true;
-              ++echunk;
+          const bool staged = p.resid || p.gate;
+          const uint32_t eb = echunk & 1u;
+          if (staged) {
+            if (!mbar_wait(&efull[eb], (echunk >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) dead = true;
+            ++echunk;
+          }
+          uint8_t* sg = smem + Cfg::OFF_GATE + eb * EPI_TILE + row * 128;
+          if (p.row_gate && !row_gate_vec) {  // by element into the gate chunk's place, which only p.gate uses
+#pragma unroll 1
+            for (int e = 0; e < 32; ++e) {
+              bf16 t = __float2bfloat16(0.f);
+              if (m < p.M && colw + e < n_out) t = p.row_gate[(m % p.row_gate_mod) * p.ldg + colw + e];
+              *reinterpret_cast<bf16*>(sg + ((uint32_t(ch * 4 + (e >> 3)) ^ rsw) << 4) + (e & 7) * 2) = t;
             }
           }
-          if (p.gate) {
-            if (staged) {
-              const uint8_t* sg = smem + Cfg::OFF_GATE + eb * EPI_TILE + row * 128;
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                const uint4 u = *reinterpret_cast<const uint4*>(sg + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
-                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
-                  v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
-                }
-              }
-            } else {
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
-                if (nvalid <= 0) continue;
-                float t8[8];
-                load8_bf16(p.gate + m * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[g * 8 + e] *= sigmoidf_fast(t8[e]);
-              }
-            }
-          }
-          if (row_gate_vec) {
+          if (p.gate || p.row_gate) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              const uint32_t w4[4] = {rg[g].x, rg[g].y, rg[g].z, rg[g].w};
+              const uint4 u = row_gate_vec ? rg[g] : *reinterpret_cast<const uint4*>(sg + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
+              const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
                 v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
               }
             }
-            if (c + 1 < nch) fetch_row_gate(c + 1);
-          } else if (p.row_gate) {  // gate shared by rows with equal (row % mod): AdaLN-Zero conditioning of several samples
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
-              if (nvalid <= 0) continue;
-              float t8[8];
-              load8_bf16(p.row_gate + (m % p.row_gate_mod) * p.ldg + col, t8, nvalid, (p.ldg & 7) == 0);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[g * 8 + e] *= sigmoidf_fast(t8[e]);
-            }
+            if (row_gate_vec && c + 1 < nch) fetch_row_gate(c + 1);
           }
           if (p.resid) {
-            if (staged) {
-              const uint8_t* sr = smem + Cfg::OFF_RES + eb * EPI_TILE + row * 128;
+            const uint8_t* sr = smem + Cfg::OFF_RES + eb * EPI_TILE + row * 128;
 #pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                const uint4 u = *reinterpret_cast<const uint4*>(sr + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
-                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+            for (int g = 0; g < 4; ++g) {
+              const uint4 u = *reinterpret_cast<const uint4*>(sr + ((uint32_t(ch * 4 + g) ^ rsw) << 4));
+              const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  v[g * 8 + 2 * e] += bf16_lo(w4[e]);
-                  v[g * 8 + 2 * e + 1] += bf16_hi(w4[e]);
-                }
-              }
-            } else {
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                const int col = colw + g * 8, nvalid = rvalid ? n_out - col : 0;
-                if (nvalid <= 0) continue;
-                float t8[8];
-                load8_bf16(p.resid + m * p.ldr + col, t8, nvalid, (p.ldr & 7) == 0);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[g * 8 + e] += t8[e];
+              for (int e = 0; e < 4; ++e) {
+                v[g * 8 + 2 * e] += bf16_lo(w4[e]);
+                v[g * 8 + 2 * e + 1] += bf16_hi(w4[e]);
               }
             }
           }

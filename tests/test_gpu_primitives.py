@@ -97,7 +97,7 @@ def test_linear_gate_residual(ops, M, K, N):
 
 
 @pytest.mark.parametrize("M", [1, 15, 16, 17, 77, 128, 129, 300, 640])  # 8, 8, .. 8, 4, 2 and 1 CTAs to a tile
-@pytest.mark.parametrize("K,N", [(1024, 768), (1544, 392), (256, 72)])
+@pytest.mark.parametrize("K,N", [(1024, 768), (1544, 392), (256, 72), (64, 72)])  # the last: K too short, gates by element
 def test_linear_gate_residual_split_k(ops, M, K, N):
     x, w, resid = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(M, N, seed=4)
     mod = max(1, M // 3)
