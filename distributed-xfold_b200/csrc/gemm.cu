@@ -201,6 +201,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     pdl_wait();
     pdl_launch();
+    const uint32_t go = elect_one();
     const int q = warp & 3;          // TMEM lane quarter this warp may read
     const int ch = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
     const int row = q * 32 + lane;
@@ -320,7 +321,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         // the TMA store that last used this staging buffer (two chunks ago) must have read it out
-        if (lane == 0) tma_store_wait_read<1>();
+        tma_store_wait_read<1>();
         __syncwarp();
         if constexpr (EPI == EPI_COLS) {
           // Every row needs all 32 elements of the column vectors: they pass through the free staging buffer.  (Loaded by
@@ -360,16 +361,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
-          if (colw < n_out && tm * BM + q * 32 < p.M) tma_store_3d(&tmO, so, colw, tm * BM + q * 32, b);
-          tma_store_commit();  // an empty group counts too: the wait above is by number
-        }
+        tma_store_3d_if(colw < n_out && tm * BM + q * 32 < p.M ? go : 0u, &tmO, so, colw, tm * BM + q * 32, b);
+        tma_store_commit();  // empty groups (the other lanes', parts outside the output) count too: the wait is by number
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
     }
-    if (lane == 0) tma_store_wait_all();  // written, not only read out: the next kernel may be waiting already
+    tma_store_wait_all();  // written, not only read out: the next kernel may be waiting already
   }
 
   tc_fence_before();

@@ -11,7 +11,7 @@
 // 77 rows 1215 -> 986 us with S = 8, 231 rows 1195 -> 1014 with 4, 384 rows 1406 -> 1230 and 512 rows 1467 -> 1314 with 2.
 // The projections before them (K = 768, 24 to 64 tiles) gain nothing: what the shorter loop saves the exchange costs.
 //
-//   warp 0 TMA producer, warp 1 tcgen05.mma issuer (warp-uniform, see attention.cu), warps 2..9 exchange and epilogue.
+//   warp 0 TMA producer, warp 1 tcgen05.mma issuer (both warp-uniform, see attention.cu), warps 2..9 exchange and epilogue.
 #include "internal.h"
 #include "umma.cuh"
 
@@ -90,31 +90,26 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int kb0 = rank * KB / split, kb1 = (rank + 1) * KB / split;  // split <= KB: never empty
 
   if (warp == 0) {
-    if (lane == 0) {
-      auto load_b = [&](int s, int kb) {
-        uint8_t* sB = smem + s * STAGE_BYTES + A_BYTES;
-        mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-        tma_load_3d(sB, &tmB, &full[s], kb * 64, tn * BN, 0);
-      };
-      int pre = 0;  // stages whose weights are on their way before the wait for the previous kernel
-      if (p.static_b)
-        for (; pre < stages && kb0 + pre < kb1; ++pre) load_b(pre, kb0 + pre);
-      pdl_wait();
-      pdl_launch();
-      int s = 0;
-      uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (kb - kb0 >= pre) {
-          if (!mbar_wait(&empty[s], phase ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-          load_b(s, kb);
-        }
-        tma_load_3d(smem + s * STAGE_BYTES, &tmA, &full[s], kb * 64, tm * 128, 0);
-        if (++s == stages) { s = 0; phase ^= 1u; }
-      }
-    }
-    __syncwarp();
+    const uint32_t go = elect_one();
+    auto load_b = [&](int s, int kb) {
+      mbar_arrive_expect_tx_if(go, &full[s], STAGE_BYTES);
+      tma_load_3d_if(go, smem + s * STAGE_BYTES + A_BYTES, &tmB, &full[s], kb * 64, tn * BN, 0);
+    };
+    int pre = 0;  // stages whose weights are on their way before the wait for the previous kernel
+    if (p.static_b)
+      for (; pre < stages && kb0 + pre < kb1; ++pre) load_b(pre, kb0 + pre);
     pdl_wait();
     pdl_launch();
+    int s = 0;
+    uint32_t phase = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (kb - kb0 >= pre) {
+        if (!mbar_wait_warp(&empty[s], phase ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+        load_b(s, kb);
+      }
+      tma_load_3d_if(go, smem + s * STAGE_BYTES, &tmA, &full[s], kb * 64, tm * 128, 0);
+      if (++s == stages) { s = 0; phase ^= 1u; }
+    }
     cluster_wait();
   } else if (warp == 1) {
     pdl_wait();
