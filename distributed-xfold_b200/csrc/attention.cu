@@ -205,55 +205,54 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
     // ------------------------------------------------------------------------------------------------ TMA producer
     // V is loaded two blocks later than K, so that waiting for a V buffer (free after P V) never holds up the keys of
     // the block before it; V goes first, because the wait for Q's buffer may depend on it.
-    if (lane == 0) {
-      const uint64_t my_items = n_items > blockIdx.x ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-      const uint64_t total = my_items * uint64_t(NB);
-      uint32_t kst = 0, kph = 0, vst = 0, vph = 0, it = 0, item_k = blockIdx.x, item_v = blockIdx.x;
-      int ks = 0, vs = 0, qt = 0, h = 0, b = 0, vqt, vh, vb;
-      decode(item_v, vqt, vh, vb);
-      bool okay = true;
-      for (uint64_t t = 0; t < total + 2 && okay; ++t) {
-        if (t >= 2) {
-          if (!mbar_wait(&v_empty[vst], vph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-          mbar_arrive_expect_tx(&v_full[vst], Cfg::VSTAGE);
-          tma_load_3d(smem + Cfg::OFF_V + vst * Cfg::VSTAGE, &tmkv, &v_full[vst], p.v_col0 + vh * D, vs * 64, vb);
-          if (++vst == NV) { vst = 0; vph ^= 1u; }
-          if (++vs == NB) {
-            vs = 0;
-            item_v += gridDim.x;
-            decode(item_v, vqt, vh, vb);
-          }
+    const uint32_t go = elect_one();  // warp-uniform, like the issuers
+    const uint64_t my_items = n_items > blockIdx.x ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const uint64_t total = my_items * uint64_t(NB);
+    uint32_t kst = 0, kph = 0, vst = 0, vph = 0, it = 0, item_k = blockIdx.x, item_v = blockIdx.x;
+    int ks = 0, vs = 0, qt = 0, h = 0, b = 0, vqt, vh, vb;
+    decode(item_v, vqt, vh, vb);
+    bool okay = true;
+    for (uint64_t t = 0; t < total + 2 && okay; ++t) {
+      if (t >= 2) {
+        if (!mbar_wait_warp(&v_empty[vst], vph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+        mbar_arrive_expect_tx_if(go, &v_full[vst], Cfg::VSTAGE);
+        tma_load_3d_if(go, smem + Cfg::OFF_V + vst * Cfg::VSTAGE, &tmkv, &v_full[vst], p.v_col0 + vh * D, vs * 64, vb);
+        if (++vst == NV) { vst = 0; vph ^= 1u; }
+        if (++vs == NB) {
+          vs = 0;
+          item_v += gridDim.x;
+          decode(item_v, vqt, vh, vb);
         }
-        if (t < total) {
-          if (ks == 0) {
-            decode(item_k, qt, h, b);
-            const uint32_t qb = it & 1u;
-            if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-            mbar_arrive_expect_tx(&q_full[qb], (ROWS ? NS : ns) * Cfg::QT);
-            uint8_t* sq = smem + Cfg::OFF_Q + qb * (NS * Cfg::QT);
-            if constexpr (ROWS) tma_load_3d(sq, &tmq, &q_full[qb], p.q_col0 + h * D, qt * 128, b);
-            else
-              for (int s = 0; s < ns; ++s) tma_load_3d(sq + s * Cfg::QT, &tmq, &q_full[qb], p.q_col0 + h * D, (qt + s) * 128, b);
-            ++it;
-          }
-          if (!mbar_wait(&k_empty[kst], kph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-          uint8_t* sb = smem + Cfg::OFF_K + kst * Cfg::KSTAGE;
-          uint8_t* sk = sb + Cfg::B_BYTES;
-          uint8_t* sm = sk + Cfg::K_BYTES;
-          int nm = 1;  // mask tiles: one per batch row of the item
-          if constexpr (ROWS) nm = p.mext_batch_stride == 0 ? 1 : (p.B - b < NS ? p.B - b : NS);
-          mbar_arrive_expect_tx(&k_full[kst], (ROWS ? 1 : ns) * Cfg::BT + Cfg::K_BYTES + nm * Cfg::MT);
-          tma_load_3d(sk, &tmkv, &k_full[kst], p.k_col0 + h * D, ks * 64, b);
-          if constexpr (ROWS) tma_load_3d(sb, &tmb, &k_full[kst], ks * 64, qt * 128, h);
+      }
+      if (t < total) {
+        if (ks == 0) {
+          decode(item_k, qt, h, b);
+          const uint32_t qb = it & 1u;
+          if (!mbar_wait_warp(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+          mbar_arrive_expect_tx_if(go, &q_full[qb], (ROWS ? NS : ns) * Cfg::QT);
+          uint8_t* sq = smem + Cfg::OFF_Q + qb * (NS * Cfg::QT);
+          if constexpr (ROWS) tma_load_3d_if(go, sq, &tmq, &q_full[qb], p.q_col0 + h * D, qt * 128, b);
           else
-            for (int s = 0; s < ns; ++s) tma_load_3d(sb + s * Cfg::BT, &tmb, &k_full[kst], ks * 64, (qt + s) * 128, h);
-          const uint8_t* mrow = p.mext + (long long)b * p.mext_batch_stride + (long long)ks * Cfg::MT;
-          for (int s = 0; s < nm; ++s) bulk_load(sm + s * Cfg::MT, mrow + s * p.mext_batch_stride, Cfg::MT, &k_full[kst]);
-          if (++kst == NK) { kst = 0; kph ^= 1u; }
-          if (++ks == NB) {
-            ks = 0;
-            item_k += gridDim.x;
-          }
+            for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sq + s * Cfg::QT, &tmq, &q_full[qb], p.q_col0 + h * D, (qt + s) * 128, b);
+          ++it;
+        }
+        if (!mbar_wait_warp(&k_empty[kst], kph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+        uint8_t* sb = smem + Cfg::OFF_K + kst * Cfg::KSTAGE;
+        uint8_t* sk = sb + Cfg::B_BYTES;
+        uint8_t* sm = sk + Cfg::K_BYTES;
+        int nm = 1;  // mask tiles: one per batch row of the item
+        if constexpr (ROWS) nm = p.mext_batch_stride == 0 ? 1 : (p.B - b < NS ? p.B - b : NS);
+        mbar_arrive_expect_tx_if(go, &k_full[kst], (ROWS ? 1 : ns) * Cfg::BT + Cfg::K_BYTES + nm * Cfg::MT);
+        tma_load_3d_if(go, sk, &tmkv, &k_full[kst], p.k_col0 + h * D, ks * 64, b);
+        if constexpr (ROWS) tma_load_3d_if(go, sb, &tmb, &k_full[kst], ks * 64, qt * 128, h);
+        else
+          for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sb + s * Cfg::BT, &tmb, &k_full[kst], ks * 64, (qt + s) * 128, h);
+        const uint8_t* mrow = p.mext + (long long)b * p.mext_batch_stride + (long long)ks * Cfg::MT;
+        for (int s = 0; s < nm; ++s) bulk_load_if(go, sm + s * Cfg::MT, mrow + s * p.mext_batch_stride, Cfg::MT, &k_full[kst]);
+        if (++kst == NK) { kst = 0; kph ^= 1u; }
+        if (++ks == NB) {
+          ks = 0;
+          item_k += gridDim.x;
         }
       }
     }

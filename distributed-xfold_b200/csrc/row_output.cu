@@ -122,31 +122,30 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int it = 0; it < mine; ++it) {
-        const uint32_t s = it & 1;
-        int j, i;
-        coords(it, j, i);
-        if (!mbar_wait(&empty[s], ((uint32_t(it) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-        mbar_arrive_expect_tx(&full[s], RO_TILE * (1 + (p.resid ? 1 : 0) + (p.gate ? 1 : 0)));
-        uint8_t* sx = smem + s * RO_STAGE;
-        if constexpr (CM) {
+    const uint32_t go = elect_one();  // warp-uniform, like the issuers
+    for (int it = 0; it < mine; ++it) {
+      const uint32_t s = it & 1;
+      int j, i;
+      coords(it, j, i);
+      if (!mbar_wait_warp(&empty[s], ((uint32_t(it) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+      mbar_arrive_expect_tx_if(go, &full[s], RO_TILE * (1 + (p.resid ? 1 : 0) + (p.gate ? 1 : 0)));
+      uint8_t* sx = smem + s * RO_STAGE;
+      if constexpr (CM) {
 #pragma unroll
-          for (int kb = 0; kb < 2; ++kb)
+        for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
-            for (int x = 0; x < 2; ++x) tma_load_3d(sx + kb * 16384 + x * 8192, &tmx, &full[s], j + x * 64, kb * 64, i);
-        } else {
-          tma_load_3d(sx, &tmx, &full[s], 0, j, i);
-          tma_load_3d(sx + 16384, &tmx, &full[s], 64, j, i);
-        }
-        if (p.gate) {
-          tma_load_3d(sx + 2 * RO_TILE, &tmg, &full[s], 0, j, i);
-          tma_load_3d(sx + 2 * RO_TILE + 16384, &tmg, &full[s], 64, j, i);
-        }
-        if (p.resid) {
-          tma_load_3d(sx + RO_TILE, &tmz, &full[s], 0, j, i);
-          tma_load_3d(sx + RO_TILE + 16384, &tmz, &full[s], 64, j, i);
-        }
+          for (int x = 0; x < 2; ++x) tma_load_3d_if(go, sx + kb * 16384 + x * 8192, &tmx, &full[s], j + x * 64, kb * 64, i);
+      } else {
+        tma_load_3d_if(go, sx, &tmx, &full[s], 0, j, i);
+        tma_load_3d_if(go, sx + 16384, &tmx, &full[s], 64, j, i);
+      }
+      if (p.gate) {
+        tma_load_3d_if(go, sx + 2 * RO_TILE, &tmg, &full[s], 0, j, i);
+        tma_load_3d_if(go, sx + 2 * RO_TILE + 16384, &tmg, &full[s], 64, j, i);
+      }
+      if (p.resid) {
+        tma_load_3d_if(go, sx + RO_TILE, &tmz, &full[s], 0, j, i);
+        tma_load_3d_if(go, sx + RO_TILE + 16384, &tmz, &full[s], 64, j, i);
       }
     }
   } else if (warp == 1) {

@@ -156,36 +156,33 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   auto unit_g = [](int g) { return !ATTN && g % 3 == 2; };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t bytes = 0;
-      for (int u = 0; u < U; ++u) bytes += unit_g(u0 + u) ? Cfg::W_UNIT / 2 : Cfg::W_UNIT;
-      mbar_arrive_expect_tx(w_full, bytes);
-      for (int u = 0; u < U; ++u) {
-        uint8_t* sw = smem + Cfg::OFF_W + u * Cfg::W_UNIT;
-        const int g = u0 + u;
-        // first 64 and last 64 weight rows of the unit (g: 64 in all)
-        const int r0 = ATTN ? g * 128 : unit_g(g) ? 512 + (g / 3) * 64 : (g / 3) * 256 + (g % 3) * 64, r1 = ATTN ? r0 + 64 : r0 + 128;
+    const uint32_t go = elect_one();  // warp-uniform, like the issuers
+    uint32_t bytes = 0;
+    for (int u = 0; u < U; ++u) bytes += unit_g(u0 + u) ? Cfg::W_UNIT / 2 : Cfg::W_UNIT;
+    mbar_arrive_expect_tx_if(go, w_full, bytes);
+    for (int u = 0; u < U; ++u) {
+      uint8_t* sw = smem + Cfg::OFF_W + u * Cfg::W_UNIT;
+      const int g = u0 + u;
+      // first 64 and last 64 weight rows of the unit (g: 64 in all)
+      const int r0 = ATTN ? g * 128 : unit_g(g) ? 512 + (g / 3) * 64 : (g / 3) * 256 + (g % 3) * 64, r1 = ATTN ? r0 + 64 : r0 + 128;
 #pragma unroll
-        for (int kh = 0; kh < 2; ++kh) {
-          tma_load_3d(sw + kh * 16384, &tmw, w_full, kh * 64, r0, 0);
-          if (!unit_g(g)) tma_load_3d(sw + kh * 16384 + 8192, &tmw, w_full, kh * 64, r1, 0);
-        }
-      }
-      pdl_wait();
-      pdl_launch();
-      for (int it = 0; it < mine; ++it) {
-        const int t = t0 + it * step;
-        const uint32_t xb = it & 1;
-        if (!mbar_wait(&x_free[xb], ((uint32_t(it) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-        mbar_arrive_expect_tx(&x_full[xb], Cfg::X_TILE);
-        uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
-        const int c1 = p.mode1 ? t % p.dim1 : t * 128, c2 = p.mode1 ? t / p.dim1 * 128 : 0;
-        tma_load_3d(sx, &tmx, &x_full[xb], 0, c1, c2);
-        tma_load_3d(sx + 16384, &tmx, &x_full[xb], 64, c1, c2);
+      for (int kh = 0; kh < 2; ++kh) {
+        tma_load_3d_if(go, sw + kh * 16384, &tmw, w_full, kh * 64, r0, 0);
+        if (!unit_g(g)) tma_load_3d_if(go, sw + kh * 16384 + 8192, &tmw, w_full, kh * 64, r1, 0);
       }
     }
     pdl_wait();
     pdl_launch();
+    for (int it = 0; it < mine; ++it) {
+      const int t = t0 + it * step;
+      const uint32_t xb = it & 1;
+      if (!mbar_wait_warp(&x_free[xb], ((uint32_t(it) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+      mbar_arrive_expect_tx_if(go, &x_full[xb], Cfg::X_TILE);
+      uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
+      const int c1 = p.mode1 ? t % p.dim1 : t * 128, c2 = p.mode1 ? t / p.dim1 * 128 : 0;
+      tma_load_3d_if(go, sx, &tmx, &x_full[xb], 0, c1, c2);
+      tma_load_3d_if(go, sx + 16384, &tmx, &x_full[xb], 64, c1, c2);
+    }
   } else if (warp == 1) {
     pdl_wait();
     pdl_launch();

@@ -105,54 +105,51 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
 
   if (warp == 0) {
     if (!p.static_w) pdl_wait();
-    if (lane == 0) {
-      const long long nblk = (long long)mine * NBK;
-      int hb1 = 0, hb2 = 0, t = blockIdx.x, xt = 0;
-      bool okay = true;
-      auto load_w1 = [&](long long i) {
-        const uint32_t st = uint32_t(i) & 1u;
-        if (!mbar_wait(&w1_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
-        mbar_arrive_expect_tx(&w1_full[st], TR_W1);
-        uint8_t* sw = smem + TR_OFF_W1 + st * TR_W1;
-        const int r0 = (hb1 >> 1) * 256 + (hb1 & 1) * 64;  // 64 SiLU units and their 64 linear partners
+    const uint32_t go = elect_one();  // warp-uniform, like the issuers
+    const long long nblk = (long long)mine * NBK;
+    int hb1 = 0, hb2 = 0, t = blockIdx.x, xt = 0;
+    bool okay = true;
+    auto load_w1 = [&](long long i) {
+      const uint32_t st = uint32_t(i) & 1u;
+      if (!mbar_wait_warp(&w1_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
+      mbar_arrive_expect_tx_if(go, &w1_full[st], TR_W1);
+      uint8_t* sw = smem + TR_OFF_W1 + st * TR_W1;
+      const int r0 = (hb1 >> 1) * 256 + (hb1 & 1) * 64;  // 64 SiLU units and their 64 linear partners
 #pragma unroll
-        for (int kh = 0; kh < 2; ++kh) {
-          tma_load_3d(sw + kh * 16384, &tmw1, &w1_full[st], kh * 64, r0, 0);
-          tma_load_3d(sw + kh * 16384 + 8192, &tmw1, &w1_full[st], kh * 64, r0 + 128, 0);
-        }
-        if (++hb1 == NBK) hb1 = 0;
-      };
-      auto load_w2 = [&](long long i) {
-        const uint32_t st = uint32_t(i) & 1u;
-        if (!mbar_wait(&w2_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
-        mbar_arrive_expect_tx(&w2_full[st], TR_W2);
-        tma_load_3d(smem + TR_OFF_W2 + st * TR_W2, &tmw2, &w2_full[st], hb2 * 64, 0, 0);
-        if (++hb2 == NBK) hb2 = 0;
-      };
-      load_w1(0);  // (weights that no kernel of the call writes: on their way before the wait for the previous kernel)
-      pdl_wait();
-      pdl_launch();
-      // W2 runs one block behind W1, and the next item's x goes out with the item's last blocks: no load waits for a
-      // buffer that is freed later than the one after it needs
-      for (long long i = 0; i <= nblk && okay; ++i) {
-        if (xt < mine && (long long)xt * NBK <= i) {  // i == first block of item xt: its W1 is on its way
-          for (int s = 0; s < NT && okay; ++s) {
-            if (!mbar_wait(&n_empty[s], (uint32_t(xt) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
-            mbar_arrive_expect_tx(&x_full[s], TR_TILE);
-            uint8_t* sx = smem + TR_OFF_N + s * TR_TILE;
-            const int r = (t * NT + s) * 128;
-            tma_load_3d(sx, &tmx, &x_full[s], 0, r, 0);
-            tma_load_3d(sx + 16384, &tmx, &x_full[s], 64, r, 0);
-          }
-          t += gridDim.x;
-          ++xt;
-        }
-        if (okay && i > 0) load_w2(i - 1);
-        if (okay && i + 1 < nblk) load_w1(i + 1);
+      for (int kh = 0; kh < 2; ++kh) {
+        tma_load_3d_if(go, sw + kh * 16384, &tmw1, &w1_full[st], kh * 64, r0, 0);
+        tma_load_3d_if(go, sw + kh * 16384 + 8192, &tmw1, &w1_full[st], kh * 64, r0 + 128, 0);
       }
-    }
+      if (++hb1 == NBK) hb1 = 0;
+    };
+    auto load_w2 = [&](long long i) {
+      const uint32_t st = uint32_t(i) & 1u;
+      if (!mbar_wait_warp(&w2_empty[st], ((uint32_t(i) >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; return; }
+      mbar_arrive_expect_tx_if(go, &w2_full[st], TR_W2);
+      tma_load_3d_if(go, smem + TR_OFF_W2 + st * TR_W2, &tmw2, &w2_full[st], hb2 * 64, 0, 0);
+      if (++hb2 == NBK) hb2 = 0;
+    };
+    load_w1(0);  // (weights that no kernel of the call writes: on their way before the wait for the previous kernel)
     pdl_wait();
     pdl_launch();
+    // W2 runs one block behind W1, and the next item's x goes out with the item's last blocks: no load waits for a
+    // buffer that is freed later than the one after it needs
+    for (long long i = 0; i <= nblk && okay; ++i) {
+      if (xt < mine && (long long)xt * NBK <= i) {  // i == first block of item xt: its W1 is on its way
+        for (int s = 0; s < NT && okay; ++s) {
+          if (!mbar_wait_warp(&n_empty[s], (uint32_t(xt) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) { okay = false; break; }
+          mbar_arrive_expect_tx_if(go, &x_full[s], TR_TILE);
+          uint8_t* sx = smem + TR_OFF_N + s * TR_TILE;
+          const int r = (t * NT + s) * 128;
+          tma_load_3d_if(go, sx, &tmx, &x_full[s], 0, r, 0);
+          tma_load_3d_if(go, sx + 16384, &tmx, &x_full[s], 64, r, 0);
+        }
+        t += gridDim.x;
+        ++xt;
+      }
+      if (okay && i > 0) load_w2(i - 1);
+      if (okay && i + 1 < nblk) load_w1(i + 1);
+    }
   } else if (warp == 1) {
     pdl_wait();
     pdl_launch();

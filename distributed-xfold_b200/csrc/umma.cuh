@@ -210,6 +210,14 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                : "memory");
 }
 
+__device__ __forceinline__ void bulk_load_if(uint32_t go, void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}"
+      ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "r"(go)
+      : "memory");
+}
+
 // ------------------------------------------------------------------------------------
 // tcgen05: TMEM allocation, MMA, commit, loads
 // ------------------------------------------------------------------------------------
