@@ -50,7 +50,7 @@ struct RpCfg {
   static constexpr int UNITS = ATTN ? 4 : 6, NSET = ATTN ? 3 : 4, MIN_PARTS = ATTN ? 1 : 2;
   static constexpr int THREADS = (10 + 4 * NSET) * 32;
   static constexpr uint32_t W_UNIT = 32768, X_TILE = 32768;      // [2 K halves][128 rows][64], swizzled
-  static constexpr uint32_t STG = 128 * 32 * 2;                  // a set's staging tile [128 rows][32 columns]
+  static constexpr uint32_t STG = 128 * 32 * 2;                  // a set's staging tiles, [32 rows][32 columns] per warp
   static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + UNITS / MIN_PARTS * W_UNIT, OFF_STG = OFF_X + 2 * X_TILE,
                             OFF_WB = OFF_STG + NSET * STG, OFF_GB = OFF_WB + (ATTN ? 4096 : 0), OFF_SC = OFF_GB + 1024,
                             OFF_CB = OFF_SC + (ATTN ? 2048 : 0), OFF_ST = OFF_CB + (ATTN ? 128 : 0),
@@ -317,29 +317,28 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     pdl_launch();
     const int set = (warp - 10) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t laddr = tmem_base + set * 128 + (uint32_t(quarter * 32) << 16);
-    uint8_t* stg = smem + Cfg::OFF_STG + set * Cfg::STG;
-    const bool elected = ((warp - 10) & 3) == 0 && lane == 0;
+    uint8_t* stg = smem + Cfg::OFF_STG + set * Cfg::STG + quarter * 2048;
+    const uint32_t go = elect_one();
     uint32_t k = 0;  // units this set has taken
     for (int n = set; n < mine * U; n += NSET, ++k) {
       const int it = n / U, g = u0 + n % U, t = t0 + it * step;
       const int c1 = p.mode1 ? t % p.dim1 : t * 128, c2 = p.mode1 ? t / p.dim1 * 128 : 0;
-      const uint32_t rsw = uint32_t(row >> 1) & 3u;  // 64-byte swizzle of the staging tile
+      const uint32_t rsw = uint32_t(lane >> 1) & 3u;  // 64-byte swizzle of the staging tile
       if (ATTN || unit_g(g)) {
         const int chunks = ATTN ? 4 : 2, col0 = ATTN ? g * 128 : (g / 3) * 64;
-        mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through: the set meets at barriers)
+        mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through)
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < chunks; ++c) {
           uint32_t r[32];
           tmem_ld32(laddr + c * 32, r);
-          if (elected) tma_store_wait_read<0>();
-          named_bar_sync(1 + set, 128);
           tmem_ld_wait();
           if (c == chunks - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&t_empty[set]);
           }
+          uint4 o4[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint32_t o[4];
@@ -354,14 +353,19 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
               const __half2 h2 = __floats2half2_rn(v0, v1);  // the v columns leave as fp16
               o[e] = ATTN && g == 2 ? *reinterpret_cast<const uint32_t*>(&h2) : pack_bf16x2(v0, v1);
             }
-            *reinterpret_cast<uint4*>(stg + row * 64 + ((uint32_t(q) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+            o4[q] = make_uint4(o[0], o[1], o[2], o[3]);
           }
+          // a warp stages and stores its own rows; its store before has mostly been read out by now
+          tma_store_wait_read<0>();
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(stg + lane * 64 + ((uint32_t(q) ^ rsw) << 4)) = o4[q];
           fence_proxy_async_smem();
-          named_bar_sync(1 + set, 128);
-          if (elected) {
-            tma_store_3d(&tmo, stg, col0 + c * 32, c1, c2);
-            tma_store_commit();
-          }
+          __syncwarp();
+          const int y = p.mode1 ? c1 : c1 + quarter * 32, x = p.mode1 ? c2 + quarter * 32 : c2;
+          const bool inside = p.mode1 ? (long long)x * p.ntok < p.rows : (long long)y < p.rows;
+          tma_store_3d_if(inside ? go : 0u, &tmo, stg, col0 + c * 32, y, x);
+          tma_store_commit();
         }
       } else {
         // where this thread's token goes, and its mask value, before the wait
@@ -403,7 +407,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
         }
       }
     }
-    if (elected) tma_store_wait_all();
+    tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -450,11 +454,11 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   bool ok;
   if (!transposed) {
     ok = make_tmap_bf16_3d(&tmx, z, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) &&
-         make_tmap_bf16_3d(&tmo, out_g, 128, M, 1, 128, (uint64_t)128 * M, 32, 128, 1, 64);
+         make_tmap_bf16_3d(&tmo, out_g, 128, M, 1, 128, (uint64_t)128 * M, 32, 32, 1, 64);
     a.tiles = (int)((M + 127) / 128);
   } else {  // tile rows step along the first token axis, second axis fixed: a[j][c][i]
     ok = make_tmap_bf16_3d(&tmx, z, 128, N, R, 128, (uint64_t)128 * N, 64, 1, 128) &&
-         make_tmap_bf16_3d(&tmo, out_g, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 128, 64);
+         make_tmap_bf16_3d(&tmo, out_g, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 32, 64);
     a.mode1 = 1;
     a.dim1 = N;
     a.tiles = N * ((R + 127) / 128);
@@ -482,7 +486,7 @@ int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, int norm, const
   CUtensorMap tmx, tmw, tmo;
   RowProjectArgs a = {};
   if (!make_tmap_bf16_3d(&tmx, z, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) ||
-      !make_tmap_bf16_3d(&tmo, qkvg, 512, M, 1, 512, (uint64_t)512 * M, 32, 128, 1, 64) ||
+      !make_tmap_bf16_3d(&tmo, qkvg, 512, M, 1, 512, (uint64_t)512 * M, 32, 32, 1, 64) ||
       !make_tmap_bf16_3d(&tmw, w_qkvg, 128, 512, 1, 128, 128 * 512, 64, 64, 1))
     return fail(c, XFOLD_ERR_ARG, "triattn: cannot encode projection tensor maps");
   a.tiles = (int)((M + 127) / 128);
