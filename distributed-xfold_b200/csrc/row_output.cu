@@ -32,6 +32,7 @@ struct RowOutputArgs {
   const float *gamma, *beta;
   long long tiles;
   int tiles_j;        // tiles per row (row mode), or 0: flat tokens
+  int extent;         // tokens of a row
   int gate, resid, static_w;
   int* status;
 };
@@ -47,7 +48,7 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   // a stage's token statistics (-mean, rstd) go over its operand tile once the product has read that
   auto rstat = [&](uint32_t s) { return reinterpret_cast<float2*>(smem + s * RO_STAGE); };
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + RO_OFF_BAR);  // [2]
-  uint64_t* empty = full + 2;    // [2] both halves of the result have left shared memory
+  uint64_t* empty = full + 2;    // [2] the result has left shared memory (8 warps)
   uint64_t* t_full = empty + 2;  // [2] product complete
   uint64_t* t_empty = t_full + 2;  // [2] accumulator read (8 warps)
   uint64_t* st_full = t_empty + 2;  // [2] statistics written (8 warps)
@@ -59,7 +60,7 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 2);
+      mbar_init(&empty[s], 8);
       mbar_init(&t_full[s], 1);
       mbar_init(&t_empty[s], 8);
       mbar_init(&st_full[s], 8);
@@ -215,10 +216,11 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const int set = (warp - 10) >> 2, s = set & 1, half = set >> 1, quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t rsw = uint32_t(row & 7), laddr = tmem_base + s * 128 + half * 64 + (uint32_t(quarter * 32) << 16);
     uint8_t* sz = smem + s * RO_STAGE + RO_TILE + half * 16384 + row * 128;
+    const uint32_t go = elect_one();
     const uint8_t* sg = sz + RO_TILE;
     for (int it = s; it < mine; it += 2) {
       const uint32_t ph = (uint32_t(it) >> 1) & 1u;
-      mbar_wait(&full[s], ph, ab, XF_ERR_WAIT_FULL);  // (a failed wait runs through: the set meets at a barrier)
+      mbar_wait(&full[s], ph, ab, XF_ERR_WAIT_FULL);  // (a failed wait runs through)
       if (CM) mbar_wait(&st_full[s], ph, ab, XF_ERR_WAIT_FULL);
       mbar_wait(&t_full[s], ph, ab, XF_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
@@ -260,18 +262,19 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
           *reinterpret_cast<uint4*>(sz + at) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
+      // a warp's rows leave by themselves
       fence_proxy_async_smem();
-      named_bar_sync(1 + set, 128);
-      if (((warp - 10) & 3) == 0 && lane == 0) {
-        int j, i;
-        coords(it, j, i);
-        tma_store_3d(&tmo, smem + s * RO_STAGE + RO_TILE + half * 16384, half * 64, j, i);
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(&empty[s]);
-      }
+      __syncwarp();
+      int j, i;
+      coords(it, j, i);
+      j += quarter * 32;
+      tma_store_3d_if(j < p.extent ? go : 0u, &tmo, smem + s * RO_STAGE + RO_TILE + half * 16384 + quarter * 4096, half * 64, j, i);
+      tma_store_commit();
+      tma_store_wait_read<0>();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
     }
-    if (((warp - 10) & 3) == 0 && lane == 0) tma_store_wait_all();
+    tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -311,11 +314,12 @@ int launch_row_output(Ctx* c, const bf16* x, long long M, const bf16* w, const b
   CUtensorMap tmx, tmz, tmo;
   if (!make_tmap_bf16_3d(&tmx, x, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) ||
       !make_tmap_bf16_3d(&tmz, resid ? resid : out, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) ||
-      !make_tmap_bf16_3d(&tmo, out, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1))
+      !make_tmap_bf16_3d(&tmo, out, 128, M, 1, 128, (uint64_t)128 * M, 64, 32, 1))
     return fail(c, XFOLD_ERR_ARG, "row output: cannot encode tensor maps");
   RowOutputArgs a = {};
   a.w = w;
   a.tiles = (M + 127) / 128;
+  a.extent = (int)M;
   a.resid = resid != nullptr;
   return launch_ro<false>(c, tmx, tmz, tmz, tmo, a, st);
 }
@@ -331,7 +335,7 @@ int launch_row_output_cm(Ctx* c, const bf16* o, long long o_cs, long long o_rs, 
   CUtensorMap tmx, tmz, tmg, tmo;
   if (!make_tmap_bf16_3d(&tmx, o, J, 128, I, o_cs, flat ? (uint64_t)o_cs * 128 : (uint64_t)o_rs, 64, 64, 1) ||
       !make_tmap_bf16_3d(&tmz, resid ? resid : out, 128, J, I, 128, 128 * J, 64, 128, 1) ||
-      !make_tmap_bf16_3d(&tmg, g, 128, J, I, 128, 128 * J, 64, 128, 1) || !make_tmap_bf16_3d(&tmo, out, 128, J, I, 128, 128 * J, 64, 128, 1))
+      !make_tmap_bf16_3d(&tmg, g, 128, J, I, 128, 128 * J, 64, 128, 1) || !make_tmap_bf16_3d(&tmo, out, 128, J, I, 128, 128 * J, 64, 32, 1))
     return fail(c, XFOLD_ERR_ARG, "row output: cannot encode tensor maps");
   RowOutputArgs a = {};
   a.w = w;
@@ -339,6 +343,7 @@ int launch_row_output_cm(Ctx* c, const bf16* o, long long o_cs, long long o_rs, 
   a.beta = beta;
   a.tiles_j = flat ? 0 : (N + 127) / 128;
   a.tiles = flat ? (long long)(J + 127) / 128 : (long long)a.tiles_j * R;
+  a.extent = (int)J;
   a.gate = 1;
   a.resid = resid != nullptr;
   return launch_ro<true>(c, tmx, tmz, tmg, tmo, a, st);
