@@ -23,18 +23,24 @@ adaln_kernel(const bf16* x, bf16* __restrict__ y, int rows, const bf16* scale, c
   constexpr int V = C / 128;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const bool valid = row < rows;
+  uint2 rx[V], ra[V], rb[V];
+  // The modulation was written at least two launches ago (the gate projection or a whole sub-layer lies between) and has
+  // landed when this kernel starts: a kernel lets its successor start only after its own pdl_wait().  So it is fetched
+  // while the predecessor still runs.
+  if (valid) {
+    const long long mr = (long long)(row % mod) * ldm;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      ra[k] = __ldcg(reinterpret_cast<const uint2*>(scale + mr) + lane + 32 * k);
+      rb[k] = __ldcg(reinterpret_cast<const uint2*>(shift + mr) + lane + 32 * k);
+    }
+  }
   pdl_wait();
   pdl_launch();
-  if (row >= rows) return;
-  const long long mr = (long long)(row % mod) * ldm;
-  uint2 rx[V], ra[V], rb[V];
+  if (!valid) return;
 #pragma unroll
   for (int k = 0; k < V; ++k) rx[k] = reinterpret_cast<const uint2*>(x + (long long)row * C)[lane + 32 * k];
-#pragma unroll
-  for (int k = 0; k < V; ++k) {
-    ra[k] = reinterpret_cast<const uint2*>(scale + mr)[lane + 32 * k];
-    rb[k] = reinterpret_cast<const uint2*>(shift + mr)[lane + 32 * k];
-  }
   float v[V][4], s = 0.f;
 #pragma unroll
   for (int k = 0; k < V; ++k) {
