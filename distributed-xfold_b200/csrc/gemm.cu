@@ -227,6 +227,15 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if constexpr (EPI == EPI_GATE_RESID)
         if (row_gate_vec) fetch_row_gate(0);
+      // COLS: this lane's element of the column vectors, likewise
+      float cb = 0.f, cs = 1.f;
+      auto fetch_cols = [&](int c) {
+        const int col = tn * BN + c * 64 + ch * 32 + lane;
+        cb = p.col_bias && col < p.N ? p.col_bias[col] : 0.f;
+        cs = p.col_scale && col < p.N ? p.col_scale[col] : 1.f;
+        if (col - lane < p.log2e_cols) cs *= 1.4426950408889634f;
+      };
+      if constexpr (EPI == EPI_COLS) fetch_cols(0);
       if (!mbar_wait(&tfull[buf], aphase, ab, XF_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(q * 32) << 16);
@@ -249,12 +258,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int colw = col0 + ch * 32;              // first output column of this warp
         uint8_t* so = smem + Cfg::OFF_OUT + ((warp - 2) * 2 + (ochunk & 1u)) * OUT_TILE;
         float v[32];
-        float cb = 0.f, cs = 1.f;  // this lane's element of the column vectors
-        if constexpr (EPI == EPI_COLS) {
-          if (p.col_bias && colw + lane < n_out) cb = p.col_bias[colw + lane];
-          if (p.col_scale && colw + lane < n_out) cs = p.col_scale[colw + lane];
-          if (colw < p.log2e_cols) cs *= 1.4426950408889634f;
-        }
         if constexpr (EPI == EPI_SWIGLU) {
           uint32_t ra[32], rb[32];
           tmem_ld32(taddr + c * 64 + ch * 32, ra);
@@ -331,6 +334,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           sv[lane] = cb;
           sv[32 + lane] = cs;
           __syncwarp();
+          if (c + 1 < nch) fetch_cols(c + 1);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const float4 fb = reinterpret_cast<const float4*>(sv)[e], fs = reinterpret_cast<const float4*>(sv)[8 + e];
