@@ -12,13 +12,15 @@ reference's own wrappers (``prototypes/*.py``) run unchanged on GPU tensors:
   GridSelfAttention.py:47-49): sequence axes rounded up to 64, TriangleMultiplication's two token axes to 32;
 * the schemas are defined here only when no extension has defined them already.
 
-Weights are re-packed into the kernel layouts on first use and cached per (storage, version).
+Weights are re-packed into the kernel layouts on first use and cached as long as their storage lives, unchanged.
 """
 from __future__ import annotations
 
 from typing import Dict, Tuple
 
 import torch
+
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import ops
 
@@ -55,16 +57,30 @@ def _pad_to(n: int, block: int) -> int:
 
 
 def _key(*ts) -> Tuple:
-    return tuple((t.data_ptr(), t._version, tuple(t.shape)) for t in ts)
+    return tuple((t.untyped_storage()._cdata, t.data_ptr(), t._version, t.dtype, tuple(t.shape), t.stride()) for t in ts)
 
 
 def _cached(name, tensors, make):
+    """The packed form of ``tensors`` (``make`` returns copies: an alias would keep the storage alive).  An entry holds weak
+    references to their storages: while those live, no other storage can have the same identity, so an equal key is the
+    same memory, read in the same way, not written since.  An entry whose storage has gone is never returned and leaves the
+    cache with the next new one."""
     k = (name,) + _key(*tensors)
-    v = _CACHE.get(k)
-    if v is None:
-        if len(_CACHE) > 4096:
-            _CACHE.clear()
-        v = _CACHE[k] = make()
+    hit = _CACHE.get(k)
+    if hit is not None and not any(r.expired() for r in hit[1]):
+        return hit[0]
+    v = make()
+    on_gpu = tensors[0].is_cuda
+    if on_gpu:
+        torch.cuda.current_stream(tensors[0].device).synchronize()   # any stream may use the packed form from now on
+    gone = [e for e, (_, refs) in list(_CACHE.items()) if any(r.expired() for r in refs)]
+    if len(_CACHE) - len(gone) > 4096:
+        gone = list(_CACHE)
+    if gone and on_gpu:
+        torch.cuda.synchronize(tensors[0].device)                    # and may still be using those that go
+    for e in gone:
+        _CACHE.pop(e, None)
+    _CACHE[k] = (v, [StorageWeakRef(t.untyped_storage()) for t in tensors])
     return v
 
 
@@ -152,8 +168,7 @@ def _transition(act, transition1, transition2, layernorm_weight, layernorm_bias)
 
     def pack():   # the op takes the matrices as [in, out] (kernel_test/transition.py:31-36)
         state = {"transition1.weight": transition1.detach().float().T, "transition2.weight": transition2.detach().float().T,
-                 "input_layer_norm.weight": layernorm_weight.detach().float(),
-                 "input_layer_norm.bias": layernorm_bias.detach().float()}
+                 "input_layer_norm.weight": layernorm_weight.clone(), "input_layer_norm.bias": layernorm_bias.clone()}
         return ops.PackedTransition(state, "", act.device)
 
     w = _cached("tr", (transition1, transition2, layernorm_weight, layernorm_bias), pack)
@@ -190,9 +205,11 @@ def _traingle_multiplication(act, mask, equation_flag, left_norm_input_weight, l
             out[0::2], out[1::2] = w[:c], w[c:]
             return out
         state = {"projection.weight": interleave(projection_weight), "gate.weight": interleave(gate_weight),
-                 "gating_linear.weight": gating_linear_weight, "output_projection.weight": output_projection_weight,
-                 "left_norm_input.weight": left_norm_input_weight, "left_norm_input.bias": left_norm_input_bias,
-                 "center_norm.weight": center_norm_weight, "center_norm.bias": center_norm_bias}
+                 "gating_linear.weight": gating_linear_weight,
+                 "output_projection.weight": output_projection_weight.clone(),
+                 "left_norm_input.weight": left_norm_input_weight.clone(),
+                 "left_norm_input.bias": left_norm_input_bias.clone(),
+                 "center_norm.weight": center_norm_weight.clone(), "center_norm.bias": center_norm_bias.clone()}
         return ops.PackedTriMul(state, "", dev)
 
     w = _cached("tm", (left_norm_input_weight, left_norm_input_bias, projection_weight, gate_weight, center_norm_weight,

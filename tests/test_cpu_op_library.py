@@ -24,6 +24,28 @@ def test_meta_shapes(pkg):
     assert tuple(ops.transition_forward(m(3, 7, 128), m(128, 1024), f(512, 128), m(128), m(128)).shape) == (3, 7, 128)
 
 
+def test_packed_weights_follow_the_tensors_they_were_made_from(pkg):
+    """The cache of packed weights answers for the very memory it was filled from: not for another storage at the same
+    address, another view of it, another reading of its bits, or later contents."""
+    from distributed_xfold_b200 import op_library as L
+    buf = bytearray(torch.arange(12, dtype=torch.float32).numpy().tobytes())
+    get = lambda t: L._cached("test", (t,), lambda: t.clone())
+    w = torch.frombuffer(buf, dtype=torch.float32).view(3, 4)
+    first = get(w)
+    assert get(w) is first and get(w.view(3, 4)) is first
+    assert torch.equal(get(w.as_strided((3, 4), (1, 3))), w.as_strided((3, 4), (1, 3)))
+    assert get(w.view(torch.int32)).dtype == torch.int32
+    w += 1
+    assert torch.equal(get(w), w)
+    del w
+    other = torch.frombuffer(buf, dtype=torch.float32).view(3, 4)    # a new storage, same address, version and shape
+    other.numpy()[:] = 7
+    assert torch.equal(get(other), other)
+    del other
+    get(torch.zeros(5))
+    assert sum(k[0] == "test" for k in L._CACHE) <= 1                # what has gone leaves with the next new entry
+
+
 _WRAPPER_SCRIPT = r"""
 import sys, torch
 repo, ref_src = sys.argv[1], sys.argv[2]
