@@ -66,7 +66,8 @@ class DiffusionBlockWeights(C.Structure):
 
 class DiffusionWeights(C.Structure):
     _fields_ = [(n, ci) for n in ("C", "C_cond", "H", "Dp", "F", "num_blocks")] + \
-               [(n, vp) for n in ("w_mod", "b_mod", "w_gate", "b_gate")] + [("blocks", C.POINTER(DiffusionBlockWeights))]
+               [(n, vp) for n in ("w_mod", "b_mod", "w_gate", "b_gate")] + [("blocks", C.POINTER(DiffusionBlockWeights)),
+                ("ln_cond", vp)]
 
 
 class ShardDesc(C.Structure):

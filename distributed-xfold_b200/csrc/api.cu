@@ -100,6 +100,32 @@ int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const
   return gemm_rows(c, cols ? EPI_COLS : EPI_PLAIN, x, ldx, M, K, w, N, K, a, bn, st);
 }
 
+// out[m][b * N + n] = sum_k x[b][m][k] w[b][n][k] + bias[b * N + n]
+int linear_batched(Ctx* c, const bf16* x, int M, int K, int batches, const bf16* w, int N, const float* bias, bf16* out,
+                   long long ldo, cudaStream_t st) {
+  if ((K & 7) || (N & 7)) return fail(c, XFOLD_ERR_ARG, "batched linear: K and N must be multiples of 8");
+  GemmArgs a;
+  const int bn = gemm_tile_n(c, M, N, K, batches, 256, 64);
+  CUtensorMap tA, tB;
+  if (!make_tmap_bf16_3d(&tA, x, K, M, batches, K, (uint64_t)M * K, 64, 128, 1) ||
+      !make_tmap_bf16_3d(&tB, w, K, N, batches, K, (uint64_t)N * K, 64, bn, 1))
+    return fail(c, XFOLD_ERR_ARG, "batched linear: cannot encode tensor maps (16-byte aligned bases?)");
+  a.static_b = c->static_weights;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.batches = batches;
+  a.b_batched = 1;
+  a.tiles_m = (M + 127) / 128;
+  a.tiles_n = (N + bn - 1) / bn;
+  a.out = out;
+  a.ldo = ldo;
+  a.out_batch_stride = N;
+  a.col_bias = bias;
+  a.status = c->d_status;
+  return launch_gemm(c, EPI_COLS, bn, tA, tB, a, st);
+}
+
 int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N,
                              const bf16* gate, long long ldg, int row_gate_mod, const bf16* resid, long long ldr,
                              bf16* out, long long ldo, cudaStream_t st) {

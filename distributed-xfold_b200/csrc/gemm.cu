@@ -117,11 +117,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // Weights that no kernel of this call writes are fetched before the wait for the previous kernel: with a few rows
     // of activations the launch is a latency chain and the weights' trip from HBM is the longest link of it.
     int pre = 0;
-    if (p.static_b && (long long)blockIdx.x < total)
+    if (p.static_b && (long long)blockIdx.x < total) {
+      const int b0 = p.b_batched ? int(blockIdx.x / (p.tiles_n * p.tiles_m)) : 0;
       for (; pre < STAGES && pre < KB; ++pre) {
         mbar_arrive_expect_tx_if(go, &full[pre], Cfg::STAGE_BYTES);
-        load_b(smem + pre * Cfg::STAGE_BYTES + Cfg::A_BYTES, &full[pre], pre, int(blockIdx.x % p.tiles_n), 0);
+        load_b(smem + pre * Cfg::STAGE_BYTES + Cfg::A_BYTES, &full[pre], pre, int(blockIdx.x % p.tiles_n), b0);
       }
+    }
     pdl_wait();
     pdl_launch();
     for (long long t = blockIdx.x; t < total && okay; t += gridDim.x) {
@@ -231,8 +233,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       float cb = 0.f, cs = 1.f;
       auto fetch_cols = [&](int c) {
         const int col = tn * BN + c * 64 + ch * 32 + lane;
-        cb = p.col_bias && col < p.N ? p.col_bias[col] : 0.f;
-        cs = p.col_scale && col < p.N ? p.col_scale[col] : 1.f;
+        cb = p.col_bias && col < p.N ? p.col_bias[b * p.N + col] : 0.f;
+        cs = p.col_scale && col < p.N ? p.col_scale[b * p.N + col] : 1.f;
         if (col - lane < p.log2e_cols) cs *= 1.4426950408889634f;
       };
       if constexpr (EPI == EPI_COLS) fetch_cols(0);
@@ -416,7 +418,7 @@ static int launch_one(Ctx* c, const CUtensorMap& tmA, const CUtensorMap& tmB, co
   const int grid = (int)(total < sms ? total : sms);
   const int tag = EPI == EPI_SWIGLU ? XFOLD_K_LINEAR_SWIGLU
                   : EPI == EPI_GATE_RESID ? XFOLD_K_LINEAR_GATE_RESID
-                  : (a.batches > 1 ? XFOLD_K_TRIMUL_CONTRACT : XFOLD_K_LINEAR);
+                  : (EPI == EPI_PLAIN && a.batches > 1 ? XFOLD_K_TRIMUL_CONTRACT : XFOLD_K_LINEAR);
   ProfScope ps(c, tag, st);
   launch_pdl(kern, grid, GEMM_THREADS, Cfg::SMEM_BYTES, st, tmA, tmB, tmO, tmR, tmG, a);
   return check_launch(c, "gemm_tn_kernel");

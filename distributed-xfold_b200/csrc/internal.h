@@ -82,9 +82,9 @@ int check_launch(Ctx* c, const char* what);
 
 // Launch that may start while the previous kernel of the stream still runs (see pdl_wait in umma.cuh).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args&&... args) {
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -136,7 +136,7 @@ struct GemmArgs {
   // output (row-major, all epilogues)
   bf16* out = nullptr;
   long long ldo = 0, out_batch_stride = 0;
-  const float* col_bias = nullptr;  // COLS: (product + col_bias) * col_scale
+  const float* col_bias = nullptr;  // COLS: (product + col_bias) * col_scale; N of them for each entry of the batch
   const float* col_scale = nullptr;
   int f16_col0 = 0, f16_col1 = 0;  // COLS: output columns [f16_col0, f16_col1) are stored as fp16 (multiples of 32)
   int log2e_cols = 0;  // COLS: output columns [0, log2e_cols) times log2(e) (a multiple of 32): the attention works in base 2

@@ -63,6 +63,8 @@ int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cuda
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,
                  const float* scale, bf16* out, long long ldo, cudaStream_t st, int f16_col0 = 0, int f16_col1 = 0,
                  int log2e_cols = 0);
+int linear_batched(Ctx* c, const bf16* x, int M, int K, int batches, const bf16* w, int N, const float* bias, bf16* out,
+                   long long ldo, cudaStream_t st);
 int linear_gate_resid(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const bf16* gate,
                       long long ldg, int row_gate_mod, const bf16* resid, long long ldr, bf16* out, long long ldo,
                       cudaStream_t st);

@@ -3,7 +3,7 @@
 24 blocks in 6 super-blocks; per block  act += AttentionPairBias(act, mask, pair_logits, single_cond)
 and  act += DiffusionTransition(act, single_cond).  A step is one C-ABI call (``xfold_diffusion_transformer_fwd``):
 
-    conditioning             -> one LayerNorm of single_cond and two GEMMs for the modulations and gates of many blocks
+    conditioning             -> the LayerNorms of single_cond and two GEMMs for the modulations and gates of many blocks
     AdaptiveLayerNorm        -> LayerNorm with fused modulation
     q/k/v/gate projections   -> one GEMM with query bias and D^-0.5 folded into the epilogue
     attention (16 x 48 -> 64)-> flash kernel with the prepared pair logits
@@ -50,20 +50,20 @@ class _PackedAdaLN:
 
 
 def _conditioning(state: State, p_att: str, p_tr: str):
-    """The conditioning projections of one block: (mod [4c, c_cond], its bias [4c], gate [2c, c_cond], its bias [2c]).  The
-    scale of the conditioning's LayerNorm goes into the columns of the first, so that all blocks share one LayerNorm."""
-    mod, mod_b, gate, gate_b = [], [], [], []
+    """The conditioning projections of one block: (modulations [4c, c_cond], their bias [4c], gates [2c, c_cond], their
+    bias [2c], scales of the two LayerNorms of the conditioning [2, c_cond])."""
+    mod, mod_b, gate, gate_b, ln_g = [], [], [], [], []
     for p in (p_att, p_tr):
         ln = p + "adaptive_layernorm."
-        g = state[ln + "single_cond_layer_norm.weight"].detach().float()
+        ln_g.append(state[ln + "single_cond_layer_norm.weight"].detach().float()[None])
         scale_b = state[ln + "single_cond_scale.bias"].detach().float()
-        mod += [state[ln + n + ".weight"].detach().float() * g for n in ("single_cond_scale", "single_cond_bias")]
+        mod += [state[ln + n + ".weight"].detach().float() for n in ("single_cond_scale", "single_cond_bias")]
         mod_b += [scale_b, torch.zeros_like(scale_b)]
         w = state[p + "adaptive_zero_init.adaptive_zero_cond.weight"].detach().float()
         b = state.get(p + "adaptive_zero_init.adaptive_zero_cond.bias")
         gate.append(w)
         gate_b.append(w.new_zeros(w.shape[0]) if b is None else b.detach().float())
-    return mod, mod_b, gate, gate_b
+    return mod, mod_b, gate, gate_b, ln_g
 
 
 class PackedDiffusionBlock:
@@ -86,14 +86,14 @@ class PackedDiffusionTransformer:
         names = [(prefix + f"self_attention.{i}.", prefix + f"transition_block.{i}.") for i in range(num_blocks)]
         self.blocks = [PackedDiffusionBlock(state, p_att, p_tr, device, num_head) for p_att, p_tr in names]
         parts = [_conditioning(state, p_att, p_tr) for p_att, p_tr in names]
-        stack = [torch.cat([t for p in parts for t in p[k]], 0) for k in range(4)]
+        stack = [torch.cat([t for p in parts for t in p[k]], 0) for k in range(5)]
         self.w_mod, self.w_gate = ops._b16(stack[0], device), ops._b16(stack[2], device)
-        self.b_mod, self.b_gate = ops._f32(stack[1], device), ops._f32(stack[3], device)
+        self.b_mod, self.b_gate, self.ln_cond = (ops._f32(stack[k], device) for k in (1, 3, 4))
         a = self.blocks[0].att
         self._arr = (_cabi.DiffusionBlockWeights * num_blocks)(*[b.c for b in self.blocks])
         self.c = _cabi.DiffusionWeights(a.C, self.w_mod.shape[1], a.H, a.Dp, self.blocks[0].tr_w2.shape[1], num_blocks,
                                         ops._ptr(self.w_mod), ops._ptr(self.b_mod), ops._ptr(self.w_gate),
-                                        ops._ptr(self.b_gate), self._arr)
+                                        ops._ptr(self.b_gate), self._arr, ops._ptr(self.ln_cond))
 
     def pair_logits(self, pair_cond: torch.Tensor) -> List[torch.Tensor]:
         """[N, N, 128] bf16 -> per super-block float16 [super_block_size, heads, N, pad8(N)], the prepared operand of the

@@ -195,8 +195,9 @@ int xfold_grid_attention_fwd(xfold_ctx* ctx, const void* x, int B, int S, int C,
                              const void* w_out, int C_out, void* out, int SP, void* ws, size_t ws_bytes, void* stream);
 /* All blocks of the DiffusionTransformer (nn/d_diffusion_transformer.py:267-310) for one denoising step of S samples, in
  * place on act bf16 [S][N][C].  The conditioning projections of all blocks are stacked:
- *   w_mod  bf16 [num_blocks * 4C][C_cond]: per block scale, shift (attention), scale, shift (transition), every column
- *          multiplied by the block's single_cond_layer_norm scale; b_mod float32 [num_blocks * 4C] (zero for the shifts)
+ *   w_mod  bf16 [num_blocks * 4C][C_cond]: per block scale, shift (attention), scale, shift (transition); b_mod float32
+ *          [num_blocks * 4C] (zero for the shifts); ln_cond float32 [num_blocks * 2][C_cond]: the scales of the
+ *          single_cond_layer_norm before them (attention, transition)
  *   w_gate bf16 [num_blocks * 2C][C_cond]: per block the AdaLN-Zero gates of attention and transition; b_gate or null
  * w_qkvg / w_out as for xfold_attention_pair_bias_core_fwd (heads padded to Dp), w1_packed [2F][C], w2 [C][F] as for
  * xfold_linear_swiglu_fwd; pair_logits: per block the prepared bias [H][N][pad8(N)]; mask float32 [N] or null. */
@@ -215,6 +216,7 @@ typedef struct {
   const void* w_gate;
   const float* b_gate;
   const xfold_diffusion_block_weights* blocks;
+  const float* ln_cond;
 } xfold_diffusion_weights;
 size_t xfold_diffusion_workspace_bytes(int S, int N, const xfold_diffusion_weights* w);
 int xfold_diffusion_transformer_fwd(xfold_ctx* ctx, void* act, int S, int N, const float* mask, const void* single_cond,

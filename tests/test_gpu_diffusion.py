@@ -60,6 +60,40 @@ def test_diffusion_single_sample_2d_input(ops, oracle):
     assert relf(a.float().cpu(), ref) < 2e-2
 
 
+@pytest.mark.parametrize("n,samples,blocks", [(40, 1, 2), (300, 2, 24), (1900, 1, 3)])
+def test_step_is_the_composition_of_its_operators(ops, oracle, n, samples, blocks):
+    """The one-call step against the same blocks put together from the single operators: the same roundings at the same
+    places, hence the same bits.  The conditioning of 24 blocks at 300 tokens comes in two groups, the second one shorter;
+    of three blocks at 1900 tokens in groups of two and one."""
+    from distributed_xfold_b200 import diffusion
+    c, heads = 768, 16
+    g = torch.Generator().manual_seed(n + blocks)
+    st = oracle.make_diffusion_transformer_state(g, "", c, 384, 128, heads, blocks, 1)
+    for k, v in st.items():
+        if k.endswith("single_cond_layer_norm.weight"):
+            st[k] = 1.0 + 0.3 * torch.randn(v.shape, generator=g)
+    model = diffusion.PackedDiffusionTransformer(st, "", "cuda", heads, blocks, 1)
+    act = torch.randn(samples, n, c, generator=g).to(BF).cuda()
+    cond = torch.randn(n, 384, generator=g).to(BF).cuda()
+    mask = (torch.rand(n, generator=g) > 0.1).float().cuda()
+    logits = [torch.randn(1, heads, n, n, device="cuda") for _ in range(blocks)]
+    prepared = [ops.prepare_pair_bias(t[0])[None] for t in logits]
+    got = model.forward(act.clone(), mask, cond, prepared)
+    want = act.clone()
+    for i, blk in enumerate(model.blocks):
+        for part, p in enumerate((f"self_attention.{i}.", f"transition_block.{i}.")):
+            xn = diffusion._PackedAdaLN(st, p + "adaptive_layernorm.", "cuda")(want, cond)
+            wc = st[p + "adaptive_zero_init.adaptive_zero_cond.weight"].to(BF).cuda()
+            gate = ops.linear(cond, wc, st[p + "adaptive_zero_init.adaptive_zero_cond.bias"].cuda())
+            if part == 0:
+                o, w = ops.attention_pair_bias_core(xn, blk.att, prepared[i][0], mask), blk.att.w_out
+            else:
+                o, w = ops.linear_swiglu(xn, blk.tr_w1), blk.tr_w2
+            ops.linear_gate_residual(o, w, gate, want, row_gate_mod=n, out=want)
+    ops.synchronize_and_check()
+    assert torch.isfinite(got).all() and torch.equal(got, want)
+
+
 def test_sampler_loop_around_the_gpu_transformer(ops, oracle):
     """The sampler of d_alphafold3.py:316-404 (host arithmetic in diffusion_head.py) driving the DiffusionTransformer on
     the GPU, against the same loop around the CPU oracle's transformer.  The atom encoder / decoder of the reference's
