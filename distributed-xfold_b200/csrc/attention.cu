@@ -4,7 +4,7 @@
 // Bound: the exponential unit (16 results per clock and SM): N^2 heads rows exponentials, 0.98 ms for a TriangleAttention of
 // 1024 tokens.  Everything else is arranged so that the softmax threads do little besides exponentiate and rarely wait:
 //   * The logits arrive complete.  The tensor core adds the pair bias (bias tile x 16 x 16 identity blocks, fp16, exact) and
-//     the key mask (a rank-1 product) to Q K^T, and Q was scaled by log2(e) where it was projected, so a logit in tensor
+//     the key mask (ones x its three bf16 pieces) to Q K^T, and Q was scaled by log2(e) where it was projected, so a logit in tensor
 //     memory is the base-2 exponent: per pair of keys one packed subtraction of the reference exponent, two exponentials,
 //     one pack, one packed addition to the row sum.
 //   * Per block of 64 keys and slot the softmax warps wait once (logits complete) and arrive once (P stored).  Logits and P
@@ -178,14 +178,14 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
     tma_prefetch_desc(&tmb);
   }
   // Constant operands, un-swizzled 8 x 16-byte core matrices.  ID: the 16 x 16 fp16 identity.  E1: columns 0..7 of a
-  // [128][16] matrix whose column 0 is all ones.  ZERO: columns 8..15 of E1 and of the mask tiles.
+  // [128][16] matrix whose columns 0..2 are all ones.  ZERO: columns 8..15 of E1 and of the mask tiles.
   for (uint32_t i = threadIdx.x; i < (512 + 2048 + 2048) / 4; i += Cfg::THREADS) {
     uint32_t v = 0;
     if (i < 128) {
       const uint32_t core = i >> 5, row = (i & 31) >> 2, pr = i & 3;  // core = (row group, column group)
       if ((core == 0 || core == 3) && (row >> 1) == pr) v = (row & 1) ? 0x3C000000u : 0x00003C00u;
     } else if (i < 640) {
-      if ((i & 3) == 0) v = 0x00003F80u;
+      v = (i & 3) == 0 ? 0x3F803F80u : (i & 3) == 1 ? 0x00003F80u : 0u;
     }
     reinterpret_cast<uint32_t*>(smem + Cfg::OFF_ID)[i] = v;
   }
@@ -480,11 +480,13 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
   }
 }
 
-// Mask-bias tiles: out[b][ks] is a [64 keys][8] bf16 tile (8-key groups of 128 bytes, 16 bytes per key) whose column 0
-// holds 1e9 * (mask[b][k] - 1) for k < S and -1e30 for the padding of the last tile; its other columns are zero.
-// 1e9 * (mask - 1) as in the reference, floored at -60000: any such logit still exponentiates to exactly 0 next to an
-// unmasked one, while a row whose keys are ALL masked keeps fp32-resolvable logits (at 1e9 the fp32 spacing is 64).
-// additive: the mask is given as that additive bias.
+// Mask-bias tiles: out[b][ks] is a [64 keys][8] bf16 tile (8-key groups of 128 bytes, 16 bytes per key) whose first columns
+// add up to the bias of a key k < S, -1e30 for the padding of the last tile; its other columns are zero.
+// A mask: 1e9 * (mask[b][k] - 1) as in the reference, in one column, floored at -60000: any such logit still exponentiates to
+// exactly 0 next to an unmasked one, while a row whose keys are ALL masked keeps fp32-resolvable logits (at 1e9 the fp32
+// spacing is 64).
+// additive: the bias itself.  Times log2(e) like the logits it is added to, in three columns (float32's 24 bits), kept within
+// +-60000 like the pair bias.
 __global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restrict__ out, int B, int S, int KS, int additive) {
   pdl_wait();
   pdl_launch();
@@ -493,11 +495,18 @@ __global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restr
     const long long bb = idx / (KS * 64);
     const int k = int(idx - bb * (KS * 64));
     float v = -1.0e30f;
+    uint32_t p[3] = {0, 0, 0};
     if (k < S) {
       v = mask ? mask[bb * mask_ld + k] : additive ? 0.f : 1.f;
-      v = fminf(fmaxf(additive ? v : 1.0e9f * (v - 1.f), -60000.f), additive ? 0.f : 3.0e38f);
+      v = fminf(fmaxf(additive ? v * 1.4426950408889634f : 1.0e9f * (v - 1.f), -60000.f), additive ? 60000.f : 3.0e38f);
     }
-    out[idx] = make_uint4(uint32_t(__bfloat16_as_ushort(__float2bfloat16(v))), 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const bf16 h = __float2bfloat16(v);
+      p[i] = __bfloat16_as_ushort(h);
+      v = additive ? v - __bfloat162float(h) : 0.f;
+    }
+    out[idx] = make_uint4(p[0] | p[1] << 16, p[2], 0, 0);
   }
 }
 

@@ -113,7 +113,9 @@ def _grid_self_attn(q_data, bias, nonbatched_bias, query_w, key_w, value_w, gati
 
     w_qkvg, scale, w_out = _cached("gsa", (query_w, key_w, value_w, gating_w, output_w), pack)
     x = q_data.to(BF16).contiguous()
-    bias = bias.float().reshape(-1, s).contiguous()      # additive: 1e9 * (mask - 1), per batch entry or shared
+    bias = bias.float().reshape(-1, s).contiguous()      # additive, as 1e9 * (mask - 1): one row per batch entry, or one
+    if 1 < bias.shape[0] < b:
+        raise ops._cabi.XfoldError(f"grid_self_attn_forward: a bias of {bias.shape[0]} rows for {b} batch entries")
     nb = nonbatched_bias.float().contiguous() if nonbatched_bias.numel() else torch.zeros(h, s, s, device=dev)
     lib = load()
     di = dev.index if dev.index is not None else torch.cuda.current_device()

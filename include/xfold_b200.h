@@ -186,8 +186,9 @@ int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* ctx, const void* xn, 
                                                 size_t ws_bytes, void* stream);
 
 /* The TriangleAttention operator on already normalised rows (csrc/Alpha_Attention.cpp:50-70): x bf16 [B][S][C], w_qkvg bf16
- * [4 * H * 32][C] (heads padded to 32), qkvg_scale float32 [4 * H * 32] or null, pair_bias float32 [H][S][S], mask_bias the
- * ADDITIVE mask 1e9 * (mask - 1), float32, row b at mask_bias + b * mask_ld (0: one row for all; null: no mask), w_out bf16
+ * [4 * H * 32][C] (heads padded to 32), qkvg_scale float32 [4 * H * 32] or null, pair_bias float32 [H][S][S], mask_bias an
+ * additive bias of the keys (the mask as 1e9 * (mask - 1)), float32, row b at mask_bias + b * mask_ld (0: one row for all;
+ * null: none); magnitudes beyond 41500 count as 41500, w_out bf16
  * [C_out][H * 32] -> out bf16 [B][SP][C_out], rows S..SP-1 zero. */
 size_t xfold_grid_attention_workspace_bytes(int B, int S, int SP, int H);
 int xfold_grid_attention_fwd(xfold_ctx* ctx, const void* x, int B, int S, int C, int H, const void* w_qkvg,

@@ -134,3 +134,29 @@ def test_op_grid_self_attention_shapes(lib, oracle, b, s, c, h, d, shared):
     ref = oracle.gated_attention(rb(x), bias, nb, rb(ws["query_w"]), rb(ws["key_w"]), rb(ws["value_w"]), rb(ws["gating_w"]),
                                  rb(ws["output_w"]))
     assert relf(out[:, :s].float().cpu(), ref) < 2e-2
+
+
+@pytest.mark.parametrize("b,s,shared", [(5, 70, False), (3, 129, True), (2, 40, False)])
+def test_op_grid_self_attention_adds_the_bias_as_given(lib, oracle, b, s, shared):
+    """A bias of the keys that is no mask: moderate values of either sign, some keys pushed up or out, one batch entry with
+    every key far below zero.  Slots over batch rows and over query tiles."""
+    c, h, d = 128, 4, 32
+    g = torch.Generator().manual_seed(80 + s)
+    ws = _attn_weights(g, c, h, d, True)
+    x = torch.randn(b, s, c, generator=g)
+    bias = 3.0 * torch.randn(1 if shared else b, 1, 1, s, generator=g)
+    bias[..., 3] += 12.0
+    bias[..., 5::7] = -1e9
+    bias[-1] -= 300.0
+    nb = torch.randn(h, s, s, generator=g)
+    args = [x.to(BF).cuda(), bias.cuda(), nb.cuda(), *(ws[n].to(BF).cuda() for n in (
+        "query_w", "key_w", "value_w", "gating_w", "output_w")), d, d]
+    out = lib.grid_self_attn_forward(*args)
+    torch.cuda.synchronize()
+    ref = oracle.gated_attention(rb(x), bias, nb, rb(ws["query_w"]), rb(ws["key_w"]), rb(ws["value_w"]), rb(ws["gating_w"]),
+                                 rb(ws["output_w"]))
+    assert relf(out[:, :s].float().cpu(), ref) < 2e-2
+    if b > 2 and not shared:   # neither one row for all nor one for each
+        args[1] = bias[:2].cuda()
+        with pytest.raises(RuntimeError):
+            lib.grid_self_attn_forward(*args)
