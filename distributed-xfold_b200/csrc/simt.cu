@@ -348,7 +348,7 @@ ln128_tc_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ld
   uint8_t* sW = smem + LNTC_OFF_W;                                     // [2 halves][16 heads][128 B], swizzled
   float* colsum = reinterpret_cast<float*>(smem + LNTC_OFF_MISC);      // [16]
   float* colbias = colsum + 16;                                        // [16]
-  float2* rstat = reinterpret_cast<float2*>(smem + LNTC_OFF_MISC + 128);  // [128] (mean, rstd) of the tile's rows
+  float2* rstat = reinterpret_cast<float2*>(smem + LNTC_OFF_MISC + 128);  // [128] (-mean, rstd) of the tile's rows
   uint64_t* mma_bar = reinterpret_cast<uint64_t*>(smem + LNTC_OFF_MISC + 128 + 1024);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_bar + 1);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -450,44 +450,50 @@ ln128_tc_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ld
       umma_commit(mma_bar);
     }
     if (t + gridDim.x < ntiles) fetch(t + gridDim.x, buf ^ 1);
-    // row statistics (and the normalised rows, when asked for) while the product runs
-    constexpr int UNR = 2;
-#pragma unroll UNR
-    for (int it = 0; it < 8; ++it) {
-      const int r = warp * 16 + it * 2 + half;
-      const long long prow = t * 128 + r;
-      const bool valid = prow < rows;
-      const uint4 rawv = *reinterpret_cast<const uint4*>(piece(buf, r, l16));
-      const uint32_t w4[4] = {rawv.x, rawv.y, rawv.z, rawv.w};
-      float v[8];
-      float s0 = 0.f, s1 = 0.f;
+    // Row statistics (and the normalised rows, when asked for) while the product runs.  Two threads per row, adding in the
+    // order of row_project_kernel: the row shards, which normalise here, then have the bits of the one-GPU block, which does
+    // there.
+    {
+      const int r = warp * 16 + l16;
+      uint32_t xr[32];
+      float2 s2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.bf16 %0, lo, %0;\n\tadd.rn.f32.bf16 %1, hi, %1;\n\t}"
-            : "+f"(s0), "+f"(s1) : "r"(w4[e]));
-      float sm = s0 + s1;
+      for (int q = 0; q < 8; ++q) {
+        const uint4 u = *reinterpret_cast<const uint4*>(piece(buf, r, half * 8 + q));
+        xr[q * 4] = u.x; xr[q * 4 + 1] = u.y; xr[q * 4 + 2] = u.z; xr[q * 4 + 3] = u.w;
+      }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
-      const float mean = sm * (1.f / 128);
-      const float nmean = -mean;
-      float ss = 0.f;
+      for (int e = 0; e < 32; ++e) sum2(xr[e], s2[e & 1]);
+      float sm = (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
+      sm += __shfl_xor_sync(0xffffffffu, sm, 16);
+      const float nmean = -sm * (1.f / 128);
+      float2 sq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.bf16 %0, lo, %3;\n\tadd.rn.f32.bf16 %1, hi, %3;\n\t}"
-            : "=f"(v[2 * e]), "=f"(v[2 * e + 1]) : "r"(w4[e]), "f"(nmean));
+      for (int e = 0; e < 32; ++e) {
+        const float2 v = centre2(xr[e], nmean);
+        sq[e & 1] = ffma2(v, v, sq[e & 1]);
+      }
+      sm = (sq[0].x + sq[0].y) + (sq[1].x + sq[1].y);
+      sm += __shfl_xor_sync(0xffffffffu, sm, 16);
+      if (half == 0) rstat[r] = make_float2(nmean, rsqrtf(sm * (1.f / 128) + eps));
+    }
+    if (y) {
+      __syncwarp();
+#pragma unroll 2
+      for (int it = 0; it < 8; ++it) {
+        const int r = warp * 16 + it * 2 + half;  // rows of this warp
+        const long long prow = t * 128 + r;
+        if (prow >= rows) continue;
+        const float2 st = rstat[r];
+        const uint4 rawv = *reinterpret_cast<const uint4*>(piece(buf, r, l16));
+        const uint32_t w4[4] = {rawv.x, rawv.y, rawv.z, rawv.w};
+        uint32_t o[4];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float rstd = rsqrtf(ss * (1.f / 128) + eps);
-      if (l16 == 0) rstat[r] = make_float2(mean, rstd);
-      if (y && valid) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = fmaf(v[e] * rstd, gm[e], bt[e]);
-        uint4 u;
-        u.x = pack_bf16x2(v[0], v[1]); u.y = pack_bf16x2(v[2], v[3]);
-        u.z = pack_bf16x2(v[4], v[5]); u.w = pack_bf16x2(v[6], v[7]);
-        *reinterpret_cast<uint4*>(y + srow_of(prow) * ldy + c0) = u;
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = centre2(w4[e], st.x);
+          o[e] = pack_bf16x2(fmaf(v.x * st.y, gm[2 * e], bt[2 * e]), fmaf(v.y * st.y, gm[2 * e + 1], bt[2 * e + 1]));
+        }
+        *reinterpret_cast<uint4*>(y + srow_of(prow) * ldy + c0) = make_uint4(o[0], o[1], o[2], o[3]);
       }
     }
     __syncthreads();  // statistics of all 128 rows are in shared memory
@@ -512,7 +518,7 @@ ln128_tc_kernel(const bf16* x, long long ldx, bf16* __restrict__ y, long long ld
           for (int j = 0; j < 8; ++j) {
             const int h = hsel * 8 + j;
             if (h < H) {
-              const float val = fmaf(st.y, __uint_as_float(d[j]) - st.x * colsum[h], colbias[h]);
+              const float val = fmaf(st.y, fmaf(st.x, colsum[h], __uint_as_float(d[j])), colbias[h]);
               proj_bf16[(long long)h * proj_plane + o] = bias16(val);
             }
           }

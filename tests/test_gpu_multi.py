@@ -47,6 +47,50 @@ def test_row_sharded_block_single_shard(ops, oracle, n, pad):
     assert relf((zd.float().cpu() - z.float())[pm > 0], (rz - z.float())[pm > 0]) < 3e-2
 
 
+@pytest.mark.parametrize("n,pad", [(96, 0.0), (131, 0.1), (264, 0.1)])
+def test_row_sharded_block_has_the_bits_of_the_one_gpu_block(ops, oracle, n, pad):
+    """The row-shard stages and the one-GPU block round at the same places and add in the same order."""
+    from distributed_xfold_b200 import row_sharded
+    g = torch.Generator().manual_seed(850 + n)
+    st = oracle.make_pairformer_block_state(g, "")
+    for k, v in st.items():
+        if v.dim() == 1 and "norm" in k:
+            st[k] = v + 0.1 * torch.randn(v.shape, generator=g)
+    z, s, pm, sm = (t.cuda() for t in oracle.make_inputs(851 + n, n, pad_frac=pad))
+    w = ops.PackedPairformerBlock(st, "", "cuda")
+    z0, s0 = z.to(BF).contiguous(), s.to(BF).contiguous()
+    z1, s1 = z0.clone(), s0.clone()
+    zs, ss = row_sharded.pairformer_block(row_sharded.RowSharding(n), row_sharded.CudaStages(), z0, s0, pm,
+                                          pm.t().contiguous(), sm, w)
+    ops.pairformer_block_(z1, s1, pm, sm, w)
+    ops.synchronize_and_check()
+    assert torch.equal(zs, z1) and torch.equal(ss, s1)
+
+
+@pytest.mark.parametrize("ending", [False, True])
+@pytest.mark.parametrize("n,cuts", [(128, (0, 64, 128)), (131, (0, 66, 131)), (200, (0, 1, 3, 200))])
+def test_triangle_attention_by_rows_has_the_bits_of_the_whole(ops, oracle, n, cuts, ending):
+    """What the ranks compute, one after the other: each its rows' part of the pair bias, then attention of its rows."""
+    g = torch.Generator().manual_seed(870 + n)
+    w = ops.PackedTriAttn(oracle.make_grid_attention_state(g, ""), "", "cuda")
+    z = (1.5 * torch.randn(n, n, 128, generator=g) + 0.4).to(BF).cuda()
+    mask = (torch.rand(n, n, generator=g) > 0.2).float().cuda()
+    want = ops.triangle_attention_(z.clone(), mask, w, ending)
+    rows = [slice(a, b) for a, b in zip(cuts, cuts[1:])]
+    shards = [(z.transpose(0, 1) if ending else z)[r].contiguous() for r in rows]
+    xs, bias = zip(*(ops.stage_triattn_bias(t, w, ending) for t in shards))
+    ldq = (n + 7) // 8 * 8
+    if ending:
+        bias = torch.nn.functional.pad(torch.cat(bias, 2), (0, ldq - n)).contiguous()
+    else:
+        bias = torch.cat(bias, 1).contiguous()
+    for t, x, r in zip(shards, xs, rows):
+        ops.stage_triattn_core(x, bias, mask[r], w, t)
+    ops.synchronize_and_check()
+    got = torch.cat(shards, 0)
+    assert torch.equal(got.transpose(0, 1) if ending else got, want)
+
+
 def _rank_main(rank, world, port, n, pad, use_peer, channel, ret):
     sys.path.insert(0, ROOT)
     import __graft_entry__ as ge
