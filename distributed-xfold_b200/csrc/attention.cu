@@ -79,12 +79,16 @@ __device__ __forceinline__ float ex2f_(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {  // (fminf and fmaxf would lose a NaN)
+  asm("max.NaN.f32 %0, %0, %1;\n\tmin.NaN.f32 %0, %0, %2;" : "+f"(x) : "f"(lo), "f"(hi));
+  return x;
+}
 // 2^y for a pair of float32 on the FMA pipe: y = n + f with n the nearest integer, 2^f by a degree-5 polynomial on
-// [-1/2, 1/2] (minimax in relative error, 7.5e-8, fitted with the Remez exchange), n added to the exponent field.
+// [-1/2, 1/2] (minimax in relative error, 7.5e-8, fitted with the Remez exchange), times 2^n.  0 from -127 down, NaN for NaN.
 __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   const float magic = 12582912.f;  // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
-  y.x = fminf(fmaxf(y.x, -126.f), 127.f);
-  y.y = fminf(fmaxf(y.y, -126.f), 127.f);
+  y.x = clamp_nan(y.x, -127.f, 127.f);
+  y.y = clamp_nan(y.y, -127.f, 127.f);
   const float2 t = fadd2(y, make_float2(magic, magic));
   const float2 n = fadd2(t, make_float2(-magic, -magic));
   const float2 f = ffma2(n, make_float2(-1.f, -1.f), y);
@@ -93,8 +97,9 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   q = ffma2(q, f, make_float2(0.24022120237350464f, 0.24022120237350464f));
   q = ffma2(q, f, make_float2(0.6931469440460205f, 0.6931469440460205f));
   q = ffma2(q, f, make_float2(1.0000001192092896f, 1.0000001192092896f));
-  return make_float2(__uint_as_float(__float_as_uint(q.x) + (__float_as_uint(t.x) << 23)),
-                     __uint_as_float(__float_as_uint(q.y) + (__float_as_uint(t.y) << 23)));
+  // 2^n from the exponent field (0 for n = -127)
+  return make_float2(q.x * __uint_as_float(__float_as_uint(t.x) * 0x800000u + 0x3F800000u),
+                     q.y * __uint_as_float(__float_as_uint(t.y) * 0x800000u + 0x3F800000u));
 }
 __device__ __forceinline__ void tmem_st16_(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(

@@ -316,6 +316,27 @@ def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
     assert torch.isfinite(out).all() and relf(out, ref) < 4e-2
 
 
+@pytest.mark.parametrize("C,d,key", [(384, 24, 5), (384, 24, 14), (384, 24, 31), (768, 48, 62), (768, 48, 40)])
+def test_attention_passes_nan_on(ops, oracle, C, d, key):
+    """A key whose logits are NaN (infinite in both signs) makes every query's result NaN, whichever way its exponential is
+    taken; its value row is finite."""
+    g = torch.Generator().manual_seed(key)
+    st = oracle.make_self_attention_state(g, "", C, 0, False)
+    S, H = 70, 16
+    xn = torch.randn(2, S, C, generator=g)
+    xn[:, :, 0] = 0.0
+    for n in ("q_projection", "k_projection", "v_projection", "gating_query"):
+        st[n + ".weight"][:, 0] = 3e38 if n[0] == "k" else 0.0
+    w = ops.PackedSelfAttention(st, "", "cuda", H)
+    pb = torch.randn(H, S, S, generator=g).cuda()
+    run = lambda: ops.attention_pair_bias_core(xn.to(BF).cuda().contiguous(), w, pb, None).float().cpu().reshape(2, S, H, w.Dp)[..., :d]
+    assert torch.isfinite(run()).all()
+    xn[0, key, 0] = 4.0
+    out = run()
+    ops.synchronize_and_check()
+    assert torch.isnan(out[0]).all() and torch.isfinite(out[1]).all()
+
+
 @pytest.mark.parametrize("n", [129, 137, 310])
 def test_triangle_multiplication_ragged_contraction_tiles(ops, oracle, n):
     """Token counts whose last 256-wide contraction tile is mostly empty, and row counts that are no multiple of a tile."""
