@@ -84,7 +84,9 @@ __device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {  // (f
   return x;
 }
 // 2^y for a pair of float32 on the FMA pipe: y = n + f with n the nearest integer, 2^f by a degree-5 polynomial on
-// [-1/2, 1/2] (minimax in relative error, 7.5e-8, fitted with the Remez exchange), times 2^n.  0 from -127 down, NaN for NaN.
+// [-1/2, 1/2], times 2^n.  0 from -127 down, NaN for NaN.  Coefficients: minimax in relative error with constant term 1 (a
+// linear program over the interval, each coefficient rounded to float32 before the next is fitted), 9.3e-8; evaluated in
+// float32 the relative error is at most 1.6e-7.
 __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   const float magic = 12582912.f;  // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
   y.x = clamp_nan(y.x, -127.f, 127.f);
@@ -92,11 +94,11 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   const float2 t = fadd2(y, make_float2(magic, magic));
   const float2 n = fadd2(t, make_float2(-magic, -magic));
   const float2 f = ffma2(n, make_float2(-1.f, -1.f), y);
-  float2 q = ffma2(f, make_float2(0.0013276472454890609f, 0.0013276472454890609f), make_float2(0.009675540961325169f, 0.009675540961325169f));
-  q = ffma2(q, f, make_float2(0.05550713092088699f, 0.05550713092088699f));
-  q = ffma2(q, f, make_float2(0.24022120237350464f, 0.24022120237350464f));
-  q = ffma2(q, f, make_float2(0.6931469440460205f, 0.6931469440460205f));
-  q = ffma2(q, f, make_float2(1.0000001192092896f, 1.0000001192092896f));
+  float2 q = ffma2(f, make_float2(0.0013269521296024323f, 0.0013269521296024323f), make_float2(0.009671291336417198f, 0.009671291336417198f));
+  q = ffma2(q, f, make_float2(0.0555071085691452f, 0.0555071085691452f));
+  q = ffma2(q, f, make_float2(0.24022246897220612f, 0.24022246897220612f));
+  q = ffma2(q, f, make_float2(0.6931470036506653f, 0.6931470036506653f));
+  q = ffma2(q, f, make_float2(1.f, 1.f));
   // 2^n from the exponent field (0 for n = -127)
   return make_float2(q.x * __uint_as_float(__float_as_uint(t.x) * 0x800000u + 0x3F800000u),
                      q.y * __uint_as_float(__float_as_uint(t.y) * 0x800000u + 0x3F800000u));
