@@ -241,7 +241,7 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const PairLogitsArgs
           }
           const float2 a = *reinterpret_cast<const float2*>(&cs[hb + e]), b = *reinterpret_cast<const float2*>(&cb[hb + e]);
           const float2 v = ffma2(rl2, make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), ffma2(nm2, a, b));
-          const __half2 own2 = __hmax2(__hmin2(__floats2half2_rn(v.x, v.y), lim), __hneg2(lim));
+          const __half2 own2 = __hmin2(__hmax2(__floats2half2_rn(v.x, v.y), __hneg2(lim)), lim);  // (NaN: -60000)
           const uint32_t own = *reinterpret_cast<const uint32_t*>(&own2);
           const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
           if (kstore) *reinterpret_cast<uint32_t*>(d) = __byte_perm(own, other, sel) & keep;

@@ -158,3 +158,17 @@ def test_pair_logits_prepared(ops, n, h):
     ref = ref.permute(2, 0, 1) * 1.4426950408889634
     assert relf(out[..., :n].cpu(), ref) < 4e-4  # float16 output rounding only
     assert float(out[..., n:].float().abs().sum()) == 0.0
+
+
+def test_pair_logits_of_undefined_tokens(ops):
+    """A token that holds NaN or infinities gets logits of -60000 (its key is left out), as from ``prepare_pair_bias``."""
+    g = torch.Generator().manual_seed(3)
+    pair = torch.randn(20, 20, 128, generator=g)
+    pair[4, 7, 3], pair[5, 11, 60], pair[19, 19, 127] = float("nan"), float("inf"), float("-inf")
+    out = ops.pair_logits_prepared(pair.to(BF).cuda(), None, None, torch.randn(32, 128, generator=g).cuda())
+    want = ops.prepare_pair_bias(torch.full((1, 8, 8), float("nan"), device="cuda"))
+    ops.synchronize_and_check()
+    assert (want == -60000).all()
+    bad = torch.zeros(20, 24, dtype=torch.bool, device="cuda")
+    bad[4, 7] = bad[5, 11] = bad[19, 19] = True
+    assert (out[:, bad] == -60000).all() and (out[:, ~bad].abs() < 1000).all()
