@@ -335,15 +335,18 @@ def prepare_pair_bias(pair_bias: torch.Tensor) -> torch.Tensor:
 
 def pair_logits_prepared(pair: torch.Tensor, gamma, beta, w: torch.Tensor) -> torch.Tensor:
     """pair bf16 [N, N, 128], w float32 [H, 128] -> float16 [H, N, pad8(N)]: the projection of LayerNorm(pair) to H heads in
-    the form of ``prepare_pair_bias``."""
+    the form of ``prepare_pair_bias``.  (The kernel takes heads in sixteens: others are filled up with zero weights.)"""
     _need_cuda(pair, gamma, beta, w)
+    h = w.shape[0]
+    if h % 16:
+        w = torch.nn.functional.pad(w, (0, 0, 0, -h % 16))
     assert pair.dtype == BF16 and pair.is_contiguous() and pair.shape[0] == pair.shape[1] and pair.shape[2] == 128
     dev = _dev(pair)
-    n, h = pair.shape[0], w.shape[0]
-    out = torch.empty(h, n, (n + 7) // 8 * 8, dtype=torch.float16, device=pair.device)
-    check(load().xfold_pair_logits_prepared_fwd(ctx(dev), _ptr(pair), n, _ptr(gamma), _ptr(beta), _ptr(w), h, _ptr(out),
+    n, hp = pair.shape[0], w.shape[0]
+    out = torch.empty(hp, n, (n + 7) // 8 * 8, dtype=torch.float16, device=pair.device)
+    check(load().xfold_pair_logits_prepared_fwd(ctx(dev), _ptr(pair), n, _ptr(gamma), _ptr(beta), _ptr(w), hp, _ptr(out),
                                                 _stream(dev)), dev, "xfold_pair_logits_prepared_fwd")
-    return out
+    return out[:h]
 
 
 def attention_pair_bias_core(xn: torch.Tensor, w: PackedSelfAttention, pair_bias: torch.Tensor,

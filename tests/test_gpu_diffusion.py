@@ -40,6 +40,24 @@ def test_diffusion_transformer(ops, oracle, n, samples, blocks):
     assert relf((got - act.float())[:, valid], (ref - act.float())[:, valid]) < 3e-2
 
 
+@pytest.mark.parametrize("blocks,super_block", [(3, 1), (4, 2)])
+def test_diffusion_transformer_of_four_heads(ops, oracle, blocks, super_block):
+    """Head counts that do not fill the sixteens in which the pair logits are computed; a narrow model."""
+    from distributed_xfold_b200 import diffusion
+    n, samples, c, heads = 70, 3, 128, 4
+    g = torch.Generator().manual_seed(blocks)
+    st = oracle.make_diffusion_transformer_state(g, "", c, 384, 128, heads, blocks, super_block)
+    act, cond = torch.randn(samples, n, c, generator=g).to(BF), torch.randn(n, 384, generator=g).to(BF)
+    pair, mask = torch.randn(n, n, 128, generator=g).to(BF), (torch.rand(n, generator=g) > 0.1).float()
+    with torch.no_grad():
+        ref = oracle.diffusion_transformer({k: v.to(BF).float() for k, v in st.items()}, "", act.float(), mask, cond.float(),
+                                           pair.float(), heads, blocks, super_block)
+    model = diffusion.PackedDiffusionTransformer(st, "", "cuda", heads, blocks, super_block)
+    got = model.forward(act.cuda(), mask.cuda(), cond.cuda(), model.pair_logits(pair.cuda()))
+    ops.synchronize_and_check()
+    assert relf(got.float().cpu()[:, mask > 0], ref[:, mask > 0]) < 2e-2
+
+
 def test_diffusion_single_sample_2d_input(ops, oracle):
     """[N, 768] activations (use_batch_infer False in the reference) take the same path."""
     from distributed_xfold_b200 import diffusion
@@ -143,7 +161,7 @@ def test_sampler_loop_around_the_gpu_transformer(ops, oracle):
     assert relf(got, ref) < 2e-2
 
 
-@pytest.mark.parametrize("n,h", [(1, 16), (77, 64), (128, 144), (130, 128), (257, 384)])
+@pytest.mark.parametrize("n,h", [(1, 16), (77, 64), (128, 144), (130, 128), (257, 384), (50, 4), (65, 12), (130, 132)])
 def test_pair_logits_prepared(ops, n, h):
     """LayerNorm + projection to the prepared pair bias at tile edges, ragged rows and head counts that fill the last
     group of heads only in part; rows with a mean well away from zero; zero in the padding columns."""
