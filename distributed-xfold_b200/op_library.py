@@ -57,7 +57,7 @@ def _pad_to(n: int, block: int) -> int:
 
 
 def _key(*ts) -> Tuple:
-    return tuple((t.untyped_storage()._cdata, t.data_ptr(), t._version, t.dtype, tuple(t.shape), t.stride()) for t in ts)
+    return tuple((t.untyped_storage()._cdata, t.data_ptr(), t._version, t.dtype, t.shape, t.stride()) for t in ts)
 
 
 def _cached(name, tensors, make):
@@ -124,7 +124,7 @@ def _grid_self_attn(q_data, bias, nonbatched_bias, query_w, key_w, value_w, gati
     out = torch.empty(b, sp, w_out.shape[0], dtype=BF16, device=dev)
     rc = lib.xfold_grid_attention_fwd(ctx(di), x.data_ptr(), b, s, c, h, w_qkvg.data_ptr(), scale.data_ptr(), nb.data_ptr(),
                                       bias.data_ptr(), s if bias.shape[0] >= b else 0, w_out.data_ptr(), w_out.shape[0],
-                                      out.data_ptr(), sp, ws.data_ptr(), ws.numel(), torch.cuda.current_stream(di).cuda_stream)
+                                      out.data_ptr(), sp, ws.data_ptr(), ws.numel(), ops._stream(di))
     check(rc, di, "xfold_grid_attention_fwd")
     return out.to(q_data.dtype)
 
@@ -183,7 +183,7 @@ def _transition(act, transition1, transition2, layernorm_weight, layernorm_bias)
     lib = load()
     ws = ops._Workspace.get(di, lib.xfold_transition_workspace_bytes(rows, w.C, w.F))
     rc = lib.xfold_transition_update_fwd(ctx(di), x.data_ptr(), upd.data_ptr(), rows, w.C, w.F, C.byref(w.c), ws.data_ptr(),
-                                         ws.numel(), torch.cuda.current_stream(di).cuda_stream)
+                                         ws.numel(), ops._stream(di))
     check(rc, di, "xfold_transition_update_fwd")
     return upd.to(act.dtype)
 
@@ -225,7 +225,7 @@ def _traingle_multiplication(act, mask, equation_flag, left_norm_input_weight, l
     outgoing = 1 if int(equation_flag) == 0 else 0   # flag 0: "ikc,jkc->ijc" (TriangleMultiplication.py:37-41)
     rc = lib.xfold_triangle_multiplication_update_fwd(ctx(di), z.data_ptr(), upd.data_ptr(), m.data_ptr(), n, outgoing,
                                                       C.byref(w.c), ws.data_ptr(), ws.numel(),
-                                                      torch.cuda.current_stream(di).cuda_stream)
+                                                      ops._stream(di))
     check(rc, di, "xfold_triangle_multiplication_update_fwd")
     np_ = _pad_to(n, TRI_BLOCKSIZE)
     if np_ != n:

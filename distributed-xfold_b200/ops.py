@@ -6,7 +6,9 @@ the CPU and nothing falls back to eager PyTorch.
 from __future__ import annotations
 
 import ctypes as C
-from typing import Dict, Optional
+import threading
+from collections import OrderedDict
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -21,8 +23,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+def _stream(device: int) -> int:
+    return torch._C._cuda_getCurrentRawStream(device)   # (without the Stream object of torch.cuda.current_stream)
 
 
 def _need_cuda(*ts):
@@ -36,17 +38,36 @@ def _dev(t: torch.Tensor) -> int:
 
 
 class _Workspace:
-    """Grow-only scratch buffer per device, reused by every operator call on that device."""
-    _bufs: Dict[int, torch.Tensor] = {}
+    """Scratch of the operator calls: one grow-only buffer per device and stream, allocated on that stream, so that calls on
+    different streams never share one and a buffer that is given up is reused behind the calls that still read it.  The
+    streams used last keep theirs (``KEEP``); ``release`` gives all back.  A call that is being captured into a graph gets
+    memory of the graph's own."""
+    KEEP = 8
+    _bufs: "OrderedDict[Tuple[int, int], torch.Tensor]" = OrderedDict()
+    _lock = threading.Lock()
 
     @classmethod
     def get(cls, device: int, nbytes: int) -> torch.Tensor:
-        b = cls._bufs.get(device)
-        if b is None or b.numel() < nbytes:
-            cls._bufs[device] = None
-            b = torch.empty(int(nbytes), dtype=torch.uint8, device=f"cuda:{device}")
-            cls._bufs[device] = b
-        return b
+        new = lambda: torch.empty(int(nbytes), dtype=torch.uint8, device=f"cuda:{device}")
+        if torch._C._cuda_isCurrentStreamCapturing():
+            return new()
+        key = (device, _stream(device))
+        with cls._lock:
+            b = cls._bufs.get(key)
+            if b is None or b.numel() < nbytes:
+                cls._bufs.pop(key, None)
+                b = None   # the former one is free before the new one is asked for
+                b = cls._bufs[key] = new()
+                if len(cls._bufs) > cls.KEEP:
+                    cls._bufs.popitem(last=False)
+            else:
+                cls._bufs.move_to_end(key)
+            return b
+
+    @classmethod
+    def release(cls) -> None:
+        with cls._lock:
+            cls._bufs.clear()
 
 
 def synchronize_and_check(device: Optional[int] = None) -> None:
