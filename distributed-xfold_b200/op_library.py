@@ -57,7 +57,11 @@ def _pad_to(n: int, block: int) -> int:
 
 
 def _key(*ts) -> Tuple:
-    return tuple((t.untyped_storage()._cdata, t.data_ptr(), t._version, t.dtype, t.shape, t.stride()) for t in ts)
+    return tuple([(t.untyped_storage()._cdata, t.data_ptr(), t._version, t.dtype, t.shape, t.stride()) for t in ts])
+
+
+def _gone(refs) -> bool:
+    return any(map(torch.UntypedStorage._expired, [r.cdata for r in refs]))   # (r.expired(), at a sixth of the time)
 
 
 def _cached(name, tensors, make):
@@ -67,13 +71,13 @@ def _cached(name, tensors, make):
     cache with the next new one."""
     k = (name,) + _key(*tensors)
     hit = _CACHE.get(k)
-    if hit is not None and not any(r.expired() for r in hit[1]):
+    if hit is not None and not _gone(hit[1]):
         return hit[0]
     v = make()
     on_gpu = tensors[0].is_cuda
     if on_gpu:
         torch.cuda.current_stream(tensors[0].device).synchronize()   # any stream may use the packed form from now on
-    gone = [e for e, (_, refs) in list(_CACHE.items()) if any(r.expired() for r in refs)]
+    gone = [e for e, (_, refs) in list(_CACHE.items()) if _gone(refs)]
     if len(_CACHE) - len(gone) > 4096:
         gone = list(_CACHE)
     if gone and on_gpu:
