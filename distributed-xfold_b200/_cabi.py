@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from typing import Optional
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -170,21 +171,25 @@ class XfoldError(RuntimeError):
 
 
 _ctxs = {}
+_ctxs_lock = threading.Lock()
 
 
 def ctx(device: int) -> int:
     """Per-device context handle (created on first use; needs an sm_100 GPU)."""
     h = _ctxs.get(device)
-    if h is None:
-        lib = load()
-        out = vp()
-        rc = lib.xfold_ctx_create(device, C.byref(out))
-        if rc != XFOLD_OK or not out.value:
-            raise XfoldError(f"xfold_ctx_create(device={device}) failed with status {rc}: an sm_100 (B200) GPU "
-                             "and a CUDA 12.x driver are required")
-        h = out.value
-        _ctxs[device] = h
-    return h
+    if h is not None:
+        return h
+    with _ctxs_lock:
+        h = _ctxs.get(device)
+        if h is None:
+            lib = load()
+            out = vp()
+            rc = lib.xfold_ctx_create(device, C.byref(out))
+            if rc != XFOLD_OK or not out.value:
+                raise XfoldError(f"xfold_ctx_create(device={device}) failed with status {rc}: an sm_100 (B200) GPU "
+                                 "and a CUDA 12.x driver are required")
+            h = _ctxs[device] = out.value
+        return h
 
 
 def check(rc: int, device: int, what: str) -> None:

@@ -589,10 +589,8 @@ static int pairformer_fwd(Ctx* c, bf16* z, bf16* s, const float* pair_mask, cons
   StaticWeights sw(c);
   // (a stream that is being captured keeps to itself: the second stream would stay in capture after this call)
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  bool side = s && num_blocks > 1 && c->side && !c->prof_on &&
-              cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-  std::unique_lock<std::mutex> lock(c->side_mu, std::defer_lock);
-  if (side) lock.lock();
+  const bool side = s && num_blocks > 1 && c->side && !c->prof_on &&
+                    cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
   bool behind = false;  // the second stream has work that the first has not waited for
   int rc;
   auto all = [&]() -> int {
@@ -679,13 +677,16 @@ long long xfold_launch_count(xfold_ctx* c) { return c ? c->launch_count : 0; }
 
 int xfold_profile_enable(xfold_ctx* c, int on) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   c->prof_on = on;
   return XFOLD_OK;
 }
 
 int xfold_profile_read(xfold_ctx* c, int kernel_class, float* ms_total, int* launches) {
   if (!c || !ms_total || !launches) return XFOLD_ERR_ARG;
-  if (cudaDeviceSynchronize() != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "profile read: device error");
+  const bool synced = cudaDeviceSynchronize() == cudaSuccess;
+  CallLock call(c);
+  if (!synced) return fail(c, XFOLD_ERR_LAUNCH, "profile read: device error");
   float total = 0.f;
   int n = 0;
   std::vector<ProfRec> keep;
@@ -707,10 +708,13 @@ int xfold_check_status(xfold_ctx* c, void* stream) {
   int h = 0;
   cudaError_t e = cudaMemcpyAsync(&h, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "status read: %s", cudaGetErrorString(e));
-  if (h != 0) {
+  if (e == cudaSuccess && h != 0) {
     cudaMemsetAsync(c->d_status, 0, sizeof(int), st);
     cudaStreamSynchronize(st);
+  }
+  CallLock call(c);
+  if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "status read: %s", cudaGetErrorString(e));
+  if (h != 0) {
     return fail(c, XFOLD_ERR_TIMEOUT, "in-kernel bounded wait ran out (code %d)", h);
   }
   return XFOLD_OK;
@@ -721,6 +725,7 @@ int xfold_layernorm_fwd(xfold_ctx* c, const void* x, long long ldx, void* y, lon
                         float* proj, long long proj_plane, const void* mod_scale, const void* mod_shift, int mod_rows,
                         void* stream) {
   if (!c || !x) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (num_proj > 0 && (!proj_w || !proj)) return fail(c, XFOLD_ERR_ARG, "layernorm: projection requested without buffers");
   if ((mod_scale != nullptr) != (mod_shift != nullptr) || (mod_scale && mod_rows <= 0))
     return fail(c, XFOLD_ERR_ARG, "layernorm: modulation needs scale, shift and mod_rows");
@@ -730,12 +735,14 @@ int xfold_layernorm_fwd(xfold_ctx* c, const void* x, long long ldx, void* y, lon
 
 int xfold_swiglu_fwd(xfold_ctx* c, const void* in, void* out, long long rows, int F, void* stream) {
   if (!c || !in || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return launch_swiglu(c, (const bf16*)in, (bf16*)out, rows, F, (cudaStream_t)stream);
 }
 
 int xfold_linear_fwd(xfold_ctx* c, const void* x, long long ldx, long long M, int K, const void* w, int N,
                      const float* bias, const float* scale, void* out, long long ldo, void* stream) {
   if (!c || !x || !w || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return linear_plain(c, (const bf16*)x, ldx, M, K, (const bf16*)w, N, bias, scale, (bf16*)out, ldo, (cudaStream_t)stream);
 }
 
@@ -743,6 +750,7 @@ int xfold_linear_gate_residual_fwd(xfold_ctx* c, const void* x, long long ldx, l
                                    const void* gate, long long ldg, int row_gate_mod, const void* resid, long long ldr,
                                    void* out, long long ldo, void* stream) {
   if (!c || !x || !w || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return linear_gate_resid(c, (const bf16*)x, ldx, M, K, (const bf16*)w, N, (const bf16*)gate, ldg, row_gate_mod,
                            (const bf16*)resid, ldr, (bf16*)out, ldo, (cudaStream_t)stream);
 }
@@ -750,6 +758,7 @@ int xfold_linear_gate_residual_fwd(xfold_ctx* c, const void* x, long long ldx, l
 int xfold_linear_swiglu_fwd(xfold_ctx* c, const void* x, long long ldx, long long M, int K, const void* w_packed, int F,
                             void* out, long long ldo, void* stream) {
   if (!c || !x || !w_packed || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return linear_swiglu(c, (const bf16*)x, ldx, M, K, (const bf16*)w_packed, F, (bf16*)out, ldo, (cudaStream_t)stream);
 }
 
@@ -757,6 +766,7 @@ int xfold_batched_contract_fwd(xfold_ctx* c, const void* a, const void* b, void*
                                long long ld, long long chan_stride_a, long long chan_stride_b, long long ldo,
                                long long chan_stride_o, void* stream) {
   if (!c || !a || !b || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return batched_contract(c, (const bf16*)a, (const bf16*)b, (bf16*)out, channels, Mi, Nj, Kk, ld, chan_stride_a,
                           chan_stride_b, ldo, chan_stride_o, (cudaStream_t)stream);
 }
@@ -765,6 +775,7 @@ size_t xfold_trimul_workspace_bytes(int N) { return carve_trimul(nullptr, 0, N).
 int xfold_triangle_multiplication_fwd(xfold_ctx* c, void* z, const float* mask, int N, int outgoing,
                                       const xfold_trimul_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return trimul_fwd(c, (bf16*)z, mask, N, outgoing, w, ws, ws_bytes, (cudaStream_t)stream);
 }
 
@@ -772,6 +783,7 @@ size_t xfold_triattn_workspace_bytes(int N) { return carve_triattn(nullptr, 0, N
 int xfold_triangle_attention_fwd(xfold_ctx* c, void* z, const float* mask, int N, int transpose,
                                  const xfold_triattn_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return triattn_fwd(c, (bf16*)z, mask, N, transpose, w, ws, ws_bytes, (cudaStream_t)stream);
 }
 
@@ -781,6 +793,7 @@ size_t xfold_transition_workspace_bytes(long long rows, int C, int F) {
 int xfold_transition_fwd(xfold_ctx* c, void* x, long long rows, int C, int F, const xfold_transition_weights* w, void* ws,
                          size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return transition_fwd(c, (bf16*)x, rows, C, F, w, ws, ws_bytes, (cudaStream_t)stream);
 }
 
@@ -790,6 +803,7 @@ int xfold_attention_pair_bias_core_fwd(xfold_ctx* c, const void* xn, int B, int 
                                        const float* pair_bias, const float* mask, void* out, void* ws, size_t ws_bytes,
                                        void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return apb_core_fwd(c, (const bf16*)xn, B, S, C, H, Dp, (const bf16*)w_qkvg, qkvg_bias, qkvg_scale, pair_bias, nullptr,
                       mask, (bf16*)out, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -798,12 +812,14 @@ size_t xfold_pairformer_workspace_bytes(int N) { return carve_pairformer(nullptr
 int xfold_pairformer_block_fwd(xfold_ctx* c, void* z, void* s, const float* pair_mask, const float* seq_mask, int N,
                                const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (!w) return fail(c, XFOLD_ERR_ARG, "pairformer: null argument");
   return pairformer_fwd(c, (bf16*)z, (bf16*)s, pair_mask, seq_mask, N, w, 1, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 int xfold_pair_bias_prepare_fwd(xfold_ctx* c, const float* pair_bias, int H, int S, void* prepared, void* stream) {
   if (!c || !pair_bias || !prepared) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return launch_bias_transpose(c, pair_bias, (bf16*)prepared, H, S, pad8(S), (cudaStream_t)stream);
 }
 
@@ -812,6 +828,7 @@ int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* c, const void* xn, in
                                                 const void* prepared_bias, const float* mask, void* out, void* ws,
                                                 size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return apb_core_fwd(c, (const bf16*)xn, B, S, C, H, Dp, (const bf16*)w_qkvg, qkvg_bias, qkvg_scale, nullptr,
                       (const bf16*)prepared_bias, mask, (bf16*)out, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -820,6 +837,7 @@ int xfold_gated_attention_core_fwd(xfold_ctx* c, const void* xn, int B, int S, i
                                    const float* qkvg_bias, const float* qkvg_scale, const float* pair_bias,
                                    const float* mask, long long mask_ld, void* out, void* ws, size_t ws_bytes, void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return apb_core_fwd(c, (const bf16*)xn, B, S, C, H, Dp, (const bf16*)w_qkvg, qkvg_bias, qkvg_scale, pair_bias, nullptr,
                       mask, (bf16*)out, ws, ws_bytes, (cudaStream_t)stream, mask_ld);
 }
@@ -831,6 +849,7 @@ int xfold_grid_attention_fwd(xfold_ctx* c, const void* x, int B, int S, int C, i
                              const float* pair_bias, const float* mask_bias, long long mask_ld, const void* w_out, int C_out,
                              void* out, int SP, void* ws, size_t ws_bytes, void* stream) {
   if (!c || !x || !w_qkvg || !pair_bias || !w_out || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return grid_attention_fwd(c, (const bf16*)x, B, S, C, H, (const bf16*)w_qkvg, qkvg_scale, pair_bias, mask_bias, mask_ld,
                             (const bf16*)w_out, C_out, (bf16*)out, SP, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -839,6 +858,7 @@ int xfold_pairformer_stack_fwd(xfold_ctx* c, void* z, void* s, const float* pair
                                const xfold_pairformer_weights* blocks, int num_blocks, void* ws, size_t ws_bytes,
                                void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (num_blocks < 0 || (num_blocks > 0 && !blocks)) return fail(c, XFOLD_ERR_ARG, "pairformer stack: no weights for %d blocks", num_blocks);
   return pairformer_fwd(c, (bf16*)z, (bf16*)s, pair_mask, seq_mask, N, blocks, num_blocks, ws, ws_bytes, (cudaStream_t)stream);
 }
@@ -847,6 +867,7 @@ int xfold_pairformer_stack_fwd(xfold_ctx* c, void* z, void* s, const float* pair
 int xfold_trimul_project_fwd(xfold_ctx* c, const void* z, const float* mask, int R, int N, const xfold_trimul_weights* w,
                              void* x_scratch, void* a, void* b, void* g, int ld, void* stream) {
   if (!c || !z || !w || !x_scratch || !a || !b || !g) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (ld < N || (ld & 7)) return fail(c, XFOLD_ERR_ARG, "trimul project: ld must be >= N and a multiple of 8");
   return trimul_project(c, (const bf16*)z, mask, R, N, 0, w, (bf16*)a, (bf16*)b, (bf16*)g, ld,
                         (long long)128 * ld, (cudaStream_t)stream);
@@ -854,6 +875,7 @@ int xfold_trimul_project_fwd(xfold_ctx* c, const void* z, const float* mask, int
 int xfold_trimul_contract_fwd(xfold_ctx* c, const void* a, const void* b_full, int R, int Nj, int K, int ld, void* o, int ldo,
                               void* stream) {
   if (!c || !a || !b_full || !o) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if ((ld & 7) || (ldo & 7)) return fail(c, XFOLD_ERR_ARG, "contract: leading dimensions must be multiples of 8");
   return trimul_contract(c, (const bf16*)a, ld, (long long)128 * ld, (const bf16*)b_full, ld, (long long)128 * ld, R, Nj, K,
                          (bf16*)o, ldo, (long long)128 * ldo, (cudaStream_t)stream);
@@ -861,6 +883,7 @@ int xfold_trimul_contract_fwd(xfold_ctx* c, const void* a, const void* b_full, i
 int xfold_trimul_contract_planes_fwd(xfold_ctx* c, const void* a, const void* b, int channels, int Ni, int Nj, int K, int ld,
                                      void* o, int ldo, void* stream) {
   if (!c || !a || !b || !o) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if ((ld & 7) || (ldo & 7) || channels < 1) return fail(c, XFOLD_ERR_ARG, "contract: leading dimensions must be multiples of 8");
   return trimul_contract(c, (const bf16*)a, (long long)Ni * ld, ld, (const bf16*)b, (long long)Nj * ld, ld, Ni, Nj, K, (bf16*)o,
                          (long long)Ni * ldo, ldo, (cudaStream_t)stream, channels);
@@ -868,11 +891,13 @@ int xfold_trimul_contract_planes_fwd(xfold_ctx* c, const void* a, const void* b,
 int xfold_trimul_output_fwd(xfold_ctx* c, const void* o, int ldo, const void* g, int R, int N, const xfold_trimul_weights* w,
                             void* x_scratch, void* z, void* stream) {
   if (!c || !o || !g || !w || !x_scratch || !z) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return trimul_output(c, (const bf16*)o, ldo, (long long)128 * ldo, (const bf16*)g, R, N, w, (bf16*)z, (cudaStream_t)stream);
 }
 int xfold_triattn_bias_fwd(xfold_ctx* c, const void* z, int R, int N, const xfold_triattn_weights* w, void* x, void* biasT,
                            int pitch, long long plane, int rows_are_keys, void* stream) {
   if (!c || !z || !w || !x || !biasT) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return triattn_bias(c, (const bf16*)z, R, N, w, (bf16*)x, (bf16*)biasT, pitch, plane, rows_are_keys, (cudaStream_t)stream);
 }
 size_t xfold_triattn_core_scratch_bytes(int R, int N, size_t* mext_bytes) {
@@ -883,12 +908,14 @@ int xfold_triattn_core_fwd(xfold_ctx* c, void* x, const void* biasT, int ldq, co
                            int N, const xfold_triattn_weights* w, void* qkvg_scratch, void* mext_scratch, void* z,
                            void* stream) {
   if (!c || !x || !biasT || !w || !qkvg_scratch || !mext_scratch || !z) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return triattn_core(c, (bf16*)x, (const bf16*)biasT, ldq, mask, mask_ld, R, N, 0, w, (bf16*)qkvg_scratch,
                       (bf16*)mext_scratch, (bf16*)z, (cudaStream_t)stream);
 }
 int xfold_pair_logits_fwd(xfold_ctx* c, const void* z, int R, int N, const float* ln_gamma, const float* ln_beta,
                           const float* w16, void* plT, int pitch, long long plane, int rows_are_keys, void* stream) {
   if (!c || !z || !w16 || !plT) return XFOLD_ERR_ARG;
+  CallLock call(c);
   const long long M = (long long)R * N;
   return launch_ln_rows(c, (const bf16*)z, 128, nullptr, 128, M, 128, ln_gamma, ln_beta, 1e-5f, 16, w16, nullptr, plane,
                         nullptr, nullptr, 0, (cudaStream_t)stream, (bf16*)plT, rows_are_keys ? R : -N, rows_are_keys ? N : 0,
@@ -898,6 +925,7 @@ size_t xfold_single_update_workspace_bytes(int N) { return single_ws_bytes(N); }
 int xfold_single_update_fwd(xfold_ctx* c, void* s, const void* plT, int ldq, const float* seq_mask, int N,
                             const xfold_pairformer_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c || !s || !plT || !w) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return single_update(c, (bf16*)s, (const bf16*)plT, ldq, seq_mask, N, w, ws, ws_bytes, (cudaStream_t)stream);
 }
 
@@ -907,16 +935,19 @@ int xfold_triangle_multiplication_update_fwd(xfold_ctx* c, const void* z, void* 
                                              int outgoing, const xfold_trimul_weights* w, void* ws, size_t ws_bytes,
                                              void* stream) {
   if (!c || !update) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return trimul_fwd(c, (bf16*)const_cast<void*>(z), mask, N, outgoing, w, ws, ws_bytes, (cudaStream_t)stream, (bf16*)update);
 }
 int xfold_triangle_attention_update_fwd(xfold_ctx* c, const void* z, void* update, const float* mask, int N, int transpose,
                                         const xfold_triattn_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c || !update) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return triattn_fwd(c, (bf16*)const_cast<void*>(z), mask, N, transpose, w, ws, ws_bytes, (cudaStream_t)stream, (bf16*)update);
 }
 int xfold_transition_update_fwd(xfold_ctx* c, const void* x, void* update, long long rows, int C, int F,
                                 const xfold_transition_weights* w, void* ws, size_t ws_bytes, void* stream) {
   if (!c || !update) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return transition_fwd(c, (bf16*)const_cast<void*>(x), rows, C, F, w, ws, ws_bytes, (cudaStream_t)stream, (bf16*)update);
 }
 
@@ -932,6 +963,7 @@ size_t xfold_transition_static_max_bytes(void) { return XFOLD_STATIC_SCRATCH_BYT
 int xfold_transition_static_fwd(xfold_ctx* c, void* x, long long rows, int C, int F, const xfold_transition_weights* w,
                                 void* stream) {
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (rows < 0 || C <= 0 || F <= 0 || rows >= (1ll << 31))
     return fail(c, XFOLD_ERR_ARG, "transition (static scratch): bad shape (%lld rows, C=%d, F=%d)", rows, C, F);
   const size_t need = xfold_transition_workspace_bytes(rows, C, F);

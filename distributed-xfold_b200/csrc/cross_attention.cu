@@ -232,6 +232,7 @@ int xfold_cross_attention_fwd(xfold_ctx* cx, const void* q_data, const void* m_d
                               const float* bias, void* out, void* ws, size_t ws_bytes, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !q_data || !m_data || !w_qg || !w_kv || !bias || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (D != 16 && D != 32 && D != 64) return fail(c, XFOLD_ERR_ARG, "cross attention: head dimension 16, 32 or 64");
   if (B <= 0 || S <= 0 || K <= 0) return XFOLD_OK;
   const int W = H * D;

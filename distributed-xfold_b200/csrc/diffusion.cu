@@ -234,6 +234,7 @@ int xfold_diffusion_transformer_fwd(xfold_ctx* cx, void* act, int S, int N, cons
                                     size_t ws_bytes, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !act || !single_cond || !w || !w->blocks || !w->w_mod || !w->b_mod || !w->w_gate || !w->ln_cond || !pair_logits) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return diffusion_fwd(c, (bf16*)act, S, N, mask, (const bf16*)single_cond, w, pair_logits, ws, ws_bytes, (cudaStream_t)stream);
 }
 

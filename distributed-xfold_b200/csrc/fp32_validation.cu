@@ -417,6 +417,7 @@ int xfold_pairformer_stack_f32_fwd(xfold_ctx* cx, float* z, float* s, const floa
                                    void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (num_blocks < 0 || (num_blocks > 0 && !blocks)) return fail(c, XFOLD_ERR_ARG, "fp32 validation: no weights for %d blocks", num_blocks);
   if (N <= 0 || N > 2048) return fail(c, XFOLD_ERR_ARG, "fp32 validation: 1 to 2048 tokens");
   for (int i = 0; i < num_blocks; ++i) {

@@ -20,7 +20,12 @@ struct ProfRec {
   int tag;
 };
 
+// Everything below that changes after creation (counters, the error text, what a call sets for its launches, the second
+// stream and its events) belongs to the call that holds `mu`: every entry point takes it (CallLock) while it issues its
+// launches, so several host threads may use one context.  The launches of a call are then together in its stream, and calls
+// of several threads on one stream may use the same scratch.
 struct Ctx {
+  std::mutex mu;
   int device = 0;
   int sm_count = 148;
   int* d_status = nullptr;  // one word: first in-kernel error code (0 = ok)
@@ -36,11 +41,15 @@ struct Ctx {
   int gemm_sms = 0;      // SMs a GEMM launch may take (0: all)
   int peer_cta_cap = 0;  // CTAs of a peer exchange kernel (0: its own default)
   std::vector<ProfRec> prof_recs, prof_pool;
-  // Second stream of the one-GPU trunk: the single representation's kernels of a block run beside the next block's.  One
-  // call at a time uses it (side_mu is held while the call issues its work; events are captured by the waits as they are issued).
+  // Second stream of the one-GPU trunk: the single representation's kernels of a block run beside the next block's.  (Events
+  // are captured by the waits as they are issued: the next call may use them again.)
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  std::mutex side_mu;
+};
+
+struct CallLock {
+  std::lock_guard<std::mutex> lock;
+  explicit CallLock(Ctx* c) : lock(c->mu) {}
 };
 
 // Brackets one kernel launch with events on its stream while profiling is enabled, and counts it.

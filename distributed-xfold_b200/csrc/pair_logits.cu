@@ -297,5 +297,6 @@ extern "C" int xfold_pair_logits_prepared_fwd(xfold_ctx* cx, const void* pair, i
                                               const float* w, int H, void* prepared, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !pair || !w || !prepared) return XFOLD_ERR_ARG;
+  CallLock call(c);
   return launch_pair_logits(c, (const bf16*)pair, N, ln_gamma, ln_beta, w, H, prepared, (cudaStream_t)stream);
 }

@@ -271,6 +271,7 @@ int xfold_transpose_scatter_fwd(xfold_ctx* cx, const void* z, int R, int N, int 
                                 const int* col_starts, int world, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !z || !peer_bufs || !col_starts) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (world < 1 || world > MAX_PEERS) return fail(c, XFOLD_ERR_ARG, "transpose: 1 to %d ranks supported, got %d", MAX_PEERS, world);
   return launch_transpose_scatter(c, (const bf16*)z, R, N, row0, peer_bufs, col_starts, world, (cudaStream_t)stream);
 }
@@ -279,6 +280,7 @@ int xfold_trimul_scatter_channels_fwd(xfold_ctx* cx, const void* a, const void* 
                                       void* const* peer_a, void* const* peer_b, int world, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !a || !b || !peer_a || !peer_b) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (world < 1 || world > MAX_PEERS || 128 % world) return fail(c, XFOLD_ERR_ARG, "channel scatter: the rank count must divide 128 (1, 2, 4, 8), got %d", world);
   if (ld & 7) return fail(c, XFOLD_ERR_ARG, "channel scatter: ld must be a multiple of 8");
   return launch_channel_scatter(c, (const bf16*)a, (const bf16*)b, R, N, ld, row0, peer_a, peer_b, world, (cudaStream_t)stream);
@@ -288,6 +290,7 @@ int xfold_trimul_scatter_rows_fwd(xfold_ctx* cx, const void* o, int channels, in
                                   void* const* peer_o, const int* row_starts, int world, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !o || !peer_o || !row_starts) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (world < 1 || world > MAX_PEERS) return fail(c, XFOLD_ERR_ARG, "row scatter: 1 to %d ranks supported, got %d", MAX_PEERS, world);
   if ((ldo & 7) || chan0 < 0 || chan0 + channels > 128) return fail(c, XFOLD_ERR_ARG, "row scatter: bad channel range or ldo");
   return launch_row_scatter(c, (const bf16*)o, channels, chan0, N, ldo, peer_o, row_starts, world, (cudaStream_t)stream);
@@ -297,6 +300,7 @@ int xfold_peer_allgather_fwd(xfold_ctx* cx, const void* src, long long bytes, lo
                              int world, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !src || !peer_dst) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (world < 1 || world > MAX_PEERS) return fail(c, XFOLD_ERR_ARG, "peer all-gather: 1 to %d ranks supported, got %d", MAX_PEERS, world);
   if ((bytes & 15) || (offset_bytes & 15) || (reinterpret_cast<uintptr_t>(src) & 15))
     return fail(c, XFOLD_ERR_ARG, "peer all-gather: block, offset and source must be multiples of 16 bytes");
@@ -317,6 +321,7 @@ int xfold_peer_allgather_fwd(xfold_ctx* cx, const void* src, long long bytes, lo
 int xfold_peer_barrier(xfold_ctx* cx, void* const* peer_flags, int me, int world, int epoch, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !peer_flags) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (world < 1 || world > MAX_PEERS || me < 0 || me >= world) return fail(c, XFOLD_ERR_ARG, "peer barrier: bad rank %d / world %d", me, world);
   return launch_peer_barrier(c, peer_flags, me, world, epoch, (cudaStream_t)stream);
 }

@@ -240,6 +240,7 @@ void xfold_shard_ctx_destroy(xfold_shard_ctx* sc);
 int xfold_shard_ctx_create(xfold_ctx* cx, const xfold_shard_desc* d, xfold_shard_ctx** out) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !d || !out) return XFOLD_ERR_ARG;
+  CallLock call(c);
   *out = nullptr;
   if (d->world < 2 || d->world > SH_MAX || 128 % d->world || d->rank < 0 || d->rank >= d->world)
     return fail(c, XFOLD_ERR_ARG, "shard context: the rank count must be 2, 4 or 8 (it divides the 128 channels), got rank %d of %d",
@@ -304,6 +305,7 @@ int xfold_pairformer_stack_sharded_fwd(xfold_ctx* cx, xfold_shard_ctx* sc, int z
                                        void* ws, size_t ws_bytes, void* stream, int* z_slot_out) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !sc || !z_slot_out || (num_blocks > 0 && !blocks)) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if (z_slot != 0 && z_slot != 1) return fail(c, XFOLD_ERR_ARG, "sharded stack: z_slot must be 0 or 1");
   const ShardWs W = carve_shard(ws, ws_bytes, *sc);
   if (!ws || W.bytes > ws_bytes) return fail(c, XFOLD_ERR_ARG, "sharded stack: workspace too small (%zu < %zu)", ws_bytes, W.bytes);
@@ -321,6 +323,7 @@ int xfold_trimul_contract_planes_incoming_fwd(xfold_ctx* cx, const void* a, cons
                                               int ld, void* o, int ldo, void* stream) {
   Ctx* c = reinterpret_cast<Ctx*>(cx);
   if (!c || !a || !b || !o) return XFOLD_ERR_ARG;
+  CallLock call(c);
   if ((ld & 7) || (ldo & 7) || channels < 1) return fail(c, XFOLD_ERR_ARG, "contract: leading dimensions must be multiples of 8");
   return trimul_contract_mn(c, (const bf16*)b, (long long)Nk * ld, ld, (const bf16*)a, (long long)Nk * ld, ld, Ni, Nj, Nk,
                             (bf16*)o, (long long)Ni * ldo, ldo, (cudaStream_t)stream, channels);

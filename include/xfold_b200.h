@@ -7,6 +7,8 @@
  *  - all tensor arguments are DEVICE pointers owned by the caller; activations and weights are
  *    bf16 (passed as void*), masks / LayerNorm parameters / biases are float32;
  *  - `stream` is a cudaStream_t passed as void*; calls are asynchronous on that stream;
+ *  - several host threads may use one context: a call holds its lock while it issues its launches, which are then together
+ *    in the stream (xfold_last_error() is about the last call that failed, whichever thread made it);
  *  - the library allocates nothing except the context (one status word on the device); scratch
  *    memory is passed in by the caller (`ws`, size from the matching *_workspace_bytes function);
  *  - kernels never wait unboundedly: a wait that runs out records a code in the context's status

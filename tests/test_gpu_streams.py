@@ -61,6 +61,36 @@ def test_calls_on_several_streams(ops, oracle, path, size):
             assert all(torch.equal(a, b) for a, b in zip(out, want[i]))
 
 
+@pytest.mark.parametrize("own_stream", [True, False])
+@pytest.mark.parametrize("paths", [(0, 0, 2), (1, 2, 2)])
+def test_calls_of_several_threads(ops, oracle, paths, own_stream):
+    """Threads with a stream each, or all on one stream (whose scratch they share)."""
+    import threading
+    calls = [CALLS[i][0](ops, oracle, **CALLS[i][1]) for i in paths]
+    want = [_alone(make, call, seed) for seed, (make, call) in enumerate(calls)]
+    inputs = [make(seed) for seed, (make, _) in enumerate(calls)]
+    torch.cuda.synchronize()
+    got, gate = [[] for _ in calls], threading.Barrier(len(calls))
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream() if own_stream else torch.cuda.default_stream()):
+            gate.wait()
+            for _ in range(20):
+                got[i].append(calls[i][1](*(t.clone() for t in inputs[i])))
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    ops.synchronize_and_check()
+    for i in range(len(calls)):
+        assert len(got[i]) == 20
+        for out in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(out, want[i]))
+
+
 def test_scratch_is_bounded_and_given_back(ops):
     ops._Workspace.release()
     streams = [torch.cuda.Stream() for _ in range(ops._Workspace.KEEP + 3)]
