@@ -91,6 +91,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  if (!p.static_w) pdl_wait();  // the parameters read below may come from the kernel before
   if (threadIdx.x >= 64 && threadIdx.x < 192) {
     gb[threadIdx.x - 64] = p.gamma ? p.gamma[threadIdx.x - 64] : 1.f;
     gb[threadIdx.x + 64] = p.beta ? p.beta[threadIdx.x - 64] : 0.f;
@@ -104,7 +105,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   const int mine = (p.items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
 
   if (warp == 0) {
-    if (!p.static_w) pdl_wait();
     const uint32_t go = elect_one();  // warp-uniform, like the issuers
     const long long nblk = (long long)mine * NBK;
     int hb1 = 0, hb2 = 0, t = blockIdx.x, xt = 0;

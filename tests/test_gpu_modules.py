@@ -366,3 +366,28 @@ def test_transition_tile_pairs(ops, oracle, rows):
     ops.transition_(xd, w)
     ops.synchronize_and_check()
     check_update(x, xd, ref)
+
+
+def test_transition_parameters_written_just_before(ops, oracle):
+    """LayerNorm parameters that the kernel right before the call writes are the new ones: here the last values of a long
+    projection, a kernel that lets its successor start early."""
+    from distributed_xfold_b200 import _cabi
+    g = torch.Generator().manual_seed(11)
+    st = oracle.make_transition_state(g, "", 128)
+    w = ops.PackedTransition(st, "", "cuda")
+    x = torch.randn(300, 128, generator=g).to(BF)
+    rows = 300_000
+    src, pw = torch.randn(rows, 128, generator=g).to(BF).cuda(), (torch.randn(4, 128, generator=g) / 11).cuda()
+    proj = torch.empty(4, rows, device="cuda")
+    w.c.ln_gamma, w.c.ln_beta = proj[0, -128:].data_ptr(), proj[1, -128:].data_ptr()
+    for _ in range(3):
+        xd = x.cuda()
+        proj.fill_(9.0)
+        rc = _cabi.load().xfold_layernorm_fwd(_cabi.ctx(0), src.data_ptr(), 128, None, 128, rows, 128, None, None, 1e-5, 4,
+                                              pw.data_ptr(), proj.data_ptr(), rows, None, None, 0, ops._stream(0))
+        ops.transition_(xd, w)
+        ops.synchronize_and_check()
+        st["input_layer_norm.weight"], st["input_layer_norm.bias"] = proj[0, -128:].cpu(), proj[1, -128:].cpu()
+        assert rc == 0 and float(proj.abs().max()) < 9.0
+        r = {k: v if v.dim() == 1 else v.to(BF).float() for k, v in st.items()}
+        check_update(x, xd, x.float() + oracle.transition(r, "", x.float()))
