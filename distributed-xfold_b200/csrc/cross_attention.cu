@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256, D == 64 ? 1 : 2) xattn_kernel(XAttnArgs p
       asm volatile("cp.async.commit_group;" ::: "memory");
       // meanwhile the bias, into the accumulators of the logits
       float s[16][4];
-      const bool pairs = (p.K & 1) == 0;
+      const bool pairs = ((p.K & 1) | (reinterpret_cast<uintptr_t>(p.bias) & 7)) == 0;  // two floats at a time where every row starts so
       if (active) {
 #pragma unroll
         for (int t = 0; t < 16; ++t) {

@@ -264,6 +264,23 @@ def test_cross_attention_tile_edges(ops, oracle, B, S, K, H, D):
     assert relf(out.float().cpu(), ref) < 2e-2
 
 
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_cross_attention_bias_at_any_element(ops, offset):
+    """A bias that is a view into a larger buffer starts at any float."""
+    g = torch.Generator().manual_seed(offset)
+    B, S, K, H, D, c = 3, 32, 128, 4, 32, 128
+    qw, kw, vw, gw = (torch.randn(c, H, D, generator=g) / 11 for _ in range(4))
+    w = ops.PackedCrossAttention(qw, torch.randn(1, H, D, generator=g), kw, vw, gw, "cuda")
+    qd, md = torch.randn(B, S, c, generator=g).to(BF).cuda(), torch.randn(B, K, c, generator=g).to(BF).cuda()
+    buf = torch.randn(B * H * S * K + 4, generator=g).cuda()
+    bias = buf[offset:offset + B * H * S * K].view(B, H, S, K)
+    assert bias.is_contiguous()
+    out = ops.cross_attention(qd, md, bias, w)
+    want = ops.cross_attention(qd, md, bias.clone(), w)
+    ops.synchronize_and_check()
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("B,S,C,H", [(4, 65, 384, 16), (3, 33, 384, 16), (1, 129, 384, 16), (2, 1100, 384, 16), (1, 64, 768, 16),
                                      (3, 400, 768, 16)])
 def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
