@@ -281,6 +281,26 @@ def test_cross_attention_bias_at_any_element(ops, offset):
     assert torch.equal(out, want)
 
 
+def test_cross_attention_result_at_any_element(ops):
+    """The C entry point writes to whatever element the caller's result starts at."""
+    from distributed_xfold_b200 import _cabi
+    g = torch.Generator().manual_seed(5)
+    B, S, K, H, D, c = 2, 19, 45, 4, 32, 128
+    qw, kw, vw, gw = (torch.randn(c, H, D, generator=g) / 11 for _ in range(4))
+    w = ops.PackedCrossAttention(qw, torch.randn(1, H, D, generator=g), kw, vw, gw, "cuda")
+    qd, md = torch.randn(B, S, c, generator=g).to(BF).cuda(), torch.randn(B, K, c, generator=g).to(BF).cuda()
+    bias = torch.randn(B, H, S, K, generator=g).cuda()
+    want = ops.cross_attention(qd, md, bias, w)
+    buf = torch.full((B * S * H * D + 2,), 9.0, dtype=BF, device="cuda")
+    lib = _cabi.load()
+    ws = ops._Workspace.get(0, lib.xfold_cross_attention_workspace_bytes(B, S, K, H, D))
+    rc = lib.xfold_cross_attention_fwd(_cabi.ctx(0), qd.data_ptr(), md.data_ptr(), B, S, K, c, c, H, D, w.w_qg.data_ptr(),
+                                       w.bias.data_ptr(), w.scale.data_ptr(), w.w_kv.data_ptr(), bias.data_ptr(),
+                                       buf[1:].data_ptr(), ws.data_ptr(), ws.numel(), ops._stream(0))
+    ops.synchronize_and_check()
+    assert rc == 0 and torch.equal(buf[1:-1].view_as(want), want) and buf[0] == 9.0 and buf[-1] == 9.0
+
+
 @pytest.mark.parametrize("B,S,C,H", [(4, 65, 384, 16), (3, 33, 384, 16), (1, 129, 384, 16), (2, 1100, 384, 16), (1, 64, 768, 16),
                                      (3, 400, 768, 16)])
 def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
