@@ -299,6 +299,7 @@ static int launch_ro(Ctx* c, const CUtensorMap& tmx, const CUtensorMap& tmz, con
     if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "row output smem attribute: %s", cudaGetErrorString(e));
     attr_done[c->device & 7] = true;
   }
+  if (reinterpret_cast<uintptr_t>(a.w) & 15) return fail(c, XFOLD_ERR_ARG, "row output: the weights must be 16-byte aligned");
   const int sms = c->gemm_sms > 0 && c->gemm_sms < c->sm_count ? c->gemm_sms : c->sm_count;
   a.static_w = c->static_weights;
   a.status = c->d_status;

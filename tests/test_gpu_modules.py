@@ -428,3 +428,23 @@ def test_transition_parameters_written_just_before(ops, oracle):
         assert rc == 0 and float(proj.abs().max()) < 9.0
         r = {k: v if v.dim() == 1 else v.to(BF).float() for k, v in st.items()}
         check_update(x, xd, x.float() + oracle.transition(r, "", x.float()))
+
+
+@pytest.mark.parametrize("kind", ["multiplication", "attention"])
+def test_unaligned_output_weights_are_refused(ops, oracle, kind):
+    """Weights that are a slice of a larger bf16 buffer, not at a multiple of 16 bytes: an error, and z as it was."""
+    from distributed_xfold_b200 import _cabi
+    g = torch.Generator().manual_seed(21)
+    st = {k: v.to(BF).cuda() for k, v in (oracle.make_trimul_state(g, "") if kind == "multiplication" else
+                                          oracle.make_grid_attention_state(g, "")).items()}
+    name = "output_projection.weight"
+    buf = torch.zeros(128 * 128 + 8, dtype=BF, device="cuda")
+    buf[1:-7] = st[name].flatten()
+    st[name] = buf[1:-7].view(128, 128)
+    z = torch.randn(40, 40, 128, generator=g).to(BF).cuda()
+    w = (ops.PackedTriMul if kind == "multiplication" else ops.PackedTriAttn)(st, "", "cuda")
+    before = z.clone()
+    with pytest.raises(_cabi.XfoldError, match="aligned"):
+        (ops.triangle_multiplication_ if kind == "multiplication" else ops.triangle_attention_)(z, None, w, True)
+    ops.synchronize_and_check()
+    assert torch.equal(z, before)
