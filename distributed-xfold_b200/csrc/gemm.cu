@@ -216,7 +216,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int b = int(t / ((long long)p.tiles_n * p.tiles_m));
       const uint32_t buf = it & 1u, aphase = (it >> 1) & 1u;
       // GATE_RESID with a gate row per (row % mod): the first chunk's gate values, fetched before the wait as well
-      const bool row_gate_vec = EPI == EPI_GATE_RESID && p.row_gate && (p.ldg & 7) == 0 && (p.N & 31) == 0;
+      const bool row_gate_vec = EPI == EPI_GATE_RESID && p.row_gate && (p.ldg & 7) == 0 && (p.N & 31) == 0 &&
+                                (reinterpret_cast<uintptr_t>(p.row_gate) & 15) == 0;
       uint4 rg[4];
       auto fetch_row_gate = [&](int c) {
         const long long m = (long long)tm * BM + row;

@@ -111,6 +111,20 @@ def test_linear_gate_residual_split_k(ops, M, K, N):
     assert relf(y.float().cpu(), resid.float() + x.float() @ w.float().T) < 4e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 96, 128), (300, 768, 1024), (4000, 768, 128)])
+def test_row_gate_at_any_element(ops, M, N, K):
+    """A gate of one row per (row % mod) that is a view into a larger buffer starts at any element."""
+    x, w, resid = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5), rnd(M, N, seed=4)
+    mod = 100
+    buf = rnd(1, mod * N + 8, seed=8).cuda().flatten()
+    for offset in (1, 4):
+        gate = buf[offset:offset + mod * N].view(mod, N)
+        y = ops.linear_gate_residual(x.cuda(), w.cuda(), gate, resid.cuda(), row_gate_mod=mod)
+        ops.synchronize_and_check()
+        ref = resid.float() + (x.float() @ w.float().T) * torch.sigmoid(gate.float().cpu()[torch.arange(M) % mod])
+        assert relf(y.float().cpu(), ref) < 4e-3
+
+
 @pytest.mark.parametrize("M,K,F", [(900, 128, 512), (260, 384, 1536), (100, 768, 1536)])
 def test_linear_swiglu(ops, M, K, F):
     x, w1 = rnd(M, K, seed=1), rnd(2 * F, K, seed=2, scale=K ** -0.5)
