@@ -184,6 +184,11 @@ static int diffusion_fwd(Ctx* c, bf16* act, int S, int N, const float* mask, con
   if ((long long)S * N >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "diffusion: too many tokens");
   if ((w->Dp != 32 && w->Dp != 64) || (w->H * w->Dp) % 128)
     return fail(c, XFOLD_ERR_ARG, "diffusion: H x Dp must be a multiple of 128 with Dp 32 or 64");
+  for (int b = 0; b < w->num_blocks; ++b) {
+    const xfold_diffusion_block_weights& k = w->blocks[b];
+    if (!logits[b] || !k.w_qkvg || !k.w_out || !k.w1_packed || !k.w2)
+      return fail(c, XFOLD_ERR_ARG, "diffusion: block %d has no pair logits or no weights", b);
+  }
   const DiffWs D = carve_diffusion(ws, ws_bytes, S, N, w);
   if (!ws || D.bytes > ws_bytes) return fail(c, XFOLD_ERR_ARG, "diffusion: workspace too small (%zu < %zu)", ws_bytes, D.bytes);
   StaticWeights sw(c);  // the first kernel is not a GEMM

@@ -105,22 +105,27 @@ class PackedDiffusionTransformer:
     def forward(self, act: torch.Tensor, mask: Optional[torch.Tensor], single_cond: torch.Tensor,
                 pair_logits: List[torch.Tensor]) -> torch.Tensor:
         """act bf16 [S, N, 768] or [N, 768] (updated in place and returned); single_cond bf16 [N, 384]."""
-        ops._need_cuda(act, mask, single_cond, *pair_logits)
+        ops._need_cuda(act, mask, single_cond)
         assert act.dtype == BF16 and act.is_contiguous() and act.shape[-1] == self.c.C
         assert single_cond.dtype == BF16 and single_cond.is_contiguous()
         s = 1 if act.dim() == 2 else act.shape[0]
         n = act.shape[-2]
         assert tuple(single_cond.shape) == (n, self.c.C_cond)
-        shape = (self.sb, self.num_head, n, (n + 7) // 8 * 8)
-        if any(t.dtype == torch.float32 for t in pair_logits):   # plain logits [super_block_size, heads, N, N]
-            pair_logits = [ops.prepare_pair_bias(t.reshape(-1, n, n).contiguous()).reshape(shape)
-                           if t.dtype == torch.float32 else t for t in pair_logits]
-        ptrs = (C.c_void_p * self.num_blocks)()
-        for i, t in enumerate(pair_logits):
-            assert t.dtype == torch.float16 and tuple(t.shape) == shape and t.is_contiguous()
+        shape = (self.num_head, n, (n + 7) // 8 * 8)
+        ptrs, held = (C.c_void_p * self.num_blocks)(), []
+        for i in range(0, self.num_blocks, self.sb):
+            t, blocks = pair_logits[i // self.sb], min(self.sb, self.num_blocks - i)
+            if not isinstance(t, torch.Tensor):
+                t = torch.stack(list(t))
+            ops._need_cuda(t)
+            if t.dtype == torch.float32:   # plain logits [super_block_size, heads, N, N]
+                t = ops.prepare_pair_bias(t.reshape(-1, n, n).contiguous()).reshape(-1, *shape)
+            assert t.dtype == torch.float16 and t.shape[0] >= blocks and tuple(t.shape[1:]) == shape
+            assert t.is_contiguous() or t[0].is_contiguous()
             base, step = t.data_ptr(), t.stride(0) * 2
-            for j in range(self.sb):
-                ptrs[i * self.sb + j] = base + j * step
+            for j in range(blocks):
+                ptrs[i + j] = base + j * step
+            held.append(t)
         if mask is not None:
             mask = mask.to(torch.float32).contiguous()
         dev = ops._dev(act)

@@ -112,6 +112,34 @@ def test_step_is_the_composition_of_its_operators(ops, oracle, n, samples, block
     assert torch.isfinite(got).all() and torch.equal(got, want)
 
 
+def test_pair_logits_come_in_any_list_that_covers_the_blocks(ops, oracle):
+    """Per super-block a tensor or its blocks one by one, prepared or plain, more than the blocks need; too few are an error
+    before anything runs, in Python and in C."""
+    import ctypes
+    from distributed_xfold_b200 import _cabi, diffusion
+    n, blocks, sb = 40, 5, 2
+    g = torch.Generator().manual_seed(8)
+    st = oracle.make_diffusion_transformer_state(g, "", 768, 384, 128, 16, blocks, sb)
+    model = diffusion.PackedDiffusionTransformer(st, "", "cuda", 16, blocks, sb)
+    act, cond = torch.randn(n, 768, generator=g).to(BF).cuda(), torch.randn(n, 384, generator=g).to(BF).cuda()
+    plain = [torch.randn(sb, 16, n, n, generator=g).cuda() for _ in range(4)]
+    prepared = [ops.prepare_pair_bias(t.reshape(-1, n, n)).reshape(sb, 16, n, n) for t in plain]
+    want = model.forward(act.clone(), None, cond, prepared[:3])
+    for logits in (prepared, plain, [prepared[0], plain[1], prepared[2]], [list(t) for t in prepared], torch.stack(prepared),
+                   prepared[:2] + [prepared[2][:1]], [torch.stack([t, t], 1)[:, 0] for t in prepared]):
+        assert torch.equal(model.forward(act.clone(), None, cond, logits), want)
+    with pytest.raises(IndexError):
+        model.forward(act.clone(), None, cond, prepared[:2])
+    lib = _cabi.load()
+    ws = ops._Workspace.get(0, lib.xfold_diffusion_workspace_bytes(1, n, ctypes.byref(model.c)))
+    ptrs = (ctypes.c_void_p * blocks)(*[t.data_ptr() for t in prepared])
+    assert not ptrs[4]
+    rc = lib.xfold_diffusion_transformer_fwd(_cabi.ctx(0), act.data_ptr(), 1, n, None, cond.data_ptr(), ctypes.byref(model.c),
+                                             ptrs, ws.data_ptr(), ws.numel(), ops._stream(0))
+    assert rc == _cabi.XFOLD_ERR_ARG
+    ops.synchronize_and_check()
+
+
 def test_sampler_loop_around_the_gpu_transformer(ops, oracle):
     """The sampler of d_alphafold3.py:316-404 (host arithmetic in diffusion_head.py) driving the DiffusionTransformer on
     the GPU, against the same loop around the CPU oracle's transformer.  The atom encoder / decoder of the reference's
