@@ -142,7 +142,6 @@ cond_ln_kernel(const bf16* x, bf16* y, int rows, const float* gamma, int copies)
 }
 
 static int launch_cond_ln(Ctx* c, const bf16* x, bf16* y, int rows, int C, const float* gamma, int copies, cudaStream_t st) {
-  if (((uintptr_t)x | (uintptr_t)gamma) & 15) return fail(c, XFOLD_ERR_ARG, "diffusion: single_cond and ln_cond must be 16-byte aligned");
   ProfScope ps(c, XFOLD_K_LAYERNORM, st);
   const dim3 grid((rows + 3) / 4, (copies + 1) / 2);
   switch (C) {
@@ -184,6 +183,8 @@ static int diffusion_fwd(Ctx* c, bf16* act, int S, int N, const float* mask, con
   if ((long long)S * N >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "diffusion: too many tokens");
   if ((w->Dp != 32 && w->Dp != 64) || (w->H * w->Dp) % 128)
     return fail(c, XFOLD_ERR_ARG, "diffusion: H x Dp must be a multiple of 128 with Dp 32 or 64");
+  if (((uintptr_t)act | (uintptr_t)cond | (uintptr_t)w->ln_cond) & 15)
+    return fail(c, XFOLD_ERR_ARG, "diffusion: act, single_cond and ln_cond must be 16-byte aligned");
   for (int b = 0; b < w->num_blocks; ++b) {
     const xfold_diffusion_block_weights& k = w->blocks[b];
     if (!logits[b] || !k.w_qkvg || !k.w_out || !k.w1_packed || !k.w2)

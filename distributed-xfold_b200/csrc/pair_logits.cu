@@ -270,6 +270,7 @@ static int launch_pair_logits(Ctx* c, const bf16* pair, int N, const float* gamm
                               void* out, cudaStream_t st) {
   if (N <= 0 || H <= 0) return XFOLD_OK;
   if (H & 15) return fail(c, XFOLD_ERR_ARG, "pair logits: the number of heads must be a multiple of 16, got %d", H);
+  if (reinterpret_cast<uintptr_t>(out) & 15) return fail(c, XFOLD_ERR_ARG, "pair logits: the result must be 16-byte aligned");
   CUtensorMap tmx;
   if (!make_tmap_bf16_3d(&tmx, pair, 128, N, N, 128, (uint64_t)128 * N, 64, 128, 1))
     return fail(c, XFOLD_ERR_ARG, "pair logits: cannot encode the tensor map");

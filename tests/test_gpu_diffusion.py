@@ -140,6 +140,23 @@ def test_pair_logits_come_in_any_list_that_covers_the_blocks(ops, oracle):
     ops.synchronize_and_check()
 
 
+@pytest.mark.parametrize("which", ["act", "cond"])
+def test_unaligned_inputs_are_refused(ops, oracle, which):
+    """Activations or conditioning that start at an odd element: an error before anything runs."""
+    from distributed_xfold_b200 import _cabi, diffusion
+    n = 24
+    g = torch.Generator().manual_seed(9)
+    model = diffusion.PackedDiffusionTransformer(oracle.make_diffusion_transformer_state(g, "", 768, 384, 128, 16, 1, 1), "",
+                                                 "cuda", 16, 1, 1)
+    buf = torch.ones(n * 768 + 8, dtype=BF, device="cuda")
+    shift = lambda width, by: buf[by:by + n * width].view(n, width)
+    act, cond = shift(768, int(which == "act")), shift(384, int(which == "cond"))
+    with pytest.raises(_cabi.XfoldError, match="aligned"):
+        model.forward(act, None, cond, [torch.zeros(1, 16, n, n, device="cuda")])
+    ops.synchronize_and_check()
+    assert (buf == 1).all()
+
+
 def test_sampler_loop_around_the_gpu_transformer(ops, oracle):
     """The sampler of d_alphafold3.py:316-404 (host arithmetic in diffusion_head.py) driving the DiffusionTransformer on
     the GPU, against the same loop around the CPU oracle's transformer.  The atom encoder / decoder of the reference's
