@@ -303,7 +303,7 @@ def test_cross_attention_result_at_any_element(ops):
 
 @pytest.mark.parametrize("B,S,C,H", [(4, 65, 384, 16), (3, 33, 384, 16), (1, 129, 384, 16), (2, 1100, 384, 16), (1, 64, 768, 16),
                                      (3, 400, 768, 16)])
-def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
+def test_attention_reference_exponent_moves_far(ops, oracle, B, S, C, H):
     """Logits of several hundred that grow along the keys: the running reference exponent has to move (output and stored
     probabilities rescaled) in every row, for slots over batch rows and over query tiles, at block edges and remainders."""
     g = torch.Generator().manual_seed(900 + S)
@@ -315,7 +315,8 @@ def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
     r = rounded(st)
     d = C // H
     shp = (C, H, d)
-    ref = oracle.gated_attention(xn.float(), 1e9 * (mask[None, None, None, :] - 1), pb.half().float(),
+    stored = (pb * 1.4426950408889634).half().float() / 1.4426950408889634   # as the kernel holds it
+    ref = oracle.gated_attention(xn.float(), 1e9 * (mask[None, None, None, :] - 1), stored,
                                  r["q_projection.weight"].T.reshape(shp), r["k_projection.weight"].T.reshape(shp),
                                  r["v_projection.weight"].T.reshape(shp), r["gating_query.weight"].T.reshape(shp), None,
                                  query_b=st["q_projection.bias"].reshape(H, d))
@@ -323,8 +324,7 @@ def test_attention_reference_exponent_moves(ops, oracle, B, S, C, H):
     out = ops.attention_pair_bias_core(xn.cuda().contiguous(), w, pb.cuda().contiguous(), mask.cuda())
     ops.synchronize_and_check()
     out = out.float().cpu().reshape(B, S, H, w.Dp)[..., :d]
-    # the prepared bias is fp16 times log2(e): an absolute error of up to 0.18 in a logit near 300 * log2(e)
-    assert torch.isfinite(out).all() and relf(out, ref) < 0.15
+    assert torch.isfinite(out).all() and relf(out, ref) < 2e-2
 
 
 @pytest.mark.parametrize("B,S,C,H", [(4, 65, 384, 16), (3, 33, 384, 16), (1, 129, 384, 16), (2, 1100, 384, 16), (1, 64, 768, 16),
