@@ -577,7 +577,7 @@ static PairformerWs carve_pairformer(void* ws, size_t cap, int N) {
 }
 
 // The blocks in order.  The masks' bias tiles are made once.  The single representation follows the pair representation
-// and nothing of the pair path reads it, so its eight small kernels of a block run on the context's second stream beside
+// and nothing of the pair path reads it, so its seven small kernels of a block run on the context's second stream beside
 // the next block's pair path (a block of 40 tokens: 155 us, 45 of them single path; 1024 tokens: 0.14 of 6.8 ms).  The
 // pair logits are the only buffer between the two; the next block's logits wait for the single path of this one.
 static int pairformer_fwd(Ctx* c, bf16* z, bf16* s, const float* pair_mask, const float* seq_mask, int N,

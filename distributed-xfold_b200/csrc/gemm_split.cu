@@ -1,12 +1,13 @@
 // out = [sigmoid(gate) *] (A B^T) + resid for products with few output tiles and a long K: the CTAs of a cluster share one
 // tile, each takes a part of K, and the parts are added through distributed shared memory.
 //
-// What bounds such a product is one CTA's latency, not a rate: a 64-wide step of K costs about 0.25 us (the operands' trip
-// through a ring of a few stages, four products, the hand-over), so that K = 1536 takes 6 us on a dozen SMs while the
-// others idle.  With K cut into S parts a CTA has most of its part in flight at once.  The exchange moves each fp32 partial
-// sum once: the 128 rows of the tile are dealt out to the S CTAs, every CTA stores its rows of another's share straight
-// from tensor memory into that CTA's shared memory, and after one cluster barrier each CTA adds S addends in the order of
-// their ranks (the result does not depend on timing) and runs the epilogue on its 128 / S rows.
+// What bounds such a product is one CTA's latency, not a rate: a 64-wide step of K cost about 0.25 us when this was measured
+// (0.14 since the producers lost their lane branches; the operands' trip through a ring of a few stages, four products, the
+// hand-over), so that K = 1536 takes 6 us on a dozen SMs while the others idle.  With K cut into S parts a CTA has most of its
+// part in flight at once.  The exchange moves each fp32 partial sum once: the 128 rows of the tile are dealt out to the S CTAs,
+// every CTA stores its rows of another's share straight from tensor memory into that CTA's shared memory, and after one cluster
+// barrier each CTA adds S addends in the order of their ranks (the result does not depend on timing) and runs the epilogue on
+// its 128 / S rows.
 // Measured on the diffusion transformer's two output projections (768 columns, K = 1024 and 1536, 24 blocks of a step):
 // 77 rows 1215 -> 986 us with S = 8, 231 rows 1195 -> 1014 with 4, 384 rows 1406 -> 1230 and 512 rows 1467 -> 1314 with 2.
 // The projections before them (K = 768, 24 to 64 tiles) gain nothing: what the shorter loop saves the exchange costs.

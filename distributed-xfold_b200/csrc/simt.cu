@@ -18,8 +18,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 // y = LN(x) * gamma + beta  (gamma/beta may be null), rows of C bf16; optional
 // proj[h][row] = sum_c y[c] * pw[h][c]  (fp32, computed from the un-rounded y)
 // proj_bf16 (instead of proj) is the attention kernel's pair-bias operand: 16-bit, holding FP16 values (the buffer
-// is only typed bf16) multiplied by log2(e), because the head-dim-32 attention kernel exponentiates in base 2 and adds
-// the bias tile, as it is, to fp16x2 exponent arguments.
+// is only typed bf16) multiplied by log2(e), because the attention kernel exponentiates in base 2 and its tensor-core
+// products add the bias tile, as it is, to the logits.
 // optional modulation: y = sigmoid(scale[row % mod_rows][c]) * y + shift[row % mod_rows][c]  (AdaLN)
 // ---------------------------------------------------------------------------------------------
 constexpr float kBiasLog2e = 1.4426950408889634f;

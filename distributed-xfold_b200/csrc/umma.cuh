@@ -143,12 +143,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, c
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -169,13 +163,6 @@ __device__ __forceinline__ void tma_load_3d_if(uint32_t go, void* dst, const CUt
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
       "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
       ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(go)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
-                                            int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 
@@ -203,13 +190,7 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// plain (untiled) bulk copy global -> shared; addresses and size are multiples of 16 bytes
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
+// plain (untiled) bulk copy global -> shared, by the lanes with go != 0; addresses and size are multiples of 16 bytes
 __device__ __forceinline__ void bulk_load_if(uint32_t go, void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
@@ -244,17 +225,6 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]: A is read from tensor memory (lane = row, each 32-bit column holds two
-// consecutive 16-bit K elements), so an operand produced by the CUDA cores never passes through shared memory.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The same, issued by the lanes with go != 0 (one, elected by the caller) of a converged warp: no branch, so that operands
 // can stay in uniform registers.
 __device__ __forceinline__ void umma_ss_if(uint32_t go, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -266,6 +236,8 @@ __device__ __forceinline__ void umma_ss_if(uint32_t go, uint32_t d_tmem, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(go)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem]: A is read from tensor memory (lane = row, each 32-bit column holds two
+// consecutive 16-bit K elements), so an operand produced by the CUDA cores never passes through shared memory.
 __device__ __forceinline__ void umma_ts_if(uint32_t go, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
   asm volatile(
@@ -454,13 +426,6 @@ __device__ __forceinline__ void row_normalise(uint8_t* tile, int row, float nmea
     }
     *row_piece(tile, row, g) = make_uint4(o[0], o[1], o[2], o[3]);
   }
-}
-
-// Byte offset of element (row, col) inside a K-major / MN-major 128B-swizzled tile whose rows are
-// 64 bf16 wide: 16-byte chunk index is XORed with (row & 7).  The tile base must be 1024 B aligned.
-__device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t col_elem) {
-  const uint32_t chunk = (col_elem >> 3) ^ (row & 7u);
-  return row * 128u + (chunk << 4) + ((col_elem & 7u) << 1);
 }
 
 }  // namespace xf

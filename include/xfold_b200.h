@@ -285,7 +285,7 @@ int xfold_pairformer_stack_fwd(xfold_ctx* ctx, void* z, void* s, const float* pa
  *
  * a, b: bf16 [rows][128][ld], element (row i, channel c, k) at (i * 128 + c) * ld + k, so a rank's rows
  * are one contiguous block and the all-gather of b (nn/d_triangle_multiplication.py:74-79) is a
- * concatenation.  g: bf16 [R * N][128].  o: bf16 [R][128][ldo]. */
+ * concatenation.  g: bf16 [R * N][128].  o: bf16 [R][128][ldo].  x_scratch (here and below): not null, not used any more. */
 int xfold_trimul_project_fwd(xfold_ctx* ctx, const void* z, const float* mask, int R, int N,
                              const xfold_trimul_weights* w, void* x_scratch, void* a, void* b, void* g, int ld,
                              void* stream);
