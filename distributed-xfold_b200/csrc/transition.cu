@@ -4,7 +4,8 @@
 // Bound: the tensor core.  Per tile of 128 rows 25 M multiply-adds (6100 clocks) and 65536 sigmoids (4096 clocks of the
 // special-function unit); the weights are 384 KB at F = 512, so two tiles share each block of them.  The only HBM traffic is
 // x itself.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) the normalised rows and the hidden activations made six
-// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows; this kernel 0.47 ms (one tile at a time: 0.49 ms).
+// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows; this kernel 0.46 ms by itself (one tile at a time: 0.49),
+// 0.49 back to back, 0.53 in a recycle at the power limit.
 //
 // Persistent CTAs, a pair of tiles (A, B) of 128 rows at a time, hidden units in blocks of 64; per tile
 //     D1 = LN(x) W1(block)^T   [128 x (64 SiLU | 64 linear)]      tensor memory
