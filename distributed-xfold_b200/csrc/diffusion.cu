@@ -177,12 +177,15 @@ static DiffWs carve_diffusion(void* ws, size_t cap, int S, int N, const xfold_di
   return d;
 }
 
+static bool sizes_ok(const xfold_diffusion_weights* w) {
+  return w->C > 0 && w->C_cond > 0 && w->H > 0 && w->F > 0 && (w->Dp == 32 || w->Dp == 64) && (w->H * w->Dp) % 128 == 0;
+}
+
 static int diffusion_fwd(Ctx* c, bf16* act, int S, int N, const float* mask, const bf16* cond, const xfold_diffusion_weights* w,
                          const void* const* logits, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (S <= 0 || N <= 0 || w->num_blocks <= 0) return XFOLD_OK;
   if ((long long)S * N >= (1ll << 31)) return fail(c, XFOLD_ERR_ARG, "diffusion: too many tokens");
-  if ((w->Dp != 32 && w->Dp != 64) || (w->H * w->Dp) % 128)
-    return fail(c, XFOLD_ERR_ARG, "diffusion: H x Dp must be a multiple of 128 with Dp 32 or 64");
+  if (!sizes_ok(w)) return fail(c, XFOLD_ERR_ARG, "diffusion: positive widths, and H x Dp a multiple of 128 with Dp 32 or 64");
   if (((uintptr_t)act | (uintptr_t)cond | (uintptr_t)w->ln_cond) & 15)
     return fail(c, XFOLD_ERR_ARG, "diffusion: act, single_cond and ln_cond must be 16-byte aligned");
   for (int b = 0; b < w->num_blocks; ++b) {
@@ -232,7 +235,7 @@ using namespace xf;
 extern "C" {
 
 size_t xfold_diffusion_workspace_bytes(int S, int N, const xfold_diffusion_weights* w) {
-  return w && S > 0 && N > 0 ? carve_diffusion(nullptr, 0, S, N, w).bytes : 0;
+  return w && S > 0 && N > 0 && w->num_blocks > 0 && sizes_ok(w) ? carve_diffusion(nullptr, 0, S, N, w).bytes : 0;
 }
 
 int xfold_diffusion_transformer_fwd(xfold_ctx* cx, void* act, int S, int N, const float* mask, const void* single_cond,

@@ -66,3 +66,16 @@ def test_swiglu_weight_packing_roundtrip(pkg):
     p = pack_swiglu_weight(w)
     assert torch.equal(p[:128], w[:128]) and torch.equal(p[128:256], w[256:384])
     assert torch.equal(p[256:384], w[128:256]) and torch.equal(p[384:], w[384:])
+
+
+def test_diffusion_workspace_of_sizes_that_cannot_be(pkg):
+    """Zero bytes for widths and counts that the step refuses; they divide in the sizing."""
+    import ctypes
+    cabi = pkg._cabi
+    good = dict(C=768, C_cond=384, H=16, Dp=64, F=1536, num_blocks=24)
+    size = lambda s, n, **kw: cabi.load().xfold_diffusion_workspace_bytes(
+        s, n, ctypes.byref(cabi.DiffusionWeights(**{**good, **kw})))
+    assert size(1, 100) > 0 and size(2, 100) > size(1, 100)
+    assert size(0, 100) == size(1, 0) == 0
+    for kw in (dict(C=0), dict(C=-1), dict(C_cond=0), dict(H=0), dict(Dp=48), dict(F=0), dict(num_blocks=0)):
+        assert size(1, 100, **kw) == 0, kw
