@@ -325,8 +325,8 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // the call writes -- overlaps the predecessor's tail.  Rules that keep it safe:
 //   * every thread calls pdl_wait() before it touches anything a predecessor wrote or still reads, so that the completion
 //     of a kernel implies the completion of all before it;
-//     (what a kernel two or more places ahead wrote may be read, through L2, before pdl_wait(): the predecessor let this
-//     kernel start only after its own pdl_wait(); adaln_kernel does so)
+//     (what a kernel two or more places ahead wrote may be read, through L2, and what it read may be overwritten, before
+//     pdl_wait(): the predecessor let this kernel start only after its own pdl_wait(); adaln_kernel and cond_ln_kernel do so)
 //   * pdl_launch() comes after the tensor memory allocation (a successor that got the tensor memory first would wait for
 //     this kernel, and this kernel for the tensor memory) and after pdl_wait(): L1 is invalidated when a kernel starts, and
 //     a kernel two places ahead must not start while this kernel's predecessor still reads what this kernel overwrites;

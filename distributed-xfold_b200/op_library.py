@@ -75,6 +75,8 @@ def _cached(name, tensors, make):
         return hit[0]
     v = make()
     on_gpu = tensors[0].is_cuda
+    if on_gpu and torch._C._cuda_isCurrentStreamCapturing():
+        return v   # packed by the graph, for the graph: nothing is there yet for another call
     if on_gpu:
         torch.cuda.current_stream(tensors[0].device).synchronize()   # any stream may use the packed form from now on
     gone = [e for e, (_, refs) in list(_CACHE.items()) if _gone(refs)]

@@ -160,3 +160,28 @@ def test_op_grid_self_attention_adds_the_bias_as_given(lib, oracle, b, s, shared
         args[1] = bias[:2].cuda()
         with pytest.raises(RuntimeError):
             lib.grid_self_attn_forward(*args)
+
+
+def test_first_call_of_an_operator_under_capture(lib, oracle):
+    """Weights that are packed inside a captured call belong to the graph: its replays follow the weights, and a later call
+    outside packs for itself."""
+    g = torch.Generator().manual_seed(64)
+    st = oracle.make_transition_state(g, "", 128)
+    x = torch.randn(9, 21, 128, generator=g)
+    args = [x.to(BF).cuda(), st["transition1.weight"].T.contiguous().to(BF).cuda(), st["transition2.weight"].T.contiguous().to(BF).cuda(),
+            st["input_layer_norm.weight"].to(BF).cuda(), st["input_layer_norm.bias"].to(BF).cuda()]
+    lib.transition_forward(torch.randn(4, 128).to(BF).cuda(), *(t.clone() for t in args[1:]))   # the library is loaded
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = lib.transition_forward(*args)
+    eager = lib.transition_forward(*args)
+    ref = oracle.transition({k: rb(v) for k, v in st.items()}, "", rb(x))
+    assert relf(eager.float().cpu(), ref) < 2e-2
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+    args[2].neg_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, -eager) and torch.equal(lib.transition_forward(*args), -eager)
