@@ -228,6 +228,286 @@ static int launch_xattn(Ctx* c, const XAttnArgs& a, cudaStream_t st) {
   return check_launch(c, "xattn_kernel");
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// The model's own windows (four heads of 32, 128 channels, up to 32 queries and 128 keys) in one kernel: projections and
+// attention of a window by two CTAs, one for each pair of heads, two CTAs per SM.
+// Bound: latency.  A window brings 104 KB (64 of them bias) for 0.04 GFLOP; what counts is the chain of trips -- as two
+// projection launches and xattn_kernel, with queries, keys and values through memory, 257 windows took 27.6 us.
+// The projections come out transposed (D = W x^T, lane = channel), so that the 32 queries are the tile's narrow side, the
+// query bias and scale are one number per thread, and a thread's row of keys leaves in 16-byte pieces:
+//   warp 4     : TMA and tcgen05.mma -- weights once, [q | gate] and [k | v] rows of the pair of heads; then per window
+//                [128 x 32 queries] and [128 x 128 keys]
+//   warps 0-3  : tensor memory -> bf16 [channel][token] over the window's inputs, then one head and 16 queries per warp as
+//                in xattn_kernel, from the same roundings in the same order (the same bits).  The bias is on its way while
+//                the rest is prepared.
+// 257 windows, back to back: 13.8 us (one call at a time from an idle GPU, host included: 44 -> 32).
+constexpr uint32_t XW_OFF_W = 0, XW_OFF_M = 65536, XW_OFF_Q = XW_OFF_M + 32768, XW_OFF_BAR = XW_OFF_Q + 8192,
+                   XW_SMEM = XW_OFF_BAR + 64 + 1024;
+constexpr int XW_THREADS = 160;
+
+struct XWinArgs {
+  const float *qg_bias, *qg_scale, *bias;
+  bf16* out;
+  int B, S, K;
+  int* status;
+};
+
+__global__ void __launch_bounds__(XW_THREADS, 2)
+xwin_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmm,
+            const __grid_constant__ CUtensorMap tmwq, const __grid_constant__ CUtensorMap tmwk, const XWinArgs p) {
+  constexpr float LOG2E = 1.4426950408889634f;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + XW_OFF_BAR);
+  uint64_t* x_full = w_full + 1;   // the window's inputs have landed
+  uint64_t* x_empty = x_full + 1;  // the attention has read what replaced them
+  uint64_t* t_full = x_empty + 1;  // projections complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_full + 1);
+  volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = int(__reduce_max_sync(0xffffffffu, threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const AbortCtx ab{cta_abort, p.status};
+  if (threadIdx.x == 0) {
+    mbar_init(w_full, 1);
+    mbar_init(x_full, 1);
+    mbar_init(x_empty, 4);
+    mbar_init(t_full, 1);
+    *cta_abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmq);
+    tma_prefetch_desc(&tmm);
+    tma_prefetch_desc(&tmwq);
+    tma_prefetch_desc(&tmwk);
+  }
+  if (warp == 4) {
+    tmem_alloc(tmem_slot, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __reduce_max_sync(0xffffffffu, *tmem_slot);  // [k | v]: 128 columns, [q | gate]: 32
+  const uint32_t base = smem_u32(smem);
+  const int hp = int(blockIdx.x) & 1, b0 = int(blockIdx.x) >> 1, step = int(gridDim.x) >> 1;
+  pdl_wait();
+  pdl_launch();
+
+  if (warp == 4) {
+    const uint32_t go = elect_one();
+    auto load_x = [&](int b) {
+      mbar_arrive_expect_tx_if(go, x_full, 32768 + 8192);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh) {
+        tma_load_3d_if(go, smem + XW_OFF_M + kh * 16384, &tmm, x_full, kh * 64, 0, b);
+        tma_load_3d_if(go, smem + XW_OFF_Q + kh * 4096, &tmq, x_full, kh * 64, 0, b);
+      }
+    };
+    if (b0 < p.B) load_x(b0);
+    mbar_arrive_expect_tx_if(go, w_full, 65536);
+#pragma unroll
+    for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {  // rows of the pair's q or k, then of its gate or v
+        tma_load_3d_if(go, smem + XW_OFF_W + kh * 16384 + part * 8192, &tmwk, w_full, kh * 64, part * 128 + hp * 64, 0);
+        tma_load_3d_if(go, smem + XW_OFF_W + 32768 + kh * 16384 + part * 8192, &tmwq, w_full, kh * 64, part * 128 + hp * 64, 0);
+      }
+    bool okay = mbar_wait_warp(w_full, 0, ab, XF_ERR_WAIT_FULL);
+    uint32_t ph = 0;
+    for (int b = b0; b < p.B && okay; b += step, ph ^= 1u) {
+      if (!mbar_wait_warp(x_full, ph, ab, XF_ERR_WAIT_FULL)) break;
+      tc_fence_after();
+      const uint64_t md = make_sdesc(base + XW_OFF_M, 16, 1024), qd = make_sdesc(base + XW_OFF_Q, 16, 1024);
+      const uint64_t wk = make_sdesc(base + XW_OFF_W, 16, 1024), wq = make_sdesc(base + XW_OFF_W + 32768, 16, 1024);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          umma_ss_if(go, tmem_base, wk + uint64_t(kh * 1024 + 2 * j), md + uint64_t(kh * 1024 + 2 * j), make_idesc(128, 128), (kh | j) ? 1u : 0u);
+#pragma unroll
+      for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          umma_ss_if(go, tmem_base + 128, wq + uint64_t(kh * 1024 + 2 * j), qd + uint64_t(kh * 256 + 2 * j), make_idesc(128, 32), (kh | j) ? 1u : 0u);
+      umma_commit_if(go, t_full);
+      // (the next window overwrites what the attention reads, and its products the accumulators)
+      if (!mbar_wait_warp(x_empty, ph, ab, XF_ERR_WAIT_EMPTY)) break;
+      if (b + step < p.B) load_x(b + step);
+    }
+  } else {
+    const int row = warp * 32 + lane;                       // channel: q | gate, or k | v, of the pair of heads
+    const int col = (row >> 6) * 128 + hp * 64 + (row & 63);  // its row of w_qg
+    const float qb = p.qg_bias ? p.qg_bias[col] : 0.f, qs = p.qg_scale ? p.qg_scale[col] : 1.f;
+    const int hh = warp & 1, h = hp * 2 + hh, q0 = (warp >> 1) * 16;
+    const int r0 = q0 + (lane >> 2), r1 = r0 + 8, cl = (lane & 3) * 2;
+    const uint32_t laddr = tmem_base + (uint32_t(warp * 32) << 16);
+    uint8_t* skv = smem + XW_OFF_M + row * 256;   // [128 channels][128 keys], 16-byte chunks swizzled over 8 rows
+    uint8_t* sqg = smem + XW_OFF_Q + row * 64;    // [128 channels][32 queries]
+    const uint32_t rsw = uint32_t(row & 7), rsw4 = uint32_t(row >> 1) & 3u;
+    auto kv_at = [&](int ch, int chunk) { return base + XW_OFF_M + uint32_t(ch * 256 + ((chunk ^ (ch & 7)) << 4)); };
+    auto qg_at = [&](int ch, int chunk) { return base + XW_OFF_Q + uint32_t(ch * 64 + ((chunk ^ ((ch >> 1) & 3)) << 4)); };
+    const bool active = q0 < p.S;
+    uint32_t ph = 0;
+    for (int b = b0; b < p.B; b += step, ph ^= 1u) {
+      const float* b_r0 = p.bias + (((long long)b * 4 + h) * p.S + (r0 < p.S ? r0 : 0)) * p.K;
+      const float* b_r1 = p.bias + (((long long)b * 4 + h) * p.S + (r1 < p.S ? r1 : 0)) * p.K;
+      float s[16][4];
+      if (active) {
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+          const int k = t * 8 + cl;
+          const float2 none = make_float2(-INFINITY, -INFINITY);
+          const float2 u = k < p.K ? *reinterpret_cast<const float2*>(b_r0 + k) : none;
+          const float2 v = k < p.K ? *reinterpret_cast<const float2*>(b_r1 + k) : none;
+          s[t][0] = u.x; s[t][1] = u.y; s[t][2] = v.x; s[t][3] = v.y;
+        }
+      }
+      mbar_wait_warp(t_full, ph, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through: these warps meet at a barrier)
+      tc_fence_after();
+      {
+        uint32_t r[32];
+        tmem_ld32(laddr + 128, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            o[e] = pack_bf16x2((__uint_as_float(r[c * 8 + 2 * e]) + qb) * qs, (__uint_as_float(r[c * 8 + 2 * e + 1]) + qb) * qs);
+          *reinterpret_cast<uint4*>(sqg + ((uint32_t(c) ^ rsw4) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+          tmem_ld32(laddr + g * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(__uint_as_float(r[c * 8 + 2 * e]), __uint_as_float(r[c * 8 + 2 * e + 1]));
+            *reinterpret_cast<uint4*>(skv + ((uint32_t(g * 4 + c) ^ rsw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        }
+      }
+      tc_fence_before();
+      named_bar_sync(1, 128);
+      if (active) {
+        uint32_t qa[2][4], gg[2][4];  // A fragments of the queries; gates of (r0, r1) x pairs of channels, two groups of 8 each
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int d = hh * 32 + k * 16 + (lane & 7);
+          ldsm4_t(qg_at(d + ((lane >> 4) << 3), (q0 >> 3) + ((lane >> 3) & 1)), qa[k]);
+          ldsm4_t(qg_at(64 + d + ((lane >> 4) << 3), (q0 >> 3) + ((lane >> 3) & 1)), gg[k]);
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t += 2)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            uint32_t bk[4];
+            ldsm4_t(kv_at(hh * 32 + k * 16 + (((lane >> 3) & 1) << 3) + (lane & 7), t + (lane >> 4)), bk);
+            mma16816(s[t], qa[k], bk[0], bk[1]);
+            mma16816(s[t + 1], qa[k], bk[2], bk[3]);
+          }
+        float c0 = -INFINITY, c1 = -INFINITY, l0 = 0.f, l1 = 0.f, o[4][4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[d][e] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+          c0 = fmaxf(c0, fmaxf(s[t][0], s[t][1]));
+          c1 = fmaxf(c1, fmaxf(s[t][2], s[t][3]));
+        }
+#pragma unroll
+        for (int x = 1; x < 4; x <<= 1) {
+          c0 = fmaxf(c0, __shfl_xor_sync(0xffffffffu, c0, x));
+          c1 = fmaxf(c1, __shfl_xor_sync(0xffffffffu, c1, x));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {  // 16 keys: exponentials, three bf16 pieces, products
+          uint32_t pa[3][4];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int t = 2 * j + u;
+            float e0 = exp2f((s[t][0] - c0) * LOG2E), e1 = exp2f((s[t][1] - c0) * LOG2E);
+            float e2 = exp2f((s[t][2] - c1) * LOG2E), e3 = exp2f((s[t][3] - c1) * LOG2E);
+            l0 += e0 + e1;
+            l1 += e2 + e3;
+#pragma unroll
+            for (int piece = 0; piece < 3; ++piece) {
+              const uint32_t x0 = pack_bf16x2(e0, e1), x1 = pack_bf16x2(e2, e3);
+              pa[piece][u * 2] = x0;
+              pa[piece][u * 2 + 1] = x1;
+              e0 -= bf16_lo(x0); e1 -= bf16_hi(x0);
+              e2 -= bf16_lo(x1); e3 -= bf16_hi(x1);
+            }
+          }
+#pragma unroll
+          for (int d = 0; d < 4; d += 2) {
+            uint32_t bv[4];
+            ldsm4(kv_at(64 + hh * 32 + d * 8 + ((lane >> 4) << 3) + (lane & 7), j * 2 + ((lane >> 3) & 1)), bv);
+#pragma unroll
+            for (int piece = 0; piece < 3; ++piece) {
+              mma16816(o[d], pa[piece], bv[0], bv[1]);
+              mma16816(o[d + 1], pa[piece], bv[2], bv[3]);
+            }
+          }
+        }
+#pragma unroll
+        for (int x = 1; x < 4; x <<= 1) {
+          l0 += __shfl_xor_sync(0xffffffffu, l0, x);
+          l1 += __shfl_xor_sync(0xffffffffu, l1, x);
+        }
+        const float i0 = 1.f / l0, i1 = 1.f / l1;
+        bf16* o_r0 = p.out + ((long long)b * p.S + r0) * 128 + h * 32 + cl;
+        bf16* o_r1 = o_r0 + 8 * 128;
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+          const uint32_t g0 = gg[d >> 1][(d & 1) * 2], g1 = gg[d >> 1][(d & 1) * 2 + 1];
+          if (r0 < p.S)
+            *reinterpret_cast<uint32_t*>(o_r0 + d * 8) =
+                pack_bf16x2(o[d][0] * i0 * sigmoidf_fast(bf16_lo(g0)), o[d][1] * i0 * sigmoidf_fast(bf16_hi(g0)));
+          if (r1 < p.S)
+            *reinterpret_cast<uint32_t*>(o_r1 + d * 8) =
+                pack_bf16x2(o[d][2] * i1 * sigmoidf_fast(bf16_lo(g1)), o[d][3] * i1 * sigmoidf_fast(bf16_hi(g1)));
+        }
+      }
+      fence_proxy_async_smem();  // read here, written by TMA next
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x_empty);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*cta_abort && threadIdx.x == 0) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {}
+  }
+  __syncthreads();
+  if (warp == 4) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+
+static int launch_xwin(Ctx* c, const bf16* q, const bf16* m, const bf16* w_qg, const bf16* w_kv, const XWinArgs& a, cudaStream_t st) {
+  CUtensorMap tmq, tmm, tmwq, tmwk;
+  if (!make_tmap_bf16_3d(&tmq, q, 128, a.S, a.B, 128, (uint64_t)128 * a.S, 64, 32, 1) ||
+      !make_tmap_bf16_3d(&tmm, m, 128, a.K, a.B, 128, (uint64_t)128 * a.K, 64, 128, 1) ||
+      !make_tmap_bf16_3d(&tmwq, w_qg, 128, 256, 1, 128, 128 * 256, 64, 64, 1) ||
+      !make_tmap_bf16_3d(&tmwk, w_kv, 128, 256, 1, 128, 128 * 256, 64, 64, 1))
+    return fail(c, XFOLD_ERR_ARG, "cross attention: cannot encode tensor maps (16-byte aligned bases?)");
+  static bool attr_done[8] = {false};
+  if (!attr_done[c->device & 7]) {
+    cudaError_t e = cudaFuncSetAttribute(xwin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XW_SMEM);
+    if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "cross attention smem attribute: %s", cudaGetErrorString(e));
+    attr_done[c->device & 7] = true;
+  }
+  ProfScope ps(c, XFOLD_K_APB_ATTENTION, st);
+  launch_pdl(xwin_kernel, 2 * (a.B < c->sm_count ? a.B : c->sm_count), XW_THREADS, XW_SMEM, st, tmq, tmm, tmwq, tmwk, a);
+  return check_launch(c, "xwin_kernel");
+}
+
 }  // namespace xf
 
 using namespace xf;
@@ -247,18 +527,24 @@ int xfold_cross_attention_fwd(xfold_ctx* cx, const void* q_data, const void* m_d
   if (D != 16 && D != 32 && D != 64) return fail(c, XFOLD_ERR_ARG, "cross attention: head dimension 16, 32 or 64");
   if (B <= 0 || S <= 0 || K <= 0) return XFOLD_OK;
   const int W = H * D;
+  const bool pairs = !((K & 1) || (reinterpret_cast<uintptr_t>(bias) & 7) || (reinterpret_cast<uintptr_t>(out) & 3));
   Carver cv(ws, ws_bytes);
   bf16* qg = (bf16*)cv.take((size_t)B * S * 2 * W * 2);
   bf16* kv = (bf16*)cv.take((size_t)B * K * 2 * W * 2);
   if (!ws || !cv.ok()) return fail(c, XFOLD_ERR_ARG, "cross attention: workspace too small (%zu < %zu)", ws_bytes, cv.off);
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
+  // The model's window is one tile of xwin_kernel; more queries, keys, heads or channels take the general kernels, and so do
+  // a bias and a result that pairs of elements cannot be read from or written to.
+  if (H == 4 && D == 32 && Ca == 128 && Cm == 128 && S <= 32 && K <= XA_KC && pairs)
+    return launch_xwin(c, (const bf16*)q_data, (const bf16*)m_data, (const bf16*)w_qg, (const bf16*)w_kv,
+                       XWinArgs{qg_bias, qg_scale, bias, (bf16*)out, B, S, K, c->d_status}, st);
   if ((rc = linear_plain(c, (const bf16*)q_data, Ca, (long long)B * S, Ca, (const bf16*)w_qg, 2 * W, qg_bias, qg_scale, qg,
                              2 * W, st))) return rc;
   if ((rc = linear_plain(c, (const bf16*)m_data, Cm, (long long)B * K, Cm, (const bf16*)w_kv, 2 * W, nullptr, nullptr, kv,
                              2 * W, st))) return rc;
   XAttnArgs a{qg, kv, bias, (bf16*)out, B, S, K, H};
-  if ((K & 1) || (reinterpret_cast<uintptr_t>(bias) & 7) || (reinterpret_cast<uintptr_t>(out) & 3))
+  if (!pairs)
     return D == 16 ? launch_xattn<16, false>(c, a, st) : D == 32 ? launch_xattn<32, false>(c, a, st) : launch_xattn<64, false>(c, a, st);
   return D == 16 ? launch_xattn<16, true>(c, a, st) : D == 32 ? launch_xattn<32, true>(c, a, st) : launch_xattn<64, true>(c, a, st);
 }

@@ -264,6 +264,23 @@ def test_cross_attention_tile_edges(ops, oracle, B, S, K, H, D):
     assert relf(out.float().cpu(), ref) < 2e-2
 
 
+@pytest.mark.parametrize("B,S,K", [(1, 1, 2), (2, 16, 8), (3, 17, 126), (149, 32, 128), (400, 31, 100)])
+def test_cross_attention_windows_have_the_bits_of_the_general_kernels(ops, B, S, K):
+    """The one-kernel form for windows of up to 32 x 128, from one entry to several windows per CTA, against the same call
+    with a bias that starts at an odd float, which the general kernels take."""
+    g = torch.Generator().manual_seed(B + S + K)
+    w = ops.PackedCrossAttention(*(torch.randn(128, 4, 32, generator=g) / 11 if i != 1 else torch.randn(1, 4, 32, generator=g)
+                                   for i in range(5)), "cuda")
+    qd, md = torch.randn(B, S, 128, generator=g).to(BF).cuda(), torch.randn(B, K, 128, generator=g).to(BF).cuda()
+    keep = torch.rand(B, 1, 1, K, generator=g) > 0.2
+    keep[..., 0] = True
+    bias = (torch.randn(B, 4, S, K, generator=g) + 1e9 * (keep.float() - 1)).cuda()
+    odd = torch.zeros(bias.numel() + 1, device="cuda")[1:].view_as(bias).copy_(bias)
+    out, want = ops.cross_attention(qd, md, bias, w), ops.cross_attention(qd, md, odd, w)
+    ops.synchronize_and_check()
+    assert torch.isfinite(out).all() and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("offset", [0, 1, 2, 3])
 def test_cross_attention_bias_at_any_element(ops, offset):
     """A bias that is a view into a larger buffer starts at any float."""
