@@ -166,6 +166,14 @@ __device__ __forceinline__ void tma_load_3d_if(uint32_t go, void* dst, const CUt
       : "memory");
 }
 
+// the box on its way to L2 (no completion is signalled)
+__device__ __forceinline__ void tma_prefetch_3d_if(uint32_t go, const CUtensorMap* m, int c0, int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];\n\t}" ::"l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(go)
+      : "memory");
+}
+
 // TMA store shared -> global (bulk async-group completion); rows / columns outside the tensor are clipped
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* src, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
