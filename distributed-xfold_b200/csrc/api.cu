@@ -281,14 +281,15 @@ int trimul_contract_mn(Ctx* c, const bf16* at, long long at_cs, long long at_rs,
 }
 
 // z (+)= Linear(LN_c(o)) * sigmoid(g); o: channel-major.  upd given: write the update alone there and leave z untouched.
+// g null: the gate is projected here, from z, which has to be what a and b were projected from.
 int trimul_output(Ctx* c, const bf16* o, long long o_cs, long long o_rs, const bf16* g, int R, int N, const xfold_trimul_weights* w,
                   bf16* z, cudaStream_t st, bf16* upd) {
-  return launch_row_output_cm(c, o, o_cs, o_rs, R, N, w->ln_c_gamma, w->ln_c_beta, (const bf16*)w->w_out, g, upd ? nullptr : z,
-                              upd ? upd : z, st);
+  return launch_row_output_cm(c, o, o_cs, o_rs, R, N, w->ln_c_gamma, w->ln_c_beta, (const bf16*)w->w_out, g, w->ln_in_gamma,
+                              w->ln_in_beta, (const bf16*)w->w_in + 512 * 128, z, upd ? 0 : 1, upd ? upd : z, st);
 }
 
 struct TriMulWs {
-  bf16 *a, *b, *g, *o;
+  bf16 *a, *b, *o;
   int ld;
   size_t bytes;
 };
@@ -296,9 +297,7 @@ static TriMulWs carve_trimul(void* ws, size_t cap, int N) {
   TriMulWs w;
   Carver cv(ws, cap);
   w.ld = pad8(N);
-  const size_t tok = (size_t)N * N * 128 * 2;
   const size_t cm = (size_t)128 * N * w.ld * 2;
-  w.g = (bf16*)cv.take(tok);
   w.a = (bf16*)cv.take(cm);
   w.b = (bf16*)cv.take(cm);
   w.o = (bf16*)cv.take(cm);
@@ -315,12 +314,12 @@ static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, c
   // incoming: a and b are stored transposed, so that o[i][c][j] = sum_k bT[i][c][k] aT[j][c][k] is the same product
   // one GPU: plain channel-major planes [128][N][ld] (rows of a tile are 2 KB apart, best DRAM locality)
   const long long cs = (long long)N * W.ld, rs = W.ld;
-  int rc = trimul_project(c, z, mask, N, N, outgoing ? 0 : 1, w, W.a, W.b, W.g, cs, rs, st);
+  int rc = trimul_project(c, z, mask, N, N, outgoing ? 0 : 1, w, W.a, W.b, nullptr, cs, rs, st);
   if (rc) return rc;
   StaticWeights sw(c);
   rc = trimul_contract(c, outgoing ? W.a : W.b, cs, rs, outgoing ? W.b : W.a, cs, rs, N, N, N, W.o, cs, rs, st);
   if (rc) return rc;
-  return trimul_output(c, W.o, cs, rs, W.g, N, N, w, z, st, upd);
+  return trimul_output(c, W.o, cs, rs, nullptr, N, N, w, z, st, upd);
 }
 
 struct TriAttnWs {

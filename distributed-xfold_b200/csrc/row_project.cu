@@ -1,9 +1,10 @@
 // LayerNorm of the pair representation fused with the projections behind it:
-//   trimul : a, b = gated projections (channel planes), g = gating rows         (640 x 128 weights)
+//   trimul : a, b = gated projections (channel planes)                          (512 x 128 weights),
+//            for the row-shard stages also g = gating rows                        (640 x 128)
 //   attn   : q, k, v, gate (row-major [rows][512]) and the 4-head pair bias     (512 x 128 weights)
 //
-// Bound: HBM.  256 bytes of a row come in and 768 (trimul) or 1032 (attn) leave.  As two launches the normalised rows made an
-// extra round trip, and the projections' epilogues -- eight warps in lock-step over two staging buffers -- left HBM half idle.
+// Bound: HBM.  256 bytes of a row come in and 512 (trimul), 768 (with g) or 1032 (attn) leave.  As two launches the
+// normalised rows made an extra round trip, and the projections' epilogues -- eight warps in lock-step over two staging buffers -- left HBM half idle.
 //
 // Persistent CTAs keep the weights in shared memory and walk over tiles of 128 rows:
 //   warp 0              : TMA (weights once, then x tiles, two in flight)
@@ -13,7 +14,7 @@
 //   then NSET x 4 warps : epilogue, one set of four per unit of the ring, each set on its own: no set waits for another
 // A unit is 128 weight rows; for the gated projections [64 projection rows | 64 gate rows], so that both halves of 64 outputs
 // meet in one accumulator; g is two units of 64.  With few tiles the units are divided over several CTAs per tile (`parts`;
-// each normalises the tile for itself), so that a short sequence still uses the whole chip.  trimul has at least two parts
+// each normalises the tile for itself), so that a short sequence still uses the whole chip.  With g there are at least two parts
 // (a with half of g, b with the other half): 160 KB of weights would leave no room for a second x tile, and with one, its
 // load and normalisation stood between a tile's last product and the next tile's first (11 700 clocks per tile instead of
 // the 7200 that HBM needs in the attn form).
@@ -44,13 +45,15 @@ struct RowProjectArgs {
   int* status;
 };
 
-template <bool ATTN>
+enum RpMode : int { RP_TRIMUL = 0, RP_TRIMUL_G = 1, RP_ATTN = 2 };
+template <int MODE>
 struct RpCfg {
-  // units: attn q, k, v, gate; trimul a0, a1, g0, b0, b1, g1 (g: 64 columns)
-  static constexpr int UNITS = ATTN ? 4 : 6, NSET = ATTN ? 3 : 4, MIN_PARTS = ATTN ? 1 : 2;
+  static constexpr bool ATTN = MODE == RP_ATTN, G = MODE == RP_TRIMUL_G;
+  // units: attn q, k, v, gate; trimul a0, a1, b0, b1, with g a0, a1, g0, b0, b1, g1 (g: 64 columns)
+  static constexpr int UNITS = G ? 6 : 4, NSET = ATTN ? 3 : 4, MIN_PARTS = G ? 2 : 1;
   static constexpr int THREADS = (10 + 4 * NSET) * 32;
   static constexpr uint32_t W_UNIT = 32768, X_TILE = 32768;      // [2 K halves][128 rows][64], swizzled
-  static constexpr uint32_t STG = 128 * 32 * 2;                  // a set's staging tiles, [32 rows][32 columns] per warp
+  static constexpr uint32_t STG = ATTN || G ? 128 * 32 * 2 : 0;                  // a set's staging tiles, [32 rows][32 columns] per warp
   static constexpr uint32_t OFF_W = 0, OFF_X = OFF_W + UNITS / MIN_PARTS * W_UNIT, OFF_STG = OFF_X + 2 * X_TILE,
                             OFF_WB = OFF_STG + NSET * STG, OFF_GB = OFF_WB + (ATTN ? 4096 : 0), OFF_SC = OFF_GB + 1024,
                             OFF_CB = OFF_SC + (ATTN ? 2048 : 0), OFF_ST = OFF_CB + (ATTN ? 128 : 0),
@@ -58,12 +61,13 @@ struct RpCfg {
   static_assert(SMEM <= 232448, "shared memory");
 };
 
-template <bool ATTN>
-__global__ void __launch_bounds__(RpCfg<ATTN>::THREADS, 1)
+template <int MODE>
+__global__ void __launch_bounds__(RpCfg<MODE>::THREADS, 1)
 row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
                    const __grid_constant__ CUtensorMap tmo, const RowProjectArgs p) {
-  using Cfg = RpCfg<ATTN>;
-  constexpr int NSET = Cfg::NSET, UNITS = Cfg::UNITS;
+  using Cfg = RpCfg<MODE>;
+  constexpr int NSET = Cfg::NSET, UNITS = Cfg::UNITS, PER = UNITS / 2;  // PER: units of a (or b) and its part of g
+  constexpr bool ATTN = Cfg::ATTN;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -153,7 +157,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   const int t0 = int(blockIdx.x) / p.parts, step = int(gridDim.x) / p.parts;
   const int mine = t0 < p.tiles ? (p.tiles - t0 + step - 1) / step : 0;
   const bool with_bias = ATTN && part == 0 && p.w_bias;
-  auto unit_g = [](int g) { return !ATTN && g % 3 == 2; };
+  auto unit_g = [](int g) { return Cfg::G && g % 3 == 2; };
 
   if (warp == 0) {
     const uint32_t go = elect_one();  // warp-uniform, like the issuers
@@ -164,7 +168,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       uint8_t* sw = smem + Cfg::OFF_W + u * Cfg::W_UNIT;
       const int g = u0 + u;
       // first 64 and last 64 weight rows of the unit (g: 64 in all)
-      const int r0 = ATTN ? g * 128 : unit_g(g) ? 512 + (g / 3) * 64 : (g / 3) * 256 + (g % 3) * 64, r1 = ATTN ? r0 + 64 : r0 + 128;
+      const int r0 = ATTN ? g * 128 : unit_g(g) ? 512 + (g / 3) * 64 : (g / PER) * 256 + (g % PER) * 64, r1 = ATTN ? r0 + 64 : r0 + 128;
 #pragma unroll
       for (int kh = 0; kh < 2; ++kh) {
         tma_load_3d_if(go, sw + kh * 16384, &tmw, w_full, kh * 64, r0, 0);
@@ -247,26 +251,9 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       }
       uint8_t* sx = smem + Cfg::OFF_X + xb * Cfg::X_TILE;
       uint32_t xr[32];
-      float2 sm[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const uint4 u = *row_piece(sx, row, half * 8 + q);
-        xr[q * 4] = u.x; xr[q * 4 + 1] = u.y; xr[q * 4 + 2] = u.z; xr[q * 4 + 3] = u.w;
-      }
-#pragma unroll
-      for (int e = 0; e < 32; ++e) sum2(xr[e], sm[e & 1]);
-      float s = (sm[0].x + sm[0].y) + (sm[1].x + sm[1].y);
-      s += __shfl_xor_sync(0xffffffffu, s, 16);
-      const float nmean = -s * (1.f / 128);
-      float2 sq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        const float2 v = centre2(xr[e], nmean);
-        sq[e & 1] = ffma2(v, v, sq[e & 1]);
-      }
-      s = (sq[0].x + sq[0].y) + (sq[1].x + sq[1].y);
-      s += __shfl_xor_sync(0xffffffffu, s, 16);
-      const float rstd = rsqrtf(s * (1.f / 128) + 1e-5f);
+      load_half_row(sx, row, half, xr);
+      float nmean, rstd;
+      half_row_stats(xr, nmean, rstd);
       if (with_bias) {
         // (by tile parity: a warp may be one tile ahead of the readers, not two -- the barrier is in between)
         float2* rstat = reinterpret_cast<float2*>(smem + Cfg::OFF_ST) + xb * 128;
@@ -295,19 +282,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
           }
         }
       }
-      const float2 r2 = make_float2(rstd, rstd);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        uint32_t o[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int c = half * 64 + q * 8 + 2 * e;
-          const float2 ga = *reinterpret_cast<const float2*>(gb + c), be = *reinterpret_cast<const float2*>(gb + 128 + c);
-          const float2 v = ffma2(ffma2(centre2(xr[q * 4 + e], nmean), r2, make_float2(0.f, 0.f)), ga, be);
-          o[e] = pack_bf16x2(v.x, v.y);
-        }
-        *row_piece(sx, row, half * 8 + q) = make_uint4(o[0], o[1], o[2], o[3]);
-      }
+      store_half_row(sx, row, half, xr, nmean, rstd, gb);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&n_full[xb]);
@@ -383,7 +358,7 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
           off = (long long)c1 * p.row_stride + i;
           if (valid && p.mask) mk = p.mask[i * p.ntok + c1];
         }
-        bf16* dst = (g < 3 ? p.out_a : p.out_b) + off + (long long)(g % 3 * 64) * p.chan_stride;
+        bf16* dst = (g < PER ? p.out_a : p.out_b) + off + (long long)(g % PER * 64) * p.chan_stride;
         mbar_wait(&t_full[set], k & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
         tc_fence_after();
 #pragma unroll 1
@@ -423,13 +398,13 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   }
 }
 
-template <bool ATTN>
+template <int MODE>
 static int launch_row_project(Ctx* c, const CUtensorMap& tmx, const CUtensorMap& tmw, const CUtensorMap& tmo, RowProjectArgs& a,
                               cudaStream_t st) {
-  using Cfg = RpCfg<ATTN>;
+  using Cfg = RpCfg<MODE>;
   static bool attr_done[8] = {false};
   if (!attr_done[c->device & 7]) {
-    cudaError_t e = cudaFuncSetAttribute(row_project_kernel<ATTN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(row_project_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "row projection smem attribute: %s", cudaGetErrorString(e));
     attr_done[c->device & 7] = true;
   }
@@ -440,11 +415,12 @@ static int launch_row_project(Ctx* c, const CUtensorMap& tmx, const CUtensorMap&
   const int groups = a.tiles < sms / a.parts ? a.tiles : sms / a.parts;
   a.static_w = c->static_weights;
   a.status = c->d_status;
-  ProfScope ps(c, ATTN ? XFOLD_K_LINEAR : XFOLD_K_TRIMUL_PROJ, st);
-  launch_pdl(row_project_kernel<ATTN>, groups * a.parts, Cfg::THREADS, Cfg::SMEM, st, tmx, tmw, tmo, a);
+  ProfScope ps(c, Cfg::ATTN ? XFOLD_K_LINEAR : XFOLD_K_TRIMUL_PROJ, st);
+  launch_pdl(row_project_kernel<MODE>, groups * a.parts, Cfg::THREADS, Cfg::SMEM, st, tmx, tmw, tmo, a);
   return check_launch(c, "row_project_kernel");
 }
 
+// out_g null: a and b alone
 int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, int N, int transposed, const float* gamma,
                               const float* beta, const bf16* w_in, bf16* out_a, bf16* out_b, bf16* out_g, long long chan_stride,
                               long long row_stride, cudaStream_t st) {
@@ -454,11 +430,11 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   bool ok;
   if (!transposed) {
     ok = make_tmap_bf16_3d(&tmx, z, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) &&
-         make_tmap_bf16_3d(&tmo, out_g, 128, M, 1, 128, (uint64_t)128 * M, 32, 32, 1, 64);
+         make_tmap_bf16_3d(&tmo, out_g ? out_g : z, 128, M, 1, 128, (uint64_t)128 * M, 32, 32, 1, 64);
     a.tiles = (int)((M + 127) / 128);
   } else {  // tile rows step along the first token axis, second axis fixed: a[j][c][i]
     ok = make_tmap_bf16_3d(&tmx, z, 128, N, R, 128, (uint64_t)128 * N, 64, 1, 128) &&
-         make_tmap_bf16_3d(&tmo, out_g, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 32, 64);
+         make_tmap_bf16_3d(&tmo, out_g ? out_g : z, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 32, 64);
     a.mode1 = 1;
     a.dim1 = N;
     a.tiles = N * ((R + 127) / 128);
@@ -475,7 +451,7 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   a.row_stride = row_stride;
   a.ntok = N;
   a.mask = mask;
-  return launch_row_project<false>(c, tmx, tmw, tmo, a, st);
+  return out_g ? launch_row_project<RP_TRIMUL_G>(c, tmx, tmw, tmo, a, st) : launch_row_project<RP_TRIMUL>(c, tmx, tmw, tmx, a, st);
 }
 
 // norm = 0: z is normalised already, and w_bias (then null) has no output
@@ -500,7 +476,7 @@ int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, int norm, const
   a.pitch = pitch;
   a.inner = N;
   a.plane = plane;
-  return launch_row_project<true>(c, tmx, tmw, tmo, a, st);
+  return launch_row_project<RP_ATTN>(c, tmx, tmw, tmo, a, st);
 }
 
 }  // namespace xf

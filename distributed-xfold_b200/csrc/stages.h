@@ -57,7 +57,8 @@ int launch_row_project_attn(Ctx* c, const bf16* z, int R, int N, int norm, const
 // output projections of the pair representation (row_output.cu)
 int launch_row_output(Ctx* c, const bf16* x, long long M, const bf16* w, const bf16* resid, bf16* out, cudaStream_t st);
 int launch_row_output_cm(Ctx* c, const bf16* o, long long o_cs, long long o_rs, int R, int N, const float* gamma, const float* beta,
-                         const bf16* w, const bf16* g, const bf16* resid, bf16* out, cudaStream_t st);
+                         const bf16* w, const bf16* g, const float* g_gamma, const float* g_beta, const bf16* wg, const bf16* z,
+                         int resid, bf16* out, cudaStream_t st);
 int launch_swiglu(Ctx* c, const bf16* in, bf16* out, long long rows, int F, cudaStream_t st);
 // ---- linear layers on the GEMM kernel (api.cu) -----------------------------------------------------------
 int linear_plain(Ctx* c, const bf16* x, long long ldx, long long M, int K, const bf16* w, int N, const float* bias,

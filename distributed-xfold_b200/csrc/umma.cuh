@@ -419,6 +419,47 @@ __device__ __forceinline__ void row_stats(uint8_t* tile, int row, float& nmean, 
   }
   rstd = rsqrtf((sq.x + sq.y) * (1.f / 128) + 1e-5f);
 }
+// The same by two threads of a warp, lanes l and l + 16, with half a row each in registers: xr = columns [64 half, 64 half + 64).
+__device__ __forceinline__ void load_half_row(uint8_t* tile, int row, int half, uint32_t (&xr)[32]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint4 u = *row_piece(tile, row, half * 8 + q);
+    xr[q * 4] = u.x; xr[q * 4 + 1] = u.y; xr[q * 4 + 2] = u.z; xr[q * 4 + 3] = u.w;
+  }
+}
+__device__ __forceinline__ void half_row_stats(const uint32_t (&xr)[32], float& nmean, float& rstd) {
+  float2 sm[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int e = 0; e < 32; ++e) sum2(xr[e], sm[e & 1]);
+  float s = (sm[0].x + sm[0].y) + (sm[1].x + sm[1].y);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  nmean = -s * (1.f / 128);
+  float2 sq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    const float2 v = centre2(xr[e], nmean);
+    sq[e & 1] = ffma2(v, v, sq[e & 1]);
+  }
+  s = (sq[0].x + sq[0].y) + (sq[1].x + sq[1].y);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  rstd = rsqrtf(s * (1.f / 128) + 1e-5f);
+}
+__device__ __forceinline__ void store_half_row(uint8_t* tile, int row, int half, const uint32_t (&xr)[32], float nmean, float rstd,
+                                               const float* gb) {
+  const float2 r2 = make_float2(rstd, rstd);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = half * 64 + q * 8 + 2 * e;
+      const float2 ga = *reinterpret_cast<const float2*>(gb + c), be = *reinterpret_cast<const float2*>(gb + 128 + c);
+      const float2 v = ffma2(ffma2(centre2(xr[q * 4 + e], nmean), r2, make_float2(0.f, 0.f)), ga, be);
+      o[e] = pack_bf16x2(v.x, v.y);
+    }
+    *row_piece(tile, row, half * 8 + q) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
 __device__ __forceinline__ void row_normalise(uint8_t* tile, int row, float nmean, float rstd, const float* gb) {
   const float2 r2 = make_float2(rstd, rstd);
 #pragma unroll 4
