@@ -24,8 +24,9 @@
 //         tokens, and 131 KB of keys and values).
 //   TILES: the slots are neighbouring query tiles of one batch row and head; they share the keys and values.
 // CTAs are persistent and run their items' key blocks as one continuous sequence.
-//   warp 0         : TMA producer.  Two rings of 64-key stages: {K, bias, mask} is free again when the block's logits are
-//                    complete, {V} when its P V product is.
+//   warp 0         : TMA producer.  A ring of stages {K, bias, mask of block u, V of block u - 2}: what an issuer needs for
+//                    one step, with one barrier each way.  (As two rings, an issuer waited and committed twice as often:
+//                    41 -> 40 us at 255 tokens, 1-2 % at 1024.)
 //   warps 1 .. NS  : one issuer of tcgen05.mma per slot (warp-uniform code, one elected lane).
 //   warps 4 ..     : one softmax warpgroup per slot, one thread per query row.
 // Tensor memory per slot: 128 columns of logits / probabilities, D columns of output.
@@ -58,19 +59,19 @@ struct AttnArgs {
 template <int D, bool ROWS>
 struct AttnCfg {
   static constexpr int NS = ROWS ? 3 : 2;
-  static constexpr int NK = ROWS ? 4 : 3, NV = 4;               // stages of the two rings, 64 keys each
+  static constexpr int NK = ROWS ? 4 : 3;                      // stages of the ring, 64 keys each
   static constexpr int THREADS = (4 + 4 * NS) * 32;
   static constexpr uint32_t KT = 64 * D * 2;                   // one [64 keys][D] tile
   static constexpr uint32_t BT = 128 * 64 * 2;                 // one [128 queries][64 keys] bias tile
   static constexpr uint32_t MT = 1024;                         // one [64 keys][8] mask tile
   static constexpr uint32_t QT = 128 * D * 2;
   static constexpr uint32_t K_BYTES = (ROWS ? NS : 1) * KT, B_BYTES = (ROWS ? 1 : NS) * BT, M_BYTES = (ROWS ? NS : 1) * MT;
-  static constexpr uint32_t KSTAGE = B_BYTES + K_BYTES + M_BYTES, VSTAGE = K_BYTES;
-  static constexpr uint32_t OFF_K = 0, OFF_V = OFF_K + NK * KSTAGE, OFF_Q = OFF_V + NV * VSTAGE, OFF_ID = OFF_Q + 2 * NS * QT,
+  static constexpr uint32_t STAGE = B_BYTES + 2 * K_BYTES + M_BYTES;
+  static constexpr uint32_t OFF_V = B_BYTES + K_BYTES + M_BYTES, OFF_Q = NK * STAGE, OFF_ID = OFF_Q + 2 * NS * QT,
                             OFF_E1 = OFF_ID + 512, OFF_ZERO = OFF_E1 + 2048, OFF_BAR = OFF_ZERO + 2048,
                             SMEM = OFF_BAR + 512 + 1024;
   static constexpr uint32_t TM_O = NS * 128;                   // output columns behind the logits
-  static_assert(KSTAGE % 1024 == 0 && VSTAGE % 1024 == 0 && QT % 1024 == 0, "swizzled tiles start at multiples of 1 KB");
+  static_assert(STAGE % 1024 == 0 && K_BYTES % 1024 == 0 && QT % 1024 == 0, "swizzled tiles start at multiples of 1 KB");
   static_assert(SMEM <= 232448, "shared memory");
 };
 
@@ -126,16 +127,14 @@ __global__ void __launch_bounds__(AttnCfg<D, ROWS>::THREADS, 1)
 attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmkv,
             const __grid_constant__ CUtensorMap tmb, const AttnArgs p) {
   using Cfg = AttnCfg<D, ROWS>;
-  constexpr int NS = Cfg::NS, NK = Cfg::NK, NV = Cfg::NV;
+  constexpr int NS = Cfg::NS, NK = Cfg::NK;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* k_full = bars;              // [NK] K, bias and mask of a stage have landed
-  uint64_t* k_empty = k_full + NK;      // [NK] every slot's logits of the stage are complete
-  uint64_t* v_full = k_empty + NK;      // [NV]
-  uint64_t* v_empty = v_full + NV;      // [NV] every slot's P V product of the stage is complete
-  uint64_t* q_full = v_empty + NV;      // [2] (Q of the next item arrives while this one's is in use)
+  uint64_t* full = bars;                // [NK] a stage's tiles have landed
+  uint64_t* empty = full + NK;          // [NK] every slot's products that read the stage are complete
+  uint64_t* q_full = empty + NK;       // [2] (Q of the next item arrives while this one's is in use)
   uint64_t* q_empty = q_full + 2;       // [2] every slot's last logits of the item are complete
   uint64_t* s_full = q_empty + 2;       // [NS][2] a block's logits are complete
   uint64_t* p_ready = s_full + 2 * NS;  // [NS][2] the block's P is in tensor memory
@@ -160,12 +159,8 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NK; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], ns);
-    }
-    for (int s = 0; s < NV; ++s) {
-      mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], ns);
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], ns);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&q_full[s], 1);
@@ -210,58 +205,53 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------------ TMA producer
-    // V is loaded two blocks later than K, so that waiting for a V buffer (free after P V) never holds up the keys of
-    // the block before it; V goes first, because the wait for Q's buffer may depend on it.
+    // Stage u holds keys, bias and mask of block u and the values of block u - 2: what the issuers need for one step.
     const uint32_t go = elect_one();  // warp-uniform, like the issuers
     const uint64_t my_items = n_items > blockIdx.x ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const uint64_t total = my_items * uint64_t(NB);
-    uint32_t kst = 0, kph = 0, vst = 0, vph = 0, it = 0, item_k = blockIdx.x, item_v = blockIdx.x;
+    uint32_t st = 0, ph = 0, it = 0, item_k = blockIdx.x, item_v = blockIdx.x;
     int ks = 0, vs = 0, qt = 0, h = 0, b = 0, vqt, vh, vb;
     decode(item_v, vqt, vh, vb);
-    bool okay = true;
-    for (uint64_t t = 0; t < total + 2 && okay; ++t) {
-      if (t >= 2) {
-        if (!mbar_wait_warp(&v_empty[vst], vph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-        mbar_arrive_expect_tx_if(go, &v_full[vst], Cfg::VSTAGE);
-        tma_load_3d_if(go, smem + Cfg::OFF_V + vst * Cfg::VSTAGE, &tmkv, &v_full[vst], p.v_col0 + vh * D, vs * 64, vb);
-        if (++vst == NV) { vst = 0; vph ^= 1u; }
+    for (uint64_t u = 0; u < (total ? total + 2 : 0); ++u) {
+      if (u < total && ks == 0) {
+        decode(item_k, qt, h, b);
+        const uint32_t qb = it & 1u;
+        if (!mbar_wait_warp(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+        mbar_arrive_expect_tx_if(go, &q_full[qb], (ROWS ? NS : ns) * Cfg::QT);
+        uint8_t* sq = smem + Cfg::OFF_Q + qb * (NS * Cfg::QT);
+        if constexpr (ROWS) tma_load_3d_if(go, sq, &tmq, &q_full[qb], p.q_col0 + h * D, qt * 128, b);
+        else
+          for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sq + s * Cfg::QT, &tmq, &q_full[qb], p.q_col0 + h * D, (qt + s) * 128, b);
+        ++it;
+      }
+      if (!mbar_wait_warp(&empty[st], ph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
+      uint8_t* sb = smem + st * Cfg::STAGE;
+      uint8_t* sk = sb + Cfg::B_BYTES;
+      uint8_t* sm = sk + Cfg::K_BYTES;
+      int nm = 1;  // mask tiles: one per batch row of the item
+      if constexpr (ROWS) nm = p.mext_batch_stride == 0 ? 1 : (p.B - b < NS ? p.B - b : NS);
+      mbar_arrive_expect_tx_if(go, &full[st], (u < total ? (ROWS ? 1 : ns) * Cfg::BT + Cfg::K_BYTES + nm * Cfg::MT : 0) + (u >= 2 ? Cfg::K_BYTES : 0));
+      if (u < total) {
+        tma_load_3d_if(go, sk, &tmkv, &full[st], p.k_col0 + h * D, ks * 64, b);
+        if constexpr (ROWS) tma_load_3d_if(go, sb, &tmb, &full[st], ks * 64, qt * 128, h);
+        else
+          for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sb + s * Cfg::BT, &tmb, &full[st], ks * 64, (qt + s) * 128, h);
+        const uint8_t* mrow = p.mext + (long long)b * p.mext_batch_stride + (long long)ks * Cfg::MT;
+        for (int s = 0; s < nm; ++s) bulk_load_if(go, sm + s * Cfg::MT, mrow + s * p.mext_batch_stride, Cfg::MT, &full[st]);
+        if (++ks == NB) {
+          ks = 0;
+          item_k += gridDim.x;
+        }
+      }
+      if (u >= 2) {
+        tma_load_3d_if(go, sb + Cfg::OFF_V, &tmkv, &full[st], p.v_col0 + vh * D, vs * 64, vb);
         if (++vs == NB) {
           vs = 0;
           item_v += gridDim.x;
           decode(item_v, vqt, vh, vb);
         }
       }
-      if (t < total) {
-        if (ks == 0) {
-          decode(item_k, qt, h, b);
-          const uint32_t qb = it & 1u;
-          if (!mbar_wait_warp(&q_empty[qb], ((it >> 1) & 1u) ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-          mbar_arrive_expect_tx_if(go, &q_full[qb], (ROWS ? NS : ns) * Cfg::QT);
-          uint8_t* sq = smem + Cfg::OFF_Q + qb * (NS * Cfg::QT);
-          if constexpr (ROWS) tma_load_3d_if(go, sq, &tmq, &q_full[qb], p.q_col0 + h * D, qt * 128, b);
-          else
-            for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sq + s * Cfg::QT, &tmq, &q_full[qb], p.q_col0 + h * D, (qt + s) * 128, b);
-          ++it;
-        }
-        if (!mbar_wait_warp(&k_empty[kst], kph ^ 1u, ab, XF_ERR_WAIT_EMPTY)) break;
-        uint8_t* sb = smem + Cfg::OFF_K + kst * Cfg::KSTAGE;
-        uint8_t* sk = sb + Cfg::B_BYTES;
-        uint8_t* sm = sk + Cfg::K_BYTES;
-        int nm = 1;  // mask tiles: one per batch row of the item
-        if constexpr (ROWS) nm = p.mext_batch_stride == 0 ? 1 : (p.B - b < NS ? p.B - b : NS);
-        mbar_arrive_expect_tx_if(go, &k_full[kst], (ROWS ? 1 : ns) * Cfg::BT + Cfg::K_BYTES + nm * Cfg::MT);
-        tma_load_3d_if(go, sk, &tmkv, &k_full[kst], p.k_col0 + h * D, ks * 64, b);
-        if constexpr (ROWS) tma_load_3d_if(go, sb, &tmb, &k_full[kst], ks * 64, qt * 128, h);
-        else
-          for (int s = 0; s < ns; ++s) tma_load_3d_if(go, sb + s * Cfg::BT, &tmb, &k_full[kst], ks * 64, (qt + s) * 128, h);
-        const uint8_t* mrow = p.mext + (long long)b * p.mext_batch_stride + (long long)ks * Cfg::MT;
-        for (int s = 0; s < nm; ++s) bulk_load_if(go, sm + s * Cfg::MT, mrow + s * p.mext_batch_stride, Cfg::MT, &k_full[kst]);
-        if (++kst == NK) { kst = 0; kph ^= 1u; }
-        if (++ks == NB) {
-          ks = 0;
-          item_k += gridDim.x;
-        }
-      }
+      if (++st == NK) { st = 0; ph ^= 1u; }
     }
   } else if (warp <= ns && warp < 4) {
     // ---------------------------------------------------------------------------------------- issuer of slot s
@@ -275,61 +265,59 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
     constexpr uint32_t idesc_pv = make_idesc(128, D, 0, 1, 1);         // fp16 (the v columns are projected to fp16), V N-major
     const uint32_t base = smem_u32(smem);
     const uint32_t d_s = tmem_base + s * 128, d_o = tmem_base + Cfg::TM_O + s * D;
+    // descriptors of stage 0 (a stage further: their low words move by the stage's size in 16-byte units), hi words constant
     const uint64_t qd0 = make_sdesc_d<D>(base + Cfg::OFF_Q + s * Cfg::QT);
     const uint64_t idd = make_sdesc_noswizzle(base + Cfg::OFF_ID, 128, 256);
     const uint64_t e1d = make_sdesc_noswizzle(base + Cfg::OFF_E1, Cfg::OFF_ZERO - Cfg::OFF_E1, 128);
-    const uint32_t bias_off = ROWS ? 0 : s * Cfg::BT, k_off = Cfg::B_BYTES + (ROWS ? s * Cfg::KT : 0);
-    const uint32_t m_off = Cfg::B_BYTES + Cfg::K_BYTES + (ROWS && p.mext_batch_stride != 0 ? s * Cfg::MT : 0);
-    const uint32_t v_off = Cfg::OFF_V + (ROWS ? s * Cfg::KT : 0);
-    uint32_t kst = 0, kph = 0, vst = 0, vph = 0, it_s = 0, gs = 0;
-    int jb = 0;  // block whose logits are issued next, within its item (gs: within the sequence of blocks)
-    auto issue_s = [&]() -> bool {
-      const uint32_t qb = it_s & 1u;
-      if (jb == 0 && !mbar_wait_warp(&q_full[qb], (it_s >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) return false;
-      if (!mbar_wait_warp(&k_full[kst], kph, ab, XF_ERR_WAIT_FULL)) return false;
-      tc_fence_after();
-      const uint32_t st = base + Cfg::OFF_K + kst * Cfg::KSTAGE, d = d_s + (gs & 1u) * 64;
-      const uint64_t qd = qd0 + uint64_t(qb * (NS * Cfg::QT / 16));
-      const uint64_t kd = make_sdesc_d<D>(st + k_off), bd = make_sdesc(st + bias_off, 16, 1024);
-      const uint64_t md = make_sdesc_noswizzle(st + m_off, base + Cfg::OFF_ZERO - (st + m_off), 128);
-#pragma unroll
-      for (int j = 0; j < D / 16; ++j) umma_ss_if(leader, d, qd + uint64_t(2 * j), kd + uint64_t(2 * j), idesc_qk, j ? 1u : 0u);
-      umma_ss_if(leader, d, e1d, md, idesc_qk, 1u);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) umma_ss_if(leader, d + j * 16, bd + uint64_t(2 * j), idd, idesc_bias, 1u);
-      umma_commit_if(leader, &s_full[2 * s + (gs & 1u)]);
-      umma_commit_if(leader, &k_empty[kst]);
-      if (++kst == NK) { kst = 0; kph ^= 1u; }
-      ++gs;
-      if (++jb == NB) {
-        jb = 0;
-        ++it_s;
-        umma_commit_if(leader, &q_empty[qb]);
-      }
-      return true;
-    };
+    const uint32_t m_at = base + Cfg::B_BYTES + Cfg::K_BYTES + (ROWS && p.mext_batch_stride != 0 ? s * Cfg::MT : 0);
+    const uint64_t kd0 = make_sdesc_d<D>(base + Cfg::B_BYTES + (ROWS ? s * Cfg::KT : 0));
+    const uint64_t bd0 = make_sdesc(base + (ROWS ? 0 : s * Cfg::BT), 16, 1024);
+    const uint64_t md0 = make_sdesc_noswizzle(m_at, base + Cfg::OFF_ZERO - m_at, 128);
+    const uint64_t vd0 = make_sdesc_d<D>(base + Cfg::OFF_V + (ROWS ? s * Cfg::KT : 0));
+    const uint32_t klo = uint32_t(kd0), khi = uint32_t(kd0 >> 32), blo = uint32_t(bd0), bhi = uint32_t(bd0 >> 32), mlo = uint32_t(md0),
+                   mhi = uint32_t(md0 >> 32), vlo = uint32_t(vd0), vhi = uint32_t(vd0 >> 32);
     const uint32_t my_items = n_items > blockIdx.x ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
     const uint32_t G = my_items * uint32_t(NB);  // (the launcher bounds it)
-    bool okay = true;
-    for (uint32_t i = 0; i < 2 && i < G && okay; ++i) okay = issue_s();
-    int kb = 0;
-    for (uint32_t g = 0; g < G && okay; ++g) {
-      if (!mbar_wait_warp(&v_full[vst], vph, ab, XF_ERR_WAIT_FULL)) break;  // it has landed long before
-      if (!mbar_wait_warp(&p_ready[2 * s + (g & 1u)], (g >> 1) & 1u, ab, XF_ERR_WAIT_ATTN)) break;
-      tc_fence_after();
-      const uint64_t vd = make_sdesc_d<D>(base + v_off + vst * Cfg::VSTAGE);
-      const uint32_t a_p = d_s + (g & 1u) * 64;
-      const int keys = p.S - kb * 64;
+    uint32_t st = 0, ph = 0, it = 0, so = 0;
+    int jb = 0, kb = 0;  // blocks of the logits and of the P V product within their items
+    // One step: P V of block u - 2, then the logits of block u over that P (products of one issuer execute in order).
+    for (uint32_t u = 0; u < (G ? G + 2 : 0); ++u) {
+      if (u < G && jb == 0 && !mbar_wait_warp(&q_full[it & 1u], (it >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) break;
+      if (!mbar_wait_warp(&full[st], ph, ab, XF_ERR_WAIT_FULL)) break;
+      const uint32_t x = u & 1u, d = d_s + x * 64;
+      if (u >= 2) {
+        if (!mbar_wait_warp(&p_ready[2 * s + x], ((u - 2) >> 1) & 1u, ab, XF_ERR_WAIT_ATTN)) break;
+        tc_fence_after();
+        const int keys = p.S - kb * 64;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {  // 16 keys = 32 D bytes of V = 8 columns of P
-        if ((j & ~1) * 16 >= keys) break;  // keys beyond the sequence are left out in steps of 32, as in the sweeps
-        umma_ts_if(leader, d_o, a_p + j * 8, vd + uint64_t(j * 2 * D), idesc_pv, (kb | j) ? 1u : 0u);
+        for (int j = 0; j < 4; ++j) {  // 16 keys = 32 D bytes of V = 8 columns of P
+          if ((j & ~1) * 16 >= keys) break;  // keys beyond the sequence are left out in steps of 32, as in the sweeps
+          umma_ts_lo_if(leader, d_o, d + j * 8, vlo + so + j * 2 * D, vhi, idesc_pv, (kb | j) ? 1u : 0u);
+        }
+        umma_commit_if(leader, &pv_done[2 * s + x]);
+        if (++kb == NB) kb = 0;
       }
-      umma_commit_if(leader, &pv_done[2 * s + (g & 1u)]);
-      umma_commit_if(leader, &v_empty[vst]);
-      if (++vst == NV) { vst = 0; vph ^= 1u; }
-      if (++kb == NB) kb = 0;
-      if (g + 2 < G) okay = issue_s();  // over P: executes behind the products that read it
+      if (u < G) {
+        tc_fence_after();
+        const uint32_t qb = it & 1u;
+        const uint64_t qd = qd0 + uint64_t(qb * (NS * Cfg::QT / 16));
+#pragma unroll
+        for (int j = 0; j < D / 16; ++j)
+          umma_ss_lo_if(leader, d, uint32_t(qd) + 2 * j, uint32_t(qd >> 32), klo + so + 2 * j, khi, idesc_qk, j ? 1u : 0u);
+        umma_ss_lo_if(leader, d, uint32_t(e1d), uint32_t(e1d >> 32), mlo - so * 65535u, mhi, idesc_qk, 1u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          umma_ss_lo_if(leader, d + j * 16, blo + so + 2 * j, bhi, uint32_t(idd), uint32_t(idd >> 32), idesc_bias, 1u);
+        umma_commit_if(leader, &s_full[2 * s + x]);
+        if (++jb == NB) {
+          jb = 0;
+          ++it;
+          umma_commit_if(leader, &q_empty[qb]);
+        }
+      }
+      umma_commit_if(leader, &empty[st]);
+      so += Cfg::STAGE / 16;
+      if (++st == NK) { st = 0; ph ^= 1u; so = 0; }
     }
   } else if (warp >= 4 && warp < 4 + 4 * ns) {
     // ------------------------------------------------------------------------------------------------ softmax warps
