@@ -194,7 +194,9 @@ __device__ __forceinline__ void tma_store_wait_read() {
 }
 // waits until this thread's bulk stores have been written (the .read form: only read out of shared memory)
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// (bar.sync counts a warp that is not converged once for each of its parts: a warp that stored with some lanes only converges first)
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
