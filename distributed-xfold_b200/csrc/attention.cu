@@ -104,14 +104,6 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   return make_float2(q.x * __uint_as_float(__float_as_uint(t.x) * 0x800000u + 0x3F800000u),
                      q.y * __uint_as_float(__float_as_uint(t.y) * 0x800000u + 0x3F800000u));
 }
-__device__ __forceinline__ void tmem_st16_(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait_() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Which of a sweep's 16 pairs take the polynomial: two.  (TriangleAttention, 1024 tokens: none 1.33 ms, two or three 1.27,
 // four or five 1.32, six 1.44 -- the FMA pipe and the issue slots are then the longer queue.)
 __host__ __device__ constexpr bool poly_pair(int e) { return (e & 7) == 7; }
@@ -377,13 +369,13 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
                       tmem_ld_wait();
 #pragma unroll
                       for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-                      tmem_st16_(o_addr + oc, o);
+                      tmem_st16(o_addr + oc, o);
                     }
                   }
                   if (c > 0) {  // so is the first half of the block's P
                     const __half2 a2 = __float2half2_rn(alpha);
                     uint32_t q[16];
-                    tmem_st_wait_();
+                    tmem_st_wait();
                     tmem_ld16(buf, q);
                     tmem_ld_wait();
 #pragma unroll
@@ -391,7 +383,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
                       const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&q[e]), a2);
                       q[e] = *reinterpret_cast<const uint32_t*>(&v);
                     }
-                    tmem_st16_(buf, q);
+                    tmem_st16(buf, q);
                   }
                 }
               }
@@ -410,11 +402,11 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
             }
             if (!okay) break;
             l2 = fadd2(l2, s2);
-            tmem_st16_(buf + c * 16, pk);  // over logits that have been read
+            tmem_st16(buf + c * 16, pk);  // over logits that have been read
           }
         }
         if (!okay) break;
-        tmem_st_wait_();
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[2 * s + (g & 1u)]);

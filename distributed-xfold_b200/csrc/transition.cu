@@ -4,17 +4,19 @@
 // Bound: the tensor core.  Per tile of 128 rows 25 M multiply-adds (6100 clocks) and 65536 sigmoids (4096 clocks of the
 // special-function unit); the weights are 384 KB at F = 512, so two tiles share each block of them.  The only HBM traffic is
 // x itself.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) the normalised rows and the hidden activations made six
-// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows; this kernel 0.46 ms by itself (one tile at a time: 0.49),
-// 0.49 back to back, 0.53 in a recycle at the power limit.
+// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows.
 //
 // Persistent CTAs, a pair of tiles (A, B) of 128 rows at a time, hidden units in blocks of 64; per tile
 //     D1 = LN(x) W1(block)^T   [128 x (64 SiLU | 64 linear)]      tensor memory
-//     h  = silu(D1a) * D1b     bf16, shared memory (K-major, 128-byte swizzle)
+//     h  = silu(D1a) * D1b     bf16, tensor memory, over the D1 it comes from
 //     D2 += h W2(block)^T      [128 x 128]                        tensor memory
 //   warp 0         : TMA -- x tiles, weight blocks of 32 KB (W1, free after D1) and 16 KB (W2), two of each
-//   warp 1         : tcgen05.mma issuer; D1 of a block is issued ahead of D2 of the block before it
+//   warp 1         : tcgen05.mma issuer, the tiles in turn: D2 of a block and right behind it D1 of the next, which goes over
+//                    the h that D2 reads (products of one issuer execute in order)
 //   warps 2 - 9    : LayerNorm in place, one thread per row
-//   warps 10 - 17  : one set of four per tile: D1 -> h; finally D2 + x -> the h buffer in two halves, which leave by TMA
+//   warps 10 - 17  : one set of four per tile: D1 -> h; finally D2 + x -> a staging tile in two halves, which leave by TMA
+// The operands' trips from shared memory bound it (128 bytes per clock): with h in tensor memory they are 21 % fewer.  (h in
+// shared memory, D1 a block ahead of it: 0.54 ms in the trunk of 1024 tokens, now 0.50.  Sixteen warps for D1 -> h: no gain.)
 // With no more tiles than SMs a CTA takes one tile (B is left out).
 #include "internal.h"
 #include "stages.h"
@@ -24,7 +26,7 @@ namespace xf {
 
 constexpr uint32_t TR_TILE = 32768;                       // [2 halves][128 rows][64 columns], swizzled
 constexpr uint32_t TR_W1 = 32768, TR_W2 = 16384;          // a block's weights: [2 K halves][128 rows][64], [128 rows][64]
-constexpr uint32_t TR_H = 16384;
+constexpr uint32_t TR_H = 16384;                          // a tile's staging, [128 rows][64 columns]
 constexpr uint32_t TR_OFF_N = 0, TR_OFF_W1 = 2 * TR_TILE, TR_OFF_W2 = TR_OFF_W1 + 2 * TR_W1, TR_OFF_H = TR_OFF_W2 + 2 * TR_W2,
                    TR_OFF_GB = TR_OFF_H + 2 * TR_H, TR_OFF_BAR = TR_OFF_GB + 1024, TR_SMEM = TR_OFF_BAR + 256 + 1024;
 constexpr int TR_THREADS = 18 * 32;
@@ -55,10 +57,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
   uint64_t* w2_full = w1_empty + 2;  // [2]
   uint64_t* w2_empty = w2_full + 2;  // [2] the block's D2 products are complete
   uint64_t* d1_full = w2_empty + 2;  // [tile]
-  uint64_t* d1_empty = d1_full + 2;  // [tile] in registers
-  uint64_t* h_full = d1_empty + 2;   // [tile]
-  uint64_t* h_empty = h_full + 2;    // [tile] D2 has read h
-  uint64_t* d2_full = h_empty + 2;   // [tile]
+  uint64_t* h_full = d1_full + 2;    // [tile] h stands over D1
+  uint64_t* d2_full = h_full + 2;    // [tile]
   uint64_t* d2_empty = d2_full + 2;  // [tile]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d2_empty + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -75,9 +75,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
       mbar_init(&w2_full[s], 1);
       mbar_init(&w2_empty[s], 1);
       mbar_init(&d1_full[s], 1);
-      mbar_init(&d1_empty[s], 4);
       mbar_init(&h_full[s], 4);
-      mbar_init(&h_empty[s], 1);
       mbar_init(&d2_full[s], 1);
       mbar_init(&d2_empty[s], 4);
     }
@@ -157,50 +155,58 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc = make_idesc(128, 128);
     uint32_t g1 = 0, g2 = 0;  // blocks whose D1 / D2 have been issued
-    auto d1 = [&](int hb, uint32_t item) -> bool {
-      const uint32_t b = g1 & 1u;
-      if (!mbar_wait_warp(&w1_full[b], (g1 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) return false;
-      const uint64_t wd = make_sdesc(base + TR_OFF_W1 + b * TR_W1, 16, 1024);
-      for (int s = 0; s < NT; ++s) {
-        if (hb == 0 && !mbar_wait_warp(&n_full[s], item & 1u, ab, XF_ERR_WAIT_FULL)) return false;
-        if (!mbar_wait_warp(&d1_empty[s], (g1 & 1u) ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint64_t nd = make_sdesc(base + TR_OFF_N + s * TR_TILE, 16, 1024);
+    // D1 of the block after g1's for tile s (the products that read the h it goes over were issued before: in order)
+    auto d1 = [&](int s) {
+      const uint64_t wd = make_sdesc(base + TR_OFF_W1 + (g1 & 1u) * TR_W1, 16, 1024);
+      const uint64_t nd = make_sdesc(base + TR_OFF_N + s * TR_TILE, 16, 1024);
 #pragma unroll
-        for (int kh = 0; kh < 2; ++kh)
+      for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_ss_if(leader, tmem_base + s * 128, nd + uint64_t(kh * 1024 + 2 * j), wd + uint64_t(kh * 1024 + 2 * j), idesc,
-                       (kh | j) ? 1u : 0u);
-        umma_commit_if(leader, &d1_full[s]);
-        if (hb == NBK - 1) umma_commit_if(leader, &n_empty[s]);
-      }
-      umma_commit_if(leader, &w1_empty[b]);
-      ++g1;
-      return true;
+        for (int j = 0; j < 4; ++j)
+          umma_ss_if(leader, tmem_base + s * 128, nd + uint64_t(kh * 1024 + 2 * j), wd + uint64_t(kh * 1024 + 2 * j), idesc,
+                     (kh | j) ? 1u : 0u);
+      umma_commit_if(leader, &d1_full[s]);
     };
-    bool okay = mine > 0 ? d1(0, 0) : true;
+    auto w1_ready = [&]() { return mbar_wait_warp(&w1_full[g1 & 1u], (g1 >> 1) & 1u, ab, XF_ERR_WAIT_FULL); };
+    bool okay = true;
     for (int it = 0; it < mine && okay; ++it) {
+      if (!w1_ready()) break;
+      for (int s = 0; s < NT && okay; ++s) {
+        okay = mbar_wait_warp(&n_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL);
+        if (!okay) break;
+        tc_fence_after();
+        d1(s);
+        if (NBK == 1) umma_commit_if(leader, &n_empty[s]);
+      }
+      if (!okay) break;
+      umma_commit_if(leader, &w1_empty[g1 & 1u]);
+      ++g1;
       for (int hb = 0; hb < NBK && okay; ++hb) {
-        // the next block's D1 first; at the item's end D2 (the next item's rows are still on their way)
-        if (hb + 1 < NBK && !d1(hb + 1, it)) { okay = false; break; }
         const uint32_t b = g2 & 1u;
+        const bool more = hb + 1 < NBK;
+        if (more && !w1_ready()) { okay = false; break; }
         if (!mbar_wait_warp(&w2_full[b], (g2 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
         const uint64_t wd = make_sdesc(base + TR_OFF_W2 + b * TR_W2, 16, 1024);
         for (int s = 0; s < NT && okay; ++s) {
           if (hb == 0 && !mbar_wait_warp(&d2_empty[s], (uint32_t(it) & 1u) ^ 1u, ab, XF_ERR_WAIT_TMEM_EMPTY)) { okay = false; break; }
           if (!mbar_wait_warp(&h_full[s], g2 & 1u, ab, XF_ERR_WAIT_FULL)) { okay = false; break; }
           tc_fence_after();
-          const uint64_t hd = make_sdesc(base + TR_OFF_H + s * TR_H, 16, 1024);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_ss_if(leader, tmem_base + 256 + s * 128, hd + uint64_t(2 * j), wd + uint64_t(2 * j), idesc, (hb | j) ? 1u : 0u);
-          umma_commit_if(leader, hb == NBK - 1 ? &d2_full[s] : &h_empty[s]);  // after the last block D2's reader reuses h
+          for (int j = 0; j < 4; ++j)  // 16 hidden units = 8 columns of h
+            umma_ts_if(leader, tmem_base + 256 + s * 128, tmem_base + s * 128 + j * 8, wd + uint64_t(2 * j), idesc, (hb | j) ? 1u : 0u);
+          if (!more) umma_commit_if(leader, &d2_full[s]);
+          else {
+            d1(s);
+            if (hb + 2 == NBK) umma_commit_if(leader, &n_empty[s]);
+          }
         }
         umma_commit_if(leader, &w2_empty[b]);
         ++g2;
+        if (more) {
+          umma_commit_if(leader, &w1_empty[g1 & 1u]);
+          ++g1;
+        }
       }
-      if (okay && it + 1 < mine) okay = d1(0, it + 1);
     }
   } else if (warp < 10) {
     pdl_wait();
@@ -221,7 +227,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const int s = (warp - 10) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t rsw = uint32_t(row & 7), laddr = tmem_base + s * 128 + (uint32_t(quarter * 32) << 16);
     uint8_t* sh = smem + TR_OFF_H + s * TR_H + row * 128;
-    uint32_t g = 0, gh = 0;  // blocks; h buffers handed to D2 with a notice (all but an item's last)
+    uint32_t g = 0;  // blocks
     int t = blockIdx.x;
     for (int it = 0; it < mine && s < NT; ++it, t += gridDim.x) {
       for (int hb = 0; hb < NBK; ++hb, ++g) {
@@ -233,30 +239,20 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
           tmem_ld32(laddr + c2 * 32, ra);
           tmem_ld32(laddr + 64 + c2 * 32, rb);
           tmem_ld_wait();
-          if (c2 == 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&d1_empty[s]);
-          }
           uint32_t o[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const float a0 = __uint_as_float(ra[2 * e]), a1 = __uint_as_float(ra[2 * e + 1]);
             o[e] = pack_bf16x2(a0 * sigmoidf_fast(a0) * __uint_as_float(rb[2 * e]), a1 * sigmoidf_fast(a1) * __uint_as_float(rb[2 * e + 1]));
           }
-          if (c2 == 0 && hb > 0) {
-            mbar_wait(&h_empty[s], gh & 1u, ab, XF_ERR_WAIT_EMPTY);
-            ++gh;
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(sh + ((uint32_t(c2 * 4 + c) ^ rsw) << 4)) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+          tmem_st16(laddr + c2 * 16, o);  // over columns that have been read
         }
-        fence_proxy_async_smem();
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&h_full[s]);
       }
-      // the tile's result: D2 + x, through the h buffer, 64 columns at a time
+      // the tile's result: D2 + x, through the staging tile, 64 columns at a time
       const long long tile_row = (long long)(t * NT + s) * 128;
       const bool valid = tile_row + row < p.rows && !p.update_only;
       const uint4* xg = reinterpret_cast<const uint4*>(p.x + (tile_row + row) * 128);
@@ -302,7 +298,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
         }
       }
       if (quarter == 0 && lane == 0) tma_store_wait_read<0>();
-      named_bar_sync(1 + s, 128);  // h is free for the next item
+      named_bar_sync(1 + s, 128);  // the staging tile is free for the next item
     }
     if (quarter == 0 && lane == 0) tma_store_wait_all();
   }
