@@ -31,10 +31,11 @@
 //   warps 4 ..     : one softmax warpgroup per slot, one thread per query row.
 // Tensor memory per slot: 128 columns of logits / probabilities, D columns of output.
 //
-// The reference exponent m_ref follows the running maximum lazily.  A sweep over 32 keys runs against the m_ref of the keys
-// before and looks at its partial sums afterwards; if one exceeds 2^12 in some row of the warp (fp16 P overflows at 2^16)
-// the warp takes the exact path: maximum of the 32 logits still in registers, O, the row sum and the block's stored P
-// rescaled where it grew by more than 2^8, the sweep repeated.  The first sweep of an item always takes it.
+// The reference exponent m_ref follows the running maximum lazily.  A block's sweep over 64 keys runs against the m_ref of the
+// blocks before and looks at its partial sums afterwards; if one exceeds 2^12 in some row of the warp (fp16 P overflows at
+// 2^16) the warp takes the exact path: maximum of the logits, which are still in registers, O and the row sum rescaled where it
+// grew by more than 2^8, the sweep repeated.  The first block of an item starts with its maximum.  The exact path stands beside
+// the sweep, not in a loop around it (a loop around each half, with a vote after each: 1.05 of the time at 1024 tokens).
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -104,9 +105,10 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   return make_float2(q.x * __uint_as_float(__float_as_uint(t.x) * 0x800000u + 0x3F800000u),
                      q.y * __uint_as_float(__float_as_uint(t.y) * 0x800000u + 0x3F800000u));
 }
-// Which of a sweep's 16 pairs take the polynomial: two.  (TriangleAttention, 1024 tokens: none 1.33 ms, two or three 1.27,
-// four or five 1.32, six 1.44 -- the FMA pipe and the issue slots are then the longer queue.)
-__host__ __device__ constexpr bool poly_pair(int e) { return (e & 7) == 7; }
+// Which of a sweep's 16 pairs take the polynomial: two, away from its ends.  (TriangleAttention, 1024 tokens: none 1.02 of the
+// time, three 1.00 to 1.02, four more; at the ends of the sweep's halves 1.01 -- with more, the FMA pipe and the issue slots
+// are the longer queue.)
+__host__ __device__ constexpr bool poly_pair(int e) { return e % 6 == 4; }
 // K-major or MN-major tile with rows of 64 bytes (D = 32) or 128 bytes (D = 64), swizzled over 8 rows
 template <int D>
 __device__ __forceinline__ uint64_t make_sdesc_d(uint32_t saddr) {
@@ -334,78 +336,70 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
         okay = __all_sync(FULL, mbar_wait(&s_full[2 * s + (g & 1u)], (g >> 1) & 1u, ab, XF_ERR_WAIT_ATTN));
         if (!okay) break;
         tc_fence_after();
-        const int chunks = p.S - kb * 64 > 32 ? 2 : 1;
+        const bool both = p.S - kb * 64 > 32;  // the block's second 32 keys exist
         uint32_t r[2][32];
         tmem_ld32(buf, r[0]);
-        if (chunks > 1) tmem_ld32(buf + 32, r[1]);
+        if (both) tmem_ld32(buf + 32, r[1]);
         tmem_ld_wait();
+        float2 s2 = make_float2(0.f, 0.f);
+        // 32 keys against m_ref: P over logits that have been read, and their sums
+        auto sweep = [&](const uint32_t(&x)[32], uint32_t at) {
+          const float2 nm = make_float2(-m_ref, -m_ref);
+          uint32_t pk[16];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          if (c < chunks) {
-            const uint32_t(&x)[32] = r[c];
-            bool exact = kb == 0 && c == 0;
-            uint32_t pk[16];
-            float2 s2;
-            for (;;) {
-              if (exact) {
-                float mx = __uint_as_float(x[0]);
-#pragma unroll
-                for (int e = 1; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(x[e]));
-                const bool grow = mx > m_ref + 8.f;
-                if (__any_sync(FULL, grow)) {
-                  const float m_new = grow ? mx : m_ref;
-                  const float alpha = ex2f_(m_ref - m_new);
-                  m_ref = m_new;
-                  l2.x *= alpha;
-                  l2.y *= alpha;
-                  if (kb > 0) {  // every earlier P V product of the item must have landed before O is rescaled
-                    okay = __all_sync(FULL, mbar_wait(&pv_done[2 * s + ((g - 1) & 1u)], ((g - 1) >> 1) & 1u, ab, XF_ERR_WAIT_ATTN));
-                    if (!okay) break;
-                    tc_fence_after();
-                    uint32_t o[16];
-#pragma unroll 1
-                    for (int oc = 0; oc < D; oc += 16) {
-                      tmem_ld16(o_addr + oc, o);
-                      tmem_ld_wait();
-#pragma unroll
-                      for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-                      tmem_st16(o_addr + oc, o);
-                    }
-                  }
-                  if (c > 0) {  // so is the first half of the block's P
-                    const __half2 a2 = __float2half2_rn(alpha);
-                    uint32_t q[16];
-                    tmem_st_wait();
-                    tmem_ld16(buf, q);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                      const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&q[e]), a2);
-                      q[e] = *reinterpret_cast<const uint32_t*>(&v);
-                    }
-                    tmem_st16(buf, q);
-                  }
-                }
-              }
-              const float2 nm = make_float2(-m_ref, -m_ref);
-              s2 = make_float2(0.f, 0.f);
-#pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const float2 y = fadd2(make_float2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), nm);
-                const float2 pe = poly_pair(e) ? ex2_poly2(y) : make_float2(ex2f_(y.x), ex2f_(y.y));
-                s2 = fadd2(s2, pe);
-                const __half2 ph = __floats2half2_rn(pe.x, pe.y);
-                pk[e] = *reinterpret_cast<const uint32_t*>(&ph);
-              }
-              if (exact || !__any_sync(FULL, fmaxf(s2.x, s2.y) > 4096.f)) break;
-              exact = true;  // some row may have outgrown the reference: exact maximum, rescale if so, sweep again
-            }
-            if (!okay) break;
-            l2 = fadd2(l2, s2);
-            tmem_st16(buf + c * 16, pk);  // over logits that have been read
+          for (int e = 0; e < 16; ++e) {
+            const float2 y = fadd2(make_float2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), nm);
+            const float2 pe = poly_pair(e) ? ex2_poly2(y) : make_float2(ex2f_(y.x), ex2f_(y.y));
+            s2 = fadd2(s2, pe);
+            const __half2 ph = __floats2half2_rn(pe.x, pe.y);
+            pk[e] = *reinterpret_cast<const uint32_t*>(&ph);
           }
+          tmem_st16(at, pk);
+        };
+        // the reference exponent follows the block's maximum where that is more than 8 above it
+        auto follow = [&]() {
+          float mx = __uint_as_float(r[0][0]);
+#pragma unroll
+          for (int e = 1; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[0][e]));
+          if (both) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(r[1][e]));
+          }
+          const bool grow = mx > m_ref + 8.f;
+          const float m_new = grow ? mx : m_ref;
+          const float alpha = ex2f_(m_ref - m_new);
+          m_ref = m_new;
+          l2.x *= alpha;
+          l2.y *= alpha;
+          return alpha;
+        };
+        if (kb == 0) follow();
+        sweep(r[0], buf);
+        if (both) sweep(r[1], buf + 16);
+        if (kb > 0 && __any_sync(FULL, fmaxf(s2.x, s2.y) > 4096.f)) {
+          // some row may have outgrown the reference: exact maximum, rescale, sweep again
+          const float alpha = follow();
+          if (__any_sync(FULL, alpha != 1.f)) {
+            // every earlier P V product of the item must have landed before O is rescaled
+            okay = __all_sync(FULL, mbar_wait(&pv_done[2 * s + ((g - 1) & 1u)], ((g - 1) >> 1) & 1u, ab, XF_ERR_WAIT_ATTN));
+            if (!okay) break;
+            tc_fence_after();
+            uint32_t o[16];
+#pragma unroll 1
+            for (int oc = 0; oc < D; oc += 16) {
+              tmem_ld16(o_addr + oc, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              tmem_st16(o_addr + oc, o);
+            }
+          }
+          s2 = make_float2(0.f, 0.f);
+          tmem_st_wait();
+          sweep(r[0], buf);
+          if (both) sweep(r[1], buf + 16);
         }
-        if (!okay) break;
+        l2 = fadd2(l2, s2);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
