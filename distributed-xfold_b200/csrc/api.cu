@@ -305,8 +305,9 @@ static TriMulWs carve_trimul(void* ws, size_t cap, int N) {
   return w;
 }
 
+// readers: an event that stands for who still reads z as it is (or null)
 static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, const xfold_trimul_weights* w, void* ws,
-                      size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr) {
+                      size_t ws_bytes, cudaStream_t st, bf16* upd = nullptr, cudaEvent_t readers = nullptr) {
   if (!z || !w || !w->w_in || !w->w_out) return fail(c, XFOLD_ERR_ARG, "trimul: null argument");
   if (N <= 0) return XFOLD_OK;
   TriMulWs W = carve_trimul(ws, ws_bytes, N);
@@ -319,6 +320,7 @@ static int trimul_fwd(Ctx* c, bf16* z, const float* mask, int N, int outgoing, c
   StaticWeights sw(c);
   rc = trimul_contract(c, outgoing ? W.a : W.b, cs, rs, outgoing ? W.b : W.a, cs, rs, N, N, N, W.o, cs, rs, st);
   if (rc) return rc;
+  if (readers && cudaStreamWaitEvent(st, readers, 0) != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "trimul: event wait");
   return trimul_output(c, W.o, cs, rs, nullptr, N, N, w, z, st, upd);
 }
 
@@ -576,9 +578,10 @@ static PairformerWs carve_pairformer(void* ws, size_t cap, int N) {
 }
 
 // The blocks in order.  The masks' bias tiles are made once.  The single representation follows the pair representation
-// and nothing of the pair path reads it, so its seven small kernels of a block run on the context's second stream beside
-// the next block's pair path (a block of 40 tokens: 155 us, 45 of them single path; 1024 tokens: 0.14 of 6.8 ms).  The
-// pair logits are the only buffer between the two; the next block's logits wait for the single path of this one.
+// and nothing of the pair path reads it, so its eight small kernels of a block, the pair logits first, run on the context's
+// second stream beside the next block's pair path (a block of 37 tokens: 135 us, 37 of them single path; with the logits on
+// the first stream four blocks took 405 us instead of 397).  They read z, which the next block writes for the first time in
+// its third kernel: that one waits for the logits.
 static int pairformer_fwd(Ctx* c, bf16* z, bf16* s, const float* pair_mask, const float* seq_mask, int N,
                           const xfold_pairformer_weights* blocks, int num_blocks, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (!z || (num_blocks > 0 && !blocks)) return fail(c, XFOLD_ERR_ARG, "pairformer: null argument");
@@ -597,21 +600,25 @@ static int pairformer_fwd(Ctx* c, bf16* z, bf16* s, const float* pair_mask, cons
     if (s && (rc = launch_mext(c, seq_mask, 0, W.mext_seq, 1, N, st))) return rc;
     for (int i = 0; i < num_blocks; ++i) {
       const xfold_pairformer_weights* w = &blocks[i];
-      if ((rc = trimul_fwd(c, z, pair_mask, N, 1, &w->tri_out, W.pair, W.pair_bytes, st))) return rc;
+      if ((rc = trimul_fwd(c, z, pair_mask, N, 1, &w->tri_out, W.pair, W.pair_bytes, st, nullptr, behind ? c->ev_pl : nullptr))) return rc;
       if ((rc = trimul_fwd(c, z, pair_mask, N, 0, &w->tri_in, W.pair, W.pair_bytes, st))) return rc;
       if ((rc = triattn_fwd(c, z, pair_mask, N, 0, &w->att_start, W.pair, W.pair_bytes, st, nullptr, W.mext))) return rc;
       if ((rc = triattn_fwd(c, z, pair_mask, N, 1, &w->att_end, W.pair, W.pair_bytes, st, nullptr, W.mext))) return rc;
       if ((rc = transition_fwd(c, z, (long long)N * N, 128, 512, &w->pair_transition, W.pair, W.pair_bytes, st))) return rc;
       if (!s || !w->spl_w) continue;
-      if (behind && cudaStreamWaitEvent(st, c->ev_join, 0) != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pairformer: event wait");
-      behind = false;
-      if ((rc = launch_ln_rows(c, z, 128, nullptr, 128, (long long)N * N, 128, w->spl_ln_gamma, w->spl_ln_beta, 1e-5f, 16, w->spl_w,
-                               nullptr, (long long)N * W.ldq, nullptr, nullptr, 0, st, W.pl, -N, 0, W.ldq))) return rc;
       const bool here = !side || i + 1 == num_blocks;
-      if (!here && (cudaEventRecord(c->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(c->side, c->ev_fork, 0) != cudaSuccess))
+      const cudaStream_t ss = here ? st : c->side;
+      if (here) {
+        if (behind && cudaStreamWaitEvent(st, c->ev_join, 0) != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pairformer: event wait");
+        behind = false;
+      } else if (cudaEventRecord(c->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(c->side, c->ev_fork, 0) != cudaSuccess) {
         return fail(c, XFOLD_ERR_LAUNCH, "pairformer: event record");
-      behind = !here;
-      if ((rc = single_update(c, s, W.pl, W.ldq, seq_mask, N, w, W.single, W.single_bytes, here ? st : c->side, W.mext_seq))) return rc;
+      }
+      behind = behind || !here;
+      if ((rc = launch_ln_rows(c, z, 128, nullptr, 128, (long long)N * N, 128, w->spl_ln_gamma, w->spl_ln_beta, 1e-5f, 16, w->spl_w,
+                               nullptr, (long long)N * W.ldq, nullptr, nullptr, 0, ss, W.pl, -N, 0, W.ldq))) return rc;
+      if (!here && cudaEventRecord(c->ev_pl, c->side) != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pairformer: event record");
+      if ((rc = single_update(c, s, W.pl, W.ldq, seq_mask, N, w, W.single, W.single_bytes, ss, W.mext_seq))) return rc;
       if (!here && cudaEventRecord(c->ev_join, c->side) != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pairformer: event record");
     }
     return XFOLD_OK;
@@ -651,7 +658,8 @@ int xfold_ctx_create(int device, xfold_ctx** out) {
   cudaMemset(c->d_status, 0, sizeof(int));
   if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_pl, cudaEventDisableTiming) != cudaSuccess) {
     xfold_ctx_destroy(c);
     return XFOLD_ERR_DEVICE;
   }
@@ -665,6 +673,7 @@ void xfold_ctx_destroy(xfold_ctx* c) {
   if (c->side) cudaStreamDestroy(c->side);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->ev_pl) cudaEventDestroy(c->ev_pl);
   for (auto& r : c->prof_recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   for (auto& r : c->prof_pool) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   delete c;

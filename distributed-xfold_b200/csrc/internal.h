@@ -44,7 +44,7 @@ struct Ctx {
   // Second stream of the one-GPU trunk: the single representation's kernels of a block run beside the next block's.  (Events
   // are captured by the waits as they are issued: the next call may use them again.)
   cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_pl = nullptr;
 };
 
 struct CallLock {
