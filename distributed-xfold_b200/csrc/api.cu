@@ -511,14 +511,13 @@ static int grid_attention_fwd(Ctx* c, const bf16* x, int B, int S, int C, int H,
   // padded rows of the attention's output: zero rows project to zero rows
   if (SP > S && cudaMemset2DAsync(W.att + (size_t)S * Wd, (size_t)SP * Wd * 2, 0, (size_t)(SP - S) * Wd * 2, B, st) != cudaSuccess)
     return fail(c, XFOLD_ERR_LAUNCH, "grid attention: memset");
+  if ((rc = launch_attn_prepare(c, pair_bias, W.biasT, H, S, ldq, mask_bias, mask_ld, W.mext, mrows, 1, st))) return rc;
+  StaticWeights sw(c);
   if (C == 128 && Wd == 128)
     rc = launch_row_project_attn(c, x, B, S, 0, nullptr, nullptr, w_qkvg, scale, nullptr, W.qkvg, nullptr, 0, 0, st);
   else
     rc = linear_plain(c, x, C, (long long)B * S, C, w_qkvg, 4 * Wd, nullptr, scale, W.qkvg, 4 * Wd, st, 2 * Wd, 3 * Wd, Wd);
   if (rc) return rc;
-  StaticWeights sw(c);
-  if ((rc = launch_bias_transpose(c, pair_bias, W.biasT, H, S, ldq, st))) return rc;
-  if ((rc = launch_mext(c, mask_bias, mask_ld, W.mext, mrows, S, st, 1))) return rc;
   if ((rc = launch_attention2(c, W.qkvg, 4 * Wd, S, B, 0, 0, Wd, 2 * Wd, 3 * Wd, H, W.biasT, ldq, W.mext, mrows, W.att, Wd,
                               (long long)SP * Wd, st, 32))) return rc;
   if (Wd == 128 && C_out == 128) return launch_row_output(c, W.att, (long long)B * SP, w_out, nullptr, out, st);

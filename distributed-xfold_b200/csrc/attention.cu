@@ -468,11 +468,10 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
 // spacing is 64).
 // additive: the bias itself.  Times log2(e) like the logits it is added to, in three columns (float32's 24 bits), kept within
 // +-60000 like the pair bias.
-__global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restrict__ out, int B, int S, int KS, int additive) {
-  pdl_wait();
-  pdl_launch();
+__device__ __forceinline__ void mext_tiles(const float* mask, long long mask_ld, uint4* out, int B, int S, int KS, int additive,
+                                           long long first, long long step) {
   const long long n = (long long)B * KS * 64;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
+  for (long long idx = first; idx < n; idx += step) {
     const long long bb = idx / (KS * 64);
     const int k = int(idx - bb * (KS * 64));
     float v = -1.0e30f;
@@ -490,6 +489,11 @@ __global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restr
     out[idx] = make_uint4(p[0] | p[1] << 16, p[2], 0, 0);
   }
 }
+__global__ void mext_kernel(const float* mask, long long mask_ld, uint4* __restrict__ out, int B, int S, int KS, int additive) {
+  pdl_wait();
+  pdl_launch();
+  mext_tiles(mask, mask_ld, out, B, S, KS, additive, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
 
 int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st, int additive) {
   const int KS = (S + 63) / 64;
@@ -504,15 +508,30 @@ int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, 
 
 // fp32 [H][S][S] -> 16-bit [H][S][ldq] (same query-major order, padded row pitch): FP16 values times log2(e), the operand
 // the kernel's pair-bias tensor map expects (the kernel works in base 2 and adds the tile as it is).
-__global__ void bias_convert_kernel(const float* in, __half* __restrict__ out, long long rows, int S, int ldq) {
-  pdl_wait();
-  pdl_launch();
+__device__ __forceinline__ void bias_convert(const float* in, __half* out, long long rows, int S, int ldq, long long first, long long step) {
   const long long n = rows * ldq;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
+  for (long long idx = first; idx < n; idx += step) {
     const long long r = idx / ldq;
     const int k = int(idx % ldq);
     out[idx] = __float2half_rn(k < S ? fminf(fmaxf(in[r * S + k] * 1.4426950408889634f, -60000.f), 60000.f) : 0.f);
   }
+}
+
+__global__ void bias_convert_kernel(const float* in, __half* __restrict__ out, long long rows, int S, int ldq) {
+  pdl_wait();
+  pdl_launch();
+  bias_convert(in, out, rows, S, ldq, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+// Both operands of a call in one launch: the first `split` blocks convert the bias, the others make the mask tiles.
+__global__ void attn_prepare_kernel(const float* bias, __half* __restrict__ bias_out, long long rows, int S, int ldq, int split,
+                                    const float* mask, long long mask_ld, uint4* __restrict__ mask_out, int B, int KS, int additive) {
+  pdl_wait();
+  pdl_launch();
+  if (int(blockIdx.x) < split)
+    bias_convert(bias, bias_out, rows, S, ldq, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)split * blockDim.x);
+  else
+    mext_tiles(mask, mask_ld, mask_out, B, S, KS, additive, (long long)(blockIdx.x - split) * blockDim.x + threadIdx.x,
+               (long long)(gridDim.x - split) * blockDim.x);
 }
 
 int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int ldq, cudaStream_t st) {
@@ -523,6 +542,18 @@ int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int 
   ProfScope ps(c, XFOLD_K_MASK_BIAS, st);
   launch_pdl(bias_convert_kernel, (int)blocks, 256, 0, st, in, reinterpret_cast<__half*>(out), rows, S, ldq);
   return check_launch(c, "bias_convert_kernel");
+}
+
+int launch_attn_prepare(Ctx* c, const float* bias, bf16* bias_out, int H, int S, int ldq, const float* mask, long long mask_ld,
+                        bf16* mask_out, int B, int additive, cudaStream_t st) {
+  if (H <= 0 || S <= 0 || B <= 0) return XFOLD_OK;
+  const int KS = (S + 63) / 64;
+  const long long rows = (long long)H * S, b1 = (rows * ldq + 255) / 256, b2 = ((long long)B * KS * 64 + 255) / 256;
+  const int split = (int)(b1 > 16384 ? 16384 : b1), rest = (int)(b2 > 8192 ? 8192 : b2);
+  ProfScope ps(c, XFOLD_K_MASK_BIAS, st);
+  launch_pdl(attn_prepare_kernel, split + rest, 256, 0, st, bias, reinterpret_cast<__half*>(bias_out), rows, S, ldq, split, mask, mask_ld,
+             reinterpret_cast<uint4*>(mask_out), B, KS, additive);
+  return check_launch(c, "attn_prepare_kernel");
 }
 
 template <int D, bool ROWS>

@@ -42,6 +42,9 @@ int launch_ln_rows(Ctx* c, const bf16* x, long long ldx, bf16* y, long long ldy,
                    int trav_outer = 0, int proj_pitch = 0);
 int launch_mext(Ctx* c, const float* mask, long long mask_ld, bf16* out, int B, int S, cudaStream_t st, int additive = 0);
 int launch_bias_transpose(Ctx* c, const float* in, bf16* out, int H, int S, int ldq, cudaStream_t st);
+// both of the above in one launch
+int launch_attn_prepare(Ctx* c, const float* bias, bf16* bias_out, int H, int S, int ldq, const float* mask, long long mask_ld,
+                        bf16* mask_out, int B, int additive, cudaStream_t st);
 int launch_attention2(Ctx* c, const bf16* qkvg, int width, int S, int B, int transposed, int q_col0, int k_col0,
                       int v_col0, int g_col0, int heads, const bf16* biasT, int ldq, const bf16* mext, int mext_rows,
                       bf16* out, long long out_seq_stride, long long out_batch_stride, cudaStream_t st, int head_dim = 32);
