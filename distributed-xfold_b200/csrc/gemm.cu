@@ -278,9 +278,11 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tmem_ld32(taddr + BN / 2 + c * 64 + ch * 32, rb);
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const float x = __uint_as_float(ra[e]);
-            v[e] = x * sigmoidf_fast(x) * __uint_as_float(rb[e]);
+          for (int e = 0; e < 32; e += 2) {
+            const float2 x = make_float2(__uint_as_float(ra[e]), __uint_as_float(ra[e + 1]));
+            const float2 h = fmul2(fmul2(x, sigmoid2(x)), make_float2(__uint_as_float(rb[e]), __uint_as_float(rb[e + 1])));
+            v[e] = h.x;
+            v[e + 1] = h.y;
           }
         } else {
           uint32_t r[32];

@@ -329,20 +329,17 @@ row_output_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int n = half * 64 + c * W + q * 8 + 2 * e;
-            float v0 = __uint_as_float(r[q * 8 + 2 * e]), v1 = __uint_as_float(r[q * 8 + 2 * e + 1]);
+            float2 v = make_float2(__uint_as_float(r[q * 8 + 2 * e]), __uint_as_float(r[q * 8 + 2 * e + 1]));
             if constexpr (CM) {
-              float g0 = bf16_lo(gw[e]), g1 = bf16_hi(gw[e]);
-              if constexpr (GZ) {
-                // (rounded as where it passes through memory, so that the stages by rows give the same bits)
-                const uint32_t g2 = pack_bf16x2(__uint_as_float(rg[q * 8 + 2 * e]), __uint_as_float(rg[q * 8 + 2 * e + 1]));
-                g0 = bf16_lo(g2);
-                g1 = bf16_hi(g2);
-              }
+              uint32_t g2 = gw[e];
+              // (rounded as where it passes through memory, so that the stages by rows give the same bits)
+              if constexpr (GZ) g2 = pack_bf16x2(__uint_as_float(rg[q * 8 + 2 * e]), __uint_as_float(rg[q * 8 + 2 * e + 1]));
               const float4 k = *reinterpret_cast<const float4*>(&cs[n]);
-              v0 = fmaf(rstd, fmaf(nmean, k.x, v0), k.y) * sigmoidf_fast(g0);
-              v1 = fmaf(rstd, fmaf(nmean, k.z, v1), k.w) * sigmoidf_fast(g1);
+              v = ffma2(make_float2(rstd, rstd), ffma2(make_float2(nmean, nmean), make_float2(k.x, k.z), v), make_float2(k.y, k.w));
+              v = fmul2(v, sigmoid2(make_float2(bf16_lo(g2), bf16_hi(g2))));
             }
-            o[e] = pack_bf16x2(v0 + bf16_lo(zw[e]), v1 + bf16_hi(zw[e]));
+            v = fadd2(v, make_float2(bf16_lo(zw[e]), bf16_hi(zw[e])));
+            o[e] = pack_bf16x2(v.x, v.y);
           }
           *reinterpret_cast<uint4*>(sz + at) = make_uint4(o[0], o[1], o[2], o[3]);
         }

@@ -374,8 +374,13 @@ row_project_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
           }
           if (valid) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              *dst = __float2bfloat16(__uint_as_float(rp[e]) * mk * sigmoidf_fast(__uint_as_float(rg[e])));
+            for (int e = 0; e < 16; e += 2) {
+              const float2 v = fmul2(make_float2(__uint_as_float(rp[e]), __uint_as_float(rp[e + 1])), make_float2(mk, mk));
+              const float2 s = fmul2(v, sigmoid2(make_float2(__uint_as_float(rg[e]), __uint_as_float(rg[e + 1]))));
+              const uint32_t o = pack_bf16x2(s.x, s.y);
+              *dst = __ushort_as_bfloat16((unsigned short)o);
+              dst += p.chan_stride;
+              *dst = __ushort_as_bfloat16((unsigned short)(o >> 16));
               dst += p.chan_stride;
             }
           }

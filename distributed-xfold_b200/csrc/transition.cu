@@ -242,8 +242,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
           uint32_t o[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const float a0 = __uint_as_float(ra[2 * e]), a1 = __uint_as_float(ra[2 * e + 1]);
-            o[e] = pack_bf16x2(a0 * sigmoidf_fast(a0) * __uint_as_float(rb[2 * e]), a1 * sigmoidf_fast(a1) * __uint_as_float(rb[2 * e + 1]));
+            const float2 a = make_float2(__uint_as_float(ra[2 * e]), __uint_as_float(ra[2 * e + 1]));
+            const float2 h = fmul2(fmul2(a, sigmoid2(a)), make_float2(__uint_as_float(rb[2 * e]), __uint_as_float(rb[2 * e + 1])));
+            o[e] = pack_bf16x2(h.x, h.y);
           }
           tmem_st16(laddr + c2 * 16, o);  // over columns that have been read
         }

@@ -401,6 +401,17 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
       "mov.b64 {%0, %1}, rd;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmul.rn.f32x2 rd, ra, rb;\n\t"
+      "mov.b64 {%0, %1}, rd;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 sigmoid2(float2 x) {  // sigmoidf_fast of a pair
+  float2 t = fmul2(x, make_float2(0.5f, 0.5f));
+  asm("tanh.approx.f32 %0, %0;\n\ttanh.approx.f32 %1, %1;" : "+f"(t.x), "+f"(t.y));
+  return ffma2(make_float2(0.5f, 0.5f), t, make_float2(0.5f, 0.5f));
+}
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 
