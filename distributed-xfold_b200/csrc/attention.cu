@@ -437,9 +437,9 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
             uint32_t ow[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float o0 = __uint_as_float(o[g8 * 8 + 2 * e]) * inv * sigmoidf_fast(bf16_lo(gw[e]));
-              const float o1 = __uint_as_float(o[g8 * 8 + 2 * e + 1]) * inv * sigmoidf_fast(bf16_hi(gw[e]));
-              ow[e] = pack_bf16x2(o0, o1);
+              const float2 y = fmul2(fmul2(make_float2(__uint_as_float(o[g8 * 8 + 2 * e]), __uint_as_float(o[g8 * 8 + 2 * e + 1])),
+                                           make_float2(inv, inv)), sigmoid2(make_float2(bf16_lo(gw[e]), bf16_hi(gw[e]))));
+              ow[e] = pack_bf16x2(y.x, y.y);
             }
             *reinterpret_cast<uint4*>(orow + oc + g8 * 8) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
           }

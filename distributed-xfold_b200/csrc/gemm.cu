@@ -315,8 +315,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                v[g * 8 + 2 * e] *= sigmoidf_fast(bf16_lo(w4[e]));
-                v[g * 8 + 2 * e + 1] *= sigmoidf_fast(bf16_hi(w4[e]));
+                const float2 x = fmul2(make_float2(v[g * 8 + 2 * e], v[g * 8 + 2 * e + 1]), sigmoid2(make_float2(bf16_lo(w4[e]), bf16_hi(w4[e]))));
+                v[g * 8 + 2 * e] = x.x;
+                v[g * 8 + 2 * e + 1] = x.y;
               }
             }
             if (row_gate_vec && c + 1 < nch) fetch_row_gate(c + 1);
@@ -329,8 +330,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                v[g * 8 + 2 * e] += bf16_lo(w4[e]);
-                v[g * 8 + 2 * e + 1] += bf16_hi(w4[e]);
+                const float2 x = fadd2(make_float2(v[g * 8 + 2 * e], v[g * 8 + 2 * e + 1]), make_float2(bf16_lo(w4[e]), bf16_hi(w4[e])));
+                v[g * 8 + 2 * e] = x.x;
+                v[g * 8 + 2 * e + 1] = x.y;
               }
             }
           }
@@ -354,10 +356,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const float4 fb = reinterpret_cast<const float4*>(sv)[e], fs = reinterpret_cast<const float4*>(sv)[8 + e];
-            v[4 * e] = (v[4 * e] + fb.x) * fs.x;
-            v[4 * e + 1] = (v[4 * e + 1] + fb.y) * fs.y;
-            v[4 * e + 2] = (v[4 * e + 2] + fb.z) * fs.z;
-            v[4 * e + 3] = (v[4 * e + 3] + fb.w) * fs.w;
+            const float2 x = fmul2(fadd2(make_float2(v[4 * e], v[4 * e + 1]), make_float2(fb.x, fb.y)), make_float2(fs.x, fs.y));
+            const float2 y = fmul2(fadd2(make_float2(v[4 * e + 2], v[4 * e + 3]), make_float2(fb.z, fb.w)), make_float2(fs.z, fs.w));
+            v[4 * e] = x.x; v[4 * e + 1] = x.y; v[4 * e + 2] = y.x; v[4 * e + 3] = y.y;
           }
           __syncwarp();
         }
