@@ -17,7 +17,9 @@
 //   warps 10 - 17  : one set of four per tile: D1 -> h; finally D2 + x -> a staging tile in two halves, which leave by TMA
 // The operands' trips from shared memory bound it (128 bytes per clock): with h in tensor memory they are 21 % fewer.  (h in
 // shared memory, D1 a block ahead of it: 0.54 ms in the trunk of 1024 tokens, now 0.50.  Sixteen warps for D1 -> h: no gain.)
-// With no more tiles than SMs a CTA takes one tile (B is left out).
+// With no more tiles than SMs a CTA takes one tile: its blocks go through the two accumulators in turn, each with its set of
+// warps, D1 two blocks ahead of D2, and a set takes one half of the result.  (One accumulator and one set: four
+// blocks of the trunk at 37 tokens 392 us instead of 379, at 100 tokens 485 instead of 471.)
 #include "internal.h"
 #include "stages.h"
 #include "umma.cuh"
@@ -155,10 +157,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc = make_idesc(128, 128);
     uint32_t g1 = 0, g2 = 0;  // blocks whose D1 / D2 have been issued
-    // D1 of the block after g1's for tile s (the products that read the h it goes over were issued before: in order)
-    auto d1 = [&](int s) {
+    // D1 of the next block, of tile `tile` into accumulator s (the products that read the h it goes over were issued before: in
+    // order)
+    auto d1 = [&](int s, int tile) {
       const uint64_t wd = make_sdesc(base + TR_OFF_W1 + (g1 & 1u) * TR_W1, 16, 1024);
-      const uint64_t nd = make_sdesc(base + TR_OFF_N + s * TR_TILE, 16, 1024);
+      const uint64_t nd = make_sdesc(base + TR_OFF_N + tile * TR_TILE, 16, 1024);
 #pragma unroll
       for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
@@ -169,13 +172,40 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     };
     auto w1_ready = [&]() { return mbar_wait_warp(&w1_full[g1 & 1u], (g1 >> 1) & 1u, ab, XF_ERR_WAIT_FULL); };
     bool okay = true;
-    for (int it = 0; it < mine && okay; ++it) {
+    if (!p.pair && mine > 0) {
+      // one tile: its blocks take the two accumulators in turn, D1 two blocks ahead of D2
+      okay = mbar_wait_warp(&n_full[0], 0, ab, XF_ERR_WAIT_FULL);
+      for (int hb = 0; hb < NBK + 2 && okay; ++hb) {
+        const int s = hb & 1;
+        if (hb >= 2) {
+          const uint32_t b = g2 & 1u;
+          if (!mbar_wait_warp(&w2_full[b], (g2 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) break;
+          if (!mbar_wait_warp(&h_full[s], (g2 >> 1) & 1u, ab, XF_ERR_WAIT_FULL)) break;
+          tc_fence_after();
+          const uint64_t wd = make_sdesc(base + TR_OFF_W2 + b * TR_W2, 16, 1024);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_ts_if(leader, tmem_base + 256, tmem_base + s * 128 + j * 8, wd + uint64_t(2 * j), idesc, (g2 | uint32_t(j)) ? 1u : 0u);
+          umma_commit_if(leader, &w2_empty[b]);
+          ++g2;
+        }
+        if (hb < NBK) {
+          if (!w1_ready()) break;
+          tc_fence_after();
+          d1(s, 0);
+          umma_commit_if(leader, &w1_empty[g1 & 1u]);
+          ++g1;
+        }
+      }
+      umma_commit_if(leader, &d2_full[0]);
+    }
+    for (int it = 0; it < (p.pair ? mine : 0) && okay; ++it) {
       if (!w1_ready()) break;
       for (int s = 0; s < NT && okay; ++s) {
         okay = mbar_wait_warp(&n_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_FULL);
         if (!okay) break;
         tc_fence_after();
-        d1(s);
+        d1(s, s);
         if (NBK == 1) umma_commit_if(leader, &n_empty[s]);
       }
       if (!okay) break;
@@ -196,7 +226,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
             umma_ts_if(leader, tmem_base + 256 + s * 128, tmem_base + s * 128 + j * 8, wd + uint64_t(2 * j), idesc, (hb | j) ? 1u : 0u);
           if (!more) umma_commit_if(leader, &d2_full[s]);
           else {
-            d1(s);
+            d1(s, s);
             if (hb + 2 == NBK) umma_commit_if(leader, &n_empty[s]);
           }
         }
@@ -227,10 +257,13 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
     const int s = (warp - 10) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t rsw = uint32_t(row & 7), laddr = tmem_base + s * 128 + (uint32_t(quarter * 32) << 16);
     uint8_t* sh = smem + TR_OFF_H + s * TR_H + row * 128;
-    uint32_t g = 0;  // blocks
+    uint32_t g = 0;  // blocks of this set
     int t = blockIdx.x;
-    for (int it = 0; it < mine && s < NT; ++it, t += gridDim.x) {
-      for (int hb = 0; hb < NBK; ++hb, ++g) {
+    // one tile: a set takes every other block, and one half of the result
+    const int h0 = p.pair ? 0 : s, hstep = p.pair ? 1 : 2, tile = p.pair ? s : 0;
+    const uint32_t daddr = tmem_base + 256 + tile * 128 + (uint32_t(quarter * 32) << 16);
+    for (int it = 0; it < mine; ++it, t += gridDim.x) {
+      for (int hb = h0; hb < NBK; hb += hstep, ++g) {
         mbar_wait(&d1_full[s], g & 1u, ab, XF_ERR_WAIT_TMEM_FULL);  // (a failed wait runs through: these warps meet at a barrier)
         tc_fence_after();
 #pragma unroll
@@ -254,16 +287,16 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
         if (lane == 0) mbar_arrive(&h_full[s]);
       }
       // the tile's result: D2 + x, through the staging tile, 64 columns at a time
-      const long long tile_row = (long long)(t * NT + s) * 128;
+      const long long tile_row = (long long)(t * NT + tile) * 128;
       const bool valid = tile_row + row < p.rows && !p.update_only;
       const uint4* xg = reinterpret_cast<const uint4*>(p.x + (tile_row + row) * 128);
 #pragma unroll 1
-      for (int hf = 0; hf < 2; ++hf) {
+      for (int hf = h0; hf < 2; hf += hstep) {
         uint4 xv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) xv[q] = valid ? __ldcg(xg + hf * 8 + q) : make_uint4(0, 0, 0, 0);
-        if (hf == 0) {
-          mbar_wait(&d2_full[s], uint32_t(it) & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
+        if (hf == h0) {
+          mbar_wait(&d2_full[tile], uint32_t(it) & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
           tc_fence_after();
         } else {
           if (quarter == 0 && lane == 0) tma_store_wait_read<0>();
@@ -272,7 +305,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t r[32];
-          tmem_ld32(laddr + 256 + hf * 64 + c * 32, r);
+          tmem_ld32(daddr + hf * 64 + c * 32, r);
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 4; ++q) {

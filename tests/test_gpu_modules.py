@@ -465,3 +465,20 @@ def test_unaligned_output_weights_are_refused(ops, oracle, kind):
         (ops.triangle_multiplication_ if kind == "multiplication" else ops.triangle_attention_)(z, None, w, True)
     ops.synchronize_and_check()
     assert torch.equal(z, before)
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128, 148 * 128 + 1])
+def test_transition_one_tile_per_cta_has_the_bits_of_pairs(ops, oracle, rows):
+    """Up to a tile per SM the hidden blocks take two accumulators in turn, beyond that a CTA has two tiles: the same sums in the
+    same order.  The rows are the first of a call that is large enough for pairs."""
+    g = torch.Generator().manual_seed(rows)
+    st = oracle.make_transition_state(g, "", 128)
+    w = ops.PackedTransition(st, "", "cuda")
+    x = torch.randn(2 * 148 * 128 + 77, 128, generator=g).to(BF).cuda()
+    want = ops.transition_(x.clone(), w)[:rows]
+    got = ops.transition_(x[:rows].clone(), w)
+    ops.synchronize_and_check()
+    assert torch.equal(got, want)
+    x = x[:min(rows, 300)].float().cpu()
+    ref = x + oracle.transition(rounded(st), "", x)
+    assert relf(got[:len(ref)].float().cpu(), ref) < TOL_Z
