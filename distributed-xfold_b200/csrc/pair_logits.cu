@@ -24,6 +24,12 @@
 // first read come from L2.  Warp 0 fetches tiles (two in flight), warp 1 issues the products into two accumulators, and two
 // sets of eight warps take the tiles in turn: row statistics from the shared-memory tile while the product runs (two threads
 // per row), then 32 heads x 64 keys per warp, staged and stored by itself.
+//
+// FEW: up to 96 heads in all.  The tensor core has no narrower rows than 128, so that form makes, converts and stages 128
+// heads whatever their number; here keys are the rows and the product is as wide as the heads, stores are 4 bytes from traded
+// halves, and in place of the staging tiles a third tile of x is in flight.  The same operands and sums, the same bits.
+// N = 1000: 16 heads 54 us (heads as rows: 87), 64 heads 78 (93), 96 heads 98 (102), 112 heads 107 (106); N = 300: 96 heads
+// 18.5 (20.7), 112 heads 19.8 (21.2); N = 40: 16 heads 4.6 (8.9).
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -33,6 +39,7 @@
 namespace xf {
 
 constexpr int PL_G = 128;      // heads per CTA at most
+constexpr int PL_FEW = 96;     // up to so many heads in all: keys as the accumulator's rows (at 112 and 1000 tokens the other form is ahead)
 constexpr int PL_XS = 2;       // tiles of x in flight
 constexpr uint32_t PL_TILE = 32768;
 constexpr uint32_t PL_STG = 4096;                                // a warp's [32 heads][64 keys], swizzled
@@ -48,19 +55,22 @@ static_assert(PL_SMEM <= 232448, "shared memory");
 
 struct PairLogitsArgs {
   const float *gamma, *beta, *w;
+  __half* out;
   int N, H, tiles_k, groups;
   int* status;
 };
 
+template <bool FEW>
 __global__ void __launch_bounds__(PL_THREADS, 1)
 pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmo, const PairLogitsArgs p) {
   constexpr float LOG2E = 1.4426950408889634f;
+  constexpr int XS = FEW ? 3 : PL_XS;  // FEW: no staging, its third tile is there
   extern __shared__ __align__(1024) uint8_t smem[];  // (no room to round up)
   uint8_t* sW = smem + PL_OFF_W;
   float* cb = reinterpret_cast<float*>(smem + PL_OFF_CB);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + PL_OFF_BAR);
-  uint64_t* empty = full + PL_XS;
-  uint64_t* tfull = empty + PL_XS;
+  uint64_t* empty = full + XS;
+  uint64_t* tfull = empty + XS;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -68,7 +78,7 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   const AbortCtx ab{cta_abort, p.status};
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < PL_XS; ++s) {
+    for (int s = 0; s < XS; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 9);  // the products' commit and the eight statistics warps
     }
@@ -79,7 +89,7 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     *cta_abort = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmx);
-    tma_prefetch_desc(&tmo);
+    if (!FEW) tma_prefetch_desc(&tmo);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 256);
@@ -91,7 +101,7 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   // split weights, one head per half-warp pass; 16 lanes x 8 channels
   {
     const int half = lane >> 4, l16 = lane & 15;
-    for (int h = warp * 2 + half; h < PL_G; h += 2 * (PL_THREADS / 32)) {
+    for (int h = warp * 2 + half; h < (FEW ? ng : PL_G); h += 2 * (PL_THREADS / 32)) {
       float s = 0.f, b = 0.f, r[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -143,11 +153,11 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       uint8_t* sx = smem + PL_OFF_X + stage * PL_TILE;
       tma_load_3d_if(go, sx, &tmx, &full[stage], 0, k0, q);
       tma_load_3d_if(go, sx + 16384, &tmx, &full[stage], 64, k0, q);
-      if (++stage == PL_XS) { stage = 0; phase ^= 1u; }
+      if (++stage == XS) { stage = 0; phase ^= 1u; }
     }
   } else if (warp == 1) {
     const uint32_t go = elect_one();
-    constexpr uint32_t idesc = make_idesc(128, 128);
+    const uint32_t idesc = make_idesc(128, FEW ? ng : 128);
     const uint64_t wd = make_sdesc(base + PL_OFF_W, 16, 1024);
     uint32_t stage = 0, phase = 0, it = 0;
     for (long long t = t0; t < total; t += step, ++it) {
@@ -162,11 +172,13 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma_ss_if(go, d, wd + uint64_t((k * 2 + hf) * (PL_G * 8) + 2 * j), xd + uint64_t(hf * 1024 + 2 * j), idesc, (k | hf | j) ? 1u : 0u);
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t wt = wd + uint64_t((k * 2 + hf) * (PL_G * 8) + 2 * j), xt = xd + uint64_t(hf * 1024 + 2 * j);
+            umma_ss_if(go, d, FEW ? xt : wt, FEW ? wt : xt, idesc, (k | hf | j) ? 1u : 0u);
+          }
       umma_commit_if(go, &empty[stage]);
       umma_commit_if(go, &tfull[buf]);
-      if (++stage == PL_XS) { stage = 0; phase ^= 1u; }
+      if (++stage == XS) { stage = 0; phase ^= 1u; }
     }
   } else {
     // two sets of eight warps take the tiles in turn, so that one set's barriers and loads pass behind the other's work
@@ -176,12 +188,12 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
     const int ldq = (p.N + 7) & ~7;
     const uint32_t go = elect_one();
     uint8_t* stg = smem + PL_OFF_STG + (warp - 2) * PL_STG;
-    const float bias = cb[quarter * 32 + lane];
+    const float bias = FEW ? 0.f : cb[quarter * 32 + lane];
     const float2 b2 = make_float2(bias, bias);
     const __half2 lim = __float2half2_rn(60000.f);
     uint32_t it = set;
     for (long long t = t0 + set * step; t < total; t += 2 * step, it += 2) {
-      const uint32_t stage = it % PL_XS, phase = (it / PL_XS) & 1u;
+      const uint32_t stage = it % XS, phase = (it / XS) & 1u;
       const int q = int(t / p.tiles_k), k0 = int(t % p.tiles_k) * 128;
       // (a failed wait does not leave the loop: these warps meet at a named barrier; further waits return at once)
       mbar_wait(&full[stage], phase, ab, XF_ERR_WAIT_FULL);
@@ -198,6 +210,36 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       named_bar_sync(1 + set, 256);
       mbar_wait(&tfull[set], (it >> 1) & 1u, ab, XF_ERR_WAIT_TMEM_FULL);
       tc_fence_after();
+      if constexpr (FEW) {
+        // thread = key, 32 heads at a time; neighbouring lanes trade halves, so that the even lane holds two keys of head e and the
+        // odd lane two of head e + 1
+        const int row = quarter * 32 + lane, k = k0 + (row & ~1);
+        const float2 rl2 = make_float2(rl[row], rl[row]);
+        const bool kstore = k < ldq;
+        const long long plane2 = 2ll * p.N * ldq;
+        const uint32_t keep = (k < p.N ? 0xffffu : 0u) | (k + 1 < p.N ? 0xffff0000u : 0u);
+        const uint32_t sel = (lane & 1) ? 0x3276u : 0x5410u;  // odd: (other.hi, own.hi), even: (own.lo, other.lo)
+#pragma unroll 1
+        for (int hb = ch * 32; hb < ng; hb += 64) {
+          uint32_t r[32];
+          tmem_ld32(tmem_base + set * 128 + hb + (uint32_t(quarter * 32) << 16), r);
+          tmem_ld_wait();
+          __half* d = p.out + ((long long)(hb + (lane & 1)) * p.N + q) * ldq + k;
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            if (e == 16 && hb + 16 >= ng) break;  // heads in sixteens
+            const float2 v = ffma2(make_float2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), rl2, *reinterpret_cast<const float2*>(&cb[hb + e]));
+            const __half2 h2 = __hmin2(__hmax2(__floats2half2_rn(v.x, v.y), __hneg2(lim)), lim);  // (NaN: -60000)
+            const uint32_t own = *reinterpret_cast<const uint32_t*>(&h2), other = __shfl_xor_sync(0xffffffffu, own, 1);
+            if (kstore) *reinterpret_cast<uint32_t*>(d) = __byte_perm(own, other, sel) & keep;
+            d += plane2;
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[set]);
+        continue;
+      }
       const int kw = k0 + ch * 64;  // this warp's first key
       const bool edge = kw + 64 > p.N;
       tma_store_wait_read<0>();  // the tile before has left the staging buffer
@@ -238,7 +280,7 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
       tma_store_3d_if(kw < ldq && quarter * 32 < ng ? go : 0u, &tmo, stg, kw, q, h0 + quarter * 32);
       tma_store_commit();
     }
-    tma_store_wait_all();
+    if (!FEW) tma_store_wait_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -253,6 +295,23 @@ pair_logits_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constan
   }
 }
 
+template <bool FEW>
+static int launch_pl(Ctx* c, const CUtensorMap& tmx, const CUtensorMap& tmo, const PairLogitsArgs& a, cudaStream_t st) {
+  static bool attr_done[8] = {false};
+  if (!attr_done[c->device & 7]) {
+    cudaError_t e = cudaFuncSetAttribute(pair_logits_kernel<FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
+    if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pair logits smem attribute: %s", cudaGetErrorString(e));
+    attr_done[c->device & 7] = true;
+  }
+  long long per_group = c->sm_count / a.groups;
+  if (per_group < 1) per_group = 1;
+  const long long total = (long long)a.N * a.tiles_k;
+  if (per_group > total) per_group = total;
+  ProfScope ps(c, XFOLD_K_LAYERNORM, st);
+  launch_pdl(pair_logits_kernel<FEW>, (int)per_group * a.groups, PL_THREADS, PL_SMEM, st, tmx, tmo, a);
+  return check_launch(c, "pair_logits_kernel");
+}
+
 static int launch_pair_logits(Ctx* c, const bf16* pair, int N, const float* gamma, const float* beta, const float* w, int H,
                               void* out, cudaStream_t st) {
   if (N <= 0 || H <= 0) return XFOLD_OK;
@@ -261,23 +320,12 @@ static int launch_pair_logits(Ctx* c, const bf16* pair, int N, const float* gamm
   CUtensorMap tmx, tmo;
   if (!make_tmap_bf16_3d(&tmx, pair, 128, N, N, 128, (uint64_t)128 * N, 64, 128, 1))
     return fail(c, XFOLD_ERR_ARG, "pair logits: cannot encode the tensor map");
+  PairLogitsArgs a{gamma, beta, w, reinterpret_cast<__half*>(out), N, H, (N + 127) / 128, (H + PL_G - 1) / PL_G, c->d_status};
+  if (H <= PL_FEW) return launch_pl<true>(c, tmx, tmx, a, st);
   // (fp16 as far as the stores go: 16-bit elements)
   const uint64_t ldq = (uint64_t)((N + 7) & ~7);
   if (!make_tmap_bf16_3d(&tmo, out, ldq, N, H, ldq, ldq * N, 64, 1, 32)) return fail(c, XFOLD_ERR_ARG, "pair logits: cannot encode the result's tensor map");
-  PairLogitsArgs a{gamma, beta, w, N, H, (N + 127) / 128, (H + PL_G - 1) / PL_G, c->d_status};
-  static bool attr_done[8] = {false};
-  if (!attr_done[c->device & 7]) {
-    cudaError_t e = cudaFuncSetAttribute(pair_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
-    if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pair logits smem attribute: %s", cudaGetErrorString(e));
-    attr_done[c->device & 7] = true;
-  }
-  long long per_group = c->sm_count / a.groups;
-  if (per_group < 1) per_group = 1;
-  const long long total = (long long)N * a.tiles_k;
-  if (per_group > total) per_group = total;
-  ProfScope ps(c, XFOLD_K_LAYERNORM, st);
-  launch_pdl(pair_logits_kernel, (int)per_group * a.groups, PL_THREADS, PL_SMEM, st, tmx, tmo, a);
-  return check_launch(c, "pair_logits_kernel");
+  return launch_pl<false>(c, tmx, tmo, a, st);
 }
 
 }  // namespace xf

@@ -223,6 +223,26 @@ def test_pair_logits_prepared(ops, n, h):
     assert float(out[..., n:].float().abs().sum()) == 0.0
 
 
+@pytest.mark.parametrize("n", [1, 40, 129, 300])
+def test_pair_logits_of_few_heads_have_the_bits_of_many(ops, n):
+    """Up to 96 heads go through the form with keys as the accumulator's rows, more through the one with heads as its rows:
+    the same operands and sums.  Rows far from zero (mean 30, deviation 1): the mean falls out of the product with weights
+    that add up to zero, whose float32 rounding leaves about 30 * 2^-24 * sqrt(128) of a weight, 2e-5; the rest is float16's
+    rounding of the result, at most 2^-11 of a value and 2.1e-4 over many."""
+    g = torch.Generator().manual_seed(n)
+    pair = (torch.randn(n, n, 128, generator=g) + 30).to(BF)
+    gamma, beta = torch.rand(128, generator=g) + 0.5, 0.3 * torch.randn(128, generator=g)
+    w = torch.randn(112, 128, generator=g) / 11
+    ref = torch.nn.functional.layer_norm(pair.double(), (128,), gamma.double(), beta.double(), 1e-5) @ w.double().T
+    ref = ref.permute(2, 0, 1) * 1.4426950408889634
+    pair, gamma, beta, w = pair.cuda(), gamma.cuda(), beta.cuda(), w.cuda()
+    many = ops.pair_logits_prepared(pair, gamma, beta, w)
+    assert relf(many[..., :n].cpu(), ref) < (5e-4 if n == 1 else 3e-4)
+    for h in (96, 80, 48, 33, 16):
+        assert torch.equal(ops.pair_logits_prepared(pair, gamma, beta, w[:h].contiguous()), many[:h])
+    ops.synchronize_and_check()
+
+
 def test_pair_logits_of_undefined_tokens(ops):
     """A token that holds NaN or infinities gets logits of -60000 (its key is left out), as from ``prepare_pair_bias``."""
     g = torch.Generator().manual_seed(3)
