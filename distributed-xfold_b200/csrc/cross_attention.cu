@@ -535,8 +535,15 @@ int xfold_cross_attention_fwd(xfold_ctx* cx, const void* q_data, const void* m_d
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
   // The model's window is one tile of xwin_kernel; more queries, keys, heads or channels take the general kernels, and so do
-  // a bias and a result that pairs of elements cannot be read from or written to.
-  if (H == 4 && D == 32 && Ca == 128 && Cm == 128 && S <= 32 && K <= XA_KC && pairs)
+  // a bias and a result that pairs of elements cannot be read from or written to, and a result that lies over an operand: the
+  // general kernels have read all of those before the first result is stored, the windows' CTAs have not.
+  const auto apart = [&](const void* x, size_t bytes) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(x), to = reinterpret_cast<uintptr_t>(out);
+    return !x || at + bytes <= to || to + (size_t)B * S * W * 2 <= at;
+  };
+  if (H == 4 && D == 32 && Ca == 128 && Cm == 128 && S <= 32 && K <= XA_KC && pairs && apart(q_data, (size_t)B * S * 256) &&
+      apart(m_data, (size_t)B * K * 256) && apart(w_qg, 256 * 256) && apart(w_kv, 256 * 256) && apart(qg_bias, 1024) &&
+      apart(qg_scale, 1024))
     return launch_xwin(c, (const bf16*)q_data, (const bf16*)m_data, (const bf16*)w_qg, (const bf16*)w_kv,
                        XWinArgs{qg_bias, qg_scale, bias, (bf16*)out, B, S, K, c->d_status}, st);
   if ((rc = linear_plain(c, (const bf16*)q_data, Ca, (long long)B * S, Ca, (const bf16*)w_qg, 2 * W, qg_bias, qg_scale, qg,

@@ -281,6 +281,33 @@ def test_cross_attention_windows_have_the_bits_of_the_general_kernels(ops, B, S,
     assert torch.isfinite(out).all() and torch.equal(out, want)
 
 
+@pytest.mark.parametrize("where,shift", [("q", 0), ("q", 64), ("q", -64), ("m", 0), ("m", 32 * 128)])
+def test_cross_attention_result_over_its_operands(ops, where, shift):
+    """The result may lie over the queries' or the keys' tokens, at the same place or some elements further: as the call with a
+    result of its own."""
+    B, S, K = 400, 32, 128
+    g = torch.Generator().manual_seed(5)
+    w = ops.PackedCrossAttention(*(torch.randn(128, 4, 32, generator=g) / 11 if i != 1 else torch.randn(1, 4, 32, generator=g)
+                                   for i in range(5)), "cuda")
+    qd, md = torch.randn(B, S, 128, generator=g).to(BF).cuda(), torch.randn(B, K, 128, generator=g).to(BF).cuda()
+    bias = torch.randn(B, 4, S, K, generator=g).cuda()
+    want = ops.cross_attention(qd, md, bias, w)
+    pad = 128
+    room = torch.zeros(pad + (qd if where == "q" else md).numel() + pad, dtype=BF, device="cuda")
+    held = room[pad:-pad].view(qd.shape if where == "q" else md.shape)
+    held.copy_(qd if where == "q" else md)
+    out = room[pad + shift:][:want.numel()].view(want.shape)
+    q, m = (held, md) if where == "q" else (qd, held)
+    lib, dev = ops.load(), qd.device.index
+    ws = torch.empty(lib.xfold_cross_attention_workspace_bytes(B, S, K, 4, 32), dtype=torch.uint8, device="cuda")
+    rc = lib.xfold_cross_attention_fwd(ops.ctx(dev), q.data_ptr(), m.data_ptr(), B, S, K, 128, 128, 4, 32, w.w_qg.data_ptr(),
+                                       w.bias.data_ptr(), w.scale.data_ptr(), w.w_kv.data_ptr(), bias.data_ptr(), out.data_ptr(),
+                                       ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    ops.check(rc, dev, "xfold_cross_attention_fwd")
+    ops.synchronize_and_check()
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("offset", [0, 1, 2, 3])
 def test_cross_attention_bias_at_any_element(ops, offset):
     """A bias that is a view into a larger buffer starts at any float."""
