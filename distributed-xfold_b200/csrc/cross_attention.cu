@@ -541,7 +541,11 @@ int xfold_cross_attention_fwd(xfold_ctx* cx, const void* q_data, const void* m_d
     const uintptr_t at = reinterpret_cast<uintptr_t>(x), to = reinterpret_cast<uintptr_t>(out);
     return !x || at + bytes <= to || to + (size_t)B * S * W * 2 <= at;
   };
-  if (H == 4 && D == 32 && Ca == 128 && Cm == 128 && S <= 32 && K <= XA_KC && pairs && apart(q_data, (size_t)B * S * 256) &&
+  // Many windows with few tokens too: a window costs xwin_kernel the same whatever it holds, and packed rows are less then
+  // (16000 windows of 1 x 2: 320 us against 403, 4 x 20: 412 and 438, 16 x 16: 489 and 473, 20 x 4: 514 and 502, 1 x 40: 448
+  // and 439; 4000 of 1 x 2: 88 and 105; 592 of 1 x 2: 18.9 both).
+  const bool windows = B <= 4 * c->sm_count || S > 16 || S + K >= 40;
+  if (H == 4 && D == 32 && Ca == 128 && Cm == 128 && S <= 32 && K <= XA_KC && windows && pairs && apart(q_data, (size_t)B * S * 256) &&
       apart(m_data, (size_t)B * K * 256) && apart(w_qg, 256 * 256) && apart(w_kv, 256 * 256) && apart(qg_bias, 1024) &&
       apart(qg_scale, 1024))
     return launch_xwin(c, (const bf16*)q_data, (const bf16*)m_data, (const bf16*)w_qg, (const bf16*)w_kv,

@@ -264,10 +264,12 @@ def test_cross_attention_tile_edges(ops, oracle, B, S, K, H, D):
     assert relf(out.float().cpu(), ref) < 2e-2
 
 
-@pytest.mark.parametrize("B,S,K", [(1, 1, 2), (2, 16, 8), (3, 17, 126), (149, 32, 128), (400, 31, 100)])
+@pytest.mark.parametrize("B,S,K", [(1, 1, 2), (2, 16, 8), (3, 17, 126), (149, 32, 128), (400, 31, 100), (592, 1, 2), (593, 1, 2),
+                                   (593, 16, 22), (593, 16, 24), (593, 17, 2)])
 def test_cross_attention_windows_have_the_bits_of_the_general_kernels(ops, B, S, K):
     """The one-kernel form for windows of up to 32 x 128, from one entry to several windows per CTA, against the same call
-    with a bias that starts at an odd float, which the general kernels take."""
+    with a bias that starts at an odd float, which the general kernels take; at the edges of the rule on many windows with few
+    tokens."""
     g = torch.Generator().manual_seed(B + S + K)
     w = ops.PackedCrossAttention(*(torch.randn(128, 4, 32, generator=g) / 11 if i != 1 else torch.randn(1, 4, 32, generator=g)
                                    for i in range(5)), "cuda")
