@@ -100,7 +100,7 @@ class PackedDiffusionTransformer:
         attention kernel (values times log2(e)): half the resident bytes of the float32 logits, and no conversion inside
         the 200 denoising steps.  ('n s (b h) -> b h n s', nn/d_diffusion_transformer.py:301-305.)"""
         prepared = ops.pair_logits_prepared(pair_cond, self.pair_ln_g, self.pair_ln_b, self.pl_w)
-        return list(prepared.reshape(-1, self.sb, self.num_head, *prepared.shape[1:]))
+        return list(prepared.reshape(-1, self.sb, self.num_head, *prepared.shape[1:]).unbind(0))
 
     def forward(self, act: torch.Tensor, mask: Optional[torch.Tensor], single_cond: torch.Tensor,
                 pair_logits: List[torch.Tensor]) -> torch.Tensor:
