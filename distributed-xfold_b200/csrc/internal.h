@@ -89,6 +89,14 @@ struct StaticWeights {
 int fail(Ctx* c, int code, const char* fmt, ...);
 int check_launch(Ctx* c, const char* what);
 
+// A kernel without room to round the start of its shared memory up to 1 KB, where swizzled tiles begin, counts on the dynamic
+// part's own alignment: nothing static may stand in front of it.
+template <typename... KArgs>
+bool only_dynamic_smem(void (*kern)(KArgs...)) {
+  cudaFuncAttributes at;
+  return cudaFuncGetAttributes(&at, kern) == cudaSuccess && at.sharedSizeBytes == 0;
+}
+
 // Launch that may start while the previous kernel of the stream still runs (see pdl_wait in umma.cuh).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, Args&&... args) {

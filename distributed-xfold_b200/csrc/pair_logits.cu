@@ -301,6 +301,7 @@ static int launch_pl(Ctx* c, const CUtensorMap& tmx, const CUtensorMap& tmo, con
   if (!attr_done[c->device & 7]) {
     cudaError_t e = cudaFuncSetAttribute(pair_logits_kernel<FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
     if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "pair logits smem attribute: %s", cudaGetErrorString(e));
+    if (!only_dynamic_smem(pair_logits_kernel<FEW>)) return fail(c, XFOLD_ERR_LAUNCH, "pair logits: shared memory does not start at 1 KB");
     attr_done[c->device & 7] = true;
   }
   long long per_group = c->sm_count / a.groups;

@@ -379,6 +379,7 @@ static int launch_ro(Ctx* c, const CUtensorMap& tmx, const CUtensorMap& tmz, con
   if (!attr_done[c->device & 7]) {
     cudaError_t e = cudaFuncSetAttribute(row_output_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, RoCfg<MODE>::SMEM);
     if (e != cudaSuccess) return fail(c, XFOLD_ERR_LAUNCH, "row output smem attribute: %s", cudaGetErrorString(e));
+    if (!only_dynamic_smem(row_output_kernel<MODE>)) return fail(c, XFOLD_ERR_LAUNCH, "row output: shared memory does not start at 1 KB");
     attr_done[c->device & 7] = true;
   }
   if (reinterpret_cast<uintptr_t>(a.w) & 15) return fail(c, XFOLD_ERR_ARG, "row output: the weights must be 16-byte aligned");
