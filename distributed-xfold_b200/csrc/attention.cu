@@ -105,8 +105,6 @@ __device__ __forceinline__ float2 ex2_poly2(float2 y) {
   return make_float2(q.x * __uint_as_float(__float_as_uint(t.x) * 0x800000u + 0x3F800000u),
                      q.y * __uint_as_float(__float_as_uint(t.y) * 0x800000u + 0x3F800000u));
 }
-// sixteen packed pairs of a row: P over logits that have been read, or rescaled output
-__device__ __forceinline__ void tmem_st16_(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
 // Which of a sweep's 16 pairs take the polynomial: two, away from its ends.  (TriangleAttention, 1024 tokens: none 1.02 of the
 // time, three 1.00 to 1.02, four more; at the ends of the sweep's halves 1.01 -- with more, the FMA pipe and the issue slots
 // are the longer queue.)
@@ -356,7 +354,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
             const __half2 ph = __floats2half2_rn(pe.x, pe.y);
             pk[e] = *reinterpret_cast<const uint32_t*>(&ph);
           }
-          tmem_st16_(at, pk);
+          tmem_st16(at, pk);
         };
         // the reference exponent follows the block's maximum where that is more than 8 above it
         auto follow = [&]() {
@@ -393,7 +391,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUt
               tmem_ld_wait();
 #pragma unroll
               for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-              tmem_st16_(o_addr + oc, o);
+              tmem_st16(o_addr + oc, o);
             }
           }
           s2 = make_float2(0.f, 0.f);

@@ -435,11 +435,11 @@ int launch_row_project_trimul(Ctx* c, const bf16* z, const float* mask, int R, i
   bool ok;
   if (!transposed) {
     ok = make_tmap_bf16_3d(&tmx, z, 128, M, 1, 128, (uint64_t)128 * M, 64, 128, 1) &&
-         make_tmap_bf16_3d(&tmo, out_g ? out_g : z, 128, M, 1, 128, (uint64_t)128 * M, 32, 32, 1, 64);
+         (!out_g || make_tmap_bf16_3d(&tmo, out_g, 128, M, 1, 128, (uint64_t)128 * M, 32, 32, 1, 64));
     a.tiles = (int)((M + 127) / 128);
   } else {  // tile rows step along the first token axis, second axis fixed: a[j][c][i]
     ok = make_tmap_bf16_3d(&tmx, z, 128, N, R, 128, (uint64_t)128 * N, 64, 1, 128) &&
-         make_tmap_bf16_3d(&tmo, out_g ? out_g : z, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 32, 64);
+         (!out_g || make_tmap_bf16_3d(&tmo, out_g, 128, N, R, 128, (uint64_t)128 * N, 32, 1, 32, 64));
     a.mode1 = 1;
     a.dim1 = N;
     a.tiles = N * ((R + 127) / 128);

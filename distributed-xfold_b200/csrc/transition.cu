@@ -206,7 +206,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant
         if (!okay) break;
         tc_fence_after();
         d1(s, s);
-        if (NBK == 1) umma_commit_if(leader, &n_empty[s]);
       }
       if (!okay) break;
       umma_commit_if(leader, &w1_empty[g1 & 1u]);
