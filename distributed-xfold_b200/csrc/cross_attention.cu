@@ -230,8 +230,8 @@ static int launch_xattn(Ctx* c, const XAttnArgs& a, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------------------------------------------
 // The model's own windows (four heads of 32, 128 channels, up to 32 queries and 128 keys) in one kernel: projections and
-// attention of a window by two CTAs, one for each pair of heads, two CTAs per SM.
-// Bound: latency.  A window brings 104 KB (64 of them bias) for 0.04 GFLOP; what counts is the chain of trips -- as two
+// attention of a window by two CTAs, one for each pair of heads, two CTAs per SM.  No scratch.
+// Bound: latency.  A window brings 104 KB (64 of them bias) for 0.013 GFLOP; what counts is the chain of trips -- as two
 // projection launches and xattn_kernel, with queries, keys and values through memory, 257 windows took 27.6 us.
 // The projections come out transposed (D = W x^T, lane = channel), so that the 32 queries are the tile's narrow side, the
 // query bias and scale are one number per thread, and a thread's row of keys leaves in 16-byte pieces:

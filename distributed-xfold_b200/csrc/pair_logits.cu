@@ -2,9 +2,12 @@
 // operand (FP16 values times log2 e, [head][query][key], pitch pad8(N)): all pair logits of the diffusion transformer
 // (24 blocks x 16 heads) in one launch.
 //
-// Bound: HBM.  128 x 2 bytes come in and 2 H leave per token; nothing else has to move.  (One fp32 plane set per
-// super-block, computed on the CUDA cores, and a conversion pass over it took 8.5 ms at N = 1000, H = 384; this kernel
-// takes 0.30 ms, 3.4 TB/s.)
+// 128 x 2 bytes come in and 2 H leave per token; nothing else has to move: 157 us of HBM at N = 1000, H = 384, and the products
+// (1500 clocks per tile of 128 keys and 128 heads) are 0.13 ms.  Neither is the bound: without its stores the kernel takes 237
+// us, 2800 clocks per tile, the chain of a set of warps (statistics, barrier, wait for the product, conversion), and the stores
+// come on top.  301 us at 1965 MHz, the first hundred calls from a cool GPU, and 353 at the 1500 MHz that calls in a row settle at
+// under the power limit.  (One fp32 plane set per super-block, computed on the CUDA cores, and a conversion pass over it took
+// 8.5 ms.)
 //
 // The product runs on the RAW rows, which are bf16 and therefore exact tensor-core operands, and keeps float32's precision
 // in the weights by splitting them:
@@ -17,7 +20,7 @@
 // in memory, so a pair of logits is one packed FMA with the keys' scales (broadcast from shared memory), one conversion and
 // the clamp, and eight leave as one 16-byte piece for TMA.  (With keys as rows, neighbouring lanes had to trade halves for
 // 4-byte stores, and every pair of logits read two pairs of column sums: the shared-memory pipe was 61 % busy, the issue
-// slots 50 %; 350 us at N = 1000, H = 384, now 300.  What is left: without the stores it would be 237.)
+// slots 50 %; 350 us at N = 1000, H = 384, cool, now 301.)
 //
 // A CTA keeps the split weights of up to 128 heads in shared memory (96 KB) and walks over tiles of 128 keys of one query
 // row; with more heads the CTAs divide into groups that read the same tiles at about the same time, so that all but the

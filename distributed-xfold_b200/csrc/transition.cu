@@ -1,10 +1,12 @@
 // Transition of the pair representation in one kernel:  x += W2 swiglu(W1 LN(x))  for rows of 128, F hidden units
 // (csrc/Alpha_Attention.cpp:72-92, kernel_test/transition.py:22-48 state the operator).
 //
-// Bound: the tensor core.  Per tile of 128 rows 25 M multiply-adds (6100 clocks) and 65536 sigmoids (4096 clocks of the
-// special-function unit); the weights are 384 KB at F = 512, so two tiles share each block of them.  The only HBM traffic is
-// x itself.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) the normalised rows and the hidden activations made six
-// passes over 128 and 512 columns: 0.84 ms for 1024 x 1024 rows.
+// Per tile of 128 rows at F = 512: 25 M multiply-adds (6100 clocks of the tensor core), 65536 sigmoids (4096 of the
+// special-function unit) and 1056 KB through shared memory (8450 clocks at 128 bytes each): operands of the products 640 KB,
+// weights on arrival 192 (384 KB in all, two tiles share each block of them), x, its LayerNorm and the result 224.  The only HBM
+// traffic is x itself.  1024 x 1024 rows take 412 us at 1965 MHz, 14 600 clocks per tile, and 470 to 480 at the 1710 MHz of the
+// power limit: shared memory is the nearest bound, at 58 %.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) the
+// normalised rows and the hidden activations made six passes over 128 and 512 columns: 0.84 ms.
 //
 // Persistent CTAs, a pair of tiles (A, B) of 128 rows at a time, hidden units in blocks of 64; per tile
 //     D1 = LN(x) W1(block)^T   [128 x (64 SiLU | 64 linear)]      tensor memory
@@ -15,8 +17,8 @@
 //                    the h that D2 reads (products of one issuer execute in order)
 //   warps 2 - 9    : LayerNorm in place, one thread per row
 //   warps 10 - 17  : one set of four per tile: D1 -> h; finally D2 + x -> a staging tile in two halves, which leave by TMA
-// The operands' trips from shared memory bound it (128 bytes per clock): with h in tensor memory they are 21 % fewer.  (h in
-// shared memory, D1 a block ahead of it: 0.54 ms in the trunk of 1024 tokens, now 0.50.  Sixteen warps for D1 -> h: no gain.)
+// With h in tensor memory 256 KB fewer of a tile's 1312 go through shared memory.  (h in shared memory, D1 a block ahead of it:
+// 0.54 ms in the trunk of 1024 tokens, now 0.50.  Sixteen warps for D1 -> h: no gain.)
 // With no more tiles than SMs a CTA takes one tile: its blocks go through the two accumulators in turn, each with its set of
 // warps, D1 two blocks ahead of D2, and a set takes one half of the result.  (One accumulator and one set: four
 // blocks of the trunk at 37 tokens 392 us instead of 379, at 100 tokens 485 instead of 471.)

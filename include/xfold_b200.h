@@ -179,7 +179,7 @@ int xfold_attention_pair_bias_core_fwd(xfold_ctx* ctx, const void* xn, int B, in
 int xfold_pair_bias_prepare_fwd(xfold_ctx* ctx, const float* pair_bias, int H, int S, void* prepared, void* stream);
 /* LayerNorm (eps 1e-5) of a whole pair representation [N][N][128] and its projection to H heads (w float32 [H][128], H a
  * multiple of 16), written as prepared pair bias [H][N][pad8(N)]: every block's logits of the diffusion transformer in one
- * launch ('n s (b h) -> b h n s', nn/d_diffusion_transformer.py:299-305). */
+ * launch ('n s (b h) -> b h n s', nn/d_diffusion_transformer.py:299-305).  pair and prepared are 16-byte aligned. */
 int xfold_pair_logits_prepared_fwd(xfold_ctx* ctx, const void* pair, int N, const float* ln_gamma, const float* ln_beta,
                                    const float* w, int H, void* prepared, void* stream);
 int xfold_attention_pair_bias_core_prepared_fwd(xfold_ctx* ctx, const void* xn, int B, int S, int C, int H, int Dp,
@@ -240,7 +240,8 @@ int xfold_gated_attention_core_fwd(xfold_ctx* ctx, const void* xn, int B, int S,
  * m_data bf16 [B][K][Cm], a float32 bias per batch entry [B][H][S][K], gate sigmoid(q_data gating_w), no output projection.
  *   w_qg bf16 [2*H*D][Ca]: the query rows (head-major) then the gating rows; qg_bias / qg_scale float32 [2*H*D]
  *   (query bias and D^-0.5 on the query rows, 0 / 1 on the gating rows); w_kv bf16 [2*H*D][Cm]: key rows then value rows.
- * out: bf16 [B][S][H*D].  D in {16, 32, 64}. */
+ * out: bf16 [B][S][H*D], which may lie over q_data or m_data.  D in {16, 32, 64}.  The workspace is asked for at every
+ * size, whether or not the call's kernels need it (the model's windows of 32 queries and 128 keys do not). */
 size_t xfold_cross_attention_workspace_bytes(int B, int S, int K, int H, int D);
 int xfold_cross_attention_fwd(xfold_ctx* ctx, const void* q_data, const void* m_data, int B, int S, int K, int Ca, int Cm,
                               int H, int D, const void* w_qg, const float* qg_bias, const float* qg_scale,

@@ -243,6 +243,24 @@ def test_pair_logits_of_few_heads_have_the_bits_of_many(ops, n):
     ops.synchronize_and_check()
 
 
+@pytest.mark.parametrize("heads", [16, 112])
+@pytest.mark.parametrize("which,offset", [("pair", 1), ("pair", 4), ("prepared", 1), ("prepared", 2), ("prepared", 4)])
+def test_pair_logits_at_unaligned_addresses_are_refused(ops, heads, which, offset):
+    """Both tensors start at multiples of 16 bytes: anything else is an error before the first launch, and nothing is written."""
+    n, lib = 20, ops.load()
+    pair = torch.zeros(n * n * 128 + 8, dtype=BF, device="cuda")
+    out = torch.full((heads * n * 24 + 8,), 7.0, dtype=torch.float16, device="cuda")
+    w = torch.ones(heads, 128, device="cuda")
+    dev = pair.device.index
+    p, o = pair[offset if which == "pair" else 0:], out[offset if which == "prepared" else 0:]
+    rc = lib.xfold_pair_logits_prepared_fwd(ops.ctx(dev), p.data_ptr(), n, None, None, w.data_ptr(), heads, o.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream)
+    with pytest.raises(RuntimeError):
+        ops.check(rc, dev, "xfold_pair_logits_prepared_fwd")
+    ops.synchronize_and_check()
+    assert (out == 7).all()
+
+
 def test_pair_logits_of_undefined_tokens(ops):
     """A token that holds NaN or infinities gets logits of -60000 (its key is left out), as from ``prepare_pair_bias``."""
     g = torch.Generator().manual_seed(3)
